@@ -1,5 +1,5 @@
 // The batched-decode product on the 5th-generation tensor cores: y[m, n] = sum_k x[m, k] * w[n, k] for 9..64 activation
-// rows per pass, weights streamed once in their stored format.
+// rows per pass, weights streamed once in their stored format. (More rows of BF16 / INT8 / FP8 products: gemm_pair.cu.)
 //
 // The weight tile is the A operand of tcgen05.mma (128 weight rows = the 128 lanes of the accumulator in tensor memory),
 // the activations are the B operand (one accumulator column per activation row and digit), K advances 32 bytes per
@@ -83,12 +83,7 @@ struct TcLayout {
 // is found by every block of the row again (the row is a few KB, from L2), which saves a second kernel. Plane j of
 // row u is column j * Mp + u. k past K is written as zero up to the end of the last stage; columns that no row owns
 // are never written (their accumulator columns are never read).
-// MODE kPrepQuant (int8 / e4m3 only): the low-precision maths of lx_gemm_w. The row is quantized once, as
-// lx_quantize_act does (scale = max|x| / 127 or / 448, values rounded to nearest even and clamped; engine/cuda/quant.cu),
-// into ONE plane, and the row's sums are multiplied by that scale.
-// MODE kPrepRound (f32 activations): every value is rounded to bf16 first and then treated as a bf16 activation, which
-// is what lx_gemm_w does with f32 activations under BF16 math (engine/cuda/gemm_w.cu:239-252: "a bf16 copy").
-enum { kPrepExact = 0, kPrepQuant = 1, kPrepRound = 2 };
+// MODE: tc.cuh.
 template <int ACT, bool XBF, int MODE = kPrepExact>
 __global__ void __launch_bounds__(128) tc_prep_kernel(const void* __restrict__ x, int ld_x, int rows, int K, int NC, int Mp, int planes,
                                                       uint8_t* __restrict__ out, float* __restrict__ inv_scales, int n_stages) {
@@ -1286,6 +1281,10 @@ int tc_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const v
                int ld_y, int M, int N, int K, float alpha, float beta, void* workspace, cudaStream_t stream, bool quantized) {
   const bool x_bf16 = x_dtype == LX_BF16;
   if (quantized && w.type != LX_W_INT8 && w.type != LX_W_FP8) return kNotSupported;
+  // More rows than one pass: pairs of SMs, same digits, same order, same bits. (FP8, 28672 x 8192: 64 rows 52 us here, 65 rows
+  // 54 us there; a second pass would add another 50.)
+  if (M > kMaxRows && w.type != LX_W_NVFP4)
+    return pair_product(x, x_dtype, ld_x, w, bias, bias_dtype, y, y_dtype, ld_y, M, N, K, alpha, beta, workspace, stream, quantized);
   const int act = act_of(w.type), elem = act_elem(act), kKS = ks_of(act);
   const int per_pass = rows_per_pass(act, true);  // f32 activations become bf16 (or quantized) values: as many planes as bf16
   const int n_stages = (K + kKS - 1) / kKS;
@@ -1424,6 +1423,7 @@ int64_t tc_workspace_bytes(int M, int K) {
       const int NC = (act_planes(act, bf != 0) * ((r + 7) / 8 * 8) + 15) / 16 * 16;
       need = std::max(need, TcLayout(NC, act, (K + ks_of(act) - 1) / ks_of(act)).total);
     }
+  if (M > kMaxRows) need = std::max(need, pair_workspace_bytes(M, K));
   return need;
 }
 

@@ -71,15 +71,15 @@ using TensorMapEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint
                                        CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 TensorMapEncodeFn tensor_map_encoder();
 
-// A 2-D map over `rows` rows of `row_bytes` bytes each (row pitch = row_bytes, a multiple of 16; base 16-byte aligned),
+// A 2-D map over `rows` rows of `row_bytes` bytes each (`pitch` bytes apart, 0 = row_bytes, a multiple of 16; base 16-byte aligned),
 // copied in boxes of box_rows x box_bytes. elem_bytes (1 or 4) is the unit the kernel gives x coordinates in. With
 // swizzle128 (boxes 128 bytes wide) the 16-byte pieces of row r land at piece ^ (r % 8).
 inline int make_tile_map(CUtensorMap* map, const void* base, int64_t row_bytes, int64_t rows, int box_bytes, int box_rows,
-                         int elem_bytes, bool swizzle128 = false) {
+                         int elem_bytes, bool swizzle128 = false, int64_t pitch = 0) {
   TensorMapEncodeFn encode = tensor_map_encoder();
   if (!encode) return kNotSupported;
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(row_bytes / elem_bytes), static_cast<cuuint64_t>(rows)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(row_bytes)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(pitch ? pitch : row_bytes)};
   const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_bytes / elem_bytes), static_cast<cuuint32_t>(box_rows)};
   const cuuint32_t estr[2] = {1, 1};
   const CUresult r = encode(map, elem_bytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_INT32 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2,
@@ -174,6 +174,10 @@ inline int math_admitted(int math, int wtype) {
 int tc_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const void* bias, int bias_dtype, void* y, int y_dtype,
                int ld_y, int M, int N, int K, float alpha, float beta, void* workspace, cudaStream_t stream, bool quantized = false);
 int64_t tc_workspace_bytes(int M, int K);
+// gemm_pair.cu: the same product for more rows than one pass of tc_product takes, on pairs of SMs.
+int pair_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const void* bias, int bias_dtype, void* y, int y_dtype, int ld_y,
+                 int M, int N, int K, float alpha, float beta, void* workspace, cudaStream_t stream, bool quantized);
+int64_t pair_workspace_bytes(int M, int K);
 bool tc_enabled();
 // Where the all-gather epilogue of a sharded product stores: every rank's copy of the whole y and arrival counter.
 struct PeerTargets {

@@ -75,6 +75,13 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
                : "r"(taddr)
                : "memory");
 }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                 "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+               : "r"(taddr)
+               : "memory");
+}
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // D[tmem] (+)= A[smem descriptor] * B[smem descriptor], one CTA.
 template <int kAct>
@@ -183,6 +190,13 @@ struct Ring {
 // ---- activation preparation ----------------------------------------------------------------------------------------
 // The same functions serve the preparation kernel (more than 8 activation rows) and the CTAs that prepare their own
 // activations (up to 8 rows), so a row's digits, and with them its sums, are the same bits on either way.
+//
+// MODE kPrepQuant (int8 / e4m3 only): the low-precision maths of lx_gemm_w. The row is quantized once, as
+// lx_quantize_act does (scale = max|x| / 127 or / 448, values rounded to nearest even and clamped; engine/cuda/quant.cu),
+// into ONE plane, and the row's sums are multiplied by that scale.
+// MODE kPrepRound (f32 activations): every value is rounded to bf16 first and then treated as a bf16 activation, which
+// is what lx_gemm_w does with f32 activations under BF16 math (engine/cuda/gemm_w.cu:239-252: "a bf16 copy").
+enum { kPrepExact = 0, kPrepQuant = 1, kPrepRound = 2 };
 
 // V consecutive activations of a row starting at k0, as f32; zero past K.
 template <bool XBF, int V>
