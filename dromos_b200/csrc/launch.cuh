@@ -48,6 +48,26 @@ int launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, 
   return kOk;
 }
 
+// One zeroed 64-bit word on the device for a call that reads a number back before it returns. The words are a fixed array
+// of the library (no allocation: after a synchronisation the stream-ordered allocator hands its memory back to the system,
+// and the next call pays for mapping it again); a word is one call's from construction to destruction, whichever threads and
+// streams call, and it is given back only after the stream is done with it. With all of them taken (more than 64 calls
+// at once on a GPU) the word comes from the stream-ordered allocator.
+struct ResultWord {
+  unsigned long long* dev = nullptr;
+  cudaStream_t stream;
+  int status;
+  explicit ResultWord(cudaStream_t s);
+  ~ResultWord();
+  int read(unsigned long long* value);  // synchronizes the stream
+  ResultWord(const ResultWord&) = delete;
+  ResultWord& operator=(const ResultWord&) = delete;
+
+ private:
+  int device = 0, slot = -1;
+  bool idle = false;  // the stream has been waited for since the last use
+};
+
 // Scratch for the stage-granular split of dense products: per device, a few regions handed out in turn (consecutive
 // launches never share one), each holding kSplitMaxCtas partial-sum slots of kSplitBytesPerCta bytes and their flags.
 // Allocated on first use and kept for the life of the process; the flags are zero whenever no kernel is running.

@@ -35,6 +35,50 @@ int* status_word() {
   return words[dev];
 }
 
+namespace {
+constexpr int kResultWords = 64;
+__device__ unsigned long long g_result_words[kResultWords * 4];  // 32 bytes apart
+std::mutex g_result_mu;
+uint64_t g_result_taken[64];  // per device, a bit per word
+}  // namespace
+
+ResultWord::ResultWord(cudaStream_t s) : stream(s) {
+  void* base = nullptr;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e == cudaSuccess && device < 64) e = cudaGetSymbolAddress(&base, g_result_words);
+  if (e == cudaSuccess && base) {
+    std::lock_guard<std::mutex> lock(g_result_mu);
+    uint64_t& taken = g_result_taken[device];
+    if (~taken) {
+      slot = __builtin_ctzll(~taken);
+      taken |= 1ull << slot;
+      dev = static_cast<unsigned long long*>(base) + 4 * slot;
+    }
+  }
+  if (e == cudaSuccess && !dev) e = cudaMallocAsync(&dev, sizeof(*dev), s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(dev, 0, sizeof(*dev), s);
+  if (e != cudaSuccess) cudaGetLastError();
+  status = static_cast<int>(e);
+}
+
+int ResultWord::read(unsigned long long* value) {
+  cudaError_t e = cudaMemcpyAsync(value, dev, sizeof(*value), cudaMemcpyDeviceToHost, stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+  idle = e == cudaSuccess;
+  if (e != cudaSuccess) cudaGetLastError();
+  return static_cast<int>(e);
+}
+
+ResultWord::~ResultWord() {
+  if (slot < 0) {
+    if (dev) cudaFreeAsync(dev, stream);
+    return;
+  }
+  if (!idle && cudaStreamSynchronize(stream) != cudaSuccess) cudaGetLastError();
+  std::lock_guard<std::mutex> lock(g_result_mu);
+  g_result_taken[device] &= ~(1ull << slot);
+}
+
 int split_scratch(float** partials, int** flags) {
   static std::mutex mu;
   static uint8_t* base[64] = {};
