@@ -149,7 +149,9 @@ class Library:
 
     def __getattr__(self, name):
         if name.startswith("lx_"):
-            return self.fn(name)
+            f = self.fn(name)
+            self.__dict__[name] = f  # found without this detour from now on
+            return f
         raise AttributeError(name)
 
 
