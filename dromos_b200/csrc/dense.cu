@@ -106,10 +106,10 @@ int launch_dense_format(const StreamParams& P, cudaStream_t stream) {
 }
 
 // ---- the decode GEMV (gemv.cuh): up to 8 rows, every format ----------------------------------------------------------
-template <int F, int NT, int CPS>
+template <int F, int NT, int CPS, bool kWide = true>
 int launch_gemv_inst(const GemvParams& P, size_t smem, cudaStream_t stream) {
-  auto kernel = gemv_kernel<F, NT, CPS>;
-  if (int e = allow_dynamic_smem<4096 + F * 64 + NT * 8 + CPS>(kernel)) return e;
+  auto kernel = gemv_kernel<F, NT, CPS, kWide>;
+  if (int e = allow_dynamic_smem<4096 + F * 64 + NT * 8 + (kWide ? 0 : 4) + CPS>(kernel)) return e;
   const int sms = sm_count();
   if (!sms) return kInvalid;
   const unsigned grid = static_cast<unsigned>(std::max(1, std::min((P.N + kGemvGranule - 1) / kGemvGranule, sms * CPS)));
@@ -193,6 +193,16 @@ int launch_gemv(GemvParams P, int variant, cudaStream_t stream) {
   }
   const bool two = variant == kGemvD4C2 || (variant < 0 && F != LX_W_BF16X);
   const int cps = (smem <= 110 * 1024 && two) ? 2 : 1;
+  if constexpr (F == LX_W_BF16 || F == LX_W_INT8 || F == LX_W_FP8) {
+    if (!aligned(P.w, 32)) {  // the same sums from 16-byte loads (rows are whole 128 bytes, so they are as aligned as the matrix)
+      switch (NT) {
+        case 1: return launch_gemv_inst<F, 1, 1, false>(P, smem, stream);
+        case 2: return launch_gemv_inst<F, 2, 1, false>(P, smem, stream);
+        case 3: return launch_gemv_inst<F, 3, 1, false>(P, smem, stream);
+      }
+      return kInvalid;
+    }
+  }
   switch (NT * 10 + cps) {
     case 11: return launch_gemv_inst<F, 1, 1>(P, smem, stream);
     case 12: return launch_gemv_inst<F, 1, 2>(P, smem, stream);

@@ -102,8 +102,19 @@ constexpr int gemv_act() {
   return kMma == kMmaBf16 ? kActBf16 : kMma == kMmaF16 ? kActF16 : kMma == kMmaE4m3 ? kActE4m3 : kActS8;
 }
 
-// 32 bytes of weights that nothing will read again: around L1. `on` = 0 leaves q as it was.
+// 32 bytes of weights that nothing will read again: around L1. `on` = 0 leaves q as it was. kWide: the address is a multiple
+// of 32 (a 256-bit load faults on any other); else of 16.
+template <bool kWide>
 __device__ __forceinline__ void ldg_stream32(uint32_t (&q)[8], const uint8_t* p, uint32_t on) {
+  if constexpr (!kWide) {
+    asm volatile(
+        "{ .reg .pred q; setp.ne.u32 q, %9, 0;\n"
+        "@q ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%8];\n"
+        "@q ld.global.nc.L1::no_allocate.v4.u32 {%4, %5, %6, %7}, [%8 + 16]; }"
+        : "+r"(q[0]), "+r"(q[1]), "+r"(q[2]), "+r"(q[3]), "+r"(q[4]), "+r"(q[5]), "+r"(q[6]), "+r"(q[7])
+        : "l"(p), "r"(on));
+    return;
+  }
   asm volatile(
       "{ .reg .pred q; setp.ne.u32 q, %9, 0;\n"
       "@q ld.global.nc.L1::no_allocate.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8]; }"
@@ -295,7 +306,8 @@ __device__ __forceinline__ void e4m3_expand4(uint32_t word, uint32_t& lo, uint32
 // i + 2 sent while batch i + 1 is multiplied) stream slower than one buffer of twice the depth; prefetching the next
 // unit into L2 slows every size down; sending the next unit's loads before the unit's sums are added up makes the
 // adding (shared-memory loads, which then queue behind them) slower than what it hides.
-template <int F, int NT, int CPS>
+// kWide: weight rows start on 32-byte boundaries (a matrix may begin on any 16).
+template <int F, int NT, int CPS, bool kWide>
 __global__ void __launch_bounds__(kGemvThreads, CPS) gemv_kernel(const GemvParams P) {
   using Fm = GemvFmt<F>;
   constexpr int kMma = Fm::kMma;
@@ -370,8 +382,8 @@ __global__ void __launch_bounds__(kGemvThreads, CPS) gemv_kernel(const GemvParam
         ldg_nc8(qb[d][4], qb[d][5], pb + blk + 128 + 32 * half + 8 * t, on);
         ldg_nc1(qb[d][6], pb + 4 * slots + (sd >> 1), on);
       } else if constexpr (kLane == 32) {
-        ldg_stream32(qa[d], pa + d * kWStep, on);
-        ldg_stream32(qb[d], pb + d * kWStep, on);
+        ldg_stream32<kWide>(qa[d], pa + d * kWStep, on);
+        ldg_stream32<kWide>(qb[d], pb + d * kWStep, on);
       } else {
         ldg_stream16(qa[d], pa + d * kWStep, on);
         ldg_stream16(qb[d], pb + d * kWStep, on);
