@@ -12,7 +12,7 @@
 //      its blocks serve every pair of that expert (one pass over the expert's rows however many tokens picked it);
 //      the blocks of the other pairs leave at once. A warp reads gate row i and up row I + i together and writes
 //      bf16(silu(gate) * up) to each member pair's row of the workspace.
-//   2. down: a block belongs to one (token, 8 output rows); a warp sums the token's top_k experts in k order in
+//   2. down: a block belongs to one (token, 16 output rows); a warp takes two and sums the token's top_k experts in k order in
 //      registers and writes out[t, l].
 // Each (pair, row) sum is one lane-ordered chain of fmaf over k followed by a fixed shuffle tree, whatever else the
 // block serves, which is what makes the rows batch-invariant and BF16X equal to bf16 bit for bit (both walk 8 values
@@ -27,6 +27,7 @@ namespace {
 constexpr int kDecodeMaxT = 8;      // moe_decode.cu:40-41 of the reference: the decode contract
 constexpr int kDecodeMaxTopK = 8;
 constexpr int kRowsPerBlock = 8;    // one warp per row
+constexpr int kDownRows = 2;        // output rows per warp of the down kernel
 constexpr int kGateUpRows = 16;     // intermediate rows a gate/up block walks (two per warp)
 constexpr int kDecodeThreads = 32 * kRowsPerBlock;
 constexpr int kScanPairs = kDecodeMaxT * kDecodeMaxTopK;  // pairs a block scans for its expert's members
@@ -216,16 +217,99 @@ __device__ __forceinline__ uint32_t row_flag(const uint8_t* row) {
   else return 0;
 }
 
+// A lane's word of a step that lies whole within the row, its address a running pointer: no bounds, no test of the alignment.
+// (`row` and k0 are for BF16X, whose three pieces of a word are found from the value's place in its record.)
+template <int F>
+__device__ __forceinline__ Raw load_whole(const uint8_t* at, const uint8_t* scale_at, const uint8_t* row, int k0, int hdr, int slots) {
+  Raw r{make_uint4(0, 0, 0, 0), 0};
+  if constexpr (F == LX_W_BF16X) {
+    const int off = k0 & 127;
+    const uint8_t* b = row + hdr + (k0 >> 7) * 192;
+    const uint2 sm = __ldg(reinterpret_cast<const uint2*>(b + off));
+    r.w = make_uint4(sm.x, sm.y, __ldg(reinterpret_cast<const uint32_t*>(b + 128 + (off >> 1))), __ldg(row + 4 * slots + (k0 >> 7)));
+  } else if constexpr (F == LX_W_NVFP4) {
+    const uint2 u = __ldg(reinterpret_cast<const uint2*>(at));
+    r.w.x = u.x, r.w.y = u.y;
+    r.s = __ldg(scale_at);
+  } else {
+    r.w = ldg16(at);
+  }
+  return r;
+}
+
 // acc[r][t] += rows[r] . x[t] over all of K: the warp's lanes take consecutive words, kSteps words of each row in
 // flight per lane. A token's sum is the same chain of operations whatever NT is.
-template <int F, int NR, int NT>
+// WHOLE (rows, scales and activations on their word's boundary): the steps all of whose 32 words lie within the row go
+// without bounds, by running pointers. The same words in the same order either way. These kernels are bound by instruction issue: at 5.4-6.4 instructions per FP8 value (where converting
+// and adding take 3) four tokens of the 64-expert case (FP8, 4096 x 1536, top 8) took 152 us, at half the copy bandwidth; 137 now.
+template <int F, int NR, int NT, bool WHOLE>
 __device__ __forceinline__ void dot_rows(const Stack& S, const uint8_t* const (&row)[NR], const uint8_t* const (&row_scale)[NR],
                                          const uint32_t (&flag)[NR], const uint16_t* const (&x)[NT], bool xvec, int lane,
                                          float (&acc)[NR][NT]) {
   constexpr int V = kLaneValues<F>;
   constexpr int kSteps = NT == 1 ? 4 : 2;
+  constexpr int kStep = 32 * V;  // values of K a step covers
   const int K = S.K;
-  for (int k_base = 0; k_base < K; k_base += 32 * V * kSteps) {
+  int k_done = 0;
+  if constexpr (WHOLE) {
+    constexpr int kWord = F == LX_W_BF16 || F == LX_W_INT8 || F == LX_W_FP8 ? 16 : 8, kStepBytes = 32 * kWord;
+    const int hdr = F == LX_W_BF16X ? x16::header_bytes(K) : 0, slots = F == LX_W_BF16X ? x16::patch_slots(K) : 0;
+    const uint8_t *at[NR], *scale_at[NR];
+    const uint16_t* xp[NT];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) at[r] = row[r] + lane * kWord, scale_at[r] = F == LX_W_NVFP4 ? row_scale[r] + lane : row[r];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) xp[t] = x[t] + lane * V;
+    for (int left = K / kStep; left > 0; left -= kSteps) {
+      Raw raw[kSteps][NR];
+#pragma unroll
+      for (int j = 0; j < kSteps; ++j) {
+        if (j >= left) break;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+          raw[j][r] = load_whole<F>(at[r] + j * kStepBytes, scale_at[r] + j * 32, row[r], k_done + j * kStep + lane * V, hdr, slots);
+          if constexpr (F == LX_W_BF16X) raw[j][r].s = flag[r];
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < kSteps; ++j) {
+        if (j >= left) break;
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          float xf[V];
+          load_x<V>(xp[t] + j * kStep, 0, V, true, xf);
+#pragma unroll
+          for (int r = 0; r < NR; ++r) acc[r][t] = dot_word<F>(raw[j][r], xf, acc[r][t], row[r], k_done + j * kStep + lane * V, K);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        at[r] += kSteps * kStepBytes;
+        if constexpr (F == LX_W_NVFP4) scale_at[r] += kSteps * 32;
+      }
+#pragma unroll
+      for (int t = 0; t < NT; ++t) xp[t] += kSteps * kStep;
+      k_done += kSteps * kStep;
+    }
+    // the last step: the lanes whose word lies in the row (whole words, but for BF16X's last)
+    const int k0 = K / kStep * kStep + lane * V, back = K / kStep * kStep - k_done;
+    if (k0 >= K) return;
+    Raw raw[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      raw[r] = load_whole<F>(at[r] + back / V * kWord, scale_at[r] + back / 16, row[r], k0, hdr, slots);
+      if constexpr (F == LX_W_BF16X) raw[r].s = flag[r];
+    }
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      float xf[V];
+      load_x<V>(x[t], k0, F == LX_W_BF16X ? K : k0 + V, true, xf);
+#pragma unroll
+      for (int r = 0; r < NR; ++r) acc[r][t] = dot_word<F>(raw[r], xf, acc[r][t], row[r], k0, K);
+    }
+    return;
+  }
+  for (int k_base = 0; k_base < K; k_base += kStep * kSteps) {
     Raw raw[kSteps][NR];
 #pragma unroll
     for (int j = 0; j < kSteps; ++j)
@@ -250,7 +334,7 @@ __device__ __forceinline__ void dot_rows(const Stack& S, const uint8_t* const (&
 }
 
 // Stage 1 for the NT member pairs of one expert: mid[pair, i] = bf16(silu(s_g * gate_i . x) * (s_u * up_i . x)).
-template <int F, int NT>
+template <int F, int NT, bool WHOLE>
 __device__ __forceinline__ void gate_up_members(const Stack& S, int e, int i, int I, const uint16_t* latent, int ld, bool xvec,
                                                 const int (&member)[NT], int count, int top_k, uint16_t* mid, int lane) {
   const int64_t ng = static_cast<int64_t>(e) * S.rows + i, nu = ng + I;
@@ -263,7 +347,7 @@ __device__ __forceinline__ void gate_up_members(const Stack& S, int e, int i, in
   float acc[2][NT];
 #pragma unroll
   for (int t = 0; t < NT; ++t) acc[0][t] = acc[1][t] = 0.0f;
-  dot_rows<F, 2, NT>(S, row, row_scale, flag, x, xvec, lane, acc);
+  dot_rows<F, 2, NT, WHOLE>(S, row, row_scale, flag, x, xvec, lane, acc);
   const float fg = stack_row_factor<F>(S, ng, e), fu = stack_row_factor<F>(S, nu, e);
 #pragma unroll
   for (int t = 0; t < NT; ++t) {
@@ -276,8 +360,8 @@ __device__ __forceinline__ void gate_up_members(const Stack& S, int e, int i, in
 // grid (ceil(I / kGateUpRows), P). dedupe: P <= 64 and the first pair of an expert serves all of its pairs, two at a
 // time (more members than two read the rows again, from L1 / L2: the registers of wider passes would halve the warps
 // an SM holds for the common case of one or two).
-template <int F>
-__global__ void __launch_bounds__(kDecodeThreads) decode_gate_up_kernel(const Stack S, const uint16_t* __restrict__ latent, int ld,
+template <int F, bool WHOLE>
+__global__ void __launch_bounds__(kDecodeThreads, WHOLE && F != LX_W_BF16X && F != LX_W_NVFP4 ? 3 : 2) decode_gate_up_kernel(const Stack S, const uint16_t* __restrict__ latent, int ld,
                                                                         int xvec, const int32_t* __restrict__ ids,
                                                                         uint16_t* __restrict__ mid, int P, int top_k, int I,
                                                                         int dedupe) {
@@ -302,17 +386,18 @@ __global__ void __launch_bounds__(kDecodeThreads) decode_gate_up_kernel(const St
       if (left) {
         member[1] = __ffsll(static_cast<long long>(left)) - 1;
         left &= left - 1;
-        gate_up_members<F, 2>(S, e, i, I, latent, ld, xvec != 0, member, 2, top_k, mid, lane);
+        gate_up_members<F, 2, WHOLE>(S, e, i, I, latent, ld, xvec != 0, member, 2, top_k, mid, lane);
       } else {
         const int m1[1] = {member[0]};
-        gate_up_members<F, 1>(S, e, i, I, latent, ld, xvec != 0, m1, 1, top_k, mid, lane);
+        gate_up_members<F, 1, WHOLE>(S, e, i, I, latent, ld, xvec != 0, m1, 1, top_k, mid, lane);
       }
     }
   }
 }
 
-// Stage 2: out[t, l] = sum over k, in order, of weights[t, k] * (s_l * down[e_k]_l . mid[t, k]). grid (ceil(L / 8), T).
-template <int F>
+// Stage 2: out[t, l] = sum over k, in order, of weights[t, k] * (s_l * down[e_k]_l . mid[t, k]). grid (ceil(L / 16), T): a warp
+// takes two rows, so that the intermediate row's conversion serves both.
+template <int F, bool WHOLE>
 __global__ void __launch_bounds__(kDecodeThreads) decode_down_kernel(const Stack S, const uint16_t* __restrict__ mid, int xvec,
                                                                      const int32_t* __restrict__ ids,
                                                                      const float* __restrict__ weights, float* __restrict__ out,
@@ -320,23 +405,33 @@ __global__ void __launch_bounds__(kDecodeThreads) decode_down_kernel(const Stack
   pdl_trigger();
   pdl_wait();  // the intermediates come from the gate/up kernel
   const int t = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int l = blockIdx.x * kRowsPerBlock + warp;
-  if (l >= L) return;
-  float total = 0.0f;
+  const int l0 = (blockIdx.x * kRowsPerBlock + warp) * kDownRows;
+  if (l0 >= L) return;
+  float total[kDownRows] = {};
 #pragma unroll 1
   for (int k = 0; k < top_k; ++k) {
     const int p = t * top_k + k, e = ids[p];
-    const int64_t n = static_cast<int64_t>(e) * S.rows + l;
-    const uint8_t* const row[1] = {S.data + n * S.row_bytes};
-    const uint8_t* const row_scale[1] = {scale_row<F>(S, n)};
-    const uint32_t flag[1] = {row_flag<F>(row[0])};
+    int64_t n[kDownRows];
+    const uint8_t *row[kDownRows], *row_scale[kDownRows];
+    uint32_t flag[kDownRows];
+    float acc[kDownRows][1];
+#pragma unroll
+    for (int r = 0; r < kDownRows; ++r) {
+      n[r] = static_cast<int64_t>(e) * S.rows + min(l0 + r, L - 1);  // (past the last row: that row again, not written)
+      row[r] = S.data + n[r] * S.row_bytes;
+      row_scale[r] = scale_row<F>(S, n[r]);
+      flag[r] = row_flag<F>(row[r]);
+      acc[r][0] = 0.0f;
+    }
     const uint16_t* const x[1] = {mid + static_cast<int64_t>(p) * S.K};
-    float acc[1][1] = {{0.0f}};
-    dot_rows<F, 1, 1>(S, row, row_scale, flag, x, xvec != 0, lane, acc);
-    const float term = __fmul_rn(weights[p], __fmul_rn(stack_row_factor<F>(S, n, e), warp_sum(acc[0][0])));
-    total = __fadd_rn(total, term);
+    dot_rows<F, kDownRows, 1, WHOLE>(S, row, row_scale, flag, x, xvec != 0, lane, acc);
+#pragma unroll
+    for (int r = 0; r < kDownRows; ++r)
+      total[r] = __fadd_rn(total[r], __fmul_rn(weights[p], __fmul_rn(stack_row_factor<F>(S, n[r], e), warp_sum(acc[r][0]))));
   }
-  if (lane == 0) out[static_cast<int64_t>(t) * L + l] = total;
+#pragma unroll
+  for (int r = 0; r < kDownRows; ++r)
+    if (lane == 0 && l0 + r < L) out[static_cast<int64_t>(t) * L + l0 + r] = total[r];
 }
 
 // ---- host ------------------------------------------------------------------------------------------------------------
@@ -353,7 +448,7 @@ Stack make_stack(int type, const void* data, const void* scale, const float* exp
     case LX_W_BF16X: S.row_bytes = x16::row_bytes(K); break;
     default: S.row_bytes = K; break;
   }
-  const int word = type == LX_W_NVFP4 ? 8 : 16;
+  const int word = type == LX_W_NVFP4 || type == LX_W_BF16X ? 8 : 16;
   S.vec = aligned(data, word) && S.row_bytes % word == 0;
   return S;
 }
@@ -363,15 +458,15 @@ int launch_gate_up(const Stack& S, const void* latent, const int32_t* ids, uint1
                    cudaStream_t s) {
   const int xvec = aligned(latent, 16) && L % 8 == 0;
   const dim3 grid(static_cast<unsigned>((I + kGateUpRows - 1) / kGateUpRows), static_cast<unsigned>(P));
-  return launch_kernel(decode_gate_up_kernel<F>, grid, dim3(kDecodeThreads), 0, s, S, static_cast<const uint16_t*>(latent), L, xvec,
+  return launch_kernel(S.vec && xvec ? decode_gate_up_kernel<F, true> : decode_gate_up_kernel<F, false>, grid, dim3(kDecodeThreads), 0, s, S, static_cast<const uint16_t*>(latent), L, xvec,
                        ids, mid, P, top_k, I, P <= kScanPairs ? 1 : 0);
 }
 template <int F>
 int launch_down(const Stack& S, const uint16_t* mid, const int32_t* ids, const float* weights, float* out, int T, int L, int I,
                 int top_k, cudaStream_t s) {
   const int xvec = aligned(mid, 16) && I % 8 == 0;
-  const dim3 grid(static_cast<unsigned>((L + kRowsPerBlock - 1) / kRowsPerBlock), static_cast<unsigned>(T));
-  return launch_kernel(decode_down_kernel<F>, grid, dim3(kDecodeThreads), 0, s, S, mid, xvec, ids, weights, out, top_k, L);
+  const dim3 grid(static_cast<unsigned>((L + kRowsPerBlock * kDownRows - 1) / (kRowsPerBlock * kDownRows)), static_cast<unsigned>(T));
+  return launch_kernel(S.vec && xvec ? decode_down_kernel<F, true> : decode_down_kernel<F, false>, grid, dim3(kDecodeThreads), 0, s, S, mid, xvec, ids, weights, out, top_k, L);
 }
 
 // Both stages on stacks already checked. The grid's second extent holds pairs (tokens): up to 65535 of them per launch.
