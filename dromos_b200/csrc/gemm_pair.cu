@@ -162,12 +162,10 @@ __device__ __forceinline__ void pair_store(const PairParams& P, Y* __restrict__ 
     }
     return P.alpha * (rf * (sum * scale) + bias);
   };
-  auto put = [&](Y* at, float v) {
-    if constexpr (sizeof(Y) == 4) {
-      *at = P.beta != 0.0f ? fmaf(P.beta, *at, v) : v;
-    } else {
-      *at = static_cast<uint16_t>(f32_to_bf16_bits(P.beta != 0.0f ? fmaf(P.beta, bf16_bits_to_f32(*at), v) : v));
-    }
+  auto put = [&](Y* at, float v, float old) {
+    if (P.beta != 0.0f) v = fmaf(P.beta, old, v);
+    if constexpr (sizeof(Y) == 4) *at = v;
+    else *at = static_cast<uint16_t>(f32_to_bf16_bits(v));
   };
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
@@ -175,13 +173,22 @@ __device__ __forceinline__ void pair_store(const PairParams& P, Y* __restrict__ 
     uint32_t raw[PLANES][16];
 #pragma unroll
     for (int p = 0; p < PLANES; ++p) tmem_ld16(d_addr + p * P.half + 16 * q, raw[p]);
-    tmem_wait_ld();
     const int left = rows - 16 * q;
+    float old[16];  // with beta: all sixteen asked for before the first is stored (see gemm_tc.cu)
+#pragma unroll
+    for (int j = 0; j < 16; ++j) old[j] = 0.0f;
+    if (P.beta != 0.0f && live) {
+      const Y* from = y;
+#pragma unroll
+      for (int j = 0; j < 16; ++j, from += ld)
+        if (j < left) old[j] = sizeof(Y) == 4 ? static_cast<float>(*from) : bf16_bits_to_f32(static_cast<uint32_t>(*from));
+    }
+    tmem_wait_ld();
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       const float scale = PLANES == 1 && kAct == kActBf16 ? 1.0f : __shfl_sync(0xffffffffu, inv[q / 2], 16 * (q & 1) + j);
       const float v = value(raw, j, scale);
-      if (live && j < left) put(y, v);
+      if (live && j < left) put(y, v, old[j]);
       y += ld;
     }
   }

@@ -155,9 +155,17 @@ __device__ __forceinline__ void expand_nvfp4(uint32_t w0, uint32_t w1, uint32_t 
 }
 
 // ---- the epilogue of a tile ---------------------------------------------------------------------------------------------
+// What y holds at rows m0 .. m0 + 7 of column n (0 past M), for beta. All eight are asked for before the first is stored: loads
+// and stores of one buffer taken in turn wait for each other, a round trip to L2 per row (37 rows x 10309 bf16 outputs with
+// beta, the copy of the old outputs and the preparation included: 30.7 us then, 24.2 now).
+__device__ __forceinline__ void load_old(const TcParams& P, int m0, int n, float (&old)[8]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) old[j] = m0 + j < P.M ? load_f32(P.y, P.y_dtype, static_cast<int64_t>(m0 + j) * P.ld_y + n) : 0.0f;
+}
+
 template <int kAct, bool kPeers>
 __device__ __forceinline__ void combine_and_store(const TcParams& P, const uint32_t (&raw)[3][8], const float (&inv)[8], int m0, int n, float rf,
-                                                  float bias) {
+                                                  float bias, const float (&old)[8]) {
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const int m = m0 + j;
@@ -177,7 +185,7 @@ __device__ __forceinline__ void combine_and_store(const TcParams& P, const uint3
       for (int g = 0; g < P.peers; ++g) store_from_f32(P.y_peer[g], P.y_dtype, at + P.col0, out);
       continue;
     }
-    if (P.beta != 0.0f) out = fmaf(P.beta, load_f32(P.y, P.y_dtype, at), out);
+    if (P.beta != 0.0f) out = fmaf(P.beta, old[j], out);
     store_from_f32(P.y, P.y_dtype, at, out);
   }
 }
@@ -218,7 +226,13 @@ __device__ __forceinline__ void finish_tile(const TcParams& P, const RowTerms& T
     if (release_bar && lane == 0) mbar_arrive(release_bar);
   };
   uint32_t raw[3][8];
+  const bool adds = !kPeers && P.beta != 0.0f && T.live;
+  float old[8] = {}, next[8] = {};  // y at this chunk and the next one
+  if (adds && chunk0 < chunks) load_old(P, chunk0 * 8, T.n, next);
   for (int c = chunk0; c < chunks; c += chunk_step) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) old[j] = next[j];
+    if (adds && c + chunk_step < chunks) load_old(P, (c + chunk_step) * 8, T.n, next);
 #pragma unroll
     for (int p = 0; p < 3; ++p)
       if (p < P.planes) tmem_ld8(d_addr + p * Mp + c * 8, raw[p]);
@@ -227,7 +241,7 @@ __device__ __forceinline__ void finish_tile(const TcParams& P, const RowTerms& T
     for (int j = 0; j < 8; ++j) inv[j] = __shfl_sync(0xffffffffu, c < 4 ? inv_lo : inv_hi, (c * 8 + j) & 31);
     tmem_wait_ld();
     if (c + chunk_step >= chunks) release();
-    if (T.live) combine_and_store<kAct, kPeers>(P, raw, inv, c * 8, T.n, T.rf, T.bias);
+    if (T.live) combine_and_store<kAct, kPeers>(P, raw, inv, c * 8, T.n, T.rf, T.bias, old);
   }
   if (chunk0 >= chunks) release();
 }
