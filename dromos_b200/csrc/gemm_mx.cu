@@ -1,0 +1,571 @@
+// lx_gemm_w on NVFP4 weights: y[m, n] = sum_k x[m, k] * w[n, k], up to 64 activation rows per pass, with the weights
+// multiplied as they are stored (tcgen05.mma kind::mxf4nvf4, block scales of 16 values applied by the tensor core).
+//
+// Why digits. No instruction multiplies e2m1 x e4m3-block-scale weights by wider activations, and expanding the weights to
+// f16 in registers was what bound the kernels before this one: eight converter warps, ~27 instructions per 16 values, 72 us
+// for 28672 x 8192 at 16 rows where the bytes take 20. So it is the activations that are taken apart, once per call, into
+// what the instruction multiplies: every block of 16 values gets the power of two of its largest magnitude as its scale and
+// seven digits in base 8 (-4..4, exact in e2m1), 21 bits below that magnitude. A bf16 value within 2^-12 of its block's
+// largest comes out exactly, a smaller one within 2^-20 of that largest. A digit is a column of its own
+// (column j * Mp + m is digit j of row m), summed on its own in f32 and put together in the epilogue, least first. (Block
+// scales reach 2^-17 of the row's largest magnitude; a block below that keeps the bits above 2^-36 of it.) Against 64 bits,
+// N(0, 1) activations: 4e-8 at every K, where the f16 expansion was off by 1e-7 (K = 512) to 2.4e-6 (K = 8192); with six
+// digits it was 4e-7, more than before at short K.
+//
+// What a product costs: an instruction covers 128 weight rows x 64 values of K (four times kind::f16's) for half a cycle per
+// column; up to 64 rows are 448 columns in two instructions of four and three digits. A launch takes up to 1024 rows in
+// chunks of at most 64, the chunks of a weight panel next to each other so that its later readers find it in L2.
+//
+// Measured (28672 x 8192; before: the f16 expansion): 16 / 32 / 64 rows 72.1 / 74.5 / 83 -> 42.5 / 47 / 75 us; 14336 x 4096, 100 / 500
+// / 1000 rows 49 / 209 / 415 -> 43 / 132 / 244. What a stage takes at 16 rows is its copies (39 us with products and scales
+// left out); at 64 rows the 60 KB of digits that every SM fetches from L2 per 12 KB of weights.
+//   * The block scales go to tensor memory with tcgen05.st. Written to shared memory for tcgen05.cp they needed the proxy fence,
+//     which waits for the thread's scale loads in flight: 84 us. With the activations' scales by tcgen05.cp: 57 us (copies
+//     and products of one pipe wait for each other).
+//   * As many stages of activations in flight as of weights: with four, 16 rows took 50 us.
+//
+// Roles (one CTA per SM, tiles of R <= 128 weight rows dealt evenly, as in gemm_tc.cu): warps 0-3 epilogue (lane = weight
+// row); warps 4-7 bring the block scales: each thread loads its weight row's 16 bytes per stage straight from memory, kAhead
+// stages ahead (a tile copy of 16 bytes per row costs the copy engine as much as one of 128), the four warps exchange rows
+// through shared memory, and every warp writes all of them to its quarter of tensor memory, the activations' beside them;
+// warp 8 weights, warp 10 activations (one thread each, bulk copies, no multicast); warp 9 issues.
+//
+// Weights and their scales stream before the dependency wait, as in gemm_tc.cu. Every wait is bounded; a role that gives up
+// leaves its loop, the producers wait (bounded) for their copies in flight, and the CTA frees its tensor memory.
+#include "tc.cuh"
+
+namespace b200 {
+namespace {
+
+constexpr int kMxStageK = 256;                  // values of K per stage: 128 bytes per weight row, four products
+constexpr int kMxDigits = 7;
+constexpr int kMxThreads = 11 * 32;
+constexpr int kMxScaleBytes = 2 * 128 * 16;     // shared memory in which the scale warps exchange rows: two stages of 128 rows x 16 bytes
+constexpr int kAhead = 8;                       // stages whose weight scales a thread has in flight
+
+struct MxParams {
+  const uint8_t* scale;     // e4m3 [N, K / 16]
+  float global;
+  int N, K, M;
+  int chunks, chunk_rows;   // the activation rows are multiplied in chunks of at most 64
+  int64_t chunk_bytes;      // a chunk's prepared activations
+  int R, box_bytes;         // weight rows per tile; shared memory of a stage's box (1024-aligned)
+  int Mp;                   // accumulator columns per digit
+  int cols0, cols1;         // columns of a step's first instruction and of its second (0: one takes all digits)
+  int sf0, sf_stages;       // where in tensor memory the scales begin, and for how many stages in turn (4, 2 or 1)
+  int x_bytes, sf_off;      // a stage's activations: digits, and from sf_off on the block scales
+  const uint8_t* xprep;
+  const float* row_scale;   // per activation row: what its sums are multiplied by
+  int buffers;              // accumulators (2 where they fit)
+  int SW, SX;
+  const void* bias;
+  int bias_dtype;
+  void* y;
+  int y_dtype, ld_y;
+  float alpha, beta;
+  int* status;
+};
+
+// ---- activations -----------------------------------------------------------------------------------------------------------
+// bf16 bits of value k of a row (f32 rows are rounded first, as lx_gemm_w does).
+template <bool XBF>
+__device__ __forceinline__ uint32_t bf16_at(const void* x, int64_t i) {
+  if constexpr (XBF) return static_cast<const uint16_t*>(x)[i];
+  else return f32_to_bf16_bits(static_cast<const float*>(x)[i]) & 0xffffu;
+}
+// Eight values as packed bf16.
+template <bool XBF>
+__device__ __forceinline__ uint4 bf16x8_at(const void* x, int64_t i, bool vec) {
+  if (vec) {
+    if constexpr (XBF) return *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(x) + i);
+    const float4 a = *reinterpret_cast<const float4*>(static_cast<const float*>(x) + i), b = *reinterpret_cast<const float4*>(static_cast<const float*>(x) + i + 4);
+    auto pack = [](float lo, float hi) { return (f32_to_bf16_bits(lo) & 0xffffu) | (f32_to_bf16_bits(hi) << 16); };
+    return make_uint4(pack(a.x, a.y), pack(a.z, a.w), pack(b.x, b.y), pack(b.z, b.w));
+  }
+  uint32_t w[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) w[j] = bf16_at<XBF>(x, i + 2 * j) | (bf16_at<XBF>(x, i + 2 * j + 1) << 16);
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+__device__ __forceinline__ uint32_t max_magnitude(uint32_t m, const uint4& v) {  // bf16 magnitudes order as integers, NaN above all
+  const uint32_t t = __vmaxu2(__vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu), __vmaxu2(v.z & 0x7fff7fffu, v.w & 0x7fff7fffu));
+  return max(m, max(t & 0xffffu, t >> 16));
+}
+// 2^e as ue4m3, e in -9..8.
+__device__ __forceinline__ uint32_t ue4m3_pow2(int e) { return e >= -6 ? static_cast<uint32_t>(e + 7) << 3 : 1u << (e + 9); }
+
+// Block (piece, row): 256 threads, each 8 values (half a scale block) of an activation row; every block finds the row's largest
+// magnitude again (a few KB, from L2), which saves a second kernel. (With 32 values per thread the seven digits of each were
+// ~1400 instructions in a row: at 16 rows the preparation took as long as an eighth of the product.)
+// Rows that are not finite: a NaN, or more than one infinity, makes the row's outputs NaN; with a single infinity the finite
+// values do not count and the outputs are the infinity times its weight (NaN where that is zero).
+constexpr int kPrepThreads = 256;
+template <bool XBF>
+__global__ void __launch_bounds__(kPrepThreads) mx_prep_kernel(const void* __restrict__ x, int ld_x, int K, int chunk_rows, int64_t chunk_bytes, int Mp, int cols0,
+                                                               int cols1, int x_bytes, int sf_off, uint8_t* __restrict__ out, float* __restrict__ row_scale) {
+  pdl_trigger();
+  pdl_wait();  // the kernel before this one may still be reading the workspace
+  __shared__ uint32_t part[kPrepThreads / 32], infinities;
+  const int row_id = blockIdx.y, chunk = row_id / chunk_rows, m = row_id - chunk * chunk_rows, tid = threadIdx.x;
+  const int64_t row = static_cast<int64_t>(row_id) * ld_x;
+  const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && ld_x % (XBF ? 8 : 4) == 0;
+  const int k0 = (blockIdx.x * kPrepThreads + tid) * 8;
+  const uint4 v = k0 < K ? bf16x8_at<XBF>(x, row + k0, vec) : make_uint4(0, 0, 0, 0);
+  uint32_t top = 0;
+#pragma unroll 4
+  for (int k = 8 * tid; k < K; k += 8 * kPrepThreads) top = max_magnitude(top, bf16x8_at<XBF>(x, row + k, vec));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+  if ((tid & 31) == 0) part[tid >> 5] = top;
+  if (tid == 0) infinities = 0;
+  uint32_t block_top = max_magnitude(0, v);
+  block_top = max(block_top, __shfl_xor_sync(0xffffffffu, block_top, 1));
+  __syncthreads();
+  top = 0;
+#pragma unroll
+  for (int i = 0; i < kPrepThreads / 32; ++i) top = max(top, part[i]);
+  const bool finite = top < 0x7f80u;
+  if (!finite) {
+    uint32_t n = 0;
+    for (int k = tid; k < K; k += kPrepThreads) n += (bf16_at<XBF>(x, row + k) & 0x7fffu) == 0x7f80u;
+    atomicAdd(&infinities, n);
+    __syncthreads();
+  }
+  const int e_row = max(static_cast<int>(top >> 7), 30) - 127;
+  if (blockIdx.x == 0 && tid == 0)
+    row_scale[row_id] = finite ? __uint_as_float(static_cast<uint32_t>(e_row - 8 + 127) << 23)
+                               : __uint_as_float(top == 0x7f80u && infinities == 1 ? 0x7f800000u : 0x7fc00000u);
+  if (k0 >= K) return;
+  constexpr int kUnit = 3 * kMxDigits - 2;  // the last digit counts in 2^(e - kUnit), the first in 2^e / 2
+  const int e = max(max(static_cast<int>(block_top >> 7), 1) - 127, e_row - 17);  // 2^-9 is the least scale
+  // 2^(kUnit - e) in two factors: the whole can be beyond f32
+  const int half = (kUnit - e) / 2;
+  const float f0 = __uint_as_float(static_cast<uint32_t>(half + 127) << 23), f1 = __uint_as_float(static_cast<uint32_t>(kUnit - e - half + 127) << 23);
+  const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+  uint32_t w[kMxDigits] = {};
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t bits = (words[i / 2] >> (16 * (i & 1))) & 0xffffu;
+    int q;
+    if (finite) q = __float2int_rn(bf16_bits_to_f32(bits) * f0 * f1);
+    else q = (bits & 0x7fffu) != 0x7f80u ? 0 : bits & 0x8000u ? -(4 << 3 * (kMxDigits - 1)) : 4 << 3 * (kMxDigits - 1);  // the first digit alone
+#pragma unroll
+    for (int j = kMxDigits - 1; j > 0; --j) {
+      const int u8 = (q + 4) & 7;  // the digit plus 4
+      w[j] |= ((0x32109abcu >> (4 * u8)) & 15u) << (4 * i);
+      q = (q + 4 - u8) >> 3;
+    }
+    w[0] |= static_cast<uint32_t>(q < 0 ? 8 - q : q) << (4 * i);
+  }
+  uint8_t* stage = out + chunk * chunk_bytes + static_cast<size_t>(k0 / kMxStageK) * x_bytes;
+  const int kb = (k0 % kMxStageK) / 2, NC = cols0 + cols1, atoms = (cols0 + 127) / 128;
+#pragma unroll
+  for (int j = 0; j < kMxDigits; ++j) *reinterpret_cast<uint32_t*>(stage + block_offset(NC, kb & ~15, j * Mp + m) + (kb & 15)) = w[j];
+  if (k0 % 16 != 0) return;
+  // scales: product k0 / 64 of the stage; 128 columns are 32 lanes of 16 bytes, a column's 4 bytes at word column / 32
+  const uint8_t sf = static_cast<uint8_t>(finite ? ue4m3_pow2(e - e_row + 8) : 0x38u);
+  uint8_t* sfs = stage + sf_off + (k0 % kMxStageK) / 64 * (atoms * 512) + (k0 % 64) / 16;
+  for (int c = m; c < cols0; c += Mp) sfs[(c >> 7) * 512 + (c & 31) * 16 + ((c >> 5) & 3) * 4] = sf;
+}
+
+// ---- instructions ------------------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr), "r"(r[0]),
+               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]),
+               "r"(r[13]), "r"(r[14]), "r"(r[15])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void mx_umma(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t sfa, uint32_t sfb,
+                                        uint32_t accumulate) {
+  asm volatile(
+      "{ .reg .pred p; .reg .b64 da, db; setp.ne.u32 p, %8, 0; mov.b64 da, {%1, %2}; mov.b64 db, {%3, %4};\n"
+      "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], da, db, %5, [%6], [%7], p; }" ::"r"(d_tmem),
+      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate)
+      : "memory");
+}
+
+// ---- the product -------------------------------------------------------------------------------------------------------------
+// ATOMS: 128-column pieces of a step's activation scales; TWO: two instructions per step.
+// Tensor memory columns of a stage's scales: 4 products x 4 columns of the weights', then 4 x 4 per piece of the activations'.
+template <int ATOMS, bool TWO>
+__global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_constant__ CUtensorMap wmap, const MxParams P) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  constexpr int kSfCols = 16 + 16 * ATOMS;
+  const int SW = P.SW, SX = P.SX, x_bytes = P.x_bytes, box_bytes = P.box_bytes;
+  // The tensor core reads 128 rows from every box, whatever R is: behind the boxes come the scales and the activations.
+  uint8_t* const sring = smem + static_cast<size_t>(SW) * box_bytes;
+  uint8_t* const xring = sring + kMxScaleBytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(xring + static_cast<size_t>(SX) * x_bytes);
+  const uint32_t bar0 = smem_u32(bars);
+  auto w_full = [&](int s) { return bar0 + 8u * s; };                       // weights landed
+  auto w_empty = [&](int s) { return bar0 + 8u * (SW + s); };               // products done
+  auto x_full = [&](int s) { return bar0 + 8u * (2 * SW + s); };
+  auto x_empty = [&](int s) { return bar0 + 8u * (2 * SW + SX + s); };
+  auto s_full = [&](int b) { return bar0 + 8u * (2 * SW + 2 * SX + b); };       // scales b are in tensor memory
+  auto s_empty = [&](int b) { return bar0 + 8u * (2 * SW + 2 * SX + 4 + b); };  // and their products are done
+  auto d_full = [&](int b) { return bar0 + 8u * (2 * SW + 2 * SX + 8 + b); };   // accumulator b is complete
+  auto d_empty = [&](int b) { return bar0 + 8u * (2 * SW + 2 * SX + 10 + b); };  // and has been read
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * SW + 2 * SX + 12);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int n_stages = P.K / kMxStageK;
+  // a tile is a panel of weight rows times a chunk; the chunks of a panel are neighbours, so that its later readers find it in L2
+  const int chunks = P.chunks;
+  const int n_tiles = (P.N + P.R - 1) / P.R * chunks;
+  const int tile_begin = static_cast<int>(static_cast<int64_t>(n_tiles) * blockIdx.x / gridDim.x);
+  const int tile_end = static_cast<int>(static_cast<int64_t>(n_tiles) * (blockIdx.x + 1) / gridDim.x);
+  const int total = (tile_end - tile_begin) * n_stages;
+
+  if (tid == 0) {
+    for (int s = 0; s < SW; ++s) {
+      mbar_init(w_full(s), 1);
+      mbar_init(w_empty(s), 1);
+    }
+    for (int s = 0; s < SX; ++s) {
+      mbar_init(x_full(s), 1);
+      mbar_init(x_empty(s), 1);
+    }
+    for (int b = 0; b < 4; ++b) {
+      mbar_init(s_full(b), 4);
+      mbar_init(s_empty(b), 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(d_full(b), 1);
+      mbar_init(d_empty(b), 4);
+    }
+    mbar_init_fence();
+  }
+  if (warp == 9) {
+    tmem_alloc(smem_u32(tmem_slot), kTmemColumns);
+    tmem_relinquish();
+    tc_fence_before();
+  }
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 8) {
+    // ================================ weights ================================
+    pdl_trigger();
+    if (lane == 0) {  // static: no wait
+      asm volatile("prefetch.tensormap [%0];" ::"l"(&wmap) : "memory");
+      Ring w;
+      bool ok = true, wrapped = false;
+      int issued = 0;
+      for (int tile = tile_begin; tile < tile_end && ok; ++tile) {
+        const int row = tile / chunks * P.R;
+        for (int s = 0; s < n_stages; ++s) {
+          if (wrapped && !tc_wait(w_empty(w.slot), w.lap ^ 1u, P.status)) {
+            ok = false;
+            break;
+          }
+          mbar_arrive_expect_tx(w_full(w.slot), P.R * 128);
+          tile_g2s(smem_u32(smem) + static_cast<uint32_t>(w.slot) * box_bytes, &wmap, s * 32, row, w_full(w.slot));
+          ++issued;
+          w.advance(SW);
+          wrapped |= w.slot == 0;
+        }
+      }
+      if (!ok)  // the copies in flight land before the CTA leaves
+        for (int i = max(0, issued - SW); i < issued; ++i) tc_wait(w_full(i % SW), (i / SW) & 1, P.status);
+    }
+  } else if (warp == 10) {
+    // ================================ activations ================================
+    if (lane == 0) {
+      pdl_wait();  // prepared by the kernel before this one
+      Ring x;
+      bool ok = true, wrapped = false;
+      int s = 0, i = 0, chunk = tile_begin % chunks;
+      const uint8_t* src = P.xprep + chunk * P.chunk_bytes;
+      for (; i < total; ++i) {
+        if (wrapped && !tc_wait(x_empty(x.slot), x.lap ^ 1u, P.status)) {
+          ok = false;
+          break;
+        }
+        mbar_arrive_expect_tx(x_full(x.slot), x_bytes);
+        bulk_g2s(smem_u32(xring) + static_cast<uint32_t>(x.slot) * x_bytes, src + static_cast<size_t>(s) * x_bytes, x_bytes, x_full(x.slot));
+        x.advance(SX);
+        wrapped |= x.slot == 0;
+        if (++s == n_stages) {
+          s = 0;
+          if (++chunk == chunks) chunk = 0;
+          src = P.xprep + chunk * P.chunk_bytes;
+        }
+      }
+      if (!ok)
+        for (int j = max(0, i - SX); j < i; ++j) tc_wait(x_full(j % SX), (j / SX) & 1, P.status);
+    }
+  } else if (warp == 9) {
+    // ================================ issuer ================================
+    if (lane == 0) {
+      const int NC = P.cols0 + P.cols1;
+      // e2m1 x e2m1, ue4m3 scales, 128 rows
+      const uint32_t idesc = (1u << 7) | (1u << 10) | (1u << 27);
+      const uint32_t idesc0 = idesc | (static_cast<uint32_t>(P.cols0 >> 3) << 17), idesc1 = idesc | (static_cast<uint32_t>(P.cols1 >> 3) << 17);
+      const uint32_t lbo = static_cast<uint32_t>(NC / 8) * 128, sbo = 128;
+      const uint32_t a_hi = (1024u >> 4) | (1u << 14) | (2u << 29), b_hi = (sbo >> 4) | (1u << 14);
+      const uint32_t a_lo0 = ((smem_u32(smem) & 0x3ffffu) >> 4) | (1u << 16);
+      const uint32_t b_lo0 = ((smem_u32(xring) & 0x3ffffu) >> 4) | ((lbo >> 4) << 16);
+      const uint32_t b_step = (2u * lbo) >> 4, b_second = static_cast<uint32_t>(P.cols0 / 8) * 128 >> 4;
+      Ring w, x;
+      bool ok = true;
+      const uint32_t sf_mask = P.sf_stages - 1, sf_shift = P.sf_stages == 4 ? 2 : P.sf_stages == 2 ? 1 : 0;
+      uint32_t i = 0;
+      for (int tile = tile_begin, t = 0; tile < tile_end && ok; ++tile, ++t) {
+        const int buf = P.buffers == 2 ? t & 1 : 0, use = P.buffers == 2 ? t >> 1 : t;  // this accumulator's use-th use
+        const uint32_t d_tmem = tmem_base + buf * NC;
+        if (use > 0 && !tc_wait(d_empty(buf), (use - 1) & 1, P.status)) break;
+        tc_fence_after();
+        for (int s = 0; s < n_stages; ++s, ++i) {
+          const uint32_t turn = i & sf_mask, sfa = tmem_base + P.sf0 + turn * kSfCols, sfb = sfa + 16;
+          if (!tc_wait(x_full(x.slot), x.lap, P.status) || !tc_wait(w_full(w.slot), w.lap, P.status) || !tc_wait(s_full(turn), (i >> sf_shift) & 1, P.status)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t x_at = (static_cast<uint32_t>(x.slot) * x_bytes) >> 4;
+          const uint32_t a_lo = a_lo0 + ((static_cast<uint32_t>(w.slot) * box_bytes) >> 4), b_lo = b_lo0 + x_at;
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks) {
+            mx_umma(d_tmem, a_lo + 2 * ks, a_hi, b_lo + ks * b_step, b_hi, idesc0, sfa + 4 * ks, sfb + 4 * ATOMS * ks, (s | ks) ? 1u : 0u);
+            if constexpr (TWO) mx_umma(d_tmem + P.cols0, a_lo + 2 * ks, a_hi, b_lo + ks * b_step + b_second, b_hi, idesc1, sfa + 4 * ks, sfb + 4 * ATOMS * ks, (s | ks) ? 1u : 0u);
+          }
+          umma_commit(w_empty(w.slot));
+          umma_commit(x_empty(x.slot));
+          umma_commit(s_empty(turn));
+          w.advance(SW);
+          x.advance(SX);
+        }
+        if (ok) umma_commit(d_full(buf));
+      }
+    }
+  } else if (warp >= 4) {
+    // ================================ weight scales ================================
+    const int r = tid - 128;
+    const int64_t pitch = P.K / 16;
+    uint4 q[kAhead];
+    int lt = tile_begin, ls = 0, lc = tile_begin % chunks;  // the stage that is loaded next, and its tile's chunk
+    int row = tile_begin / chunks * P.R + r;
+    const uint8_t* src = P.scale + row * pitch;
+    bool live = r < P.R && row < P.N;
+    auto load = [&](uint4& v) {
+      if (lt < tile_end && live) v = __ldg(reinterpret_cast<const uint4*>(src) + ls);
+      if (++ls == n_stages) {
+        ls = 0, ++lt;
+        if (++lc == chunks) {
+          lc = 0, row += P.R;
+          src = P.scale + row * pitch;
+          live = r < P.R && row < P.N;
+        }
+      }
+    };
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) {
+      q[i] = make_uint4(0, 0, 0, 0);
+      load(q[i]);
+    }
+    // Lane l of each of the four warps holds rows l, 32 + l, 64 + l and 96 + l in tensor memory: every quarter has all 128 rows.
+    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + P.sf0;
+    Ring w, x;
+    bool ok = true;
+    for (int i0 = 0; i0 < total; i0 += kAhead) {  // (a warp whose wait gave up still comes to the meetings)
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) {
+        if (i0 + i >= total) break;
+        const int turn = i & (P.sf_stages - 1), use = (i0 + i) / P.sf_stages;
+        if ((q[i].x | q[i].y | q[i].z | q[i].w) & 0x80808080u) {  // scales have no sign here: it goes to the block's values
+          ok = ok && tc_wait(w_full(w.slot), w.lap, P.status);
+          const uint32_t sc[4] = {q[i].x, q[i].y, q[i].z, q[i].w};
+          uint8_t* box = smem + static_cast<size_t>(w.slot) * box_bytes + r * 128;
+          for (int b = 0; b < 16 && ok && r < P.R; ++b)
+            if (sc[b >> 2] >> (8 * (b & 3)) & 0x80u) {
+              uint2* at = reinterpret_cast<uint2*>(box + (((b >> 1) ^ (r & 7)) << 4) + 8 * (b & 1));
+              *at = make_uint2(at->x ^ 0x88888888u, at->y ^ 0x88888888u);
+            }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor core reads what this thread wrote
+        }
+        uint4* rows = reinterpret_cast<uint4*>(sring) + (i & 1) * 128;  // (two stages in turn: one meeting per stage is enough)
+        rows[r] = make_uint4(q[i].x & 0x7f7f7f7fu, q[i].y & 0x7f7f7f7fu, q[i].z & 0x7f7f7f7fu, q[i].w & 0x7f7f7f7fu);
+        load(q[i]);
+        __syncwarp();
+        named_bar_sync(1, 128);
+        uint32_t v[16];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const uint4 u = rows[32 * c + lane];
+          v[c] = u.x, v[4 + c] = u.y, v[8 + c] = u.z, v[12 + c] = u.w;
+        }
+        // the activations' scales lie behind their digits as the four words of each lane and product
+        ok = ok && tc_wait(x_full(x.slot), x.lap, P.status);
+        const uint4* xsf = reinterpret_cast<const uint4*>(xring + static_cast<size_t>(x.slot) * x_bytes + P.sf_off) + lane;
+        uint32_t xv[ATOMS][16];
+#pragma unroll
+        for (int j = 0; j < 4 * ATOMS; ++j) {
+          const uint4 u = xsf[32 * j];
+          uint32_t* to = xv[j / 4] + 4 * (j % 4);
+          to[0] = u.x, to[1] = u.y, to[2] = u.z, to[3] = u.w;
+        }
+        if (use > 0 && ok) ok = tc_wait(s_empty(turn), (use - 1) & 1, P.status);
+        ok = __all_sync(0xffffffffu, ok);
+        if (ok) {
+          const uint32_t at = lane_addr + turn * kSfCols;
+          tc_fence_after();
+          tmem_st16(at, v);
+#pragma unroll
+          for (int a = 0; a < ATOMS; ++a) tmem_st16(at + 16 + 16 * a, xv[a]);
+          tmem_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(s_full(turn));
+        }
+        x.advance(SX);
+        w.advance(SW);
+      }
+    }
+  } else {
+    // ================================ epilogue ================================
+    const int r = tid;
+    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
+    pdl_wait();  // y and the activation scales come from earlier kernels
+    for (int tile = tile_begin, t = 0; tile < tile_end; ++tile, ++t) {
+      const int buf = P.buffers == 2 ? t & 1 : 0, use = P.buffers == 2 ? t >> 1 : t;
+      const int panel = tile / chunks, m0 = (tile - panel * chunks) * P.chunk_rows, rows = min(P.chunk_rows, P.M - m0);
+      const int n = panel * P.R + r;
+      const bool live = r < P.R && n < P.N;
+      const float inv_lo = lane < rows ? P.row_scale[m0 + lane] : 0.0f, inv_hi = 32 + lane < rows ? P.row_scale[m0 + 32 + lane] : 0.0f;
+      const float bias = live && P.bias ? load_f32(P.bias, P.bias_dtype, n) : 0.0f;
+      if (!tc_wait(d_full(buf), use & 1, P.status)) break;
+      tc_fence_after();
+      const uint32_t d_addr = lane_addr + buf * (P.cols0 + P.cols1);
+      for (int c = 0; c < rows; c += 8) {
+        uint32_t raw[kMxDigits][8];
+#pragma unroll
+        for (int j = 0; j < kMxDigits; ++j) tmem_ld8(d_addr + j * P.Mp + c, raw[j]);
+        float old[8] = {};  // with beta: all eight asked for before the first is stored (see gemm_tc.cu)
+        if (P.beta != 0.0f && live) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if (c + i < rows) old[i] = load_f32(P.y, P.y_dtype, static_cast<int64_t>(m0 + c + i) * P.ld_y + n);
+        }
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float inv = __shfl_sync(0xffffffffu, c < 32 ? inv_lo : inv_hi, (c + i) & 31);
+          if (!live || c + i >= rows) continue;
+          float sum = __uint_as_float(raw[kMxDigits - 1][i]);
+#pragma unroll
+          for (int j = kMxDigits - 2; j >= 0; --j) sum = fmaf(sum, 0.125f, __uint_as_float(raw[j][i]));
+          float out = P.alpha * (P.global * (sum * inv) + bias);
+          const int64_t at = static_cast<int64_t>(m0 + c + i) * P.ld_y + n;
+          if (P.beta != 0.0f) out = fmaf(P.beta, old[i], out);
+          store_from_f32(P.y, P.y_dtype, at, out);
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(d_empty(buf));
+    }
+  }
+  __syncthreads();
+  if (warp == 9) tmem_dealloc(tmem_base, kTmemColumns);
+}
+
+// How a pass of M rows lies in accumulator columns and in the workspace. An instruction has at most 256 columns, in whole 16s.
+struct MxLayout {
+  int Mp, cols0, cols1, sf_off, x_bytes;
+  explicit MxLayout(int M) {
+    auto whole = [](int c) { return (c + 15) / 16 * 16; };
+    Mp = (M + 7) / 8 * 8;
+    cols0 = whole(kMxDigits * Mp), cols1 = 0;
+    if (cols0 > 256) cols0 = 4 * Mp, cols1 = whole((kMxDigits - 4) * Mp);  // four digits, then the rest
+    sf_off = (cols0 + cols1) * (kMxStageK / 2);
+    x_bytes = sf_off + 4 * ((cols0 + 127) / 128) * 512;
+  }
+};
+
+}  // namespace
+
+// The most rows one launch takes (more come in launches of as many): bounds the workspace.
+constexpr int kMxMaxRows = 1024;
+
+// Chunks of the fewest that hold M rows, all of the same size (a multiple of 8).
+static int mx_chunk_rows(int M) {
+  const int chunks = (M + kMaxRows - 1) / kMaxRows;
+  return ((M + chunks - 1) / chunks + 7) / 8 * 8;
+}
+
+int64_t mx_workspace_bytes(int M, int K) {
+  int64_t need = 0;
+  for (int rows : {std::min(M, kMxMaxRows), M % kMxMaxRows}) {  // a launch of the most rows, and the last one
+    if (rows == 0) continue;
+    const int chunk = mx_chunk_rows(rows);
+    const MxLayout L(chunk);
+    need = std::max(need, static_cast<int64_t>((rows + chunk - 1) / chunk) * ((K + kMxStageK - 1) / kMxStageK) * L.x_bytes + 4 * rows + 256);
+  }
+  return need;
+}
+
+// K % 256 == 0; weights, scales and workspace (mx_workspace_bytes) on 16 bytes. even_rows: the weight rows per tile that deal N
+// out evenly over the SMs.
+int mx_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const void* bias, int bias_dtype, void* y, int y_dtype, int ld_y,
+               int M, int N, int K, float alpha, float beta, void* workspace, int even_rows, cudaStream_t stream) {
+  if (K % kMxStageK != 0) return kNotSupported;
+  const bool x_bf16 = x_dtype == LX_BF16;
+  const int sms = sm_count();
+  if (!sms) return kInvalid;
+  uint8_t* ws = static_cast<uint8_t*>(workspace);
+  MxParams P{};
+  P.scale = static_cast<const uint8_t*>(w.scale);
+  P.global = w.global;
+  P.N = N, P.K = K;
+  P.bias = bias, P.bias_dtype = bias_dtype;
+  P.y_dtype = y_dtype, P.ld_y = ld_y;
+  P.alpha = alpha, P.beta = beta;
+  P.status = status_word();
+  P.xprep = ws;
+  for (int first = 0; first < M; first += kMxMaxRows) {
+    P.M = std::min(kMxMaxRows, M - first);
+    P.chunk_rows = mx_chunk_rows(P.M);
+    P.chunks = (P.M + P.chunk_rows - 1) / P.chunk_rows;
+    const MxLayout L(P.chunk_rows);
+    P.Mp = L.Mp, P.cols0 = L.cols0, P.cols1 = L.cols1, P.sf_off = L.sf_off, P.x_bytes = L.x_bytes;
+    P.chunk_bytes = static_cast<int64_t>(K / kMxStageK) * L.x_bytes;
+    // A tile takes as long with 128 weight rows as with fewer (its steps do), so what counts is the busiest SM's tiles; rows dealt
+    // evenly where that is the same.
+    auto turns = [&](int R) { return (static_cast<int64_t>((N + R - 1) / R) * P.chunks + sms - 1) / sms; };
+    P.R = turns(kBM) < turns(even_rows) ? kBM : even_rows;
+    P.box_bytes = (P.R + 7) / 8 * 1024;
+    // tensor memory from its end: the scales, then the accumulators, more than one of each where they fit
+    const int cols = L.cols0 + L.cols1;
+    const int sf_cols = 16 + 16 * ((L.cols0 + 127) / 128);
+    P.sf_stages = cols + 4 * sf_cols <= kTmemColumns ? 4 : cols + 2 * sf_cols <= kTmemColumns ? 2 : 1;
+    P.sf0 = kTmemColumns - P.sf_stages * sf_cols;
+    P.buffers = 2 * cols <= P.sf0 ? 2 : 1;
+    float* row_scale = reinterpret_cast<float*>(ws + P.chunks * P.chunk_bytes);
+    P.row_scale = row_scale;
+    P.y = static_cast<uint8_t*>(y) + static_cast<int64_t>(first) * ld_y * (y_dtype == LX_BF16 ? 2 : 4);
+    const void* xrow = static_cast<const uint8_t*>(x) + static_cast<int64_t>(first) * ld_x * (x_bf16 ? 2 : 4);
+    alignas(64) CUtensorMap wmap;
+    if (int e = make_tile_map(&wmap, w.data, K / 2, N, 128, P.R, 4, true)) return e;
+    if (int e = launch_kernel(x_bf16 ? mx_prep_kernel<true> : mx_prep_kernel<false>, dim3((K / 8 + kPrepThreads - 1) / kPrepThreads, P.M), dim3(kPrepThreads), 0, stream, xrow, ld_x, K,
+                              P.chunk_rows, P.chunk_bytes, L.Mp, L.cols0, L.cols1, L.x_bytes, L.sf_off, ws, row_scale))
+      return e;
+    // A ring of as many stages of activations as of weights: a block of them, the same for every SM, travels as long as the weights
+    // do. Where that is fewer than four, the weights keep six.
+    constexpr int kRoom = 224 * 1024 - 1024 - kMxScaleBytes;
+    const int even = kRoom / (P.box_bytes + L.x_bytes);
+    P.SX = even >= 4 ? std::min(8, even) : std::max(2, std::min(4, (kRoom - 6 * P.box_bytes) / L.x_bytes));
+    P.SW = std::min(12, (kRoom - P.SX * L.x_bytes) / P.box_bytes);
+    if (P.SW < 2) return kNotSupported;
+    const size_t smem = std::max<size_t>(static_cast<size_t>(P.SW) * P.box_bytes + kMxScaleBytes + static_cast<size_t>(P.SX) * L.x_bytes + 1024, 120 * 1024);
+    const bool two_atoms = L.cols0 > 128;
+    auto kernel = !two_atoms ? tc_mx_kernel<1, false> : L.cols1 ? tc_mx_kernel<2, true> : tc_mx_kernel<2, false>;
+    if (int e = !two_atoms ? allow_big_smem<300>(kernel) : L.cols1 ? allow_big_smem<301>(kernel) : allow_big_smem<302>(kernel)) return e;
+    const int tiles = (N + P.R - 1) / P.R * P.chunks;
+    if (int e = launch_kernel(kernel, dim3(std::min(tiles, sms)), dim3(kMxThreads), smem, stream, wmap, P)) return e;
+  }
+  return kOk;
+}
+
+}  // namespace b200

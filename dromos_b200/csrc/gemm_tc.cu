@@ -4,7 +4,7 @@
 // The weight tile is the A operand of tcgen05.mma (128 weight rows = the 128 lanes of the accumulator in tensor memory),
 // the activations are the B operand (one accumulator column per activation row and digit), K advances 32 bytes per
 // instruction. An instruction costs the tensor pipe at least ~46 cycles whatever the column count, so what matters is
-// instructions per byte of weights, and that decides the math per format:
+// instructions per byte of weights, and that decides the math per format (NVFP4: gemm_mx.cu):
 //
 //   BF16   kind::f16, A = the bf16 weights as they land in shared memory (128-byte swizzled TMA boxes, read through a
 //          shared-memory descriptor), B = bf16 activations; f32 activations as a high and a low bf16 column.
@@ -12,9 +12,6 @@
 //          e4m3 digits in base 16; the digit columns are recombined in the epilogue.
 //   INT8   kind::i8, A = the int8 weights as they land, B = the scaled activations as three int8 digits in base 128;
 //          the s32 sums are exact.
-//   NVFP4  no kind multiplies e2m1 * e4m3-block-scale weights by wider activations, so eight converter warps expand each
-//          stage to f16 in registers (exact) and write it with tcgen05.st into tensor memory as the A operand of
-//          kind::f16 (K = 16 per instruction); B = activations as f16 after a per-row power-of-two scaling.
 //
 // Roles (one CTA per SM): a weight producer thread (2-D TMA tile copies, no multicast, ring of stages with one mbarrier
 // each), an activation producer thread (1-D bulk copies of prepared blocks through a second, shallower ring), one MMA
@@ -37,8 +34,7 @@ namespace b200 {
 namespace {
 
 struct TcParams {
-  const uint8_t* scale;   // f32 [N] (INT8 / FP8); NVFP4 block scales come through the tensor map
-  float global;
+  const uint8_t* scale;   // f32 [N] (INT8 / FP8)
   int N, K, M;            // M: activation rows of this pass
   int R;                  // weight rows per tile
   int box_bytes;          // shared memory one 128-byte-wide tile copy takes: R rounded up to 8, times 128
@@ -66,7 +62,6 @@ struct TcParams {
   float alpha, beta;
   int* status;
   int SW, SX;             // depth of the weight ring and of the activation ring
-  int SA, slot_bytes;     // (NVFP4 through shared memory) A slots, and the bytes of a weight slot (box + block scales)
   int tmem_cols, dstride; // TMEM columns the CTA takes (a power of two >= 32) and the distance between its two accumulators
 };
 
@@ -132,28 +127,6 @@ __global__ void __launch_bounds__(128) tc_prep_kernel(const void* __restrict__ x
   for (int j = 0; j < planes; ++j) *reinterpret_cast<uint4*>(block + block_offset(NC, kb, j * Mp + u)) = make_uint4(w[j][0], w[j][1], w[j][2], w[j][3]);
 }
 
-// ---- expanding NVFP4 -------------------------------------------------------------------------------------------------
-// 16 e2m1 values (8 bytes) times one e4m3 block scale
-__device__ __forceinline__ void expand_nvfp4(uint32_t w0, uint32_t w1, uint32_t scale_byte, uint32_t (&p)[8]) {
-  uint32_t s2;
-  asm("{ .reg .b16 t; cvt.u16.u32 t, %1; cvt.rn.f16x2.e4m3x2 %0, t; }" : "=r"(s2) : "r"(scale_byte & 0xffu));
-  const uint32_t s = __byte_perm(s2, s2, 0x1010);
-  const uint32_t w[2] = {w0, w1};
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    uint32_t v0, v1, v2, v3;
-    asm("{ .reg .b8 b0, b1, b2, b3; mov.b32 {b0, b1, b2, b3}, %4;\n"
-        "cvt.rn.f16x2.e2m1x2 %0, b0; cvt.rn.f16x2.e2m1x2 %1, b1; cvt.rn.f16x2.e2m1x2 %2, b2; cvt.rn.f16x2.e2m1x2 %3, b3; }"
-        : "=r"(v0), "=r"(v1), "=r"(v2), "=r"(v3)
-        : "r"(w[i]));
-    asm("mul.rn.f16x2 %0, %0, %1;" : "+r"(v0) : "r"(s));
-    asm("mul.rn.f16x2 %0, %0, %1;" : "+r"(v1) : "r"(s));
-    asm("mul.rn.f16x2 %0, %0, %1;" : "+r"(v2) : "r"(s));
-    asm("mul.rn.f16x2 %0, %0, %1;" : "+r"(v3) : "r"(s));
-    p[4 * i] = v0, p[4 * i + 1] = v1, p[4 * i + 2] = v2, p[4 * i + 3] = v3;
-  }
-}
-
 // ---- the epilogue of a tile ---------------------------------------------------------------------------------------------
 // What y holds at rows m0 .. m0 + 7 of column n (0 past M), for beta. All eight are asked for before the first is stored: loads
 // and stores of one buffer taken in turn wait for each other, a round trip to L2 per row (37 rows x 10309 bf16 outputs with
@@ -204,7 +177,6 @@ __device__ __forceinline__ RowTerms row_terms(const TcParams& P, int tile, int r
   t.rf = 1.0f, t.bias = 0.0f;
   if (t.live) {  // the weight's scales and the bias are static, like the weight
     if constexpr (F == LX_W_INT8 || F == LX_W_FP8) t.rf = reinterpret_cast<const float*>(P.scale)[t.n];
-    if constexpr (F == LX_W_NVFP4) t.rf = P.global;
     if (P.bias) t.bias = load_f32(P.bias, P.bias_dtype, t.n);
   }
   return t;
@@ -671,448 +643,6 @@ __global__ void __launch_bounds__(XMODE ? kOwnThreads : kDirectThreads, XMODE ? 
   if (warp == 5) tmem_dealloc(tmem_base, P.tmem_cols);
 }
 
-// ---- NVFP4: converter warps expand the stage into tensor memory ---------------------------------------------------------
-constexpr int kKS4 = ks_of(kActF16);  // values of K per stage
-constexpr int kChunks = kKS4 / 16;   // tcgen05.mma instructions per stage (K = 16 each)
-constexpr int kASlots = 3;           // A-operand slots in TMEM, one stage each (kKS4 / 2 columns)
-constexpr int kAColumns = kKS4 / 2;
-constexpr int kDColumn = kASlots * kAColumns;  // the accumulator's first TMEM column (128 columns remain for it)
-// Eight or sixteen converter warps (kConvWarps = 8 or 16) were both measured on the 28672 x 8192 matrix: 76.9 / 82.2 us
-// at M = 16 / 64 with eight, 80.1 / 86.2 us with sixteen, so the converters' instruction stream is not what bounds a stage
-// (ncu: 30 % of issue slots, tensor pipe 6 %). A stage writes 64 KB of f16 into tensor memory for 16 KB of weights, and
-// 2375 cycles per stage is 27 bytes per cycle and SM of tcgen05.st.
-constexpr int kConvWarps = 8, kConvParts = kConvWarps / 4;  // a part: the share of a stage's K one converter thread expands for its row
-constexpr int kConvPieces = 8 / kConvParts;                  // 16-byte pieces (32 values, two block scales) per thread and stage
-constexpr int kProducerWarp = kConvWarps, kIssuerWarp = kConvWarps + 1;
-constexpr int kConvThreads = (kConvWarps + 2) * 32;  // converter warps, then the producer warp, then the MMA issuer
-
-__global__ void __launch_bounds__(kConvThreads, 1)
-    tc_nvfp4_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap smap, const TcParams P) {
-  constexpr int F = LX_W_NVFP4;
-  using Fm = TcFmt<F>;
-  extern __shared__ __align__(1024) uint8_t smem[];
-  const int NC = P.NC, SW = P.SW, SX = P.SX;
-  const int x_bytes = P.x_bytes, box_bytes = P.box_bytes;
-  // a slot is the stage's box (R rows of 128 bytes, 1024-aligned) and, box_bytes further, its 16 block scales per row
-  uint8_t* const xring = smem + static_cast<size_t>(SW) * box_bytes * 2;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(xring + static_cast<size_t>(SX) * x_bytes);
-  const uint32_t bar0 = smem_u32(bars);
-  auto w_full = [&](int s) { return bar0 + 8u * s; };                               // weight stage landed
-  auto w_empty = [&](int s) { return bar0 + 8u * (SW + s); };                       // read by all converter warps
-  auto x_full = [&](int s) { return bar0 + 8u * (2 * SW + s); };                    // activation block landed
-  auto x_empty = [&](int s) { return bar0 + 8u * (2 * SW + SX + s); };              // its products are done
-  auto a_full = [&](int a) { return bar0 + 8u * (2 * SW + 2 * SX + a); };           // A slot written
-  auto a_empty = [&](int a) { return bar0 + 8u * (2 * SW + 2 * SX + kASlots + a); };// A slot consumed
-  const uint32_t d_full = bar0 + 8u * (2 * SW + 2 * SX + 2 * kASlots);              // the tile's accumulator is complete
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * SW + 2 * SX + 2 * kASlots + 1);
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n_stages = (P.K + kKS4 - 1) / kKS4;
-  const int n_tiles = (P.N + P.R - 1) / P.R;
-  const int tile_begin = static_cast<int>(static_cast<int64_t>(n_tiles) * blockIdx.x / gridDim.x);
-  const int tile_end = static_cast<int>(static_cast<int64_t>(n_tiles) * (blockIdx.x + 1) / gridDim.x);
-  const int total = (tile_end - tile_begin) * n_stages;
-  const int slot_bytes = 2 * box_bytes;
-
-  if (tid == 0) {
-    for (int s = 0; s < SW; ++s) {
-      mbar_init(w_full(s), 1);
-      mbar_init(w_empty(s), kConvWarps);
-    }
-    for (int s = 0; s < SX; ++s) {
-      mbar_init(x_full(s), 1);
-      mbar_init(x_empty(s), 1);
-    }
-    for (int a = 0; a < kASlots; ++a) {
-      mbar_init(a_full(a), kConvWarps);
-      mbar_init(a_empty(a), 1);
-    }
-    mbar_init(d_full, 1);
-    mbar_init_fence();
-  }
-  if (warp == kIssuerWarp) {
-    tmem_alloc(smem_u32(tmem_slot), kTmemColumns);
-    tmem_relinquish();
-    tc_fence_before();
-  }
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-
-  if (warp == kProducerWarp) {
-    // ================================ producers ================================
-    pdl_trigger();
-    if (lane == 0) {
-      asm volatile("prefetch.tensormap [%0];" ::"l"(&wmap) : "memory");
-      asm volatile("prefetch.tensormap [%0];" ::"l"(&smap) : "memory");
-    }
-    if (lane == 0) {  // weights and their scales are static: no wait
-      Ring w;
-      bool ok = true, wrapped = false;
-      for (int tile = tile_begin; tile < tile_end && ok; ++tile) {
-        for (int s = 0; s < n_stages; ++s) {
-          if (wrapped && !tc_wait(w_empty(w.slot), w.lap ^ 1u, P.status)) {
-            ok = false;
-            break;
-          }
-          const uint32_t dst = smem_u32(smem) + static_cast<uint32_t>(w.slot) * slot_bytes;
-          mbar_arrive_expect_tx(w_full(w.slot), P.R * (128 + 16));
-          tile_g2s(dst, &wmap, (s * Fm::kRowBytes) / 4, tile * P.R, w_full(w.slot));
-          tile_g2s(dst + box_bytes, &smap, s * 16, tile * P.R, w_full(w.slot));
-          w.advance(SW);
-          wrapped |= w.slot == 0;
-        }
-      }
-    } else if (lane == 1) {
-      pdl_wait();  // the prepared activations come from the kernel before this one
-      Ring x;
-      bool wrapped = false;
-      int s = 0;
-      for (int i = 0; i < total; ++i) {
-        if (wrapped && !tc_wait(x_empty(x.slot), x.lap ^ 1u, P.status)) break;
-        mbar_arrive_expect_tx(x_full(x.slot), x_bytes);
-        bulk_g2s(smem_u32(xring) + static_cast<uint32_t>(x.slot) * x_bytes, P.xprep + static_cast<size_t>(s) * x_bytes, x_bytes, x_full(x.slot));
-        x.advance(SX);
-        wrapped |= x.slot == 0;
-        if (++s == n_stages) s = 0;
-      }
-    }
-  } else if (warp == kIssuerWarp) {
-    // ================================ MMA issuer ================================
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(NC >> 3) << 17) | (static_cast<uint32_t>(kBM >> 4) << 24);  // f16 x f16 -> f32
-      const uint32_t lbo = static_cast<uint32_t>(NC / 8) * 128, sbo = 128;
-      Ring x, a;
-      int s = 0;
-      for (int i = 0; i < total; ++i) {
-        // the activations of this stage are in shared memory, the converted weights in tensor memory
-        if (!tc_wait(x_full(x.slot), x.lap, P.status) || !tc_wait(a_full(a.slot), a.lap, P.status)) break;
-        tc_fence_after();
-        const uint32_t xb = smem_u32(xring) + static_cast<uint32_t>(x.slot) * x_bytes;
-#pragma unroll
-        for (int c = 0; c < kChunks; ++c) {
-          const uint64_t bdesc = smem_desc(xb + static_cast<uint32_t>(2 * c) * lbo, lbo, sbo);
-          umma_ts(tmem_base + kDColumn, tmem_base + a.slot * kAColumns + c * 8, bdesc, idesc, (s | c) ? 1u : 0u);
-        }
-        umma_commit(a_empty(a.slot));    // the A slot may be overwritten once these products are done
-        umma_commit(x_empty(x.slot));    // and so may the activation block
-        // A tile ends here: its accumulator is complete when everything issued so far is. The next tile's first
-        // product overwrites it, but waits for an A slot the converters fill only after they have read the accumulator.
-        if (++s == n_stages) {
-          s = 0;
-          umma_commit(d_full);
-        }
-        x.advance(SX);
-        a.advance(kASlots);
-      }
-    }
-  } else {
-    // ================================ converters, then epilogue ================================
-    const int quarter = warp & 3, part = warp >> 2;
-    const int r = quarter * 32 + lane;  // weight row of the tile = TMEM lane
-    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-    Ring w, a;
-    int s = 0, t = 0;
-    bool a_wrapped = false;
-    for (int i = 0; i < total; ++i) {
-      if (!tc_wait(w_full(w.slot), w.lap, P.status) || (a_wrapped && !tc_wait(a_empty(a.slot), a.lap ^ 1u, P.status))) break;
-      tc_fence_after();
-      // Rows past R read what shared memory holds behind the box (this CTA's own, see tc_launch); their lanes are
-      // never read back.
-      const uint8_t* stage = smem + static_cast<size_t>(w.slot) * slot_bytes;
-      const uint32_t a_addr = lane_addr + a.slot * kAColumns + part * (kAColumns / kConvParts);
-      const int sw = r & 7;
-      // this part's pieces kConvPieces * part .. of the row's eight 16-byte pieces (32 values each), two block scales per piece
-      const uint8_t* box = stage + r * 128;
-      uint4 q[kConvPieces];
-#pragma unroll
-      for (int j = 0; j < kConvPieces; ++j) q[j] = *reinterpret_cast<const uint4*>(box + (((kConvPieces * part + j) ^ sw) << 4));
-      uint32_t sc[(kConvPieces + 1) / 2];
-#pragma unroll
-      for (int j = 0; j < (kConvPieces + 1) / 2; ++j)
-        sc[j] = *reinterpret_cast<const uint32_t*>(stage + box_bytes + r * 16 + part * (2 * kConvPieces) + 4 * j);
-      static_assert(kConvPieces % 2 == 0, "a thread's scale bytes are read as whole words");
-#pragma unroll
-      for (int j = 0; j < kConvPieces; ++j) {
-        uint32_t p[8];
-        const uint32_t sword = sc[j / 2];
-        expand_nvfp4(q[j].x, q[j].y, sword >> (16 * (j & 1)), p);
-        tmem_st8(a_addr + (2 * j) * 8, p);
-        expand_nvfp4(q[j].z, q[j].w, sword >> (16 * (j & 1) + 8), p);
-        tmem_st8(a_addr + (2 * j + 1) * 8, p);
-      }
-      tmem_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(w_empty(w.slot));  // the bytes are in registers / tensor memory: the stage may be refilled
-        mbar_arrive(a_full(a.slot));
-      }
-      w.advance(SW);
-      a.advance(kASlots);
-      a_wrapped |= a.slot == 0;
-      if (++s != n_stages) continue;
-      s = 0;
-      // ---- the tile is over ----
-      const RowTerms T = row_terms<F>(P, tile_begin + t, r);
-      if (!tc_wait(d_full, t & 1, P.status)) break;
-      tc_fence_after();
-      pdl_wait();  // y and the activation scales come from earlier kernels
-      const float inv_lo = lane < P.M ? P.inv_scales[lane] : 0.0f, inv_hi = 32 + lane < P.M ? P.inv_scales[32 + lane] : 0.0f;
-      finish_tile<F, false>(P, T, lane_addr + kDColumn, lane, part, kConvParts, inv_lo, inv_hi, 0u);
-      ++t;
-    }
-  }
-  __syncthreads();
-  if (warp == kIssuerWarp) tmem_dealloc(tmem_base, kTmemColumns);
-}
-
-// ---- NVFP4 with the expanded weights in shared memory ---------------------------------------------------------------
-// The kernel above is bound by tcgen05.st (27 bytes per cycle and SM measured; a stage writes 64 KB). Here the converter
-// warps write the f16 expansion into shared memory instead (st.shared takes 128 bytes per cycle), in the layout a
-// 128-byte-swizzled tile copy would have left it, and the products read both operands from shared memory like the
-// kernels of the formats that need no conversion. A weight stage (256 values of K per row, as above) is converted in two
-// halves of 128 values; an A slot holds one half: two boxes of 128 rows x 128 bytes. Converter thread (row r, part p)
-// expands kSsPieces 16-byte pieces (32 values, two block scales each) of its row per half.
-//
-// Measured on the 28672 x 8192 matrix at M = 16 / 64: 72.3 / 80.9 us, against 79.1 / 87.3 us for the kernel above in the
-// same run. Variants measured and dropped: quarter-stage slots (86 us: the per-slot handshakes cost more than the finer
-// overlap gives), sixteen converter warps (75 us), block scales fetched for four stages per copy (75 / 91 us: the 32 KB
-// they take leave fewer weight stages). Switching the conversion off (raw bytes stored) gives 67 us and issuing one
-// product in eight gives 66 us: two bounds of nearly the same height. The converters execute ~2080 warp instructions
-// per stage on dependent chains; and the sixteen products of a stage take ~2050 cycles whatever their column count: the
-// tensor core takes its 4 KB A tile (128 rows x 32 bytes) at about 32 bytes per cycle, and the f16 expansion is four
-// times the stored bytes. A faster NVFP4 product needs the weights as the B operand (256 rows per product) or a kind
-// that reads e2m1 as stored.
-constexpr int kSsWarps = 8, kSsParts = kSsWarps / 4, kSsPieces = 4 / kSsParts;
-constexpr int kSsProducer = kSsWarps, kSsIssuer = kSsWarps + 1, kSsThreads = (kSsWarps + 2) * 32;
-constexpr int kSsSlotBytes = 2 * kBM * 128;  // one half stage of f16: 128 rows x 128 values
-
-__global__ void __launch_bounds__(kSsThreads, 1)
-    tc_nvfp4_ss_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap smap, const TcParams P) {
-  constexpr int F = LX_W_NVFP4;
-  using Fm = TcFmt<F>;
-  extern __shared__ __align__(1024) uint8_t smem[];
-  const int NC = P.NC, SW = P.SW, SX = P.SX, SA = P.SA;
-  const int x_bytes = P.x_bytes, box_bytes = P.box_bytes, slot_bytes = P.slot_bytes;
-  uint8_t* const aring = smem + static_cast<size_t>(SW) * slot_bytes;
-  uint8_t* const xring = aring + static_cast<size_t>(SA) * kSsSlotBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(xring + static_cast<size_t>(SX) * x_bytes);
-  const uint32_t bar0 = smem_u32(bars);
-  auto w_full = [&](int s) { return bar0 + 8u * s; };
-  auto w_empty = [&](int s) { return bar0 + 8u * (SW + s); };
-  auto x_full = [&](int s) { return bar0 + 8u * (2 * SW + s); };
-  auto x_empty = [&](int s) { return bar0 + 8u * (2 * SW + SX + s); };
-  auto a_full = [&](int a) { return bar0 + 8u * (2 * SW + 2 * SX + a); };
-  auto a_empty = [&](int a) { return bar0 + 8u * (2 * SW + 2 * SX + SA + a); };
-  const uint32_t d_full = bar0 + 8u * (2 * SW + 2 * SX + 2 * SA);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * SW + 2 * SX + 2 * SA + 1);
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n_stages = (P.K + kKS4 - 1) / kKS4;
-  const int n_tiles = (P.N + P.R - 1) / P.R;
-  const int tile_begin = static_cast<int>(static_cast<int64_t>(n_tiles) * blockIdx.x / gridDim.x);
-  const int tile_end = static_cast<int>(static_cast<int64_t>(n_tiles) * (blockIdx.x + 1) / gridDim.x);
-  const int total = (tile_end - tile_begin) * n_stages;
-
-  if (tid == 0) {
-    for (int s = 0; s < SW; ++s) {
-      mbar_init(w_full(s), 1);
-      mbar_init(w_empty(s), kSsWarps);
-    }
-    for (int s = 0; s < SX; ++s) {
-      mbar_init(x_full(s), 1);
-      mbar_init(x_empty(s), 1);
-    }
-    for (int a = 0; a < SA; ++a) {
-      mbar_init(a_full(a), kSsWarps);
-      mbar_init(a_empty(a), 1);
-    }
-    mbar_init(d_full, 1);
-    mbar_init_fence();
-  }
-  if (warp == kSsIssuer) {
-    tmem_alloc(smem_u32(tmem_slot), kTmemColumns);
-    tmem_relinquish();
-    tc_fence_before();
-  }
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-
-  if (warp == kSsProducer) {
-    // ================================ producers ================================
-    pdl_trigger();
-    if (lane == 0) {
-      asm volatile("prefetch.tensormap [%0];" ::"l"(&wmap) : "memory");
-      asm volatile("prefetch.tensormap [%0];" ::"l"(&smap) : "memory");
-    }
-    if (lane == 0) {  // weights and their scales are static: no wait
-      Ring w;
-      bool ok = true, wrapped = false;
-      for (int tile = tile_begin; tile < tile_end && ok; ++tile) {
-        for (int s = 0; s < n_stages; ++s) {
-          if (wrapped && !tc_wait(w_empty(w.slot), w.lap ^ 1u, P.status)) {
-            ok = false;
-            break;
-          }
-          const uint32_t dst = smem_u32(smem) + static_cast<uint32_t>(w.slot) * slot_bytes;
-          mbar_arrive_expect_tx(w_full(w.slot), P.R * (128 + 16));
-          tile_g2s(dst, &wmap, (s * Fm::kRowBytes) / 4, tile * P.R, w_full(w.slot));
-          tile_g2s(dst + box_bytes, &smap, s * 16, tile * P.R, w_full(w.slot));
-          w.advance(SW);
-          wrapped |= w.slot == 0;
-        }
-      }
-    } else if (lane == 1) {
-      pdl_wait();  // the prepared activations come from the kernel before this one
-      Ring x;
-      bool wrapped = false;
-      int s = 0;
-      for (int i = 0; i < total; ++i) {
-        if (wrapped && !tc_wait(x_empty(x.slot), x.lap ^ 1u, P.status)) break;
-        mbar_arrive_expect_tx(x_full(x.slot), x_bytes);
-        bulk_g2s(smem_u32(xring) + static_cast<uint32_t>(x.slot) * x_bytes, P.xprep + static_cast<size_t>(s) * x_bytes, x_bytes, x_full(x.slot));
-        x.advance(SX);
-        wrapped |= x.slot == 0;
-        if (++s == n_stages) s = 0;
-      }
-    }
-  } else if (warp == kSsIssuer) {
-    // ================================ MMA issuer ================================
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(NC >> 3) << 17) | (static_cast<uint32_t>(kBM >> 4) << 24);  // f16 x f16 -> f32
-      const uint32_t lbo = static_cast<uint32_t>(NC / 8) * 128, sbo = 128;
-      const uint32_t a_hi = (1024u >> 4) | (1u << 14) | (2u << 29), b_hi = (sbo >> 4) | (1u << 14);
-      const uint32_t a_lo0 = ((smem_u32(aring) & 0x3ffffu) >> 4) | (1u << 16);
-      const uint32_t b_lo0 = ((smem_u32(xring) & 0x3ffffu) >> 4) | ((lbo >> 4) << 16);
-      const uint32_t b_step = (2u * lbo) >> 4;
-      Ring x, a;
-      int s = 0;
-      bool ok = true;
-      for (int i = 0; i < total && ok; ++i) {
-        if (!tc_wait(x_full(x.slot), x.lap, P.status)) break;
-        const uint32_t b_lo = b_lo0 + static_cast<uint32_t>(x.slot) * (static_cast<uint32_t>(x_bytes) >> 4);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          if (!tc_wait(a_full(a.slot), a.lap, P.status)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t a_lo = a_lo0 + static_cast<uint32_t>(a.slot) * (kSsSlotBytes >> 4);
-#pragma unroll
-          for (int b = 0; b < 2; ++b) {
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {
-              const int c = 8 * h + 4 * b + ks;  // 16 values of K per instruction
-              umma_ss_halves<kActF16>(tmem_base, a_lo + b * ((kSsSlotBytes / 2) >> 4) + ks * 2, a_hi, b_lo + c * b_step, b_hi, idesc, (s | c) ? 1u : 0u);
-            }
-          }
-          umma_commit(a_empty(a.slot));  // the half stage may be overwritten once these products are done
-          a.advance(SA);
-        }
-        if (!ok) break;
-        umma_commit(x_empty(x.slot));
-        if (++s == n_stages) {
-          s = 0;
-          umma_commit(d_full);  // the tile's accumulator is complete when everything issued so far is
-        }
-        x.advance(SX);
-      }
-    }
-  } else {
-    // ================================ converters, then epilogue ================================
-    const int quarter = warp & 3, part = warp >> 2;
-    const int r = quarter * 32 + lane;  // weight row of the tile = TMEM lane
-    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-    const int sw = r & 7;
-    Ring w, a;
-    int s = 0, t = 0;
-    bool a_wrapped = false, ok = true;
-    // The arrival for a slot is sent one half later, after the next half has been expanded into registers: the proxy
-    // fence waits for the slot's stores to complete, and that wait is what the expansion of the next half hides.
-    int owed_a = -1, owed_w = -1;  // the A slot (and, after a stage's second half, the weight slot) whose arrival is still owed
-    auto settle = [&]() {
-      if (owed_a < 0) return;
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor core reads what these threads wrote
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(a_full(owed_a));
-        if (owed_w >= 0) mbar_arrive(w_empty(owed_w));  // both halves have been read and used: the stage may be refilled
-      }
-      owed_a = owed_w = -1;
-    };
-    for (int i = 0; i < total && ok; ++i) {
-      if (!tc_wait(w_full(w.slot), w.lap, P.status)) break;
-      // Rows past R read what shared memory holds behind the box (this CTA's own); their lanes are never read back.
-      const uint8_t* stage = smem + static_cast<size_t>(w.slot) * slot_bytes;
-      const uint8_t* box = stage + r * 128;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint4 q[kSsPieces];
-#pragma unroll
-        for (int j = 0; j < kSsPieces; ++j) q[j] = *reinterpret_cast<const uint4*>(box + (((4 * h + kSsPieces * part + j) ^ sw) << 4));
-        uint32_t sc[kSsPieces];  // two scale bytes per piece
-#pragma unroll
-        for (int j = 0; j < kSsPieces; ++j)
-          sc[j] = *reinterpret_cast<const uint16_t*>(stage + box_bytes + r * 16 + 2 * (4 * h + kSsPieces * part + j));
-        uint32_t p[kSsPieces][16];
-#pragma unroll
-        for (int j = 0; j < kSsPieces; ++j) {
-          uint32_t lo[8], hi[8];
-          expand_nvfp4(q[j].x, q[j].y, sc[j], lo);
-          expand_nvfp4(q[j].z, q[j].w, sc[j] >> 8, hi);
-#pragma unroll
-          for (int z = 0; z < 8; ++z) p[j][z] = lo[z], p[j][8 + z] = hi[z];
-        }
-        settle();
-        if (a_wrapped && !tc_wait(a_empty(a.slot), a.lap ^ 1u, P.status)) {
-          ok = false;
-          break;
-        }
-        uint8_t* arow = aring + static_cast<size_t>(a.slot) * kSsSlotBytes + r * 128;
-#pragma unroll
-        for (int j = 0; j < kSsPieces; ++j) {
-          const int g = kSsPieces * part + j;  // the piece's place in the half: box g / 2, chunks 4 (g % 2) ..
-          uint8_t* dst = arow + (g >> 1) * (kSsSlotBytes / 2);
-          const int c0 = 4 * (g & 1);
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
-            *reinterpret_cast<uint4*>(dst + (((c0 + c) ^ sw) << 4)) = make_uint4(p[j][4 * c], p[j][4 * c + 1], p[j][4 * c + 2], p[j][4 * c + 3]);
-        }
-        owed_a = a.slot, owed_w = h == 1 ? w.slot : -1;
-        a.advance(SA);
-        a_wrapped |= a.slot == 0;
-      }
-      if (!ok) break;
-      w.advance(SW);
-      if (++s != n_stages) continue;
-      s = 0;
-      // ---- the tile is over ----
-      settle();
-      const RowTerms T = row_terms<F>(P, tile_begin + t, r);
-      if (!tc_wait(d_full, t & 1, P.status)) break;
-      tc_fence_after();
-      pdl_wait();  // y and the activation scales come from earlier kernels
-      const float inv_lo = lane < P.M ? P.inv_scales[lane] : 0.0f, inv_hi = 32 + lane < P.M ? P.inv_scales[32 + lane] : 0.0f;
-      finish_tile<F, false>(P, T, lane_addr, lane, part, kSsParts, inv_lo, inv_hi, 0u);
-      ++t;
-    }
-  }
-  __syncthreads();
-  if (warp == kSsIssuer) tmem_dealloc(tmem_base, kTmemColumns);
-}
-
-// LX_B200_NVFP4_TMEM=1 keeps the kernel that expands into tensor memory.
-bool nvfp4_through_tmem() {
-  static const bool on = [] {
-    const char* v = std::getenv("LX_B200_NVFP4_TMEM");
-    return v && v[0] == '1';
-  }();
-  return on;
-}
-
 // ---- launching -------------------------------------------------------------------------------------------------------
 // LX_B200_TC_SMALL=1 lets products whose rings fit take small CTAs (two per SM); LX_B200_TC_SMALL_STAGES sets the fewest
 // weight stages a small CTA must keep (default 3). Off by default: measured on C2, a product between small neighbours
@@ -1150,8 +680,7 @@ int tc_launch(const lx_weight& w, TcParams P, cudaStream_t stream, int* grid_out
   if (!sms) return kInvalid;
   P.R = tile_rows(P.N, sms);
   P.box_bytes = (P.R + 7) / 8 * 1024;
-  // NVFP4 keeps a stage's box and its block scales in a slot of twice the box, so that every box starts 1024-aligned.
-  const int w_stage = F == LX_W_NVFP4 ? 2 * P.box_bytes : kBoxes * P.box_bytes;
+  const int w_stage = kBoxes * P.box_bytes;
   constexpr int kStaging = XMODE == 0 ? 0 : own_staging_bytes(XMODE == 1);
   // Two sizes of CTA. Small: at most half of an SM's shared memory and tensor memory, so that the CTAs of the NEXT kernel
   // in the stream (launched programmatically, their weights static) move in beside this kernel's and fill their rings
@@ -1164,7 +693,7 @@ int tc_launch(const lx_weight& w, TcParams P, cudaStream_t stream, int* grid_out
   P.dstride = P.NC;
   P.tmem_cols = 32;
   while (P.tmem_cols < 2 * P.NC) P.tmem_cols *= 2;
-  const int small_sw = small_ctas() && F != LX_W_NVFP4 && P.tmem_cols <= 256 ? (kSmall - kBars - std::max(2 * P.x_bytes + kStaging, 16 * 1024)) / w_stage : 0;
+  const int small_sw = small_ctas() && P.tmem_cols <= 256 ? (kSmall - kBars - std::max(2 * P.x_bytes + kStaging, 16 * 1024)) / w_stage : 0;
   const bool small = small_sw >= small_min_stages();
   size_t smem;
   if (small) {
@@ -1175,7 +704,7 @@ int tc_launch(const lx_weight& w, TcParams P, cudaStream_t stream, int* grid_out
     if (XMODE) {
       // CTAs that prepare their own (small) activation blocks keep one ring: a block per weight stage, one barrier for both
       P.SW = P.SX = std::min(12, (kLarge - kStaging) / (w_stage + P.x_bytes));
-    } else if (F != LX_W_NVFP4 && kLarge / (w_stage + P.x_bytes) >= 4) {
+    } else if (kLarge / (w_stage + P.x_bytes) >= 4) {
       P.SW = P.SX = std::min(12, kLarge / (w_stage + P.x_bytes));  // one ring again: one commit per stage
     } else {
       // Large activation blocks (64 rows of two digits are 32 KB per stage): measured at M = 64 on the 28672 x 8192 FP8
@@ -1192,43 +721,19 @@ int tc_launch(const lx_weight& w, TcParams P, cudaStream_t stream, int* grid_out
     // all of tensor memory: exactly one CTA may live on an SM, so ask for more than half of its shared memory
     smem = std::max<size_t>(static_cast<size_t>(P.SW) * w_stage + std::max(P.SX * P.x_bytes + kStaging, 16 * 1024) + kBars, 120 * 1024);
   }
-  alignas(64) CUtensorMap wmap, smap;
+  alignas(64) CUtensorMap wmap;
   memset(&wmap, 0, sizeof(wmap));
-  memset(&smap, 0, sizeof(smap));
-  const int64_t row_bytes = F == LX_W_BF16 ? 2ll * P.K : F == LX_W_NVFP4 ? P.K / 2 : P.K;
+  const int64_t row_bytes = F == LX_W_BF16 ? 2ll * P.K : P.K;
   if (int e = make_tile_map(&wmap, w.data, row_bytes, P.N, 128, P.R, 4, true)) return e;
   const int tiles = (P.N + P.R - 1) / P.R;
   const int grid = std::min(tiles, sms);
   if (grid_out) *grid_out = grid;
-  if constexpr (F == LX_W_NVFP4) {
-    static_assert(XMODE == 0, "NVFP4 takes prepared activations");
-    if (int e = make_tile_map(&smap, w.scale, P.K / 16, P.N, 16, P.R, 1, false)) return e;
-    if (!nvfp4_through_tmem()) {
-      // weight slots of the box and 128 rows of scales; two or three half-stage A slots; two activation blocks
-      constexpr int kBudget = 224 * 1024;
-      const int slot = (P.box_bytes + kBM * 16 + 1023) / 1024 * 1024;
-      P.SX = 2;
-      int sa = 3;
-      int sw_fit = (kBudget - kBars - P.SX * P.x_bytes - sa * kSsSlotBytes) / slot;
-      if (sw_fit < 5) sa = 2, sw_fit = (kBudget - kBars - P.SX * P.x_bytes - sa * kSsSlotBytes) / slot;
-      if (sw_fit >= 2) {
-        P.SW = std::min(12, sw_fit);
-        P.SA = sa, P.slot_bytes = slot;
-        const size_t bytes = static_cast<size_t>(P.SW) * slot + static_cast<size_t>(sa) * kSsSlotBytes + P.SX * P.x_bytes + kBars;
-        if (int e = allow_big_smem<F * 4 + 1>(tc_nvfp4_ss_kernel)) return e;
-        return launch_kernel(tc_nvfp4_ss_kernel, dim3(grid), dim3(kSsThreads), bytes, stream, wmap, smap, P);
-      }
-    }
-    if (int e = allow_big_smem<F * 4>(tc_nvfp4_kernel)) return e;
-    return launch_kernel(tc_nvfp4_kernel, dim3(grid), dim3(kConvThreads), smem, stream, wmap, smap, P);
-  } else {
-    if (P.peers > 0) {
-      if (int e = allow_big_smem<64 + F * 4 + XMODE>(tc_direct_kernel<F, XMODE, true>)) return e;
-      return launch_kernel(tc_direct_kernel<F, XMODE, true>, dim3(grid), dim3(XMODE ? kOwnThreads : kDirectThreads), smem, stream, wmap, P);
-    }
-    if (int e = allow_big_smem<F * 4 + XMODE>(tc_direct_kernel<F, XMODE, false>)) return e;
-    return launch_kernel(tc_direct_kernel<F, XMODE, false>, dim3(grid), dim3(XMODE ? kOwnThreads : kDirectThreads), smem, stream, wmap, P);
+  if (P.peers > 0) {
+    if (int e = allow_big_smem<64 + F * 4 + XMODE>(tc_direct_kernel<F, XMODE, true>)) return e;
+    return launch_kernel(tc_direct_kernel<F, XMODE, true>, dim3(grid), dim3(XMODE ? kOwnThreads : kDirectThreads), smem, stream, wmap, P);
   }
+  if (int e = allow_big_smem<F * 4 + XMODE>(tc_direct_kernel<F, XMODE, false>)) return e;
+  return launch_kernel(tc_direct_kernel<F, XMODE, false>, dim3(grid), dim3(XMODE ? kOwnThreads : kDirectThreads), smem, stream, wmap, P);
 }
 
 // Activation rows one pass takes: the block of one stage stays within 48 KB.
@@ -1239,7 +744,6 @@ TcParams base_params(const lx_weight& w, const void* bias, int bias_dtype, int y
                      int act, bool x_bf16, int rows, bool quantized = false) {
   TcParams P{};
   P.scale = static_cast<const uint8_t*>(w.scale);
-  P.global = w.global;
   P.N = N, P.K = K, P.M = rows;
   P.planes = quantized ? 1 : act_planes(act, x_bf16);
   P.digit = act == kActS8 ? 0.0078125f : act == kActE4m3 ? 0.0625f : 1.0f;
@@ -1297,7 +801,11 @@ int tc_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const v
   if (quantized && w.type != LX_W_INT8 && w.type != LX_W_FP8) return kNotSupported;
   // More rows than one pass: pairs of SMs, same digits, same order, same bits. (FP8, 28672 x 8192: 64 rows 52 us here, 65 rows
   // 54 us there; a second pass would add another 50.)
-  if (M > kMaxRows && w.type != LX_W_NVFP4)
+  if (w.type == LX_W_NVFP4) {
+    const int sms = sm_count();
+    return sms ? mx_product(x, x_dtype, ld_x, w, bias, bias_dtype, y, y_dtype, ld_y, M, N, K, alpha, beta, workspace, tile_rows(N, sms), stream) : kInvalid;
+  }
+  if (M > kMaxRows)
     return pair_product(x, x_dtype, ld_x, w, bias, bias_dtype, y, y_dtype, ld_y, M, N, K, alpha, beta, workspace, stream, quantized);
   const int act = act_of(w.type), elem = act_elem(act), kKS = ks_of(act);
   const int per_pass = rows_per_pass(act, true);  // f32 activations become bf16 (or quantized) values: as many planes as bf16
@@ -1325,8 +833,6 @@ int tc_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const v
       switch (act * 2 + (x_bf16 ? 1 : 0)) {
         case kActBf16 * 2: pe = prep(tc_prep_kernel<kActBf16, false, kPrepRound>); break;
         case kActBf16 * 2 + 1: pe = prep(tc_prep_kernel<kActBf16, true>); break;
-        case kActF16 * 2: pe = prep(tc_prep_kernel<kActF16, false, kPrepRound>); break;
-        case kActF16 * 2 + 1: pe = prep(tc_prep_kernel<kActF16, true>); break;
         case kActE4m3 * 2: pe = prep(tc_prep_kernel<kActE4m3, false, kPrepRound>); break;
         case kActE4m3 * 2 + 1: pe = prep(tc_prep_kernel<kActE4m3, true>); break;
         case kActS8 * 2: pe = prep(tc_prep_kernel<kActS8, false, kPrepRound>); break;
@@ -1339,7 +845,6 @@ int tc_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const v
       case LX_W_BF16: e = tc_launch<LX_W_BF16, 0>(w, P, stream); break;
       case LX_W_INT8: e = tc_launch<LX_W_INT8, 0>(w, P, stream); break;
       case LX_W_FP8: e = tc_launch<LX_W_FP8, 0>(w, P, stream); break;
-      case LX_W_NVFP4: e = tc_launch<LX_W_NVFP4, 0>(w, P, stream); break;
       default: e = kNotSupported;
     }
     if (e) return e;
@@ -1437,6 +942,7 @@ int64_t tc_workspace_bytes(int M, int K) {
       const int NC = (act_planes(act, bf != 0) * ((r + 7) / 8 * 8) + 15) / 16 * 16;
       need = std::max(need, TcLayout(NC, act, (K + ks_of(act) - 1) / ks_of(act)).total);
     }
+  need = std::max(need, mx_workspace_bytes(M, K));
   if (M > kMaxRows) need = std::max(need, pair_workspace_bytes(M, K));
   return need;
 }

@@ -198,6 +198,10 @@ int64_t tc_workspace_bytes(int M, int K);
 int pair_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const void* bias, int bias_dtype, void* y, int y_dtype, int ld_y,
                  int M, int N, int K, float alpha, float beta, void* workspace, cudaStream_t stream, bool quantized);
 int64_t pair_workspace_bytes(int M, int K);
+// gemm_mx.cu: NVFP4 weights, multiplied as stored. even_rows: weight rows per tile (at most 128) that deal N out evenly.
+int mx_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const void* bias, int bias_dtype, void* y, int y_dtype, int ld_y,
+               int M, int N, int K, float alpha, float beta, void* workspace, int even_rows, cudaStream_t stream);
+int64_t mx_workspace_bytes(int M, int K);
 bool tc_enabled();
 // Where the all-gather epilogue of a sharded product stores: every rank's copy of the whole y and arrival counter.
 struct PeerTargets {

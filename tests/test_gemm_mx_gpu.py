@@ -1,0 +1,101 @@
+"""lx_gemm_w on NVFP4 weights (weights multiplied as stored, activations as base-8 digits): against 64-bit sums at the edges of its
+layouts (digit columns in one instruction or two, chunks of 64 rows, launches of 1024, weight panels, 256 values of K), rows that
+do not depend on the call they come in, and the values that have no digits.
+
+Bound: a value keeps 21 bits below its block's largest magnitude (2^-21 of it at most is dropped, ~2^-20 of a typical value),
+products and sums of digits are exact or f32, seven sums are put together with one f32 rounding each: 1e-6 leaves a factor of
+four."""
+
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from dromos_b200 import abi, host
+from tests import util
+
+pytestmark = pytest.mark.gpu
+
+LEVELS = [0, 0.5, 1, 1.5, 2, 3, 4, 6, -0.0, -0.5, -1, -1.5, -2, -3, -4, -6]
+
+
+def values(data, scale, glob, N, K):
+    q = data.view(N, K // 2)
+    lut = torch.tensor(LEVELS, dtype=torch.float64, device="cuda")
+    v = torch.stack((lut[(q & 15).long()], lut[(q >> 4).long()]), dim=2).view(N, K)
+    return v * scale.view(N, K // 16).view(torch.float8_e4m3fn).double().repeat_interleave(16, 1) * glob
+
+
+def product(lx, x, sw, M, N, K, beta=0.0, y=None, bias=None, alpha=1.0):
+    y = torch.full((M, N), float("nan"), device="cuda") if y is None else y
+    ws = torch.full((lx.lx_gemm_workspace_bytes(M, K, 0),), 0xFF, dtype=torch.uint8, device="cuda")
+    assert lx.lx_gemm_w(abi.ptr(x), abi.F32 if x.dtype == torch.float32 else abi.BF16, x.stride(0), sw.ref(), 0, abi.ptr(bias), abi.F32, abi.ptr(y),
+                        abi.BF16 if y.dtype == torch.bfloat16 else abi.F32, y.stride(0), M, N, K, alpha, beta, abi.ptr(ws), util.stream_ptr()) == 0
+    util.check_status(lx)
+    return y
+
+
+def weight(lx, N, K, gen):
+    return host.store_weight(lx, (torch.randn((N, K), generator=gen, device="cuda") * 0.02).to(torch.bfloat16), abi.W_NVFP4)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1, 256), (8, 31, 512), (9, 250, 1024), (16, 5000, 256), (18, 129, 2048), (32, 300, 512), (36, 1000, 1280), (37, 97, 256),
+                                   (40, 4737, 512), (48, 640, 768), (56, 200, 512), (57, 300, 512), (64, 130, 4096), (65, 300, 512), (130, 2000, 1024), (1025, 260, 256)])
+def test_against_64_bits_and_rows_alone(lx, M, N, K):
+    gen = torch.Generator(device="cuda").manual_seed(M + N)
+    sw = weight(lx, N, K, gen)
+    w64 = values(sw.data, sw.scale, sw.glob, N, K)
+    for x_f32, pad in ((False, 0), (False, 3), (True, 0)):
+        wide = torch.randn((M, K + pad), generator=gen, device="cuda")
+        x = (wide if x_f32 else wide.to(torch.bfloat16))[:, :K]
+        y = product(lx, x, sw, M, N, K)
+        want = x.to(torch.bfloat16).double() @ w64.T
+        assert float((y.double() - want).norm() / want.norm()) <= 1e-6
+        for m in {0, M // 2, M - 1}:
+            assert torch.equal(product(lx, x[m:m + 1], sw, 1, N, K)[0], y[m])
+
+
+def test_bias_alpha_beta_and_bf16_outputs(lx):
+    M, N, K = 45, 333, 512
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    sw = weight(lx, N, K, gen)
+    x = torch.randn((M, K), generator=gen, device="cuda").to(torch.bfloat16)
+    bias, old = torch.randn((N,), generator=gen, device="cuda"), torch.randn((M, N + 3), generator=gen, device="cuda")
+    want = 0.5 * (x.double() @ values(sw.data, sw.scale, sw.glob, N, K).T + bias.double()) + 0.75 * old[:, :N].double()
+    y = product(lx, x, sw, M, N, K, 0.75, old.clone()[:, :N], bias, 0.5)
+    assert float((y.double() - want).norm() / want.norm()) <= 1e-6
+    y = product(lx, x, sw, M, N, K, 0.0, torch.empty((M, N), dtype=torch.bfloat16, device="cuda"), bias, 0.5)
+    assert float((y.double() - (want - 0.75 * old[:, :N].double())).norm() / want.norm()) <= 2.0**-8
+
+
+def test_values_without_digits(lx):
+    M, N, K = 12, 200, 512
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    sw = weight(lx, N, K, gen)
+    w64 = values(sw.data, sw.scale, sw.glob, N, K)
+    x = torch.randn((M, K), generator=gen, device="cuda").to(torch.bfloat16)
+    x[1, 7], x[2, 100] = float("inf"), float("-inf")
+    x[3, 5] = float("nan")
+    x[4] = 0
+    x[5] *= 1e-30
+    x[6] *= 1e30
+    x[7, 3], x[7, 300] = 1e20, 1e-20
+    x[8, ::5] = 0
+    y = product(lx, x, sw, M, N, K).double()
+    want = x.double() @ w64.T
+    for m in (1, 2):  # an infinity times its weight, NaN where that is zero
+        assert torch.equal(torch.nan_to_num(y[m], nan=0.5, posinf=1, neginf=-1), torch.nan_to_num(want[m], nan=0.5, posinf=1, neginf=-1))
+    assert bool(torch.isnan(y[3]).all()) and bool((y[4] == 0).all())
+    for m in (0, 5, 6, 7, 8, 9, 10, 11):
+        assert float((y[m] - want[m]).norm() / want[m].norm()) <= 1e-6, m
+
+
+def test_scales_with_a_sign(lx):
+    M, N, K = 16, 140, 512
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    sw = weight(lx, N, K, gen)
+    sw.scale[::3] |= 0x80
+    x = torch.randn((M, K), generator=gen, device="cuda").to(torch.bfloat16)
+    want = x.double() @ values(sw.data, sw.scale, sw.glob, N, K).T
+    assert float((product(lx, x, sw, M, N, K).double() - want).norm() / want.norm()) <= 1e-6
