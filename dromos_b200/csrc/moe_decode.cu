@@ -140,22 +140,31 @@ __device__ __forceinline__ float dot_word(const Raw& r, const float (&xf)[kLaneV
                                           int K) {
   constexpr int V = kLaneValues<F>;
   const uint32_t w[4] = {r.w.x, r.w.y, r.w.z, r.w.w};
-  if constexpr (F == LX_W_BF16) {
+  if constexpr (F == LX_W_BF16 || F == LX_W_BF16X) {
+    uint32_t v[4] = {w[0], w[1], w[2], w[3]};
+    if constexpr (F == LX_W_BF16X) {  // four values at a time to the bf16 words they encode, then like those
+      const uint32_t base4 = w[3] * 0x01010101u;
+      uint32_t e[2] = {base4 - (w[2] & 0x0f0f0f0fu), base4 - ((w[2] >> 4) & 0x0f0f0f0fu)};
+      if (r.s) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int sh = 8 * (j & 3);
+          const uint32_t p = patched_exponent(row, K, k0 + j, (e[j >> 2] >> sh) & 0xffu);
+          e[j >> 2] = (e[j >> 2] & ~(0xffu << sh)) | (p << sh);
+        }
+      }
+      const uint2 lo = x16_assemble(w[0], e[0]), hi = x16_assemble(w[1], e[1]);
+      v[0] = lo.x, v[1] = lo.y, v[2] = hi.x, v[3] = hi.y;
+      if (k0 + 8 > K) {  // padding of the last block decodes to 2^(base - 127), not to zero
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (k0 + j >= K) v[j >> 1] &= j & 1 ? 0x0000ffffu : 0xffff0000u;
+      }
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      acc = fmaf(xf[2 * j], __uint_as_float(w[j] << 16), acc);
-      acc = fmaf(xf[2 * j + 1], __uint_as_float(w[j] & 0xffff0000u), acc);
-    }
-  } else if constexpr (F == LX_W_BF16X) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const uint32_t sm = (w[j >> 2] >> (8 * (j & 3))) & 0xffu;
-      const uint32_t code = (w[2] >> (8 * (j & 3) + 4 * (j >> 2))) & 15u;
-      uint32_t e = (w[3] - code) & 0xffu;
-      if (r.s) e = patched_exponent(row, K, k0 + j, e);
-      float v = __uint_as_float(((sm & 0x80u) << 24) | (e << 23) | ((sm & 0x7fu) << 16));
-      if (k0 + j >= K) v = 0.0f;  // padding of the last block decodes to 2^(base - 127), not to zero
-      acc = fmaf(xf[j], v, acc);
+      acc = fmaf(xf[2 * j], __uint_as_float(v[j] << 16), acc);
+      acc = fmaf(xf[2 * j + 1], __uint_as_float(v[j] & 0xffff0000u), acc);
     }
   } else if constexpr (F == LX_W_INT8) {
 #pragma unroll
@@ -240,8 +249,11 @@ __device__ __forceinline__ Raw load_whole(const uint8_t* at, const uint8_t* scal
 // acc[r][t] += rows[r] . x[t] over all of K: the warp's lanes take consecutive words, kSteps words of each row in
 // flight per lane. A token's sum is the same chain of operations whatever NT is.
 // WHOLE (rows, scales and activations on their word's boundary): the steps all of whose 32 words lie within the row go
-// without bounds, by running pointers. The same words in the same order either way. These kernels are bound by instruction issue: at 5.4-6.4 instructions per FP8 value (where converting
-// and adding take 3) four tokens of the 64-expert case (FP8, 4096 x 1536, top 8) took 152 us, at half the copy bandwidth; 137 now.
+// without bounds, by running pointers. The same words in the same order either way. These kernels are bound by instruction
+// issue: at 5.4-6.4 instructions per FP8 value (where converting and adding take 3) four tokens of the 64-expert case (FP8,
+// 4096 x 1536, top 8) took 152 us, at half the copy bandwidth; 137 now. Measured and dropped: a word asked for as soon as one
+// is used, across rows and experts (161: more registers, fewer warps); f16 activations staged in shared memory for
+// fma.rn.f32.f16 (128, but one token 61 where this takes 53: the part has no such instruction and converts both operands).
 template <int F, int NR, int NT, bool WHOLE>
 __device__ __forceinline__ void dot_rows(const Stack& S, const uint8_t* const (&row)[NR], const uint8_t* const (&row_scale)[NR],
                                          const uint32_t (&flag)[NR], const uint16_t* const (&x)[NT], bool xvec, int lane,
@@ -307,27 +319,27 @@ __device__ __forceinline__ void dot_rows(const Stack& S, const uint8_t* const (&
 #pragma unroll
       for (int r = 0; r < NR; ++r) acc[r][t] = dot_word<F>(raw[r], xf, acc[r][t], row[r], k0, K);
     }
-    return;
-  }
-  for (int k_base = 0; k_base < K; k_base += kStep * kSteps) {
-    Raw raw[kSteps][NR];
+  } else {
+    for (int k_base = 0; k_base < K; k_base += kStep * kSteps) {
+      Raw raw[kSteps][NR];
 #pragma unroll
-    for (int j = 0; j < kSteps; ++j)
+      for (int j = 0; j < kSteps; ++j)
 #pragma unroll
-      for (int r = 0; r < NR; ++r) {
-        raw[j][r] = load_raw<F>(S, row[r], row_scale[r], k_base + (32 * j + lane) * V);
-        if constexpr (F == LX_W_BF16X) raw[j][r].s = flag[r];
-      }
+        for (int r = 0; r < NR; ++r) {
+          raw[j][r] = load_raw<F>(S, row[r], row_scale[r], k_base + (32 * j + lane) * V);
+          if constexpr (F == LX_W_BF16X) raw[j][r].s = flag[r];
+        }
 #pragma unroll
-    for (int j = 0; j < kSteps; ++j) {
-      const int k0 = k_base + (32 * j + lane) * V;
-      if (k0 >= K) continue;
+      for (int j = 0; j < kSteps; ++j) {
+        const int k0 = k_base + (32 * j + lane) * V;
+        if (k0 >= K) continue;
 #pragma unroll
-      for (int t = 0; t < NT; ++t) {
-        float xf[V];
-        load_x<V>(x[t], k0, K, xvec, xf);
+        for (int t = 0; t < NT; ++t) {
+          float xf[V];
+          load_x<V>(x[t], k0, K, xvec, xf);
 #pragma unroll
-        for (int r = 0; r < NR; ++r) acc[r][t] = dot_word<F>(raw[j][r], xf, acc[r][t], row[r], k0, K);
+          for (int r = 0; r < NR; ++r) acc[r][t] = dot_word<F>(raw[j][r], xf, acc[r][t], row[r], k0, K);
+        }
       }
     }
   }
