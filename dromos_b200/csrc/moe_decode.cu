@@ -408,9 +408,10 @@ __global__ void __launch_bounds__(kDecodeThreads, WHOLE && F != LX_W_BF16X && F 
 }
 
 // Stage 2: out[t, l] = sum over k, in order, of weights[t, k] * (s_l * down[e_k]_l . mid[t, k]). grid (ceil(L / 16), T): a warp
-// takes two rows, so that the intermediate row's conversion serves both.
+// takes two rows, so that the intermediate row's conversion serves both. (Four blocks per SM: what a warp waits for is the next
+// expert's rows, and FP8's 72 registers left room for three: the call above 139 us, 123 with 64.)
 template <int F, bool WHOLE>
-__global__ void __launch_bounds__(kDecodeThreads) decode_down_kernel(const Stack S, const uint16_t* __restrict__ mid, int xvec,
+__global__ void __launch_bounds__(kDecodeThreads, WHOLE && F != LX_W_BF16X ? 4 : 1) decode_down_kernel(const Stack S, const uint16_t* __restrict__ mid, int xvec,
                                                                      const int32_t* __restrict__ ids,
                                                                      const float* __restrict__ weights, float* __restrict__ out,
                                                                      int top_k, int L) {
