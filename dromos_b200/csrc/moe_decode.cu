@@ -254,12 +254,12 @@ __device__ __forceinline__ Raw load_whole(const uint8_t* at, const uint8_t* scal
 // 4096 x 1536, top 8) took 152 us, at half the copy bandwidth; 137 now. Measured and dropped: a word asked for as soon as one
 // is used, across rows and experts (161: more registers, fewer warps); f16 activations staged in shared memory for
 // fma.rn.f32.f16 (128, but one token 61 where this takes 53: the part has no such instruction and converts both operands).
-template <int F, int NR, int NT, bool WHOLE>
+template <int F, int NR, int NT, bool WHOLE, int STEPS = 4>
 __device__ __forceinline__ void dot_rows(const Stack& S, const uint8_t* const (&row)[NR], const uint8_t* const (&row_scale)[NR],
                                          const uint32_t (&flag)[NR], const uint16_t* const (&x)[NT], bool xvec, int lane,
                                          float (&acc)[NR][NT]) {
   constexpr int V = kLaneValues<F>;
-  constexpr int kSteps = NT == 1 ? 4 : 2;
+  constexpr int kSteps = NT == 1 ? STEPS : 2;
   constexpr int kStep = 32 * V;  // values of K a step covers
   const int K = S.K;
   int k_done = 0;
@@ -345,6 +345,12 @@ __device__ __forceinline__ void dot_rows(const Stack& S, const uint8_t* const (&
   }
 }
 
+// Gate/up rows of the 8-bit formats: two steps in flight per warp and four blocks per SM (64 registers) instead of four steps and
+// three blocks (80): FP8, one / four tokens 58 / 115 -> 52 / 106 us with the rest of the call, INT8, eight 261 -> 253. BF16, whose words
+// need no conversion, is faster with more in flight (98 against 105), NVFP4 and BF16X do not fit 64 registers.
+template <int F, bool WHOLE>
+constexpr bool kLean = WHOLE && (F == LX_W_FP8 || F == LX_W_INT8);
+
 // Stage 1 for the NT member pairs of one expert: mid[pair, i] = bf16(silu(s_g * gate_i . x) * (s_u * up_i . x)).
 template <int F, int NT, bool WHOLE>
 __device__ __forceinline__ void gate_up_members(const Stack& S, int e, int i, int I, const uint16_t* latent, int ld, bool xvec,
@@ -359,7 +365,7 @@ __device__ __forceinline__ void gate_up_members(const Stack& S, int e, int i, in
   float acc[2][NT];
 #pragma unroll
   for (int t = 0; t < NT; ++t) acc[0][t] = acc[1][t] = 0.0f;
-  dot_rows<F, 2, NT, WHOLE>(S, row, row_scale, flag, x, xvec, lane, acc);
+  dot_rows<F, 2, NT, WHOLE, kLean<F, WHOLE> ? 2 : 4>(S, row, row_scale, flag, x, xvec, lane, acc);
   const float fg = stack_row_factor<F>(S, ng, e), fu = stack_row_factor<F>(S, nu, e);
 #pragma unroll
   for (int t = 0; t < NT; ++t) {
@@ -373,7 +379,7 @@ __device__ __forceinline__ void gate_up_members(const Stack& S, int e, int i, in
 // time (more members than two read the rows again, from L1 / L2: the registers of wider passes would halve the warps
 // an SM holds for the common case of one or two).
 template <int F, bool WHOLE>
-__global__ void __launch_bounds__(kDecodeThreads, WHOLE && F != LX_W_BF16X && F != LX_W_NVFP4 ? 3 : 2) decode_gate_up_kernel(const Stack S, const uint16_t* __restrict__ latent, int ld,
+__global__ void __launch_bounds__(kDecodeThreads, kLean<F, WHOLE> ? 4 : WHOLE && F == LX_W_BF16 ? 3 : 2) decode_gate_up_kernel(const Stack S, const uint16_t* __restrict__ latent, int ld,
                                                                         int xvec, const int32_t* __restrict__ ids,
                                                                         uint16_t* __restrict__ mid, int P, int top_k, int I,
                                                                         int dedupe) {
