@@ -251,9 +251,9 @@ __device__ __forceinline__ Raw load_whole(const uint8_t* at, const uint8_t* scal
 // WHOLE (rows, scales and activations on their word's boundary): the steps all of whose 32 words lie within the row go
 // without bounds, by running pointers. The same words in the same order either way. These kernels are bound by instruction
 // issue: at 5.4-6.4 instructions per FP8 value (where converting and adding take 3) four tokens of the 64-expert case (FP8,
-// 4096 x 1536, top 8) took 152 us, at half the copy bandwidth; 137 now. Measured and dropped: a word asked for as soon as one
-// is used, across rows and experts (161: more registers, fewer warps); f16 activations staged in shared memory for
-// fma.rn.f32.f16 (128, but one token 61 where this takes 53: the part has no such instruction and converts both operands).
+// 4096 x 1536, top 8) took 152 us, at half the copy bandwidth; 137 this way, 115 with the blocks per SM of the two kernels. Measured and dropped: a word asked for as soon as one
+// is used, across rows and experts (161 against 137: more registers, fewer warps); f16 activations staged in shared memory for
+// fma.rn.f32.f16 (128, but one token 61 where this took 53: the part has no such instruction and converts both operands).
 template <int F, int NR, int NT, bool WHOLE, int STEPS = 4>
 __device__ __forceinline__ void dot_rows(const Stack& S, const uint8_t* const (&row)[NR], const uint8_t* const (&row_scale)[NR],
                                          const uint32_t (&flag)[NR], const uint16_t* const (&x)[NT], bool xvec, int lane,
