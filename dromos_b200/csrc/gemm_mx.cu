@@ -5,20 +5,31 @@
 // f16 in registers was what bound the kernels before this one: eight converter warps, ~27 instructions per 16 values, 72 us
 // for 28672 x 8192 at 16 rows where the bytes take 20. So it is the activations that are taken apart, once per call, into
 // what the instruction multiplies: every block of 16 values gets the power of two of its largest magnitude as its scale and
-// seven digits in base 8 (-4..4, exact in e2m1), 21 bits below that magnitude. A bf16 value within 2^-12 of its block's
-// largest comes out exactly, a smaller one within 2^-20 of that largest. A digit is a column of its own
-// (column j * Mp + m is digit j of row m), summed on its own in f32 and put together in the epilogue, least first. (Block
-// scales reach 2^-17 of the row's largest magnitude; a block below that keeps the bits above 2^-36 of it.) Against 64 bits,
-// N(0, 1) activations: 4e-8 at every K, where the f16 expansion was off by 1e-7 (K = 512) to 2.4e-6 (K = 8192); with six
-// digits it was 4e-7, more than before at short K.
+// seven digits in base 13, 24 bits below that magnitude. (e2m1 holds 0, 1, 2, 3, 4, 6, 8, 12 halves with a sign: every residue
+// of 13. Base 8, whose digits need only -4..4, gives 21 bits from seven columns, and nine columns of it leave no room for 64
+// rows in tensor memory.) A digit is a column of its own (column j * Mp + m is digit j of row m), summed on its own in f32 and
+// put together in the epilogue, least first.
+//
+// Remainders. A bf16 value within 2^-16 of its block's largest comes out of the digits exactly; of a smaller one, what the
+// digits leave is kept too, as digits under the least block scale there is, and its stage of 256 values of K is multiplied a
+// second time from these remainders, into the same accumulators. Together the operands are exact down to 2^-33 of a row's
+// largest magnitude and rounded at 2^-41 of it below (an f16 row under one power of two: 2^-31 and 2^-39): an output whose
+// weights are zero wherever the row has its outliers is as exact as any other. Which stages have remainders, only the values
+// say: the preparation leaves a bit per row and stage, and a chunk's stage goes again if any of its rows has one. (N(0, 1)
+// values: one in 10^5 has a remainder, so ~4 % of the stages go again at 16 rows and ~17 % at 64; rows with remainders
+// everywhere take twice as long.) A row without them adds zeros, so its bits do not depend on the rows beside it.
 //
 // What a product costs: an instruction covers 128 weight rows x 64 values of K (four times kind::f16's) for half a cycle per
 // column; up to 64 rows are 448 columns in two instructions of four and three digits. A launch takes up to 1024 rows in
 // chunks of at most 64, the chunks of a weight panel next to each other so that its later readers find it in L2.
 //
-// Measured (28672 x 8192; before: the f16 expansion): 16 / 32 / 64 rows 72.1 / 74.5 / 83 -> 42.5 / 47 / 75 us; 14336 x 4096, 100 / 500
-// / 1000 rows 49 / 209 / 415 -> 43 / 132 / 244. What a stage takes at 16 rows is its copies (39 us with products and scales
-// left out); at 64 rows the 60 KB of digits that every SM fetches from L2 per 12 KB of weights.
+// Measured (replayed graphs; before: the f16 expansion): 28672 x 8192, 16 / 32 / 48 / 64 rows 70.7 / 72.1 / 74.2 / 80.3 -> 44.6 / 51.4
+// / 71.0 / 91.5 us; 14336 x 4096, 64 / 100 / 500 / 1000 rows 26.8 / 49.5 / 205 / 406 -> 28.3 / 48.1 / 148 / 267. (Base 8 without
+// remainders, 21 bits: 41.7 / 45.7 / 61.4 / 73.3 and 24.0 / 42.3 / 131 / 242. Without a stage that goes again, base 13 takes 43.3 /
+// 47.7 / 62.7 / 78.2: the more rows, the more stages do.) What a stage takes at 16 rows is its copies (39 us with products and scales
+// left out); at 64 rows the 60 KB of digits that every SM fetches from L2 per 12 KB of weights. Error against 64 bits, N(0, 1)
+// rows: 4e-8 at every K (f16: 9e-8 at K = 512, 2.3e-6 at 8192); with an outlier of 2^6 .. 2^20 in every block, outputs whose weights are
+// zero there: 5e-8 .. 7.5e-7 at K = 8192 (f16: 2.3e-6; without remainders 4e-6 .. 0.4).
 //   * The block scales go to tensor memory with tcgen05.st. Written to shared memory for tcgen05.cp they needed the proxy fence,
 //     which waits for the thread's scale loads in flight: 84 us. With the activations' scales by tcgen05.cp: 57 us (copies
 //     and products of one pipe wait for each other).
@@ -39,6 +50,8 @@ namespace {
 
 constexpr int kMxStageK = 256;                  // values of K per stage: 128 bytes per weight row, four products
 constexpr int kMxDigits = 7;
+constexpr int kMxBase = 13;
+constexpr int kMxUnit = 23;                     // a block's values are whole numbers of 2^(e - kMxUnit), e the exponent of its largest
 constexpr int kMxThreads = 11 * 32;
 constexpr int kMxScaleBytes = 2 * 128 * 16;     // shared memory in which the scale warps exchange rows: two stages of 128 rows x 16 bytes
 constexpr int kAhead = 8;                       // stages whose weight scales a thread has in flight
@@ -55,6 +68,9 @@ struct MxParams {
   int sf0, sf_stages;       // where in tensor memory the scales begin, and for how many stages in turn (4, 2 or 1)
   int x_bytes, sf_off;      // a stage's activations: digits, and from sf_off on the block scales
   const uint8_t* xprep;
+  int64_t remainders;       // from a stage's digits to those of its remainders
+  const uint8_t* again;     // [chunks][groups][64]: bit b of byte (c, g, m): row m of chunk c has remainders in stage 8 g + b
+  int groups;
   const float* row_scale;   // per activation row: what its sums are multiplied by
   int buffers;              // accumulators (2 where they fit)
   int SW, SX;
@@ -91,21 +107,52 @@ __device__ __forceinline__ uint32_t max_magnitude(uint32_t m, const uint4& v) { 
   const uint32_t t = __vmaxu2(__vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu), __vmaxu2(v.z & 0x7fff7fffu, v.w & 0x7fff7fffu));
   return max(m, max(t & 0xffffu, t >> 16));
 }
+// Digits come in pairs: for a residue u of 169, the e2m1 codes (the digit's half) of its two base-13 digits, the lower one in bits
+// 0-3, and in bit 8 what the pair carries. Residue r of 13 is the digit r, or r - 13 where e2m1 has that: 0 1 2 3 4 -8 6 -6 8 -4 -3 -2 -1.
+__device__ __forceinline__ uint32_t digit_pair(uint32_t u) {
+  constexpr uint64_t kCodes = 0x9abc6d5e43210ull;
+  auto code_of = [&](uint32_t r) { return static_cast<uint32_t>(kCodes >> (4 * r)) & 15u; };
+  const uint32_t lo = code_of(u % kMxBase), next = u / kMxBase + (lo >> 3);  // 0..13
+  const uint32_t hi = next == kMxBase ? 0u : code_of(next);
+  return lo | hi << 4 | (next == kMxBase ? 256u : hi >> 3 << 8);
+}
+// The seven digits of q, |q| < 1.246 * 2^24, as codes into bits 4 i .. 4 i + 3 of w[0..6], most significant first. (Three steps of a pair
+// from a table in shared memory; six of a digit are twice the instructions, and the preparation is bound by them.)
+__device__ __forceinline__ void put_digits(int q, int i, const uint16_t* pairs, uint32_t (&w)[kMxDigits]) {
+  constexpr uint32_t kPair = kMxBase * kMxBase, kBias = kPair << 18;  // keeps what is divided positive
+#pragma unroll
+  for (int j = kMxDigits - 1; j > 0; j -= 2) {
+    const uint32_t u = static_cast<uint32_t>(q) + kBias, t = u / kPair, c = pairs[u - t * kPair];
+    w[j] |= (c & 15u) << (4 * i);
+    w[j - 1] |= (c >> 4 & 15u) << (4 * i);
+    q = static_cast<int>(t - kBias / kPair + (c >> 8));
+  }
+  w[0] |= static_cast<uint32_t>(q < 0 ? 8 - q : q) << (4 * i);  // -4..4 is left
+}
 // 2^e as ue4m3, e in -9..8.
 __device__ __forceinline__ uint32_t ue4m3_pow2(int e) { return e >= -6 ? static_cast<uint32_t>(e + 7) << 3 : 1u << (e + 9); }
+// 2^e as f32, e in -149..127.
+__device__ __forceinline__ float exp2_of(int e) { return __uint_as_float(e >= -126 ? static_cast<uint32_t>(e + 127) << 23 : 1u << (e + 149)); }
+constexpr int kFirstDigit = 4 * 4826809;  // 4 * 13^6: the first digit alone
 
 // Block (piece, row): 256 threads, each 8 values (half a scale block) of an activation row; every block finds the row's largest
 // magnitude again (a few KB, from L2), which saves a second kernel. (With 32 values per thread the seven digits of each were
-// ~1400 instructions in a row: at 16 rows the preparation took as long as an eighth of the product.)
+// ~1400 instructions in a row: at 16 rows the preparation took as long as an eighth of the product.) A warp's values are one
+// stage's, a block's eight stages': their bits are one byte of `again`. A block without remainders gets the scale zero there, which
+// makes whatever its digits are zero.
 // Rows that are not finite: a NaN, or more than one infinity, makes the row's outputs NaN; with a single infinity the finite
 // values do not count and the outputs are the infinity times its weight (NaN where that is zero).
-constexpr int kPrepThreads = 256;
+constexpr int kPrepThreads = 256;  // (at most 40 registers each: a block fits beside the product's CTA and starts under its end. With 48,
+                                   // and 140 in the product, it did not: 14336 x 4096 at 32 rows 23 us instead of 19)
 template <bool XBF>
-__global__ void __launch_bounds__(kPrepThreads) mx_prep_kernel(const void* __restrict__ x, int ld_x, int K, int chunk_rows, int64_t chunk_bytes, int Mp, int cols0,
-                                                               int cols1, int x_bytes, int sf_off, uint8_t* __restrict__ out, float* __restrict__ row_scale) {
+__global__ void __launch_bounds__(kPrepThreads, 6) mx_prep_kernel(const void* __restrict__ x, int ld_x, int K, int chunk_rows, int64_t chunk_bytes, int Mp, int cols0,
+                                                               int cols1, int x_bytes, int sf_off, uint8_t* __restrict__ out, int64_t remainders,
+                                                               uint8_t* __restrict__ again, float* __restrict__ row_scale) {
   pdl_trigger();
+  __shared__ uint32_t part[kPrepThreads / 32], infinities, stages_again;
+  __shared__ uint16_t pairs[kMxBase * kMxBase];
+  if (threadIdx.x < kMxBase * kMxBase) pairs[threadIdx.x] = static_cast<uint16_t>(digit_pair(threadIdx.x));
   pdl_wait();  // the kernel before this one may still be reading the workspace
-  __shared__ uint32_t part[kPrepThreads / 32], infinities;
   const int row_id = blockIdx.y, chunk = row_id / chunk_rows, m = row_id - chunk * chunk_rows, tid = threadIdx.x;
   const int64_t row = static_cast<int64_t>(row_id) * ld_x;
   const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && ld_x % (XBF ? 8 : 4) == 0;
@@ -117,7 +164,7 @@ __global__ void __launch_bounds__(kPrepThreads) mx_prep_kernel(const void* __res
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
   if ((tid & 31) == 0) part[tid >> 5] = top;
-  if (tid == 0) infinities = 0;
+  if (tid == 0) infinities = stages_again = 0;
   uint32_t block_top = max_magnitude(0, v);
   block_top = max(block_top, __shfl_xor_sync(0xffffffffu, block_top, 1));
   __syncthreads();
@@ -133,39 +180,70 @@ __global__ void __launch_bounds__(kPrepThreads) mx_prep_kernel(const void* __res
   }
   const int e_row = max(static_cast<int>(top >> 7), 30) - 127;
   if (blockIdx.x == 0 && tid == 0)
-    row_scale[row_id] = finite ? __uint_as_float(static_cast<uint32_t>(e_row - 8 + 127) << 23)
-                               : __uint_as_float(top == 0x7f80u && infinities == 1 ? 0x7f800000u : 0x7fc00000u);
-  if (k0 >= K) return;
-  constexpr int kUnit = 3 * kMxDigits - 2;  // the last digit counts in 2^(e - kUnit), the first in 2^e / 2
-  const int e = max(max(static_cast<int>(block_top >> 7), 1) - 127, e_row - 17);  // 2^-9 is the least scale
-  // 2^(kUnit - e) in two factors: the whole can be beyond f32
-  const int half = (kUnit - e) / 2;
-  const float f0 = __uint_as_float(static_cast<uint32_t>(half + 127) << 23), f1 = __uint_as_float(static_cast<uint32_t>(kUnit - e - half + 127) << 23);
+    row_scale[row_id] = finite ? exp2_of(e_row - 7 - kMxUnit) : __uint_as_float(top == 0x7f80u && infinities == 1 ? 0x7f800000u : 0x7fc00000u);
+  // The block's exponent; one less for a largest value below 1.25 * 2^e, which the digits still hold. 2^-9 is the least scale.
+  const int e = max(max(static_cast<int>(block_top + 96) >> 7, 2) - 128, e_row - 17);
+  // 2^(kMxUnit - e) in two factors: the whole can be beyond f32
+  const int half = (kMxUnit - e) / 2;
+  const float f0 = exp2_of(half), f1 = exp2_of(kMxUnit - e - half), to_least = exp2_of(e - e_row + 17);
   const uint32_t words[4] = {v.x, v.y, v.z, v.w};
   uint32_t w[kMxDigits] = {};
+  int rest[8];  // what the digits leave, in units of the least scale: up to 2^16
+  bool some = false;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const uint32_t bits = (words[i / 2] >> (16 * (i & 1))) & 0xffffu;
     int q;
-    if (finite) q = __float2int_rn(bf16_bits_to_f32(bits) * f0 * f1);
-    else q = (bits & 0x7fffu) != 0x7f80u ? 0 : bits & 0x8000u ? -(4 << 3 * (kMxDigits - 1)) : 4 << 3 * (kMxDigits - 1);  // the first digit alone
-#pragma unroll
-    for (int j = kMxDigits - 1; j > 0; --j) {
-      const int u8 = (q + 4) & 7;  // the digit plus 4
-      w[j] |= ((0x32109abcu >> (4 * u8)) & 15u) << (4 * i);
-      q = (q + 4 - u8) >> 3;
+    if (finite) {
+      const float t = bf16_bits_to_f32(bits) * f0 * f1, r = rintf(t);
+      q = static_cast<int>(r);
+      rest[i] = __float2int_rn((t - r) * to_least);
+      some |= rest[i] != 0;
+    } else {
+      q = (bits & 0x7fffu) != 0x7f80u ? 0 : bits & 0x8000u ? -kFirstDigit : kFirstDigit;
+      rest[i] = 0;
     }
-    w[0] |= static_cast<uint32_t>(q < 0 ? 8 - q : q) << (4 * i);
+    put_digits(q, i, pairs, w);
   }
+  const uint32_t with_rest = __ballot_sync(0xffffffffu, some);
+  if (with_rest && (tid & 31) == 0) atomicOr(&stages_again, 1u << (tid >> 5));
+  __syncthreads();
+  if (tid == 0) again[(static_cast<int64_t>(chunk) * gridDim.x + blockIdx.x) * kMaxRows + m] = static_cast<uint8_t>(stages_again);
+  if (k0 >= K) return;
   uint8_t* stage = out + chunk * chunk_bytes + static_cast<size_t>(k0 / kMxStageK) * x_bytes;
   const int kb = (k0 % kMxStageK) / 2, NC = cols0 + cols1, atoms = (cols0 + 127) / 128;
 #pragma unroll
   for (int j = 0; j < kMxDigits; ++j) *reinterpret_cast<uint32_t*>(stage + block_offset(NC, kb & ~15, j * Mp + m) + (kb & 15)) = w[j];
+  const bool block_rest = (with_rest >> (tid & 30) & 3u) != 0;  // this thread's eight values' or its neighbour's
+  int zeros = 0;
+  if (with_rest) {
+    // Under the largest scale that keeps them whole: few columns get few more bits, and their sums stay exact. (Under the least
+    // scale every product cut off the sums of the digits above: 2.5e-6 at K = 4096 with an outlier in every block, now 6e-8.)
+    uint32_t bits = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) bits |= static_cast<uint32_t>(rest[i]);
+    bits |= __shfl_xor_sync(0xffffffffu, bits, 1);
+    if (block_rest) {
+      zeros = __ffs(static_cast<int>(bits)) - 1;
+      uint32_t d[kMxDigits] = {};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) put_digits(rest[i] >> zeros, i, pairs, d);
+#pragma unroll
+      for (int j = 0; j < kMxDigits; ++j) *reinterpret_cast<uint32_t*>(stage + remainders + block_offset(NC, kb & ~15, j * Mp + m) + (kb & 15)) = d[j];
+    }
+  }
   if (k0 % 16 != 0) return;
   // scales: product k0 / 64 of the stage; 128 columns are 32 lanes of 16 bytes, a column's 4 bytes at word column / 32
-  const uint8_t sf = static_cast<uint8_t>(finite ? ue4m3_pow2(e - e_row + 8) : 0x38u);
+  const uint8_t sf = static_cast<uint8_t>(finite ? ue4m3_pow2(e - e_row + 8) : 0x38u), sf_rest = static_cast<uint8_t>(block_rest ? ue4m3_pow2(zeros - 9) : 0u);
   uint8_t* sfs = stage + sf_off + (k0 % kMxStageK) / 64 * (atoms * 512) + (k0 % 64) / 16;
-  for (int c = m; c < cols0; c += Mp) sfs[(c >> 7) * 512 + (c & 31) * 16 + ((c >> 5) & 3) * 4] = sf;
+#pragma unroll
+  for (int j = 0; j < kMxDigits; ++j) {
+    const int c = j * Mp + m;
+    if (c >= cols0) break;
+    const int at = (c >> 7) * 512 + (c & 31) * 16 + ((c >> 5) & 3) * 4;
+    sfs[at] = sf;
+    sfs[remainders + at] = sf_rest;
+  }
 }
 
 // ---- instructions ------------------------------------------------------------------------------------------------------------
@@ -174,6 +252,25 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
                "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]),
                "r"(r[13]), "r"(r[14]), "r"(r[15])
                : "memory");
+}
+// All of `threads` threads meet at a named barrier; true for each if p was for all.
+__device__ __forceinline__ bool named_bar_and(int id, int threads, bool p) {
+  uint32_t r;
+  asm volatile(
+      "{ .reg .pred a, b; setp.ne.u32 a, %1, 0; barrier.cta.red.and.pred b, %2, %3, a; selp.u32 %0, 1, 0, b; }"
+      : "=r"(r)
+      : "r"(static_cast<uint32_t>(p)), "r"(id), "r"(threads)
+      : "memory");
+  return r != 0;
+}
+// The first stage after s whose bit is set in `again`; n if there is none.
+__device__ __forceinline__ int again_after(const uint8_t* again, int n, int s) {
+#pragma unroll 1
+  for (++s; s < n; s = (s | 7) + 1) {
+    const uint32_t b = static_cast<uint32_t>(again[s >> 3]) >> (s & 7);
+    if (b) return s + __ffs(static_cast<int>(b)) - 1;
+  }
+  return n;
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void mx_umma(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t sfa, uint32_t sfb,
@@ -206,7 +303,10 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
   auto s_empty = [&](int b) { return bar0 + 8u * (2 * SW + 2 * SX + 4 + b); };  // and their products are done
   auto d_full = [&](int b) { return bar0 + 8u * (2 * SW + 2 * SX + 8 + b); };   // accumulator b is complete
   auto d_empty = [&](int b) { return bar0 + 8u * (2 * SW + 2 * SX + 10 + b); };  // and has been read
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * SW + 2 * SX + 12);
+  const uint32_t a_full = bar0 + 8u * (2 * SW + 2 * SX + 12);                    // `again` is complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * SW + 2 * SX + 13);
+  // [chunks][groups]: the stages that a chunk multiplies again, from the preparation's bits per row
+  uint8_t* const again = reinterpret_cast<uint8_t*>(tmem_slot + 2);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_stages = P.K / kMxStageK;
@@ -215,9 +315,20 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
   const int n_tiles = (P.N + P.R - 1) / P.R * chunks;
   const int tile_begin = static_cast<int>(static_cast<int64_t>(n_tiles) * blockIdx.x / gridDim.x);
   const int tile_end = static_cast<int>(static_cast<int64_t>(n_tiles) * (blockIdx.x + 1) / gridDim.x);
-  const int total = (tile_end - tile_begin) * n_stages;
+  const int groups = P.groups;
+  // stage(s, rest) for each of a chunk's stages in turn, then for those that go again; false as soon as one gives up
+  auto all_stages = [&](int chunk, auto&& stage) __attribute__((always_inline)) {
+    for (int s = 0; s < n_stages; ++s)
+      if (!stage(s, false)) return false;
+    if (!tc_wait(a_full, 0, P.status)) return false;
+    const uint8_t* bits = again + chunk * groups;
+    for (int s = again_after(bits, n_stages, -1); s < n_stages; s = again_after(bits, n_stages, s))
+      if (!stage(s, true)) return false;
+    return true;
+  };
 
   if (tid == 0) {
+    mbar_init(a_full, 128);
     for (int s = 0; s < SW; ++s) {
       mbar_init(w_full(s), 1);
       mbar_init(w_empty(s), 1);
@@ -254,18 +365,17 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
       bool ok = true, wrapped = false;
       int issued = 0;
       for (int tile = tile_begin; tile < tile_end && ok; ++tile) {
-        const int row = tile / chunks * P.R;
-        for (int s = 0; s < n_stages; ++s) {
-          if (wrapped && !tc_wait(w_empty(w.slot), w.lap ^ 1u, P.status)) {
-            ok = false;
-            break;
-          }
+        const int row = tile / chunks * P.R, chunk = tile % chunks;
+        auto stage = [&](int s, bool) __attribute__((always_inline)) {
+          if (wrapped && !tc_wait(w_empty(w.slot), w.lap ^ 1u, P.status)) return false;
           mbar_arrive_expect_tx(w_full(w.slot), P.R * 128);
           tile_g2s(smem_u32(smem) + static_cast<uint32_t>(w.slot) * box_bytes, &wmap, s * 32, row, w_full(w.slot));
           ++issued;
           w.advance(SW);
           wrapped |= w.slot == 0;
-        }
+          return true;
+        };
+        ok = all_stages(chunk, stage);
       }
       if (!ok)  // the copies in flight land before the CTA leaves
         for (int i = max(0, issued - SW); i < issued; ++i) tc_wait(w_full(i % SW), (i / SW) & 1, P.status);
@@ -276,22 +386,20 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
       pdl_wait();  // prepared by the kernel before this one
       Ring x;
       bool ok = true, wrapped = false;
-      int s = 0, i = 0, chunk = tile_begin % chunks;
-      const uint8_t* src = P.xprep + chunk * P.chunk_bytes;
-      for (; i < total; ++i) {
-        if (wrapped && !tc_wait(x_empty(x.slot), x.lap ^ 1u, P.status)) {
-          ok = false;
-          break;
-        }
-        mbar_arrive_expect_tx(x_full(x.slot), x_bytes);
-        bulk_g2s(smem_u32(xring) + static_cast<uint32_t>(x.slot) * x_bytes, src + static_cast<size_t>(s) * x_bytes, x_bytes, x_full(x.slot));
-        x.advance(SX);
-        wrapped |= x.slot == 0;
-        if (++s == n_stages) {
-          s = 0;
-          if (++chunk == chunks) chunk = 0;
-          src = P.xprep + chunk * P.chunk_bytes;
-        }
+      int i = 0, chunk = tile_begin % chunks;
+      for (int tile = tile_begin; tile < tile_end && ok; ++tile) {
+        const uint8_t* src = P.xprep + chunk * P.chunk_bytes;
+        auto stage = [&](int s, bool rest) __attribute__((always_inline)) {
+          if (wrapped && !tc_wait(x_empty(x.slot), x.lap ^ 1u, P.status)) return false;
+          mbar_arrive_expect_tx(x_full(x.slot), x_bytes);
+          bulk_g2s(smem_u32(xring) + static_cast<uint32_t>(x.slot) * x_bytes, src + (rest ? P.remainders : 0) + static_cast<size_t>(s) * x_bytes, x_bytes, x_full(x.slot));
+          ++i;
+          x.advance(SX);
+          wrapped |= x.slot == 0;
+          return true;
+        };
+        ok = all_stages(chunk, stage);
+        if (++chunk == chunks) chunk = 0;
       }
       if (!ok)
         for (int j = max(0, i - SX); j < i; ++j) tc_wait(x_full(j % SX), (j / SX) & 1, P.status);
@@ -312,32 +420,36 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
       bool ok = true;
       const uint32_t sf_mask = P.sf_stages - 1, sf_shift = P.sf_stages == 4 ? 2 : P.sf_stages == 2 ? 1 : 0;
       uint32_t i = 0;
+      int chunk = tile_begin % chunks;
       for (int tile = tile_begin, t = 0; tile < tile_end && ok; ++tile, ++t) {
         const int buf = P.buffers == 2 ? t & 1 : 0, use = P.buffers == 2 ? t >> 1 : t;  // this accumulator's use-th use
         const uint32_t d_tmem = tmem_base + buf * NC;
         if (use > 0 && !tc_wait(d_empty(buf), (use - 1) & 1, P.status)) break;
         tc_fence_after();
-        for (int s = 0; s < n_stages; ++s, ++i) {
+        auto stage = [&](int s, bool rest) __attribute__((always_inline)) {
           const uint32_t turn = i & sf_mask, sfa = tmem_base + P.sf0 + turn * kSfCols, sfb = sfa + 16;
           if (!tc_wait(x_full(x.slot), x.lap, P.status) || !tc_wait(w_full(w.slot), w.lap, P.status) || !tc_wait(s_full(turn), (i >> sf_shift) & 1, P.status)) {
-            ok = false;
-            break;
+            return false;
           }
           tc_fence_after();
           const uint32_t x_at = (static_cast<uint32_t>(x.slot) * x_bytes) >> 4;
           const uint32_t a_lo = a_lo0 + ((static_cast<uint32_t>(w.slot) * box_bytes) >> 4), b_lo = b_lo0 + x_at;
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks) {
-            mx_umma(d_tmem, a_lo + 2 * ks, a_hi, b_lo + ks * b_step, b_hi, idesc0, sfa + 4 * ks, sfb + 4 * ATOMS * ks, (s | ks) ? 1u : 0u);
-            if constexpr (TWO) mx_umma(d_tmem + P.cols0, a_lo + 2 * ks, a_hi, b_lo + ks * b_step + b_second, b_hi, idesc1, sfa + 4 * ks, sfb + 4 * ATOMS * ks, (s | ks) ? 1u : 0u);
+            mx_umma(d_tmem, a_lo + 2 * ks, a_hi, b_lo + ks * b_step, b_hi, idesc0, sfa + 4 * ks, sfb + 4 * ATOMS * ks, (rest || (s | ks)) ? 1u : 0u);
+            if constexpr (TWO) mx_umma(d_tmem + P.cols0, a_lo + 2 * ks, a_hi, b_lo + ks * b_step + b_second, b_hi, idesc1, sfa + 4 * ks, sfb + 4 * ATOMS * ks, (rest || (s | ks)) ? 1u : 0u);
           }
           umma_commit(w_empty(w.slot));
           umma_commit(x_empty(x.slot));
           umma_commit(s_empty(turn));
           w.advance(SW);
           x.advance(SX);
-        }
+          ++i;
+          return true;
+        };
+        ok = all_stages(chunk, stage);
         if (ok) umma_commit(d_full(buf));
+        if (++chunk == chunks) chunk = 0;
       }
     }
   } else if (warp >= 4) {
@@ -345,89 +457,124 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
     const int r = tid - 128;
     const int64_t pitch = P.K / 16;
     uint4 q[kAhead];
-    int lt = tile_begin, ls = 0, lc = tile_begin % chunks;  // the stage that is loaded next, and its tile's chunk
-    int row = tile_begin / chunks * P.R + r;
-    const uint8_t* src = P.scale + row * pitch;
-    bool live = r < P.R && row < P.N;
-    auto load = [&](uint4& v) {
-      if (lt < tile_end && live) v = __ldg(reinterpret_cast<const uint4*>(src) + ls);
-      if (++ls == n_stages) {
-        ls = 0, ++lt;
-        if (++lc == chunks) {
-          lc = 0, row += P.R;
-          src = P.scale + row * pitch;
-          live = r < P.R && row < P.N;
-        }
-      }
+    auto scales_of = [&](int panel) -> const uint4* {  // this thread's row of a panel, null past the last
+      const int n = panel * P.R + r;
+      return r < P.R && n < P.N ? reinterpret_cast<const uint4*>(P.scale + n * pitch) : nullptr;
     };
+    int panel = tile_begin / chunks, chunk = tile_begin % chunks;
+    const uint4* scales = tile_begin < tile_end ? scales_of(panel) : nullptr;
 #pragma unroll
-    for (int i = 0; i < kAhead; ++i) {
-      q[i] = make_uint4(0, 0, 0, 0);
-      load(q[i]);
-    }
+    for (int i = 0; i < kAhead; ++i) q[i] = scales && i < n_stages ? __ldg(scales + i) : make_uint4(0, 0, 0, 0);
     // Lane l of each of the four warps holds rows l, 32 + l, 64 + l and 96 + l in tensor memory: every quarter has all 128 rows.
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + P.sf0;
     Ring w, x;
     bool ok = true;
-    for (int i0 = 0; i0 < total; i0 += kAhead) {  // (a warp whose wait gave up still comes to the meetings)
-#pragma unroll
-      for (int i = 0; i < kAhead; ++i) {
-        if (i0 + i >= total) break;
-        const int turn = i & (P.sf_stages - 1), use = (i0 + i) / P.sf_stages;
-        if ((q[i].x | q[i].y | q[i].z | q[i].w) & 0x80808080u) {  // scales have no sign here: it goes to the block's values
-          ok = ok && tc_wait(w_full(w.slot), w.lap, P.status);
-          const uint32_t sc[4] = {q[i].x, q[i].y, q[i].z, q[i].w};
-          uint8_t* box = smem + static_cast<size_t>(w.slot) * box_bytes + r * 128;
-          for (int b = 0; b < 16 && ok && r < P.R; ++b)
-            if (sc[b >> 2] >> (8 * (b & 3)) & 0x80u) {
-              uint2* at = reinterpret_cast<uint2*>(box + (((b >> 1) ^ (r & 7)) << 4) + 8 * (b & 1));
-              *at = make_uint2(at->x ^ 0x88888888u, at->y ^ 0x88888888u);
-            }
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor core reads what this thread wrote
-        }
-        uint4* rows = reinterpret_cast<uint4*>(sring) + (i & 1) * 128;  // (two stages in turn: one meeting per stage is enough)
-        rows[r] = make_uint4(q[i].x & 0x7f7f7f7fu, q[i].y & 0x7f7f7f7fu, q[i].z & 0x7f7f7f7fu, q[i].w & 0x7f7f7f7fu);
-        load(q[i]);
-        __syncwarp();
-        named_bar_sync(1, 128);
-        uint32_t v[16];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const uint4 u = rows[32 * c + lane];
-          v[c] = u.x, v[4 + c] = u.y, v[8 + c] = u.z, v[12 + c] = u.w;
-        }
-        // the activations' scales lie behind their digits as the four words of each lane and product
-        ok = ok && tc_wait(x_full(x.slot), x.lap, P.status);
-        const uint4* xsf = reinterpret_cast<const uint4*>(xring + static_cast<size_t>(x.slot) * x_bytes + P.sf_off) + lane;
-        uint32_t xv[ATOMS][16];
-#pragma unroll
-        for (int j = 0; j < 4 * ATOMS; ++j) {
-          const uint4 u = xsf[32 * j];
-          uint32_t* to = xv[j / 4] + 4 * (j % 4);
-          to[0] = u.x, to[1] = u.y, to[2] = u.z, to[3] = u.w;
-        }
-        if (use > 0 && ok) ok = tc_wait(s_empty(turn), (use - 1) & 1, P.status);
-        ok = __all_sync(0xffffffffu, ok);
-        if (ok) {
-          const uint32_t at = lane_addr + turn * kSfCols;
-          tc_fence_after();
-          tmem_st16(at, v);
-#pragma unroll
-          for (int a = 0; a < ATOMS; ++a) tmem_st16(at + 16 + 16 * a, xv[a]);
-          tmem_wait_st();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(s_full(turn));
-        }
-        x.advance(SX);
-        w.advance(SW);
+    uint32_t count = 0;  // stages so far
+    const uint32_t sf_mask = P.sf_stages - 1, sf_shift = P.sf_stages == 4 ? 2 : P.sf_stages == 2 ? 1 : 0;
+    // One stage: this thread's scales s to the tensor core; `fetch` asks for the ones that come later. (A warp whose wait gave up still
+    // comes to the meetings.)
+    auto stage = [&](uint4& s, auto&& fetch) __attribute__((always_inline)) {
+      const uint32_t turn = count & sf_mask, use = count >> sf_shift;
+      if ((s.x | s.y | s.z | s.w) & 0x80808080u) {  // scales have no sign here: it goes to the block's values
+        ok = ok && tc_wait(w_full(w.slot), w.lap, P.status);
+        const uint32_t sc[4] = {s.x, s.y, s.z, s.w};
+        uint8_t* box = smem + static_cast<size_t>(w.slot) * box_bytes + r * 128;
+        for (int b = 0; b < 16 && ok && r < P.R; ++b)
+          if (sc[b >> 2] >> (8 * (b & 3)) & 0x80u) {
+            uint2* at = reinterpret_cast<uint2*>(box + (((b >> 1) ^ (r & 7)) << 4) + 8 * (b & 1));
+            *at = make_uint2(at->x ^ 0x88888888u, at->y ^ 0x88888888u);
+          }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor core reads what this thread wrote
       }
+      uint4* rows = reinterpret_cast<uint4*>(sring) + (count & 1) * 128;  // (two stages in turn: one meeting per stage is enough)
+      rows[r] = make_uint4(s.x & 0x7f7f7f7fu, s.y & 0x7f7f7f7fu, s.z & 0x7f7f7f7fu, s.w & 0x7f7f7f7fu);
+      fetch(s);
+      __syncwarp();
+      named_bar_sync(1, 128);
+      uint32_t v[16];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const uint4 u = rows[32 * c + lane];
+        v[c] = u.x, v[4 + c] = u.y, v[8 + c] = u.z, v[12 + c] = u.w;
+      }
+      // the activations' scales lie behind their digits as the four words of each lane and product
+      ok = ok && tc_wait(x_full(x.slot), x.lap, P.status);
+      const uint4* xsf = reinterpret_cast<const uint4*>(xring + static_cast<size_t>(x.slot) * x_bytes + P.sf_off) + lane;
+      uint32_t xv[ATOMS][16];
+#pragma unroll
+      for (int j = 0; j < 4 * ATOMS; ++j) {
+        const uint4 u = xsf[32 * j];
+        uint32_t* to = xv[j / 4] + 4 * (j % 4);
+        to[0] = u.x, to[1] = u.y, to[2] = u.z, to[3] = u.w;
+      }
+      if (use > 0 && ok) ok = tc_wait(s_empty(turn), (use - 1) & 1, P.status);
+      ok = __all_sync(0xffffffffu, ok);
+      if (ok) {
+        const uint32_t at = lane_addr + turn * kSfCols;
+        tc_fence_after();
+        tmem_st16(at, v);
+#pragma unroll
+        for (int a = 0; a < ATOMS; ++a) tmem_st16(at + 16 + 16 * a, xv[a]);
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(s_full(turn));
+      }
+      x.advance(SX);
+      w.advance(SW);
+      ++count;
+    };
+    for (int tile = tile_begin; tile < tile_end; ++tile) {
+      const bool turns = chunk + 1 == chunks;
+      const uint4* const scales_next = tile + 1 >= tile_end ? nullptr : turns ? scales_of(panel + 1) : scales;
+      const uint8_t* const bits = again + chunk * groups;
+      for (int s0 = 0; s0 < n_stages; s0 += kAhead) {
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+          if (s0 + i >= n_stages) break;
+          stage(q[i], [&](uint4& s) {  // stage s0 + i + kAhead, or stage i of the next tile
+            const bool here = s0 + i + kAhead < n_stages;
+            const uint4* from = here ? scales : scales_next;
+            if (from) s = __ldg(from + (here ? s0 + i + kAhead : i));
+          });
+        }
+      }
+      if (!named_bar_and(1, 128, tc_wait(a_full, 0, P.status))) break;  // all four warps leave together
+      int a = again_after(bits, n_stages, -1);  // the stage that goes again next: its scales are asked for a stage ahead
+      uint4 ahead = a < n_stages && scales ? __ldg(scales + a) : make_uint4(0, 0, 0, 0);
+      while (a < n_stages) {
+        uint4 now = ahead;
+        a = again_after(bits, n_stages, a);
+        stage(now, [&](uint4&) {
+          if (a < n_stages && scales) ahead = __ldg(scales + a);
+        });
+      }
+      scales = scales_next;
+      panel += turns, chunk = turns ? 0 : chunk + 1;
     }
   } else {
     // ================================ epilogue ================================
     const int r = tid;
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
     pdl_wait();  // y and the activation scales come from earlier kernels
+    for (int i = tid; i < chunks * groups; i += 128) {
+      const uint4* rows64 = reinterpret_cast<const uint4*>(P.again + static_cast<int64_t>(i) * kMaxRows);
+      const int rows = min(P.chunk_rows, P.M - i / groups * P.chunk_rows);
+      uint32_t any = 0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint4 u = rows64[q];
+        const uint32_t four[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int z = 0; z < 4; ++z) {
+          const int left = rows - 16 * q - 4 * z;  // rows among these four
+          any |= left >= 4 ? four[z] : left > 0 ? four[z] & ((1u << (8 * left)) - 1u) : 0u;
+        }
+      }
+      any |= any >> 16;
+      again[i] = static_cast<uint8_t>(any | (any >> 8));
+    }
+    mbar_arrive(a_full);
     for (int tile = tile_begin, t = 0; tile < tile_end; ++tile, ++t) {
       const int buf = P.buffers == 2 ? t & 1 : 0, use = P.buffers == 2 ? t >> 1 : t;
       const int panel = tile / chunks, m0 = (tile - panel * chunks) * P.chunk_rows, rows = min(P.chunk_rows, P.M - m0);
@@ -453,9 +600,12 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
         for (int i = 0; i < 8; ++i) {
           const float inv = __shfl_sync(0xffffffffu, c < 32 ? inv_lo : inv_hi, (c + i) & 31);
           if (!live || c + i >= rows) continue;
-          float sum = __uint_as_float(raw[kMxDigits - 1][i]);
+          float sum = __uint_as_float(raw[kMxDigits - 1][i]), power = 1.0f;  // least first: the first digit's sum is rounded once
 #pragma unroll
-          for (int j = kMxDigits - 2; j >= 0; --j) sum = fmaf(sum, 0.125f, __uint_as_float(raw[j][i]));
+          for (int j = kMxDigits - 2; j >= 0; --j) {
+            power *= kMxBase;
+            sum = fmaf(__uint_as_float(raw[j][i]), power, sum);
+          }
           float out = P.alpha * (P.global * (sum * inv) + bias);
           const int64_t at = static_cast<int64_t>(m0 + c + i) * P.ld_y + n;
           if (P.beta != 0.0f) out = fmaf(P.beta, old[i], out);
@@ -501,7 +651,8 @@ int64_t mx_workspace_bytes(int M, int K) {
     if (rows == 0) continue;
     const int chunk = mx_chunk_rows(rows);
     const MxLayout L(chunk);
-    need = std::max(need, static_cast<int64_t>((rows + chunk - 1) / chunk) * ((K + kMxStageK - 1) / kMxStageK) * L.x_bytes + 4 * rows + 256);
+    const int stages = (K + kMxStageK - 1) / kMxStageK;
+    need = std::max(need, static_cast<int64_t>((rows + chunk - 1) / chunk) * (int64_t{2} * stages * L.x_bytes + (stages + 7) / 8 * kMaxRows) + 4 * rows + 256);
   }
   return need;
 }
@@ -542,23 +693,28 @@ int mx_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const v
     P.sf_stages = cols + 4 * sf_cols <= kTmemColumns ? 4 : cols + 2 * sf_cols <= kTmemColumns ? 2 : 1;
     P.sf0 = kTmemColumns - P.sf_stages * sf_cols;
     P.buffers = 2 * cols <= P.sf0 ? 2 : 1;
-    float* row_scale = reinterpret_cast<float*>(ws + P.chunks * P.chunk_bytes);
+    P.remainders = P.chunks * P.chunk_bytes;
+    P.groups = (K / kMxStageK + 7) / 8;
+    uint8_t* again = ws + 2 * P.remainders;
+    P.again = again;
+    float* row_scale = reinterpret_cast<float*>(again + static_cast<int64_t>(P.chunks) * P.groups * kMaxRows);
     P.row_scale = row_scale;
     P.y = static_cast<uint8_t*>(y) + static_cast<int64_t>(first) * ld_y * (y_dtype == LX_BF16 ? 2 : 4);
     const void* xrow = static_cast<const uint8_t*>(x) + static_cast<int64_t>(first) * ld_x * (x_bf16 ? 2 : 4);
     alignas(64) CUtensorMap wmap;
     if (int e = make_tile_map(&wmap, w.data, K / 2, N, 128, P.R, 4, true)) return e;
-    if (int e = launch_kernel(x_bf16 ? mx_prep_kernel<true> : mx_prep_kernel<false>, dim3((K / 8 + kPrepThreads - 1) / kPrepThreads, P.M), dim3(kPrepThreads), 0, stream, xrow, ld_x, K,
-                              P.chunk_rows, P.chunk_bytes, L.Mp, L.cols0, L.cols1, L.x_bytes, L.sf_off, ws, row_scale))
+    if (int e = launch_kernel(x_bf16 ? mx_prep_kernel<true> : mx_prep_kernel<false>, dim3(P.groups, P.M), dim3(kPrepThreads), 0, stream, xrow, ld_x, K,
+                              P.chunk_rows, P.chunk_bytes, L.Mp, L.cols0, L.cols1, L.x_bytes, L.sf_off, ws, P.remainders, again, row_scale))
       return e;
     // A ring of as many stages of activations as of weights: a block of them, the same for every SM, travels as long as the weights
     // do. Where that is fewer than four, the weights keep six.
-    constexpr int kRoom = 224 * 1024 - 1024 - kMxScaleBytes;
-    const int even = kRoom / (P.box_bytes + L.x_bytes);
-    P.SX = even >= 4 ? std::min(8, even) : std::max(2, std::min(4, (kRoom - 6 * P.box_bytes) / L.x_bytes));
-    P.SW = std::min(12, (kRoom - P.SX * L.x_bytes) / P.box_bytes);
+    const int tail = std::max(1024, 448 + P.chunks * P.groups);  // barriers, and the stages that go again
+    const int room = 224 * 1024 - kMxScaleBytes - tail;
+    const int even = room / (P.box_bytes + L.x_bytes);
+    P.SX = even >= 4 ? std::min(8, even) : std::max(2, std::min(4, (room - 6 * P.box_bytes) / L.x_bytes));
+    P.SW = std::min(12, (room - P.SX * L.x_bytes) / P.box_bytes);
     if (P.SW < 2) return kNotSupported;
-    const size_t smem = std::max<size_t>(static_cast<size_t>(P.SW) * P.box_bytes + kMxScaleBytes + static_cast<size_t>(P.SX) * L.x_bytes + 1024, 120 * 1024);
+    const size_t smem = std::max<size_t>(static_cast<size_t>(P.SW) * P.box_bytes + kMxScaleBytes + static_cast<size_t>(P.SX) * L.x_bytes + tail, 120 * 1024);
     const bool two_atoms = L.cols0 > 128;
     auto kernel = !two_atoms ? tc_mx_kernel<1, false> : L.cols1 ? tc_mx_kernel<2, true> : tc_mx_kernel<2, false>;
     if (int e = !two_atoms ? allow_big_smem<300>(kernel) : L.cols1 ? allow_big_smem<301>(kernel) : allow_big_smem<302>(kernel)) return e;

@@ -1,10 +1,9 @@
-"""lx_gemm_w on NVFP4 weights (weights multiplied as stored, activations as base-8 digits): against 64-bit sums at the edges of its
+"""lx_gemm_w on NVFP4 weights (weights multiplied as stored, activations as base-13 digits): against 64-bit sums at the edges of its
 layouts (digit columns in one instruction or two, chunks of 64 rows, launches of 1024, weight panels, 256 values of K), rows that
-do not depend on the call they come in, and the values that have no digits.
+do not depend on the call they come in, small values beside large ones, and the values that have no digits.
 
-Bound: a value keeps 21 bits below its block's largest magnitude (2^-21 of it at most is dropped, ~2^-20 of a typical value),
-products and sums of digits are exact or f32, seven sums are put together with one f32 rounding each: 1e-6 leaves a factor of
-four."""
+Bound: digits and remainders hold a value exactly, or within 2^-41 of its row's largest; products of digits are exact, their sums
+f32, and seven sums are put together with one f32 rounding each (the last at full size): 1e-6 leaves a factor of four."""
 
 import ctypes
 
@@ -99,3 +98,45 @@ def test_scales_with_a_sign(lx):
     x = torch.randn((M, K), generator=gen, device="cuda").to(torch.bfloat16)
     want = x.double() @ values(sw.data, sw.scale, sw.glob, N, K).T
     assert float((product(lx, x, sw, M, N, K).double() - want).norm() / want.norm()) <= 1e-6
+
+
+@pytest.mark.parametrize("M,N,K", [(3, 200, 512), (16, 300, 4096), (40, 130, 1024), (64, 97, 2560), (130, 300, 2048)])
+@pytest.mark.parametrize("every", [True, False], ids=["every-block", "one"])
+@pytest.mark.parametrize("factor", [64, 256, 1024, 4096, 2**13, 2**15, 2**20])
+def test_small_values_beside_outliers(lx, M, N, K, every, factor):
+    """Outputs whose weights are zero wherever the row has an outlier: what is left of the sum is as exact as any other. (Values of 0.05
+    beside 0.05 * 2^20: 2^-41 of the outlier is 2^-21 of such a value, and few are rounded at all.) The other outputs are the
+    outlier's product with thousands of small ones added to it: each of the K / 64 sums may be cut off at 2^-23 of it."""
+    gen = torch.Generator(device="cuda").manual_seed(factor + M)
+    sw = weight(lx, N, K, gen)
+    at = torch.arange(5, K, 16, device="cuda") if every else torch.tensor([K // 2 + 11], device="cuda")
+    rows = torch.arange(0, M, 2, device="cuda")  # plain rows stand beside them
+    x = torch.randn((M, K), generator=gen, device="cuda") * 0.05
+    x[rows[:, None], at[None, :]] *= factor
+    x = x.to(torch.bfloat16)
+    sw.data.view(N, K // 2)[: N // 2, at // 2] &= 0x0F  # (at is odd: the high half of its byte)
+    y = product(lx, x, sw, M, N, K)
+    want = x.double() @ values(sw.data, sw.scale, sw.glob, N, K).T
+    for part, bound in ((slice(0, N // 2), 1e-6), (slice(N // 2, N), 1e-6 + K // 64 * 2.0**-23)):
+        assert float(((y[:, part].double() - want[:, part]).norm(dim=1) / want[:, part].norm(dim=1)).max()) <= bound
+    for m in {0, 1, M - 1}:
+        assert torch.equal(product(lx, x[m:m + 1], sw, 1, N, K)[0], y[m])
+
+
+def test_one_value_of_any_size(lx):
+    """Weights that pick one activation each: 2^-33 of the row's largest and above come out as they are."""
+    M, K = 16, 512
+    N = K
+    sw = weight(lx, N, K, torch.Generator(device="cuda").manual_seed(5))
+    eye = torch.zeros((N, K // 2), dtype=torch.uint8, device="cuda")
+    k = torch.arange(K, device="cuda")
+    eye[k, k // 2] = torch.where(k % 2 == 0, 2, 0x20).to(torch.uint8)  # code 2 is 1.0
+    sw.data.copy_(eye.view(-1).view(sw.data.dtype).view(sw.data.shape))
+    sw.scale.view(torch.uint8).fill_(0x38)  # 1.0
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    x = torch.randn((M, K), generator=gen, device="cuda") * torch.exp2(-torch.randint(0, 31, (M, K), generator=gen, device="cuda").float())
+    x = x.to(torch.bfloat16)
+    x[:, 7] = 3.5
+    x = torch.where(x.abs() < 2.0**-31, torch.zeros_like(x), x)  # 2^-33 of 2 .. 4
+    y = product(lx, x, sw, M, N, K)
+    assert torch.equal(y / sw.glob, (x.double() * sw.glob).float() / sw.glob)
