@@ -57,6 +57,9 @@ constexpr int kMxScaleBytes = 2 * 128 * 16;     // shared memory in which the sc
 constexpr int kAhead = 8;                       // stages whose weight scales a thread has in flight
 
 struct MxParams {
+  const void* x;            // the activations themselves, for rows with infinities
+  int x_bf16, ld_x;
+  const uint8_t* w;         // e2m1 [N, K / 2]
   const uint8_t* scale;     // e4m3 [N, K / 16]
   float global;
   int N, K, M;
@@ -133,15 +136,13 @@ __device__ __forceinline__ void put_digits(int q, int i, const uint16_t* pairs, 
 __device__ __forceinline__ uint32_t ue4m3_pow2(int e) { return e >= -6 ? static_cast<uint32_t>(e + 7) << 3 : 1u << (e + 9); }
 // 2^e as f32, e in -149..127.
 __device__ __forceinline__ float exp2_of(int e) { return __uint_as_float(e >= -126 ? static_cast<uint32_t>(e + 127) << 23 : 1u << (e + 149)); }
-constexpr int kFirstDigit = 4 * 4826809;  // 4 * 13^6: the first digit alone
 
 // Block (piece, row): 256 threads, each 8 values (half a scale block) of an activation row; every block finds the row's largest
 // magnitude again (a few KB, from L2), which saves a second kernel. (With 32 values per thread the seven digits of each were
 // ~1400 instructions in a row: at 16 rows the preparation took as long as an eighth of the product.) A warp's values are one
 // stage's, a block's eight stages': their bits are one byte of `again`. A block without remainders gets the scale zero there, which
 // makes whatever its digits are zero.
-// Rows that are not finite: a NaN, or more than one infinity, makes the row's outputs NaN; with a single infinity the finite
-// values do not count and the outputs are the infinity times its weight (NaN where that is zero).
+// A row with a NaN has NaN outputs; one with infinities has no digits, and -0 as its scale: the epilogue adds its infinities up.
 constexpr int kPrepThreads = 256;  // (at most 40 registers each: a block fits beside the product's CTA and starts under its end. With 48,
                                    // and 140 in the product, it did not: 14336 x 4096 at 32 rows 23 us instead of 19)
 template <bool XBF>
@@ -149,7 +150,7 @@ __global__ void __launch_bounds__(kPrepThreads, 6) mx_prep_kernel(const void* __
                                                                int cols1, int x_bytes, int sf_off, uint8_t* __restrict__ out, int64_t remainders,
                                                                uint8_t* __restrict__ again, float* __restrict__ row_scale) {
   pdl_trigger();
-  __shared__ uint32_t part[kPrepThreads / 32], infinities, stages_again;
+  __shared__ uint32_t part[kPrepThreads / 32], stages_again;
   __shared__ uint16_t pairs[kMxBase * kMxBase];
   if (threadIdx.x < kMxBase * kMxBase) pairs[threadIdx.x] = static_cast<uint16_t>(digit_pair(threadIdx.x));
   pdl_wait();  // the kernel before this one may still be reading the workspace
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(kPrepThreads, 6) mx_prep_kernel(const void* __
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
   if ((tid & 31) == 0) part[tid >> 5] = top;
-  if (tid == 0) infinities = stages_again = 0;
+  if (tid == 0) stages_again = 0;
   uint32_t block_top = max_magnitude(0, v);
   block_top = max(block_top, __shfl_xor_sync(0xffffffffu, block_top, 1));
   __syncthreads();
@@ -172,38 +173,24 @@ __global__ void __launch_bounds__(kPrepThreads, 6) mx_prep_kernel(const void* __
 #pragma unroll
   for (int i = 0; i < kPrepThreads / 32; ++i) top = max(top, part[i]);
   const bool finite = top < 0x7f80u;
-  if (!finite) {
-    uint32_t n = 0;
-    for (int k = tid; k < K; k += kPrepThreads) n += (bf16_at<XBF>(x, row + k) & 0x7fffu) == 0x7f80u;
-    atomicAdd(&infinities, n);
-    __syncthreads();
-  }
   const int e_row = max(static_cast<int>(top >> 7), 30) - 127;
   if (blockIdx.x == 0 && tid == 0)
-    row_scale[row_id] = finite ? exp2_of(e_row - 7 - kMxUnit) : __uint_as_float(top == 0x7f80u && infinities == 1 ? 0x7f800000u : 0x7fc00000u);
+    row_scale[row_id] = finite ? exp2_of(e_row - 7 - kMxUnit) : __uint_as_float(top == 0x7f80u ? 0x80000000u : 0x7fc00000u);
   // The block's exponent; one less for a largest value below 1.25 * 2^e, which the digits still hold. 2^-9 is the least scale.
   const int e = max(max(static_cast<int>(block_top + 96) >> 7, 2) - 128, e_row - 17);
   // 2^(kMxUnit - e) in two factors: the whole can be beyond f32
   const int half = (kMxUnit - e) / 2;
   const float f0 = exp2_of(half), f1 = exp2_of(kMxUnit - e - half), to_least = exp2_of(e - e_row + 17);
-  const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+  const uint32_t keep = finite ? ~0u : 0u, words[4] = {v.x & keep, v.y & keep, v.z & keep, v.w & keep};
   uint32_t w[kMxDigits] = {};
-  int rest[8];  // what the digits leave, in units of the least scale: up to 2^16
   bool some = false;
+  auto value_of = [&](int i) { return bf16_bits_to_f32((words[i / 2] >> (16 * (i & 1))) & 0xffffu) * f0 * f1; };
+  auto rest_of = [&](float t) { return __float2int_rn((t - rintf(t)) * to_least); };  // what the digits leave, in units of the least scale: up to 2^16
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const uint32_t bits = (words[i / 2] >> (16 * (i & 1))) & 0xffffu;
-    int q;
-    if (finite) {
-      const float t = bf16_bits_to_f32(bits) * f0 * f1, r = rintf(t);
-      q = static_cast<int>(r);
-      rest[i] = __float2int_rn((t - r) * to_least);
-      some |= rest[i] != 0;
-    } else {
-      q = (bits & 0x7fffu) != 0x7f80u ? 0 : bits & 0x8000u ? -kFirstDigit : kFirstDigit;
-      rest[i] = 0;
-    }
-    put_digits(q, i, pairs, w);
+    const float t = value_of(i);
+    some |= rest_of(t) != 0;
+    put_digits(__float2int_rn(t), i, pairs, w);
   }
   const uint32_t with_rest = __ballot_sync(0xffffffffu, some);
   if (with_rest && (tid & 31) == 0) atomicOr(&stages_again, 1u << (tid >> 5));
@@ -221,13 +208,13 @@ __global__ void __launch_bounds__(kPrepThreads, 6) mx_prep_kernel(const void* __
     // scale every product cut off the sums of the digits above: 2.5e-6 at K = 4096 with an outlier in every block, now 6e-8.)
     uint32_t bits = 0;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) bits |= static_cast<uint32_t>(rest[i]);
+    for (int i = 0; i < 8; ++i) bits |= static_cast<uint32_t>(rest_of(value_of(i)));
     bits |= __shfl_xor_sync(0xffffffffu, bits, 1);
     if (block_rest) {
       zeros = __ffs(static_cast<int>(bits)) - 1;
       uint32_t d[kMxDigits] = {};
 #pragma unroll
-      for (int i = 0; i < 8; ++i) put_digits(rest[i] >> zeros, i, pairs, d);
+      for (int i = 0; i < 8; ++i) put_digits(rest_of(value_of(i)) >> zeros, i, pairs, d);
 #pragma unroll
       for (int j = 0; j < kMxDigits; ++j) *reinterpret_cast<uint32_t*>(stage + remainders + block_offset(NC, kb & ~15, j * Mp + m) + (kb & 15)) = d[j];
     }
@@ -280,6 +267,17 @@ __device__ __forceinline__ void mx_umma(uint32_t d_tmem, uint32_t a_lo, uint32_t
       "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], da, db, %5, [%6], [%7], p; }" ::"r"(d_tmem),
       "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate)
       : "memory");
+}
+
+// What a row with infinities gives under a weight row: the sum of the infinities' products, an infinity or NaN as IEEE has it (the
+// finite values next to them do not count). No one's hot path: one thread, all of K.
+__device__ __noinline__ float infinite_sum(const void* x, int x_bf16, const uint8_t* w, const uint8_t* scale, int K) {
+  float sum = 0.0f;
+  for (int k = 0; k < K; ++k) {
+    const uint32_t bits = x_bf16 ? bf16_at<true>(x, k) : bf16_at<false>(x, k);
+    if ((bits & 0x7fffu) == 0x7f80u) sum += bf16_bits_to_f32(bits) * (e2m1_to_f32(w[k >> 1] >> (4 * (k & 1)) & 15u) * e4m3_to_f32(scale[k >> 4]));
+  }
+  return sum;
 }
 
 // ---- the product -------------------------------------------------------------------------------------------------------------
@@ -615,6 +613,16 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(d_empty(buf));
+      // Rows with infinities: what is stored is all but their sum (NaN already if a scale is). (Left out of the stores above instead,
+      // by a test of every output, they cost 1000 rows of 14336 x 4096 12 of 267 us.)
+      auto infinite = [&](float inv) { return __ballot_sync(0xffffffffu, __float_as_uint(inv) == 0x80000000u); };
+      uint64_t left = infinite(inv_lo) | static_cast<uint64_t>(infinite(inv_hi)) << 32;
+      for (; left; left &= left - 1) {
+        if (!live) continue;
+        const int64_t m = m0 + __ffsll(static_cast<long long>(left)) - 1, n64 = n, at = m * P.ld_y + n;
+        const float sum = infinite_sum(static_cast<const uint8_t*>(P.x) + m * P.ld_x * (P.x_bf16 ? 2 : 4), P.x_bf16, P.w + n64 * (P.K / 2), P.scale + n64 * (P.K / 16), P.K);
+        store_from_f32(P.y, P.y_dtype, at, load_f32(P.y, P.y_dtype, at) + P.alpha * (P.global * sum));
+      }
     }
   }
   __syncthreads();
@@ -667,6 +675,8 @@ int mx_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const v
   if (!sms) return kInvalid;
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   MxParams P{};
+  P.x_bf16 = x_bf16, P.ld_x = ld_x;
+  P.w = static_cast<const uint8_t*>(w.data);
   P.scale = static_cast<const uint8_t*>(w.scale);
   P.global = w.global;
   P.N = N, P.K = K;
@@ -701,6 +711,7 @@ int mx_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const v
     P.row_scale = row_scale;
     P.y = static_cast<uint8_t*>(y) + static_cast<int64_t>(first) * ld_y * (y_dtype == LX_BF16 ? 2 : 4);
     const void* xrow = static_cast<const uint8_t*>(x) + static_cast<int64_t>(first) * ld_x * (x_bf16 ? 2 : 4);
+    P.x = xrow;
     alignas(64) CUtensorMap wmap;
     if (int e = make_tile_map(&wmap, w.data, K / 2, N, 128, P.R, 4, true)) return e;
     if (int e = launch_kernel(x_bf16 ? mx_prep_kernel<true> : mx_prep_kernel<false>, dim3(P.groups, P.M), dim3(kPrepThreads), 0, stream, xrow, ld_x, K,

@@ -140,3 +140,33 @@ def test_one_value_of_any_size(lx):
     x = torch.where(x.abs() < 2.0**-31, torch.zeros_like(x), x)  # 2^-33 of 2 .. 4
     y = product(lx, x, sw, M, N, K)
     assert torch.equal(y / sw.glob, (x.double() * sw.glob).float() / sw.glob)
+
+
+@pytest.mark.parametrize("M,K,x_f32", [(16, 512, False), (16, 512, True), (70, 2048, False), (1100, 256, True)])
+def test_rows_with_infinities(lx, M, K, x_f32):
+    """Any number of infinities: an infinity where all their products agree in sign, NaN where they do not or a weight is zero."""
+    N = 150
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    sw = weight(lx, N, K, gen)
+    x = torch.randn((M, K), generator=gen, device="cuda")
+    inf = float("inf")
+    x[1, 7], x[1, 200] = inf, inf
+    x[2, 3], x[2, 40] = inf, -inf
+    x[3, 5], x[3, 6], x[3, K - 1] = -inf, -inf, -inf
+    x[M - 1] = inf
+    x[M - 2, K - 1], x[M - 2, 0] = inf, 3.4e38 if x_f32 else inf  # (the largest f32 values are infinite in bf16)
+    x[M - 3, 9], x[M - 3, 10] = inf, float("nan")
+    x = x if x_f32 else x.to(torch.bfloat16)
+    y = product(lx, x, sw, M, N, K).double()
+    finite = torch.isfinite(x.to(torch.bfloat16)).all(dim=1)
+    w64 = values(sw.data, sw.scale, sw.glob, N, K)
+    want = torch.where(torch.isfinite(x.to(torch.bfloat16)), 0.0, x.to(torch.bfloat16).double())[~finite] @ w64.T
+    got = y[~finite]
+    assert torch.equal(torch.nan_to_num(got, nan=0.5, posinf=1, neginf=-1), torch.nan_to_num(want, nan=0.5, posinf=1, neginf=-1))
+    assert bool(torch.isinf(got[0]).any()) and bool(torch.isnan(got[0]).any())
+    plain = x[finite].to(torch.bfloat16).double() @ w64.T
+    assert float((y[finite] - plain).norm() / plain.norm()) <= 1e-6
+    # with everything an epilogue adds, in bf16
+    old, bias = torch.randn((M, N), generator=gen, device="cuda").to(torch.bfloat16), torch.randn((N,), generator=gen, device="cuda")
+    y = product(lx, x, sw, M, N, K, 0.75, old.clone(), bias, -0.5)[~finite].double()
+    assert torch.equal(torch.nan_to_num(y, nan=0.5, posinf=1, neginf=-1), torch.nan_to_num(-want, nan=0.5, posinf=1, neginf=-1))
