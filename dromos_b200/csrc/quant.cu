@@ -178,56 +178,55 @@ __global__ void __launch_bounds__(kBlock) quantize_nvfp4_kernel(const uint16_t* 
   }
 }
 
-// out[n, k] = bf16(element * row factor). VEC: one warp per row, eight values per lane and step (cols % 8 == 0, out on 16,
-// the elements on 8 bytes, NVFP4's on 4); else one thread per element.
-template <int F, bool VEC>
+// out[n, k] = bf16(element * row factor). WORDS > 0 (cols % 8 == 0, out on 16, the elements on 8 bytes, NVFP4's on 4): eight values per
+// lane and word, a warp takes WORDS words of 32 lanes of one row, the pieces of a row one after the other; 0: one thread per element.
+template <int F, int WORDS>
 __global__ void __launch_bounds__(kBlock) dequantize_kernel(const uint8_t* __restrict__ data, const uint8_t* __restrict__ scale,
-                                                            float global, uint16_t* __restrict__ out, int64_t rows, int cols) {
+                                                            float global, uint16_t* __restrict__ out, int64_t rows, int cols, unsigned pieces) {
   // no early trigger: what this kernel writes may be the weight of the next product, whose kernels read weights
   // before their own wait
   pdl_wait();
-  if constexpr (VEC) {
-    const int64_t row = static_cast<int64_t>(blockIdx.x) * kRowWarps + (threadIdx.x >> 5);
+  if constexpr (WORDS > 0) {
+    const unsigned group = blockIdx.x / pieces, piece = blockIdx.x - group * pieces;
+    const int64_t row = static_cast<int64_t>(group) * kRowWarps + (threadIdx.x >> 5);
     if (row >= rows) return;
-    const int lane = threadIdx.x & 31, words = cols / 8;
+    const int words = cols / 8, c0 = static_cast<int>(piece) * 32 * WORDS + static_cast<int>(threadIdx.x & 31);
     uint4* dst = reinterpret_cast<uint4*>(out + row * cols);
     float rf = 1.0f;
     if constexpr (F != LX_W_NVFP4) rf = reinterpret_cast<const float*>(scale)[row];
-    for (int c0 = lane; c0 < words; c0 += 32 * kInFlight) {
-      uint2 e[kInFlight];
-      uint32_t sb[kInFlight];
+    uint2 e[WORDS];
+    uint32_t sb[WORDS];
 #pragma unroll
-      for (int i = 0; i < kInFlight; ++i) {
-        const int c = c0 + 32 * i;
-        if (c >= words) continue;
-        if constexpr (F == LX_W_NVFP4) {
-          e[i].x = __ldg(reinterpret_cast<const uint32_t*>(data + row * (cols / 2)) + c);
-          sb[i] = __ldg(scale + row * (cols / 16) + c / 2);
-        } else {
-          e[i] = __ldg(reinterpret_cast<const uint2*>(data + row * cols) + c);
+    for (int i = 0; i < WORDS; ++i) {
+      const int c = c0 + 32 * i;
+      if (c >= words) continue;
+      if constexpr (F == LX_W_NVFP4) {
+        e[i].x = __ldg(reinterpret_cast<const uint32_t*>(data + row * (cols / 2)) + c);
+        sb[i] = __ldg(scale + row * (cols / 16) + c / 2);
+      } else {
+        e[i] = __ldg(reinterpret_cast<const uint2*>(data + row * cols) + c);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < WORDS; ++i) {
+      const int c = c0 + 32 * i;
+      if (c >= words) continue;
+      float v[8];
+      if constexpr (F == LX_W_NVFP4) {
+        const float f = e4m3_to_f32(sb[i]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = e2m1_to_f32((e[i].x >> (4 * j)) & 15u) * f * global;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const uint32_t b = ((j < 4 ? e[i].x : e[i].y) >> (8 * (j & 3))) & 0xffu;
+          v[j] = (F == LX_W_INT8 ? static_cast<float>(static_cast<int8_t>(b)) : e4m3_to_f32(b)) * rf;
         }
       }
+      uint32_t o[4];
 #pragma unroll
-      for (int i = 0; i < kInFlight; ++i) {
-        const int c = c0 + 32 * i;
-        if (c >= words) continue;
-        float v[8];
-        if constexpr (F == LX_W_NVFP4) {
-          const float f = e4m3_to_f32(sb[i]);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = e2m1_to_f32((e[i].x >> (4 * j)) & 15u) * f * global;
-        } else {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const uint32_t b = ((j < 4 ? e[i].x : e[i].y) >> (8 * (j & 3))) & 0xffu;
-            v[j] = (F == LX_W_INT8 ? static_cast<float>(static_cast<int8_t>(b)) : e4m3_to_f32(b)) * rf;
-          }
-        }
-        uint32_t o[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) o[j] = (f32_to_bf16_bits(v[2 * j]) & 0xffffu) | (f32_to_bf16_bits(v[2 * j + 1]) << 16);
-        dst[c] = make_uint4(o[0], o[1], o[2], o[3]);
-      }
+      for (int j = 0; j < 4; ++j) o[j] = (f32_to_bf16_bits(v[2 * j]) & 0xffffu) | (f32_to_bf16_bits(v[2 * j + 1]) << 16);
+      dst[c] = make_uint4(o[0], o[1], o[2], o[3]);
     }
     return;
   }
@@ -314,13 +313,23 @@ int launch_rows(const void* w, uint8_t* q, float* scale, int64_t rows, int cols,
                        static_cast<const uint16_t*>(w), q, scale, rows, cols);
 }
 
+template <int F, int WORDS>
+int launch_dequantize_words(const lx_weight& w, float global, uint16_t* out, int64_t rows, int cols, cudaStream_t s) {
+  const unsigned pieces = WORDS ? blocks_for(cols, 256 * std::max(1, WORDS)) : 1;
+  const unsigned grid = WORDS ? blocks_for(rows, kRowWarps) * pieces : blocks_for(rows * cols, kBlock);
+  return launch_kernel(dequantize_kernel<F, WORDS>, dim3(grid), dim3(kBlock), 0, s, static_cast<const uint8_t*>(w.data), static_cast<const uint8_t*>(w.scale), global, out, rows, cols, pieces);
+}
+
+// A row's values are spread over as many warps as they fill, four words a lane (14336 x 4096: FP8 27.6 us, one warp per row 30.3, one
+// thread per value 169); where that is fewer than four blocks per SM, or a row is no longer than one word a lane, one word a lane. (One warp per
+// row leaves few wide rows to few SMs: FP8 64 x 16384 11.1 us, 1 x 65536 32; now 1.7 and 1.2; one thread per value 3.2 and 1.2.
+// 100000 x 256 with one word a lane 14, with four 15.6.)
 template <int F>
 int launch_dequantize(const lx_weight& w, float global, uint16_t* out, int64_t rows, int cols, cudaStream_t s) {
-  const auto* data = static_cast<const uint8_t*>(w.data);
-  const auto* scale = static_cast<const uint8_t*>(w.scale);
-  if (cols % 8 == 0 && aligned(out, 16) && aligned(data, F == LX_W_NVFP4 ? 4 : 8))
-    return launch_kernel(dequantize_kernel<F, true>, dim3(blocks_for(rows, kRowWarps)), dim3(kBlock), 0, s, data, scale, global, out, rows, cols);
-  return launch_kernel(dequantize_kernel<F, false>, dim3(blocks_for(rows * cols, kBlock)), dim3(kBlock), 0, s, data, scale, global, out, rows, cols);
+  if (cols % 8 != 0 || !aligned(out, 16) || !aligned(w.data, F == LX_W_NVFP4 ? 4 : 8)) return launch_dequantize_words<F, 0>(w, global, out, rows, cols, s);
+  const bool few = static_cast<int64_t>(blocks_for(rows, kRowWarps)) * blocks_for(cols, 256 * kInFlight) < 148 * 4;
+  if (few || cols <= 256) return launch_dequantize_words<F, 1>(w, global, out, rows, cols, s);
+  return launch_dequantize_words<F, kInFlight>(w, global, out, rows, cols, s);
 }
 
 }  // namespace

@@ -59,6 +59,18 @@ def test_same_bytes_at_every_alignment(lx, wtype, K):
     assert np.array_equal(want[0].reshape(rows, -1)[keep], data[keep])
 
 
+@pytest.mark.parametrize("wtype", [abi.W_INT8, abi.W_FP8, abi.W_NVFP4])
+@pytest.mark.parametrize("rows,K", [(1, 16), (1, 20000), (9, 16384), (4729, 1024), (4737, 1040), (1579, 3088), (4800, 256), (5001, 272)])
+def test_expanded_values_for_few_wide_and_many_short_rows(lx, wtype, rows, K):
+    """Rows in one piece or several, of one word a lane or four (from 4 x 148 blocks of eight pieces of 1024 values on), against
+    the values one at a time (an output that is not on 16 bytes)."""
+    w = torch.randn((rows, K), generator=torch.Generator(device="cuda").manual_seed(K), device="cuda").to(torch.bfloat16)
+    want = quantize(lx, w, wtype, rows, K, 1)
+    got = quantize(lx, w, wtype, rows, K, 0)
+    for a, b in zip(want, got):
+        assert np.atleast_1d(a).tobytes() == np.atleast_1d(b).tobytes()
+
+
 @pytest.mark.parametrize("rows,K", [(5, 1000), (9, 1024), (3, 1160), (2, 1)])
 def test_bf16x_same_bytes_at_every_alignment(lx, rows, K):
     w = util.bf16_normal((rows, K), 0.02, rows)
