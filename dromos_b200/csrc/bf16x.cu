@@ -353,6 +353,7 @@ extern "C" int lx_bf16x_encode(const void* w, int64_t rows, int K, void* out, in
 extern "C" int lx_bf16x_decode(const void* data, int64_t rows, int K, void* w, void* stream) {
   if (rows <= 0) return kOk;
   if (K <= 0 || K >= (1 << 23) || !data || !w) return kInvalid;
-  return launch_kernel(whole_rows(w, K) && aligned(data, 8) ? decode_kernel<true> : decode_kernel<false>, row_grid(rows), dim3(kBlock), 0,
+  // (rows of less than a block, eight values a lane, leave most lanes idle: 50000 x 64 12.9 us, one value a lane 10.8; 40000 x 128 10.6 and 11.2)
+  return launch_kernel(whole_rows(w, K) && K >= 128 && aligned(data, 8) ? decode_kernel<true> : decode_kernel<false>, row_grid(rows), dim3(kBlock), 0,
                        static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(data), rows, K, static_cast<uint16_t*>(w));
 }

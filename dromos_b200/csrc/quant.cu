@@ -35,8 +35,8 @@ __device__ __forceinline__ uint32_t max_abs2(uint32_t m, const uint4& v) {
 __device__ __forceinline__ float max_of2(uint32_t m) { return fmaxf(__uint_as_float(m << 16), __uint_as_float(m & 0xffff0000u)); }
 
 // One warp per row: the row's absmax, then its values. kFp8: e4m3 with scale absmax / 448; else int8, absmax / 127.
-// VEC: rows of whole 16-byte words (cols % 8 == 0, w on 16 and q on 8 bytes).
-template <bool kFp8, bool VEC>
+// WORDS > 0: rows of whole 16-byte words (cols % 8 == 0, w on 16 and q on 8 bytes), so many of them in flight per lane.
+template <bool kFp8, int WORDS>
 __global__ void __launch_bounds__(kBlock) quantize_rows_kernel(const uint16_t* __restrict__ w, uint8_t* __restrict__ q,
                                                                float* __restrict__ scale, int64_t rows, int cols) {
   // no early trigger: what this kernel writes may be the weight of the next product, whose kernels read weights
@@ -49,14 +49,14 @@ __global__ void __launch_bounds__(kBlock) quantize_rows_kernel(const uint16_t* _
   const uint4* src8 = reinterpret_cast<const uint4*>(src);
   const int words = cols / 8;
   float amax = 0.0f;
-  if constexpr (VEC) {
+  if constexpr (WORDS > 0) {
     uint32_t m = 0;
-    for (int c0 = lane; c0 < words; c0 += 32 * kInFlight) {
-      uint4 v[kInFlight];
+    for (int c0 = lane; c0 < words; c0 += 32 * WORDS) {
+      uint4 v[WORDS];
 #pragma unroll
-      for (int i = 0; i < kInFlight; ++i) v[i] = c0 + 32 * i < words ? __ldg(src8 + c0 + 32 * i) : make_uint4(0, 0, 0, 0);
+      for (int i = 0; i < WORDS; ++i) v[i] = c0 + 32 * i < words ? __ldg(src8 + c0 + 32 * i) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-      for (int i = 0; i < kInFlight; ++i) m = max_abs2(m, v[i]);
+      for (int i = 0; i < WORDS; ++i) m = max_abs2(m, v[i]);
     }
     amax = max_of2(m);
   } else {
@@ -72,13 +72,13 @@ __global__ void __launch_bounds__(kBlock) quantize_rows_kernel(const uint16_t* _
     if constexpr (kFp8) return e4m3_encode(fminf(fmaxf(v, -448.0f), 448.0f)) & 0xffu;
     else return static_cast<uint32_t>(static_cast<int>(fminf(fmaxf(rintf(v), -127.0f), 127.0f))) & 0xffu;
   };
-  if constexpr (VEC) {
-    for (int c0 = lane; c0 < words; c0 += 32 * kInFlight) {
-      uint4 v[kInFlight];
+  if constexpr (WORDS > 0) {
+    for (int c0 = lane; c0 < words; c0 += 32 * WORDS) {
+      uint4 v[WORDS];
 #pragma unroll
-      for (int i = 0; i < kInFlight; ++i) v[i] = c0 + 32 * i < words ? __ldg(src8 + c0 + 32 * i) : make_uint4(0, 0, 0, 0);
+      for (int i = 0; i < WORDS; ++i) v[i] = c0 + 32 * i < words ? __ldg(src8 + c0 + 32 * i) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-      for (int i = 0; i < kInFlight; ++i) {
+      for (int i = 0; i < WORDS; ++i) {
         if (c0 + 32 * i >= words) break;
         const uint32_t u[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
         uint32_t o[2];
@@ -219,8 +219,10 @@ __global__ void __launch_bounds__(kBlock) dequantize_kernel(const uint8_t* __res
       } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const uint32_t b = ((j < 4 ? e[i].x : e[i].y) >> (8 * (j & 3))) & 0xffu;
-          v[j] = (F == LX_W_INT8 ? static_cast<float>(static_cast<int8_t>(b)) : e4m3_to_f32(b)) * rf;
+          const uint32_t word = j < 4 ? e[i].x : e[i].y;
+          if constexpr (F == LX_W_INT8)  // 2^23 + 128 + the value, as bits: the conversion instructions are a quarter as fast
+            v[j] = (__uint_as_float(__byte_perm(word ^ 0x80808080u, 0x4b000000u, 0x7440 + (j & 3))) - 8388736.0f) * rf;
+          else v[j] = e4m3_to_f32((word >> (8 * (j & 3))) & 0xffu) * rf;
         }
       }
       uint32_t o[4];
@@ -305,11 +307,13 @@ __global__ void __launch_bounds__(kBlock) quantize_act_kernel(const void* __rest
 unsigned blocks_for(int64_t n, int per_block) { return static_cast<unsigned>((n + per_block - 1) / per_block); }
 
 // 14336 x 4096, quantized and expanded again (a loader's pass; 352 / 264 MB): INT8 272 -> 104 us, FP8 265 -> 77, NVFP4 365 -> 112
-// with the copy of its maximum to the host. (INT8's quantizer is left with an IEEE division and a rounding per value.)
+// with the copy of its maximum to the host. (INT8's quantizer is left with an IEEE division and a rounding per value.) Rows shorter
+// than a word per lane go value by value (FP8 50000 x 64: 10.1 us, by words 13.4), rows of one word with one in flight (FP8 100000 x 256:
+// 26.0 us, with four 31.5, value by value 28.1).
 template <bool kFp8>
 int launch_rows(const void* w, uint8_t* q, float* scale, int64_t rows, int cols, cudaStream_t s) {
-  const bool vec = cols % 8 == 0 && aligned(w, 16) && aligned(q, 8);
-  return launch_kernel(vec ? quantize_rows_kernel<kFp8, true> : quantize_rows_kernel<kFp8, false>, dim3(blocks_for(rows, kRowWarps)), dim3(kBlock), 0, s,
+  const bool vec = cols % 8 == 0 && cols >= 256 && aligned(w, 16) && aligned(q, 8);
+  return launch_kernel(!vec ? quantize_rows_kernel<kFp8, 0> : cols <= 256 ? quantize_rows_kernel<kFp8, 1> : quantize_rows_kernel<kFp8, kInFlight>, dim3(blocks_for(rows, kRowWarps)), dim3(kBlock), 0, s,
                        static_cast<const uint16_t*>(w), q, scale, rows, cols);
 }
 

@@ -30,7 +30,7 @@ def quantize(lx, w_dev, wtype, rows, K, offset):
     return util.host(data), util.host(scale), np.float32(lw.glob), util.host(out)
 
 
-@pytest.mark.parametrize("wtype,K", [(abi.W_INT8, 1), (abi.W_INT8, 8), (abi.W_INT8, 1000), (abi.W_INT8, 1032), (abi.W_FP8, 250), (abi.W_FP8, 264),
+@pytest.mark.parametrize("wtype,K", [(abi.W_INT8, 1), (abi.W_INT8, 8), (abi.W_INT8, 248), (abi.W_INT8, 256), (abi.W_INT8, 1000), (abi.W_INT8, 1032), (abi.W_FP8, 250), (abi.W_FP8, 264),
                                      (abi.W_FP8, 2056), (abi.W_NVFP4, 16), (abi.W_NVFP4, 272), (abi.W_NVFP4, 4112)])
 def test_same_bytes_at_every_alignment(lx, wtype, K):
     rows = 35
@@ -71,7 +71,7 @@ def test_expanded_values_for_few_wide_and_many_short_rows(lx, wtype, rows, K):
         assert np.atleast_1d(a).tobytes() == np.atleast_1d(b).tobytes()
 
 
-@pytest.mark.parametrize("rows,K", [(5, 1000), (9, 1024), (3, 1160), (2, 1)])
+@pytest.mark.parametrize("rows,K", [(5, 1000), (9, 1024), (3, 1160), (2, 1), (7, 120), (6, 128)])
 def test_bf16x_same_bytes_at_every_alignment(lx, rows, K):
     w = util.bf16_normal((rows, K), 0.02, rows)
     w[0, ::3] = 0x0080  # more patches than slots
