@@ -12,7 +12,7 @@
 //      its blocks serve every pair of that expert (one pass over the expert's rows however many tokens picked it);
 //      the blocks of the other pairs leave at once. A warp reads gate row i and up row I + i together and writes
 //      bf16(silu(gate) * up) to each member pair's row of the workspace.
-//   2. down: a block belongs to one (token, 16 output rows); a warp takes two and sums the token's top_k experts in k order in
+//   2. down: a block belongs to one (token, 16 or 8 output rows); a warp takes two or one and sums the token's top_k experts in k order in
 //      registers and writes out[t, l].
 // Each (pair, row) sum is one lane-ordered chain of fmaf over k followed by a fixed shuffle tree, whatever else the
 // block serves, which is what makes the rows batch-invariant and BF16X equal to bf16 bit for bit (both walk 8 values
@@ -27,7 +27,6 @@ namespace {
 constexpr int kDecodeMaxT = 8;      // moe_decode.cu:40-41 of the reference: the decode contract
 constexpr int kDecodeMaxTopK = 8;
 constexpr int kRowsPerBlock = 8;    // one warp per row
-constexpr int kDownRows = 2;        // output rows per warp of the down kernel
 constexpr int kGateUpRows = 16;     // intermediate rows a gate/up block walks (two per warp)
 constexpr int kDecodeThreads = 32 * kRowsPerBlock;
 constexpr int kScanPairs = kDecodeMaxT * kDecodeMaxTopK;  // pairs a block scans for its expert's members
@@ -345,14 +344,17 @@ __device__ __forceinline__ void dot_rows(const Stack& S, const uint8_t* const (&
   }
 }
 
-// Gate/up rows of the 8-bit formats: two steps in flight per warp and four blocks per SM (64 registers) instead of four steps and
-// three blocks (80): FP8, one / four tokens 58 / 115 -> 52 / 106 us with the rest of the call, INT8, eight 261 -> 253. BF16, whose words
-// need no conversion, is faster with more in flight (98 against 105), NVFP4 and BF16X do not fit 64 registers.
-template <int F, bool WHOLE>
-constexpr bool kLean = WHOLE && (F == LX_W_FP8 || F == LX_W_INT8);
+// Gate/up rows of the 8-bit formats (LEAN): two steps in flight per warp and four blocks per SM (64 registers) instead of four steps and
+// two (96 to 99). Measured with the rest of the call, weights of a few experts in L2: I = 1536, L = 4096, two / four / eight FP8 tokens of 16
+// experts 43 / 65 / 105 -> 37 / 54 / 91 us. A grid of fewer than two blocks per SM has no use for the third, and more to wait for with two
+// steps: I = 768, L = 2048, one INT8 / FP8 token (192 blocks) 20.6 / 15.2 with LEAN, 14.0 / 10.9 without. BF16, whose words need no
+// conversion, is faster with more in flight (98 against 105), NVFP4 and BF16X do not fit 64 registers.
+template <int F>
+constexpr bool kLeanFormat = F == LX_W_FP8 || F == LX_W_INT8;
+constexpr unsigned kLeanBlocks = 2 * 148;
 
 // Stage 1 for the NT member pairs of one expert: mid[pair, i] = bf16(silu(s_g * gate_i . x) * (s_u * up_i . x)).
-template <int F, int NT, bool WHOLE>
+template <int F, int NT, bool WHOLE, bool LEAN>
 __device__ __forceinline__ void gate_up_members(const Stack& S, int e, int i, int I, const uint16_t* latent, int ld, bool xvec,
                                                 const int (&member)[NT], int count, int top_k, uint16_t* mid, int lane) {
   const int64_t ng = static_cast<int64_t>(e) * S.rows + i, nu = ng + I;
@@ -365,7 +367,7 @@ __device__ __forceinline__ void gate_up_members(const Stack& S, int e, int i, in
   float acc[2][NT];
 #pragma unroll
   for (int t = 0; t < NT; ++t) acc[0][t] = acc[1][t] = 0.0f;
-  dot_rows<F, 2, NT, WHOLE, kLean<F, WHOLE> ? 2 : 4>(S, row, row_scale, flag, x, xvec, lane, acc);
+  dot_rows<F, 2, NT, WHOLE, LEAN ? 2 : 4>(S, row, row_scale, flag, x, xvec, lane, acc);
   const float fg = stack_row_factor<F>(S, ng, e), fu = stack_row_factor<F>(S, nu, e);
 #pragma unroll
   for (int t = 0; t < NT; ++t) {
@@ -378,8 +380,8 @@ __device__ __forceinline__ void gate_up_members(const Stack& S, int e, int i, in
 // grid (ceil(I / kGateUpRows), P). dedupe: P <= 64 and the first pair of an expert serves all of its pairs, two at a
 // time (more members than two read the rows again, from L1 / L2: the registers of wider passes would halve the warps
 // an SM holds for the common case of one or two).
-template <int F, bool WHOLE>
-__global__ void __launch_bounds__(kDecodeThreads, kLean<F, WHOLE> ? 4 : WHOLE && F == LX_W_BF16 ? 3 : 2) decode_gate_up_kernel(const Stack S, const uint16_t* __restrict__ latent, int ld,
+template <int F, bool WHOLE, bool LEAN>
+__global__ void __launch_bounds__(kDecodeThreads, LEAN ? 4 : WHOLE && F == LX_W_BF16 ? 3 : 2) decode_gate_up_kernel(const Stack S, const uint16_t* __restrict__ latent, int ld,
                                                                         int xvec, const int32_t* __restrict__ ids,
                                                                         uint16_t* __restrict__ mid, int P, int top_k, int I,
                                                                         int dedupe) {
@@ -404,19 +406,19 @@ __global__ void __launch_bounds__(kDecodeThreads, kLean<F, WHOLE> ? 4 : WHOLE &&
       if (left) {
         member[1] = __ffsll(static_cast<long long>(left)) - 1;
         left &= left - 1;
-        gate_up_members<F, 2, WHOLE>(S, e, i, I, latent, ld, xvec != 0, member, 2, top_k, mid, lane);
+        gate_up_members<F, 2, WHOLE, LEAN>(S, e, i, I, latent, ld, xvec != 0, member, 2, top_k, mid, lane);
       } else {
         const int m1[1] = {member[0]};
-        gate_up_members<F, 1, WHOLE>(S, e, i, I, latent, ld, xvec != 0, m1, 1, top_k, mid, lane);
+        gate_up_members<F, 1, WHOLE, LEAN>(S, e, i, I, latent, ld, xvec != 0, m1, 1, top_k, mid, lane);
       }
     }
   }
 }
 
-// Stage 2: out[t, l] = sum over k, in order, of weights[t, k] * (s_l * down[e_k]_l . mid[t, k]). grid (ceil(L / 16), T): a warp
-// takes two rows, so that the intermediate row's conversion serves both. (Four blocks per SM: what a warp waits for is the next
-// expert's rows, and FP8's 72 registers left room for three: the call above 139 us, 123 with 64.)
-template <int F, bool WHOLE>
+// Stage 2: out[t, l] = sum over k, in order, of weights[t, k] * (s_l * down[e_k]_l . mid[t, k]). grid (ceil(L / (8 ROWS)), T): with two rows
+// per warp the intermediate row's conversion serves both. (Four blocks per SM: what a warp waits for is the next expert's rows, and
+// FP8's 72 registers left room for three: four FP8 tokens of 64 experts 139 us, 123 with 64.)
+template <int F, bool WHOLE, int ROWS>
 __global__ void __launch_bounds__(kDecodeThreads, WHOLE && F != LX_W_BF16X ? 4 : 1) decode_down_kernel(const Stack S, const uint16_t* __restrict__ mid, int xvec,
                                                                      const int32_t* __restrict__ ids,
                                                                      const float* __restrict__ weights, float* __restrict__ out,
@@ -424,18 +426,18 @@ __global__ void __launch_bounds__(kDecodeThreads, WHOLE && F != LX_W_BF16X ? 4 :
   pdl_trigger();
   pdl_wait();  // the intermediates come from the gate/up kernel
   const int t = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int l0 = (blockIdx.x * kRowsPerBlock + warp) * kDownRows;
+  const int l0 = (blockIdx.x * kRowsPerBlock + warp) * ROWS;
   if (l0 >= L) return;
-  float total[kDownRows] = {};
+  float total[ROWS] = {};
 #pragma unroll 1
   for (int k = 0; k < top_k; ++k) {
     const int p = t * top_k + k, e = ids[p];
-    int64_t n[kDownRows];
-    const uint8_t *row[kDownRows], *row_scale[kDownRows];
-    uint32_t flag[kDownRows];
-    float acc[kDownRows][1];
+    int64_t n[ROWS];
+    const uint8_t *row[ROWS], *row_scale[ROWS];
+    uint32_t flag[ROWS];
+    float acc[ROWS][1];
 #pragma unroll
-    for (int r = 0; r < kDownRows; ++r) {
+    for (int r = 0; r < ROWS; ++r) {
       n[r] = static_cast<int64_t>(e) * S.rows + min(l0 + r, L - 1);  // (past the last row: that row again, not written)
       row[r] = S.data + n[r] * S.row_bytes;
       row_scale[r] = scale_row<F>(S, n[r]);
@@ -443,13 +445,13 @@ __global__ void __launch_bounds__(kDecodeThreads, WHOLE && F != LX_W_BF16X ? 4 :
       acc[r][0] = 0.0f;
     }
     const uint16_t* const x[1] = {mid + static_cast<int64_t>(p) * S.K};
-    dot_rows<F, kDownRows, 1, WHOLE>(S, row, row_scale, flag, x, xvec != 0, lane, acc);
+    dot_rows<F, ROWS, 1, WHOLE>(S, row, row_scale, flag, x, xvec != 0, lane, acc);
 #pragma unroll
-    for (int r = 0; r < kDownRows; ++r)
+    for (int r = 0; r < ROWS; ++r)
       total[r] = __fadd_rn(total[r], __fmul_rn(weights[p], __fmul_rn(stack_row_factor<F>(S, n[r], e), warp_sum(acc[r][0]))));
   }
 #pragma unroll
-  for (int r = 0; r < kDownRows; ++r)
+  for (int r = 0; r < ROWS; ++r)
     if (lane == 0 && l0 + r < L) out[static_cast<int64_t>(t) * L + l0 + r] = total[r];
 }
 
@@ -477,15 +479,26 @@ int launch_gate_up(const Stack& S, const void* latent, const int32_t* ids, uint1
                    cudaStream_t s) {
   const int xvec = aligned(latent, 16) && L % 8 == 0;
   const dim3 grid(static_cast<unsigned>((I + kGateUpRows - 1) / kGateUpRows), static_cast<unsigned>(P));
-  return launch_kernel(S.vec && xvec ? decode_gate_up_kernel<F, true> : decode_gate_up_kernel<F, false>, grid, dim3(kDecodeThreads), 0, s, S, static_cast<const uint16_t*>(latent), L, xvec,
-                       ids, mid, P, top_k, I, P <= kScanPairs ? 1 : 0);
+  auto kernel = S.vec && xvec ? decode_gate_up_kernel<F, true, false> : decode_gate_up_kernel<F, false, false>;
+  if constexpr (kLeanFormat<F>)
+    if (S.vec && xvec && grid.x * grid.y >= kLeanBlocks) kernel = decode_gate_up_kernel<F, true, true>;
+  return launch_kernel(kernel, grid, dim3(kDecodeThreads), 0, s, S, static_cast<const uint16_t*>(latent), L, xvec, ids, mid, P, top_k, I, P <= kScanPairs ? 1 : 0);
 }
+template <int F, int ROWS>
+int launch_down_rows(const Stack& S, const uint16_t* mid, const int32_t* ids, const float* weights, float* out, int T, int L, int I,
+                     int top_k, cudaStream_t s) {
+  const int xvec = aligned(mid, 16) && I % 8 == 0;
+  const dim3 grid(static_cast<unsigned>((L + kRowsPerBlock * ROWS - 1) / (kRowsPerBlock * ROWS)), static_cast<unsigned>(T));
+  return launch_kernel(S.vec && xvec ? decode_down_kernel<F, true, ROWS> : decode_down_kernel<F, false, ROWS>, grid, dim3(kDecodeThreads), 0, s, S, mid, xvec, ids, weights, out, top_k, L);
+}
+// Two rows per warp where that still leaves three blocks per SM (BF16X, of which two fit: one), else one: the row's conversion is shared, but
+// an SM without blocks costs more. L = 4096, I = 1536, FP8, one / two / four tokens (256, 512, 1024 blocks of two rows): 25.0 / 37.0 / 54.1 us
+// with two rows, 22.1 / 40.4 / 60.4 with one; L = 1024, four INT8 tokens (256) 20.4 and 17.3; BF16X 127 and 142.
 template <int F>
 int launch_down(const Stack& S, const uint16_t* mid, const int32_t* ids, const float* weights, float* out, int T, int L, int I,
                 int top_k, cudaStream_t s) {
-  const int xvec = aligned(mid, 16) && I % 8 == 0;
-  const dim3 grid(static_cast<unsigned>((L + kRowsPerBlock * kDownRows - 1) / (kRowsPerBlock * kDownRows)), static_cast<unsigned>(T));
-  return launch_kernel(S.vec && xvec ? decode_down_kernel<F, true> : decode_down_kernel<F, false>, grid, dim3(kDecodeThreads), 0, s, S, mid, xvec, ids, weights, out, top_k, L);
+  const int64_t blocks = static_cast<int64_t>((L + 2 * kRowsPerBlock - 1) / (2 * kRowsPerBlock)) * T;
+  return blocks < (F == LX_W_BF16X ? 1 : 3) * 148 ? launch_down_rows<F, 1>(S, mid, ids, weights, out, T, L, I, top_k, s) : launch_down_rows<F, 2>(S, mid, ids, weights, out, T, L, I, top_k, s);
 }
 
 // Both stages on stacks already checked. The grid's second extent holds pairs (tokens): up to 65535 of them per launch.

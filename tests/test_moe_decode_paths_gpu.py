@@ -33,3 +33,32 @@ def test_same_bits_with_and_without_bounds(lx, wtype, L, I):
         util.check_status(lx)
         out.append(y)
     assert torch.equal(out[0], out[1]) and bool(torch.isfinite(out[0]).all())
+
+
+@pytest.mark.parametrize("wtype", [abi.W_BF16, abi.W_INT8, abi.W_FP8, abi.W_NVFP4, abi.W_BF16X])
+@pytest.mark.parametrize("L,I", [(888, 16), (1032, 272), (2560, 1040)])
+def test_same_bits_on_small_and_large_grids(lx, wtype, L, I):
+    """Eight tokens take two output rows per warp (from 444 blocks on; 148 for BF16X) and, for the 8-bit formats, the gate/up kernel with
+    more blocks per SM (from 296); a token alone neither."""
+    E, T, top_k = 5, 8, 4
+    step = 16 if wtype in (abi.W_INT8, abi.W_FP8, abi.W_NVFP4) else 8
+    L = L // step * step
+    gen = torch.Generator(device="cuda").manual_seed(L + I)
+    make = lambda *shape: host.store_weight(lx, (torch.randn(shape, generator=gen, device="cuda") * 0.05).to(torch.bfloat16), wtype)
+    gate_up, down = make(E, 2 * I, L), make(E, L, I)
+    ids = torch.stack([torch.randperm(E, generator=gen, device="cuda")[:top_k] for _ in range(T)]).to(torch.int32)
+    weights = torch.rand((T, top_k), generator=gen, device="cuda")
+    latent = torch.randn((T, L), generator=gen, device="cuda").to(torch.bfloat16)
+    ws = torch.empty(max(256, lx.lx_moe_decode_workspace_bytes(T, I, top_k)), dtype=torch.uint8, device="cuda")
+
+    def experts(x, i, w):
+        y = torch.full((x.shape[0], L), float("nan"), device="cuda")
+        assert lx.lx_moe_experts_decode(abi.ptr(x), abi.ptr(i), abi.ptr(w), gate_up.ref(), down.ref(), abi.ptr(y), abi.ptr(ws), x.shape[0], L, I, top_k,
+                                        util.stream_ptr()) == 0
+        return y
+
+    batch = experts(latent, ids, weights)
+    for t in range(T):
+        assert torch.equal(experts(latent[t:t + 1], ids[t:t + 1].contiguous(), weights[t:t + 1].contiguous())[0], batch[t])
+    util.check_status(lx)
+    assert bool(torch.isfinite(batch).all())
