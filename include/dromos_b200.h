@@ -102,7 +102,8 @@ LX_API int lx_quantize_w8(const void* w, int8_t* q, float* scale, int64_t rows, 
 
 /* ---- lossless bf16 (LX_W_BF16X) --------------------------------------------------------------------------
  * kernels.h:574-583 (engine/cuda/bf16x.cu:1236-1295). lx_bf16x_bytes and lx_bf16x_encode synchronize the
- * stream and are load-time calls. */
+ * stream and are load-time calls. lx_bf16x_encode answers "invalid" for a buffer too small for the overflow records
+ * after the rows have been written to it: what `out` holds after any error is not an encoded matrix. */
 LX_API int64_t lx_bf16x_row_bytes(int K);
 LX_API int64_t lx_bf16x_bytes(const void* w, int64_t rows, int K, void* stream);
 LX_API int lx_bf16x_encode(const void* w, int64_t rows, int K, void* out, int64_t out_bytes, void* stream);

@@ -117,3 +117,25 @@ def test_sizes_asked_for_from_many_threads(lx):
     for t in threads:
         t.join()
     assert not wrong
+
+
+def test_bf16x_refused_buffer_holds_no_counts(lx):
+    """A buffer one byte short of the overflow records: refused, nothing past it written, and every row in it either without patches or
+    with patches in its own slots (a reader that ignores the status follows no record)."""
+    rows, K = 300, 1000
+    w = util.bf16_normal((rows, K), 0.02, 3)
+    w[::7, ::3] = 0x0080
+    row_bytes = O.bf16x_row_bytes(K)
+    src = util.dev(w)
+    n = lx.lx_bf16x_bytes(abi.ptr(src), rows, K, util.stream_ptr())
+    assert n > rows * row_bytes
+    for size in (rows * row_bytes, n - 1):
+        enc = torch.full((n + 8,), 0xAB, dtype=torch.uint8, device="cuda")
+        assert lx.lx_bf16x_encode(abi.ptr(src), rows, K, abi.ptr(enc), size, util.stream_ptr()) == 1
+        host_bytes = util.host(enc)
+        slots = host_bytes[: rows * row_bytes].reshape(rows, row_bytes)[:, :4].copy().view(np.uint32)[:, 0]
+        assert np.all((slots == 0xFFFFFFFF) | (slots < 0x80000000))
+        assert np.all(slots[::7] == 0xFFFFFFFF)
+        assert np.all(host_bytes[rows * row_bytes:] == 0xAB)
+    assert lx.lx_bf16x_encode(abi.ptr(src), rows, K, abi.ptr(enc), n, util.stream_ptr()) == 0
+    assert np.array_equal(util.host(enc)[:n], O.bf16x_encode(w))
