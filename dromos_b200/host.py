@@ -28,10 +28,16 @@ def _stream():
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
+# torch's own short way to the current stream's handle, where this torch has it (it is not a public name)
+_raw_stream_of_device = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _raw_stream():
     """The current stream of the current device as an integer, without the Stream object that torch.cuda.current_stream()
-    builds (2 us, a tenth of a small product's call)."""
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    builds (2 us, a tenth of a small product's call) where that can be had."""
+    if _raw_stream_of_device is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream_of_device(torch.cuda.current_device())
 
 
 class StoredWeight:
