@@ -170,3 +170,30 @@ def test_rows_with_infinities(lx, M, K, x_f32):
     old, bias = torch.randn((M, N), generator=gen, device="cuda").to(torch.bfloat16), torch.randn((N,), generator=gen, device="cuda")
     y = product(lx, x, sw, M, N, K, 0.75, old.clone(), bias, -0.5)[~finite].double()
     assert torch.equal(torch.nan_to_num(y, nan=0.5, posinf=1, neginf=-1), torch.nan_to_num(-want, nan=0.5, posinf=1, neginf=-1))
+
+
+@pytest.mark.parametrize("M,N,K", [(24, 28700, 512), (64, 40000, 256), (200, 14353, 512), (300, 9000, 768), (1000, 5000, 256)])
+def test_several_tiles_per_sm(lx, M, N, K):
+    """Tiles one after the other on an SM, of one chunk and of several, beginning in the middle of a panel of weights and going on into the
+    next (300 and 1000 rows on 148 SMs), with stages that go again in some chunks and not in others."""
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    sw = weight(lx, N, K, gen)
+    x = torch.randn((M, K), generator=gen, device="cuda")
+    x[torch.arange(0, M, 70, device="cuda"), K - 3] = 3e5
+    x = x.to(torch.bfloat16)
+    y = product(lx, x, sw, M, N, K)
+    w64 = values(sw.data, sw.scale, sw.glob, N, K)
+    for m0 in range(0, M, 128):
+        want = x[m0:m0 + 128].double() @ w64.T
+        got = y[m0:m0 + 128].double()
+        assert float(((got - want).norm(dim=1) / want.norm(dim=1)).max()) <= 1e-6
+    for m in {0, 1, M // 2, 70 * ((M - 1) // 70), M - 1}:
+        assert torch.equal(product(lx, x[m:m + 1], sw, 1, N, K)[0], y[m])
+    # bf16 outputs added to old ones: half a step of bf16 (its 8 bits: at most 2^-8 of the value) and the error of the sum
+    old = torch.randn((M, N), generator=gen, device="cuda").to(torch.bfloat16)
+    bias = torch.randn((N,), generator=gen, device="cuda")
+    z = product(lx, x, sw, M, N, K, 0.75, old.clone(), bias, 0.5).double()
+    for m0 in range(0, M, 128):
+        want = 0.5 * (x[m0:m0 + 128].double() @ w64.T + bias.double()) + 0.75 * old[m0:m0 + 128].double()
+        bound = 2.0**-8 * want.abs() + 1e-6 * want.norm(dim=1, keepdim=True)
+        assert bool(((z[m0:m0 + 128] - want).abs() <= bound).all())
