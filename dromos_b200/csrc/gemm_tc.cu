@@ -799,12 +799,12 @@ int tc_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const v
                int ld_y, int M, int N, int K, float alpha, float beta, void* workspace, cudaStream_t stream, bool quantized) {
   const bool x_bf16 = x_dtype == LX_BF16;
   if (quantized && w.type != LX_W_INT8 && w.type != LX_W_FP8) return kNotSupported;
-  // More rows than one pass: pairs of SMs, same digits, same order, same bits. (FP8, 28672 x 8192: 64 rows 52 us here, 65 rows
-  // 54 us there; a second pass would add another 50.)
   if (w.type == LX_W_NVFP4) {
     const int sms = sm_count();
     return sms ? mx_product(x, x_dtype, ld_x, w, bias, bias_dtype, y, y_dtype, ld_y, M, N, K, alpha, beta, workspace, tile_rows(N, sms), stream) : kInvalid;
   }
+  // More rows than one pass: pairs of SMs, same digits, same order, same bits. (FP8, 28672 x 8192: 64 rows 52 us here, 65 rows
+  // 54 us there; a second pass would add another 50.)
   if (M > kMaxRows)
     return pair_product(x, x_dtype, ld_x, w, bias, bias_dtype, y, y_dtype, ld_y, M, N, K, alpha, beta, workspace, stream, quantized);
   const int act = act_of(w.type), elem = act_elem(act), kKS = ks_of(act);
@@ -936,7 +936,7 @@ int tc_product_allgather(const void* x, int x_dtype, int ld_x, const lx_weight& 
 int64_t tc_workspace_bytes(int M, int K) {
   const int rows = std::min(M, kMaxRows);
   int64_t need = 0;
-  for (int act = 0; act < 4; ++act)
+  for (int act : {kActBf16, kActE4m3, kActS8})
     for (int bf = 0; bf < 2; ++bf) {
       const int r = std::min(rows, rows_per_pass(act, bf != 0));
       const int NC = (act_planes(act, bf != 0) * ((r + 7) / 8 * 8) + 15) / 16 * 16;
