@@ -72,7 +72,7 @@ METRIC = "decode matmul effective HBM TB/s"
 # library on a B200 (the summaries under profiles/; bytes; mean of the captured launches). c3_fp8: tc_direct_kernel,
 # the M = 16 and M = 64 launches; c3_nvfp4: tc_mx_kernel at M = 16; c5_moe_fp8: the gate/up plus the down launch of
 # one step. The few MB written are mostly lines the setup left dirty in L2: the kernels write 0.1-7 MB of outputs.
-NCU_TRAFFIC = {"c1_bf16": 33.59e6, "c2_int8": 58.854e6 + 0.105e6, "c3_fp8": (235.69e6 + 5.20e6 + 237.49e6 + 6.77e6) / 2, "c3_nvfp4": 133.70e6 + 4.27e6,
+NCU_TRAFFIC = {"c1_bf16": 33.59e6, "c2_int8": 58.854e6 + 0.105e6, "c3_fp8": (235.69e6 + 5.20e6 + 237.49e6 + 6.77e6) / 2, "c3_nvfp4": 132.92e6 + 3.84e6,
                "c4_bf16x": 88.87e6 + 3.47e6, "c5_moe_fp8": 400.74e6 + 7.10e6 + 840.85e6 + 4.11e6}
 
 

@@ -10,26 +10,28 @@
 // rows in tensor memory.) A digit is a column of its own (column j * Mp + m is digit j of row m), summed on its own in f32 and
 // put together in the epilogue, least first.
 //
-// Remainders. A bf16 value within 2^-16 of its block's largest comes out of the digits exactly; of a smaller one, what the
-// digits leave is kept too, as digits under the least block scale there is, and its stage of 256 values of K is multiplied a
-// second time from these remainders, into the same accumulators. Together the operands are exact down to 2^-33 of a row's
-// largest magnitude and rounded at 2^-41 of it below (an f16 row under one power of two: 2^-31 and 2^-39): an output whose
-// weights are zero wherever the row has its outliers is as exact as any other. Which stages have remainders, only the values
-// say: the preparation leaves a bit per row and stage, and a chunk's stage goes again if any of its rows has one. (N(0, 1)
-// values: one in 10^5 has a remainder, so ~4 % of the stages go again at 16 rows and ~17 % at 64; rows with remainders
-// everywhere take twice as long.) A row without them adds zeros, so its bits do not depend on the rows beside it.
+// Remainders. A bf16 value within 2^-16 of its block's largest comes out of the digits exactly. What they leave of smaller ones is
+// kept too where it can be told in a result: as digits under a scale of its own, and its stage of 256 values of K is multiplied a
+// second time from these, into the same accumulators. The operands are then exact down to 2^-33 of the row's largest magnitude and
+// rounded at 2^-41 of it below (an f16 row under one power of two: 2^-31 and 2^-39), so that an output whose weights are zero
+// wherever the row has its outliers is as exact as any other. It is dropped where all that is left of 2048 values together is
+// below 2^-24 (K <= 512; in proportion to K beyond, as f32 sums of so many products) of what as many values of their geometric mean's size
+// add up to: the sums are cut off by more, for every output that is not made of a few of the smallest values alone. (N(0, 1) rows
+// and products of SwiGLU hardly ever need a second stage; one outlier channel of 3000 needs one stage of 16; an outlier of 256 and more in
+// every block all of them. Kept always, SwiGLU rows took twice as long: 28672 x 8192, 64 rows 138 us.) Which stages go
+// again, only the values say: the preparation leaves a bit per row and stage, and a chunk's stage goes again if any of its rows has
+// one. A row without them adds zeros, so its bits do not depend on the rows beside it.
 //
 // What a product costs: an instruction covers 128 weight rows x 64 values of K (four times kind::f16's) for half a cycle per
 // column; up to 64 rows are 448 columns in two instructions of four and three digits. A launch takes up to 1024 rows in
 // chunks of at most 64, the chunks of a weight panel next to each other so that its later readers find it in L2.
 //
-// Measured (replayed graphs; before: the f16 expansion): 28672 x 8192, 16 / 32 / 48 / 64 rows 70.7 / 72.1 / 74.2 / 80.3 -> 44.6 / 51.4
-// / 71.0 / 91.5 us; 14336 x 4096, 64 / 100 / 500 / 1000 rows 26.8 / 49.5 / 205 / 406 -> 28.3 / 48.1 / 148 / 267. (Base 8 without
-// remainders, 21 bits: 41.7 / 45.7 / 61.4 / 73.3 and 24.0 / 42.3 / 131 / 242. Without a stage that goes again, base 13 takes 43.3 /
-// 47.7 / 62.7 / 78.2: the more rows, the more stages do.) What a stage takes at 16 rows is its copies (39 us with products and scales
-// left out); at 64 rows the 60 KB of digits that every SM fetches from L2 per 12 KB of weights. Error against 64 bits, N(0, 1)
-// rows: 4e-8 at every K (f16: 9e-8 at K = 512, 2.3e-6 at 8192); with an outlier of 2^6 .. 2^20 in every block, outputs whose weights are
-// zero there: 5e-8 .. 7.5e-7 at K = 8192 (f16: 2.3e-6; without remainders 4e-6 .. 0.4).
+// Measured (replayed graphs; before: the f16 expansion): 28672 x 8192, 16 / 32 / 48 / 64 rows 70.7 / 72.1 / 74.2 / 80.3 -> 43.2 / 48.1
+// / 62.7 / 77.5 us; 14336 x 4096, 64 / 100 / 500 / 1000 rows 26.8 / 49.5 / 205 / 406 -> 25.4 / 43.6 / 136 / 248; with an outlier in every
+// block, 28672 x 8192, 16 / 64 rows 81 / 139. What a stage takes at 16 rows is its copies (39 us with products and scales left out); at
+// 64 rows the 60 KB of digits that every SM fetches from L2 per 12 KB of weights. Error against 64 bits, N(0, 1) rows: 4e-8 at
+// every K (f16: 9e-8 at K = 512, 2.3e-6 at 8192); with an outlier of 2^6 .. 2^20 in every block, outputs whose weights are zero there:
+// 5e-8 .. 7.5e-7 at K = 8192 (f16: 2.3e-6; seven base-8 digits alone, as this kernel began: 4e-6 .. 0.4).
 //   * The block scales go to tensor memory with tcgen05.st. Written to shared memory for tcgen05.cp they needed the proxy fence,
 //     which waits for the thread's scale loads in flight: 84 us. With the activations' scales by tcgen05.cp: 57 us (copies
 //     and products of one pipe wait for each other).
@@ -151,6 +153,8 @@ __global__ void __launch_bounds__(kPrepThreads, 6) mx_prep_kernel(const void* __
                                                                uint8_t* __restrict__ again, float* __restrict__ row_scale) {
   pdl_trigger();
   __shared__ uint32_t part[kPrepThreads / 32], stages_again;
+  __shared__ unsigned long long all_squares;
+  __shared__ int all_exponents, all_count;
   __shared__ uint16_t pairs[kMxBase * kMxBase];
   if (threadIdx.x < kMxBase * kMxBase) pairs[threadIdx.x] = static_cast<uint16_t>(digit_pair(threadIdx.x));
   pdl_wait();  // the kernel before this one may still be reading the workspace
@@ -165,7 +169,7 @@ __global__ void __launch_bounds__(kPrepThreads, 6) mx_prep_kernel(const void* __
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
   if ((tid & 31) == 0) part[tid >> 5] = top;
-  if (tid == 0) stages_again = 0;
+  if (tid == 0) stages_again = 0, all_squares = 0, all_exponents = all_count = 0;
   uint32_t block_top = max_magnitude(0, v);
   block_top = max(block_top, __shfl_xor_sync(0xffffffffu, block_top, 1));
   __syncthreads();
@@ -192,10 +196,37 @@ __global__ void __launch_bounds__(kPrepThreads, 6) mx_prep_kernel(const void* __
     some |= rest_of(t) != 0;
     put_digits(__float2int_rn(t), i, pairs, w);
   }
-  const uint32_t with_rest = __ballot_sync(0xffffffffu, some);
+  uint32_t with_rest = __ballot_sync(0xffffffffu, some);
   if (with_rest && (tid & 31) == 0) atomicOr(&stages_again, 1u << (tid >> 5));
   __syncthreads();
-  if (tid == 0) again[(static_cast<int64_t>(chunk) * gridDim.x + blockIdx.x) * kMaxRows + m] = static_cast<uint8_t>(stages_again);
+  uint32_t stages = stages_again;
+  if (stages) {
+    // Can the remainders of these 2048 values be told in a result (see above)? Sums of whole numbers: the order does not matter.
+    unsigned long long squares = 0;
+    int exponents = 0, count = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t magnitude = (words[i / 2] >> (16 * (i & 1))) & 0x7fffu, rest = static_cast<uint32_t>(abs(rest_of(value_of(i))));
+      squares += static_cast<unsigned long long>(rest) * rest;
+      if (magnitude) exponents += static_cast<int>(magnitude >> 7), ++count;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      squares += __shfl_xor_sync(0xffffffffu, squares, o);
+      exponents += __shfl_xor_sync(0xffffffffu, exponents, o);
+      count += __shfl_xor_sync(0xffffffffu, count, o);
+    }
+    if ((tid & 31) == 0) {
+      atomicAdd(&all_squares, squares);
+      atomicAdd(&all_exponents, exponents);
+      atomicAdd(&all_count, count);
+    }
+    __syncthreads();
+    const float typical = static_cast<float>(all_exponents) / static_cast<float>(all_count) - static_cast<float>(127 + e_row - 40);  // log2, in units of the least scale
+    const float long_row = fmaxf(1.0f, static_cast<float>(K) * 0x1p-9f);
+    if (static_cast<float>(all_squares) <= static_cast<float>(all_count) * exp2f(2.0f * typical) * (0x1p-48f * long_row * long_row)) with_rest = stages = 0;
+  }
+  if (tid == 0) again[(static_cast<int64_t>(chunk) * gridDim.x + blockIdx.x) * kMaxRows + m] = static_cast<uint8_t>(stages);
   if (k0 >= K) return;
   uint8_t* stage = out + chunk * chunk_bytes + static_cast<size_t>(k0 / kMxStageK) * x_bytes;
   const int kb = (k0 % kMxStageK) / 2, NC = cols0 + cols1, atoms = (cols0 + 127) / 128;

@@ -2,8 +2,9 @@
 layouts (digit columns in one instruction or two, chunks of 64 rows, launches of 1024, weight panels, 256 values of K), rows that
 do not depend on the call they come in, small values beside large ones, and the values that have no digits.
 
-Bound: digits and remainders hold a value exactly, or within 2^-41 of its row's largest; products of digits are exact, their sums
-f32, and seven sums are put together with one f32 rounding each (the last at full size): 1e-6 leaves a factor of four."""
+Bound: digits and remainders hold a value exactly, or within 2^-41 of its row's largest, or leave out what is below 2^-24 * K / 512 of the
+row's typical values; products of digits are exact, their sums f32, and seven sums are put together with one f32 rounding each (the
+last at full size): 1e-6 is twice the 4.8e-7 that may be left out at K = 4096."""
 
 import ctypes
 
@@ -124,7 +125,8 @@ def test_small_values_beside_outliers(lx, M, N, K, every, factor):
 
 
 def test_one_value_of_any_size(lx):
-    """Weights that pick one activation each: 2^-33 of the row's largest and above come out as they are."""
+    """Weights that pick one activation each, rows whose values are of every size: 2^-33 of the row's largest and above come out as
+    they are."""
     M, K = 16, 512
     N = K
     sw = weight(lx, N, K, torch.Generator(device="cuda").manual_seed(5))
@@ -197,3 +199,21 @@ def test_several_tiles_per_sm(lx, M, N, K):
         want = 0.5 * (x[m0:m0 + 128].double() @ w64.T + bias.double()) + 0.75 * old[m0:m0 + 128].double()
         bound = 2.0**-8 * want.abs() + 1e-6 * want.norm(dim=1, keepdim=True)
         assert bool(((z[m0:m0 + 128] - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("M,K", [(16, 512), (64, 4096)])
+def test_a_row_does_not_depend_on_what_its_neighbours_keep(lx, M, K):
+    """Rows that keep their remainders (an outlier beside small values) and rows that drop theirs (one small value, 2^-18 of the rest) in
+    the same stages: each as it is alone."""
+    N = 200
+    gen = torch.Generator(device="cuda").manual_seed(K)
+    sw = weight(lx, N, K, gen)
+    x = torch.randn((M, K), generator=gen, device="cuda").abs() + 0.5
+    x[:, 33] = 1.7 * 2.0**-18
+    x[::3, 40] = 2.0**14
+    x = x.to(torch.bfloat16)
+    y = product(lx, x, sw, M, N, K)
+    want = x.double() @ values(sw.data, sw.scale, sw.glob, N, K).T
+    assert float(((y.double() - want).norm(dim=1) / want.norm(dim=1)).max()) <= 1e-6
+    for m in range(M):
+        assert torch.equal(product(lx, x[m:m + 1], sw, 1, N, K)[0], y[m]), m
