@@ -15,8 +15,9 @@
 // second time from these, into the same accumulators. The operands are then exact down to 2^-33 of the row's largest magnitude and
 // rounded at 2^-41 of it below (an f16 row under one power of two: 2^-31 and 2^-39), so that an output whose weights are zero
 // wherever the row has its outliers is as exact as any other. It is dropped where all that is left of 2048 values together is
-// below 2^-24 (K <= 512; in proportion to K beyond, as f32 sums of so many products) of what as many values of their geometric mean's size
-// add up to: the sums are cut off by more, for every output that is not made of a few of the smallest values alone. (N(0, 1) rows
+// below 2^-24 (K <= 512; in proportion to K beyond, as f32 sums of so many products) of what as many values add up to that have the
+// geometric mean of the smaller of every two neighbours: the sums were cut off by more, for every output that is not made of a few of
+// the smallest values alone, be half of the weights zero and half of the values a thousand times the others. (N(0, 1) rows
 // and products of SwiGLU hardly ever need a second stage; one outlier channel of 3000 needs one stage of 16; an outlier of 256 and more in
 // every block all of them. Kept always, SwiGLU rows took twice as long: 28672 x 8192, 64 rows 138 us.) Which stages go
 // again, only the values say: the preparation leaves a bit per row and stage, and a chunk's stage goes again if any of its rows has
@@ -154,7 +155,7 @@ __global__ void __launch_bounds__(kPrepThreads, 6) mx_prep_kernel(const void* __
   pdl_trigger();
   __shared__ uint32_t part[kPrepThreads / 32], stages_again;
   __shared__ unsigned long long all_squares;
-  __shared__ int all_exponents, all_count;
+  __shared__ int all_exponents, all_pairs, all_count;
   __shared__ uint16_t pairs[kMxBase * kMxBase];
   if (threadIdx.x < kMxBase * kMxBase) pairs[threadIdx.x] = static_cast<uint16_t>(digit_pair(threadIdx.x));
   pdl_wait();  // the kernel before this one may still be reading the workspace
@@ -169,7 +170,7 @@ __global__ void __launch_bounds__(kPrepThreads, 6) mx_prep_kernel(const void* __
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
   if ((tid & 31) == 0) part[tid >> 5] = top;
-  if (tid == 0) stages_again = 0, all_squares = 0, all_exponents = all_count = 0;
+  if (tid == 0) stages_again = 0, all_squares = 0, all_exponents = all_pairs = all_count = 0;
   uint32_t block_top = max_magnitude(0, v);
   block_top = max(block_top, __shfl_xor_sync(0xffffffffu, block_top, 1));
   __syncthreads();
@@ -203,26 +204,33 @@ __global__ void __launch_bounds__(kPrepThreads, 6) mx_prep_kernel(const void* __
   if (stages) {
     // Can the remainders of these 2048 values be told in a result (see above)? Sums of whole numbers: the order does not matter.
     unsigned long long squares = 0;
-    int exponents = 0, count = 0;
+    int exponents = 0, pairs_of = 0, count = 0;  // of the smaller of each two neighbours (not zero), those pairs, all values
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const uint32_t magnitude = (words[i / 2] >> (16 * (i & 1))) & 0x7fffu, rest = static_cast<uint32_t>(abs(rest_of(value_of(i))));
+      const uint32_t rest = static_cast<uint32_t>(abs(rest_of(value_of(i))));
       squares += static_cast<unsigned long long>(rest) * rest;
-      if (magnitude) exponents += static_cast<int>(magnitude >> 7), ++count;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t a = words[i] & 0x7fffu, b = words[i] >> 16 & 0x7fffu, least = a && b ? min(a, b) : a | b;
+      if (least) exponents += static_cast<int>(least >> 7), ++pairs_of;
+      count += (a != 0) + (b != 0);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       squares += __shfl_xor_sync(0xffffffffu, squares, o);
       exponents += __shfl_xor_sync(0xffffffffu, exponents, o);
+      pairs_of += __shfl_xor_sync(0xffffffffu, pairs_of, o);
       count += __shfl_xor_sync(0xffffffffu, count, o);
     }
     if ((tid & 31) == 0) {
       atomicAdd(&all_squares, squares);
       atomicAdd(&all_exponents, exponents);
+      atomicAdd(&all_pairs, pairs_of);
       atomicAdd(&all_count, count);
     }
     __syncthreads();
-    const float typical = static_cast<float>(all_exponents) / static_cast<float>(all_count) - static_cast<float>(127 + e_row - 40);  // log2, in units of the least scale
+    const float typical = static_cast<float>(all_exponents) / static_cast<float>(all_pairs) - static_cast<float>(127 + e_row - 40);  // log2, in units of the least scale
     const float long_row = fmaxf(1.0f, static_cast<float>(K) * 0x1p-9f);
     if (static_cast<float>(all_squares) <= static_cast<float>(all_count) * exp2f(2.0f * typical) * (0x1p-48f * long_row * long_row)) with_rest = stages = 0;
   }

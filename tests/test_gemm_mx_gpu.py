@@ -102,15 +102,15 @@ def test_scales_with_a_sign(lx):
 
 
 @pytest.mark.parametrize("M,N,K", [(3, 200, 512), (16, 300, 4096), (40, 130, 1024), (64, 97, 2560), (130, 300, 2048)])
-@pytest.mark.parametrize("every", [True, False], ids=["every-block", "one"])
+@pytest.mark.parametrize("outliers", ["every-block", "every-other-value", "one"])
 @pytest.mark.parametrize("factor", [64, 256, 1024, 4096, 2**13, 2**15, 2**20])
-def test_small_values_beside_outliers(lx, M, N, K, every, factor):
+def test_small_values_beside_outliers(lx, M, N, K, outliers, factor):
     """Outputs whose weights are zero wherever the row has an outlier: what is left of the sum is as exact as any other. (Values of 0.05
     beside 0.05 * 2^20: 2^-41 of the outlier is 2^-21 of such a value, and few are rounded at all.) The other outputs are the
     outlier's product with thousands of small ones added to it: each of the K / 64 sums may be cut off at 2^-23 of it."""
     gen = torch.Generator(device="cuda").manual_seed(factor + M)
     sw = weight(lx, N, K, gen)
-    at = torch.arange(5, K, 16, device="cuda") if every else torch.tensor([K // 2 + 11], device="cuda")
+    at = {"every-block": torch.arange(5, K, 16), "every-other-value": torch.arange(1, K, 2), "one": torch.tensor([K // 2 + 11])}[outliers].cuda()
     rows = torch.arange(0, M, 2, device="cuda")  # plain rows stand beside them
     x = torch.randn((M, K), generator=gen, device="cuda") * 0.05
     x[rows[:, None], at[None, :]] *= factor
