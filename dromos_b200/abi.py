@@ -11,6 +11,11 @@ from __future__ import annotations
 import ctypes
 import os
 
+try:
+    from . import _calls  # arguments converted in C++ (csrc/calls.cpp)
+except ImportError:  # not built, or for another interpreter: ctypes converts them
+    _calls = None
+
 W_BF16, W_INT8, W_FP8, W_NVFP4, W_BF16X = 0, 1, 2, 3, 4
 MATH_BF16, MATH_INT8, MATH_FP8, MATH_FP4 = 0, 1, 2, 3
 F32, BF16 = 0, 1
@@ -23,6 +28,19 @@ class LxWeight(ctypes.Structure):
     """lx_weight (engine/cuda/kernels.h:411-417): a host struct whose pointers are device pointers."""
 
     _fields_ = [("type", c_int), ("data", c_ptr), ("scale", c_ptr), ("glob", c_f32), ("expert_global", c_ptr)]
+
+
+class WeightRef:
+    """A pointer to an LxWeight as a call argument: ctypes takes it where it takes ctypes.byref(struct)."""
+
+    __slots__ = ("struct", "address", "_as_parameter_")
+
+    def __init__(self, struct: LxWeight):
+        self.struct, self.address, self._as_parameter_ = struct, ctypes.addressof(struct), ctypes.byref(struct)
+
+
+if _calls is not None:
+    _calls.setup(c_ptr, WeightRef)
 
 
 class LxTuneProblem(ctypes.Structure):
@@ -107,10 +125,11 @@ def ptr(a):
     """A device/host address as c_void_p from a torch tensor, a numpy array, an int or None."""
     if a is None:
         return c_ptr(None)
-    if isinstance(a, (int,)):
+    data_ptr = getattr(a, "data_ptr", None)
+    if data_ptr is not None:
+        return c_ptr(data_ptr())
+    if isinstance(a, int):
         return c_ptr(a)
-    if hasattr(a, "data_ptr"):
-        return c_ptr(a.data_ptr())
     if hasattr(a, "ctypes"):
         return c_ptr(a.ctypes.data)
     if isinstance(a, c_ptr):
@@ -150,6 +169,8 @@ class Library:
     def __getattr__(self, name):
         if name.startswith("lx_"):
             f = self.fn(name)
+            if _calls is not None:
+                f = _calls.bind(name, ctypes.cast(f, c_ptr).value, f)
             self.__dict__[name] = f  # found without this detour from now on
             return f
         raise AttributeError(name)

@@ -10,6 +10,7 @@ import concurrent.futures
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -17,6 +18,8 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 OBJ = os.path.join(CSRC, "obj")
 LIB = os.path.join(HERE, "libdromos_b200.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+CALLS_SRC = os.path.join(CSRC, "calls.cpp")
+CALLS = os.path.join(HERE, "_calls" + sysconfig.get_config_var("EXT_SUFFIX"))  # the Python callables of abi.Library
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-fvisibility=hidden",
          "-I", INCLUDE, "-I", CSRC, "--expt-relaxed-constexpr"]
 
@@ -64,6 +67,13 @@ def build(force=False, verbose=False):
         if r.returncode != 0:
             print(r.stdout + r.stderr, file=sys.stderr)
             raise RuntimeError("link failed")
+    if force or not os.path.exists(CALLS) or os.path.getmtime(CALLS) < max(hdr, os.path.getmtime(CALLS_SRC)):
+        cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-I", INCLUDE, "-I", sysconfig.get_paths()["include"],
+               CALLS_SRC, "-o", CALLS]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            print(r.stdout + r.stderr, file=sys.stderr)
+            raise RuntimeError("g++ failed on calls.cpp")
     return LIB
 
 

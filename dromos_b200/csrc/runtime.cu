@@ -187,6 +187,7 @@ int lx_set_arch_override(int arch) {
 int lx_tune_get(const char* kernel, int M, int N, int K) {
   if (!kernel) return -1;
   std::lock_guard<std::mutex> lock(g_mu);
+  if (table().empty()) return -1;  // every product asks: most programs tune nothing
   auto it = table().find(TableKey{kernel, m_bucket(M), N, K});
   return it == table().end() ? -1 : it->second;
 }

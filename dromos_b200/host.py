@@ -48,9 +48,12 @@ class StoredWeight:
         self.wtype, self.data, self.scale, self.glob, self.expert_global = wtype, data, scale, float(glob), expert_global
         self.rows, self.cols = rows, cols
         self.struct = abi.make_weight(wtype, data, scale, glob, expert_global)
+        self._ref = abi.WeightRef(self.struct)
 
     def ref(self):
-        return ctypes.byref(self.struct)
+        if self._ref.struct is not self.struct:
+            self._ref = abi.WeightRef(self.struct)
+        return self._ref
 
     def nbytes(self) -> int:
         """Bytes a product streams from this weight: values and their scales (the reference's accounting,
@@ -179,8 +182,9 @@ class Experts:
         # entropy and confidence are required outputs of the reference's entry point (its kernel writes them without a null
         # check, engine/cuda/moe.cu:67), so they are always passed; the last call's values stay readable as self.stats
         self.stats = torch.empty((2, T), dtype=torch.float32, device=logits.device)
-        st = self.lib.lx_moe_route(abi.ptr(logits), abi.ptr(bias), abi.ptr(ids), abi.ptr(weights), abi.ptr(self.stats[0]), abi.ptr(self.stats[1]), T,
-                                   logits.shape[1], self.top_k, _stream())
+        stats = self.stats.data_ptr()
+        st = self.lib.lx_moe_route(logits.data_ptr(), abi.ptr(bias), ids.data_ptr(), weights.data_ptr(), stats, stats + 4 * T, T, logits.shape[1], self.top_k,
+                                   _raw_stream())
         if st:
             raise RuntimeError(f"lx_moe_route failed: {st}")
         return ids, weights
@@ -192,9 +196,8 @@ class Experts:
         need = self.lib.lx_moe_grouped_workspace_bytes(T, self.L, self.I, self.E, self.top_k, abi.MATH_BF16)
         if self._ws is None or self._ws.numel() < need:
             self._ws = torch.empty(need, dtype=torch.uint8, device=latent.device)
-        st = self.lib.lx_moe_experts_grouped(abi.ptr(latent), abi.ptr(ids), abi.ptr(weights), self.gate_up.ref(), self.down.ref(),
-                                             abi.MATH_BF16, abi.ptr(out), abi.ptr(self._ws), T, self.L, self.I, self.E,
-                                             self.top_k, _stream())
+        st = self.lib.lx_moe_experts_grouped(latent.data_ptr(), ids.data_ptr(), weights.data_ptr(), self.gate_up.ref(), self.down.ref(), abi.MATH_BF16,
+                                             out.data_ptr(), self._ws.data_ptr(), T, self.L, self.I, self.E, self.top_k, _raw_stream())
         if st:
             raise RuntimeError(f"lx_moe_experts_grouped failed: {st}")
         return out

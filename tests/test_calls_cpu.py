@@ -1,0 +1,71 @@
+"""The entry points with arguments converted in C++ (dromos_b200._calls) answer as the ctypes functions behind them: the same
+results, the same refusals of arguments. Calls of no rows, and sizes, need no GPU."""
+
+import ctypes
+
+import pytest
+import torch
+
+from dromos_b200 import abi, host
+
+calls = pytest.importorskip("dromos_b200._calls", reason="built by python -m dromos_b200.build")
+
+
+@pytest.fixture()
+def lib():
+    return abi.Library(abi.default_library_path())
+
+
+def outcome(f, args):
+    try:
+        return f(*args)
+    except Exception as e:  # noqa: BLE001 - which exception is what is compared
+        return type(e), str(e)
+
+
+WEIGHT = abi.make_weight(abi.W_BF16, torch.zeros(64, dtype=torch.uint8))
+ADDRESSES = [None, 0, 64, 2**63 + 8, -8, ctypes.c_void_p(64), ctypes.c_void_p(None), b"bytes", "text", 1.5, object()]
+WEIGHTS = [None, abi.WeightRef(WEIGHT), ctypes.byref(WEIGHT), ctypes.pointer(WEIGHT), WEIGHT, 64, ctypes.c_void_p(64)]
+NUMBERS = [0, 7, -1, True, 2**31 + 5, 2**63, 2**70, 1.0, None, "1", ctypes.c_int(3)]
+FLOATS = [0.5, 1, None, "1", ctypes.c_float(2.0), float("nan"), 1e300]
+
+
+def gemv_args(**kw):  # M = 0: answers before anything is read
+    a = dict(x=64, x_dtype=1, ld_x=64, w=abi.WeightRef(WEIGHT), bias=None, bias_dtype=1, y=64, y_dtype=0, ld_y=64, M=0, N=64, K=64, alpha=1.0, beta=0.0, stream=None)
+    assert set(kw) <= set(a)
+    a.update(kw)
+    return tuple(a.values())
+
+
+@pytest.mark.parametrize("name,values", [("x", ADDRESSES), ("w", WEIGHTS), ("ld_x", NUMBERS), ("N", NUMBERS), ("alpha", FLOATS), ("stream", ADDRESSES)])
+def test_every_kind_of_argument(lib, name, values):
+    fast, slow = lib.lx_gemv_w, lib.fn("lx_gemv_w")
+    assert type(fast) is not type(slow)
+    for v in values:
+        args = gemv_args(**{name: v})
+        assert outcome(fast, args) == outcome(slow, args), (name, v)
+
+
+def test_counts_of_arguments_and_names(lib):
+    fast, slow = lib.lx_gemm_workspace_bytes, lib.fn("lx_gemm_workspace_bytes")
+    for args in ((), (1,), (9, 4096), (9, 4096, 0), (70, 512, 2), (9, 4096, 0, 5)):
+        assert outcome(fast, args) == outcome(slow, args), args
+    with pytest.raises(TypeError):
+        fast(9, 4096, maths=0)
+    assert fast.restype is slow.restype and fast.argtypes == slow.argtypes
+    assert lib.lx_bf16x_row_bytes(4096) == 6192 and lib.lx_bf16x_row_bytes(0) == -1  # a 64-bit result with its sign
+
+
+def test_a_weight_follows_its_struct():
+    a, b = torch.zeros(64, dtype=torch.uint8), torch.zeros(64, dtype=torch.uint8)
+    w = host.StoredWeight(abi.W_BF16, a)
+    first = w.ref()
+    assert w.ref() is first and first.address == ctypes.addressof(w.struct)
+    w.struct = abi.make_weight(abi.W_BF16, b)
+    assert w.ref().address == ctypes.addressof(w.struct)
+
+
+def test_without_the_module_ctypes_converts(monkeypatch):
+    monkeypatch.setattr(abi, "_calls", None)
+    lib = abi.Library(abi.default_library_path())
+    assert lib.lx_gemv_w is lib.fn("lx_gemv_w") and lib.lx_gemv_w(*gemv_args()) == 0
