@@ -57,17 +57,10 @@ __device__ __forceinline__ uint32_t patch_mask(const uint4& v, uint32_t base, in
   return mask;
 }
 
-// One warp per row: *area += bytes of the row's overflow record, for rows with more patches than slots. (A sum of whole
-// numbers: the order in which rows add does not matter.)
+// A warp: *area += bytes of a row's overflow record if it has more patches than slots. (A sum of whole numbers: the order in
+// which rows add does not matter.)
 template <bool VEC>
-__global__ void __launch_bounds__(kBlock) count_kernel(const uint16_t* __restrict__ w, int64_t rows, int K, unsigned long long* __restrict__ area) {
-  // no early trigger: what this kernel writes may be the weight of the next product, whose kernels read weights
-  // before their own wait
-  pdl_wait();
-  const int64_t row = static_cast<int64_t>(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
-  if (row >= rows) return;
-  const int lane = threadIdx.x & 31;
-  const uint16_t* src = w + row * K;
+__device__ __forceinline__ void count_row(const uint16_t* __restrict__ src, int K, int lane, unsigned long long* __restrict__ area) {
   int n = 0;
   for (int k_base = 0; k_base < K; k_base += 256 * kInFlight) {
     uint4 v[kInFlight];
@@ -79,6 +72,15 @@ __global__ void __launch_bounds__(kBlock) count_kernel(const uint16_t* __restric
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
   if (lane == 0 && n > x16::patch_slots(K)) atomicAdd(area, static_cast<unsigned long long>(record_bytes(n)));
+}
+template <bool VEC>
+__global__ void __launch_bounds__(kBlock) count_kernel(const uint16_t* __restrict__ w, int64_t rows, int K, unsigned long long* __restrict__ area) {
+  // no early trigger: what this kernel writes may be the weight of the next product, whose kernels read weights
+  // before their own wait
+  pdl_wait();
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  count_row<VEC>(w + row * K, K, threadIdx.x & 31, area);
 }
 
 // Where a lane's patches go in its row's list: after those of the lanes below it. Returns the warp's count.
@@ -99,15 +101,25 @@ __device__ __forceinline__ int place_patches(uint32_t mask, int lane, int& befor
 // common matrix is read once, and nothing but *area has to be known before.
 // A lane holds eight consecutive values: eight sign|mantissa bytes, and one word of codes (byte j holds value j low and
 // value 4 + j high), so a block's 192 bytes leave in 16 stores of 8 and 16 of 4 bytes.
+// room: the bytes there are for overflow records. Once the rows so far have more, what is written is of no use any more, and the
+// rest are only counted (a matrix whose every row overflows then costs what counting it costs).
 template <bool VEC>
 __global__ void __launch_bounds__(kBlock) encode_kernel(const uint16_t* __restrict__ w, int64_t rows, int K, uint8_t* __restrict__ out,
-                                                        unsigned long long* __restrict__ area) {
+                                                        unsigned long long* __restrict__ area, unsigned long long room) {
   // no early trigger: what this kernel writes may be the weight of the next product, whose kernels read weights
   // before their own wait
   pdl_wait();
   const int64_t row = static_cast<int64_t>(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int lane = threadIdx.x & 31;
+  if (room != ~0ull) {
+    unsigned long long so_far = 0;
+    if (lane == 0) asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(so_far) : "l"(area) : "memory");
+    if (__shfl_sync(0xffffffffu, so_far, 0) > room) {
+      count_row<VEC>(w + row * K, K, lane, area);
+      return;
+    }
+  }
   const int H = x16::header_bytes(K), P = x16::patch_slots(K), B = x16::blocks(K);
   const uint16_t* src = w + row * K;
   uint8_t* rec = out + row * x16::row_bytes(K);
@@ -340,27 +352,49 @@ extern "C" int64_t lx_bf16x_bytes(const void* w, int64_t rows, int K, void* stre
   return rows * x16::row_bytes(K) + static_cast<int64_t>(bytes);
 }
 
+// What the two encoders share. *total: the bytes the encoding takes, as lx_bf16x_bytes answers. count_on: a buffer that turns out
+// too small is not filled any further, and what it holds is undefined; else it is left as lx_bf16x_encode leaves it.
+static int encode_matrix(const void* w, int64_t rows, int K, void* out, int64_t out_bytes, int64_t* total, bool count_on, cudaStream_t stream) {
+  const int64_t rb = x16::row_bytes(K);
+  const bool vec = whole_rows(w, K);
+  ResultWord area(stream);
+  if (area.status) return area.status;
+  const auto* src = static_cast<const uint16_t*>(w);
+  auto* dst = static_cast<uint8_t*>(out);
+  const unsigned long long room = static_cast<unsigned long long>(out_bytes - rows * rb);
+  if (int e = launch_kernel(vec ? encode_kernel<true> : encode_kernel<false>, row_grid(rows), dim3(kBlock), 0, area.stream, src, rows, K, dst, area.dev,
+                            count_on ? room : ~0ull))
+    return e;
+  unsigned long long bytes = 0;
+  if (int e = area.read(&bytes)) return e;
+  *total = rows * rb + static_cast<int64_t>(bytes);
+  if (!bytes) return kOk;
+  if (bytes > room) {
+    if (count_on) return LX_B200_ERR_SCRATCH;
+    const int e = launch_kernel(drop_counts_kernel, dim3(static_cast<unsigned>((rows + kBlock - 1) / kBlock)), dim3(kBlock), 0, area.stream, dst, rows, rb);
+    return e ? e : kInvalid;
+  }
+  if (int e = launch_kernel(place_records_kernel, dim3(1), dim3(1024), 0, area.stream, dst, rows, rb)) return e;
+  return launch_kernel(vec ? overflow_kernel<true> : overflow_kernel<false>, row_grid(rows), dim3(kBlock), 0, area.stream, src, rows, K, dst);
+}
+
 // A buffer too small for the overflow records is refused after the rows themselves (which fit) have been written: whether it is, only the
 // encoder finds out, and counting first reads the matrix once more (25 us of 14336 x 4096). Such rows are left without their patches.
 extern "C" int lx_bf16x_encode(const void* w, int64_t rows, int K, void* out, int64_t out_bytes, void* stream) {
   if (rows <= 0) return kOk;
   const int64_t rb = K > 0 && K < (1 << 23) ? x16::row_bytes(K) : 0;
   if (!rb || !w || !out || !aligned(out, 8) || out_bytes < rows * rb) return kInvalid;
-  const bool vec = whole_rows(w, K);
-  ResultWord area(static_cast<cudaStream_t>(stream));
-  if (area.status) return area.status;
-  const auto* src = static_cast<const uint16_t*>(w);
-  auto* dst = static_cast<uint8_t*>(out);
-  if (int e = launch_kernel(vec ? encode_kernel<true> : encode_kernel<false>, row_grid(rows), dim3(kBlock), 0, area.stream, src, rows, K, dst, area.dev)) return e;
-  unsigned long long bytes = 0;
-  if (int e = area.read(&bytes)) return e;
-  if (!bytes) return kOk;
-  if (rows * rb + static_cast<int64_t>(bytes) > out_bytes) {
-    const int e = launch_kernel(drop_counts_kernel, dim3(static_cast<unsigned>((rows + kBlock - 1) / kBlock)), dim3(kBlock), 0, area.stream, dst, rows, rb);
-    return e ? e : kInvalid;
-  }
-  if (int e = launch_kernel(place_records_kernel, dim3(1), dim3(1024), 0, area.stream, dst, rows, rb)) return e;
-  return launch_kernel(vec ? overflow_kernel<true> : overflow_kernel<false>, row_grid(rows), dim3(kBlock), 0, area.stream, src, rows, K, dst);
+  int64_t total = 0;
+  return encode_matrix(w, rows, K, out, out_bytes, &total, false, static_cast<cudaStream_t>(stream));
+}
+
+// Sizing and encoding in one call, the matrix read once: few matrices have overflow records at all, so a caller begins with
+// a buffer of rows * lx_bf16x_row_bytes(K) and comes back with a larger one only when the answer is LX_B200_ERR_SCRATCH. *bytes: what the
+// encoding takes (lx_bf16x_bytes), filled in with either answer.
+extern "C" int lx_b200_bf16x_encode_sized(const void* w, int64_t rows, int K, void* out, int64_t out_bytes, int64_t* bytes, void* stream) {
+  const int64_t rb = K > 0 && K < (1 << 23) ? x16::row_bytes(K) : 0;
+  if (rows <= 0 || !rb || !w || !out || !bytes || !aligned(out, 8) || out_bytes < rows * rb) return kInvalid;
+  return encode_matrix(w, rows, K, out, out_bytes, bytes, true, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int lx_bf16x_decode(const void* data, int64_t rows, int K, void* w, void* stream) {

@@ -270,6 +270,10 @@ LX_API int lx_b200_moe_sum_rows(const float* rows, float* out, int T, int L, int
  * are the caller's to serialize. A bounded wait that gives up inside this call shows in lx_b200_last_error() like any
  * other. */
 #define LX_B200_ERR_SCRATCH 804
+/* lx_bf16x_bytes and lx_bf16x_encode in one call that reads the matrix once. out_bytes >= rows * lx_bf16x_row_bytes(K), out on 8
+ * bytes. Returns 0 with the bytes of the encoding in *bytes (which lx_bf16x_bytes would answer), or LX_B200_ERR_SCRATCH when they are
+ * more than out_bytes: *bytes says how many, what out holds is undefined. Synchronizes the stream, as both do. */
+LX_API int lx_b200_bf16x_encode_sized(const void* w, int64_t rows, int K, void* out, int64_t out_bytes, int64_t* bytes, void* stream);
 LX_API int lx_b200_moe_experts_grouped_static(const void* latent, const int32_t* ids, const float* weights,
                                               const lx_weight* gate_up, const lx_weight* down, lx_math math, float* out,
                                               int T, int L, int I, int E, int top_k, void* stream);
