@@ -17,7 +17,9 @@
 //            f32 row; the k-ordered sum over a token's picks is a kernel of its own (moe.cu).
 //
 // Roles, rings, bounded waits and the two accumulators in tensor memory are those of the dense kernel (gemm_tc.cu).
-// Here every role waits for the previous kernel first: which weights a CTA streams depends on the routing.
+// Which weights a CTA streams depends on the routing, but not on the activations: the chunk tables are complete when a product
+// starts (the grouping, before the first preparation, whose blocks let their successor start only behind their own wait; later kernels
+// start later), so the weights stream while the rows are still being prepared, and the down rows while the last gate/up tiles are.
 #include "tc.cuh"
 
 namespace b200 {
@@ -65,8 +67,11 @@ __global__ void __launch_bounds__(128) expert_prep_kernel(const uint16_t* __rest
                                                           const int32_t* __restrict__ pos_col, uint8_t* __restrict__ out, int64_t chunk_stride,
                                                           float* __restrict__ inv_scales, int n_stages) {
   constexpr int kElem = act_elem(ACT), V = 16 / kElem, kKS = ks_of(ACT);
-  pdl_trigger();
+  // What the product kernels read before their wait (see there) is the grouping's, the kernel before this one in front of gate/up: that
+  // product may start only when the grouping is done.
+  if (!top_k_or_0) pdl_trigger();
   pdl_wait();
+  if (top_k_or_0) pdl_trigger();
   __shared__ float part[4];
   const int u = blockIdx.y, tid = threadIdx.x;
   if (pos_chunk[u] < 0) return;  // a row of an expert another rank owns (the whole block leaves together)
@@ -154,8 +159,6 @@ __global__ void __launch_bounds__(kExpertThreads, 1) tc_expert_kernel(const __gr
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 4 && lane == 0) pdl_trigger();
-  // The chunk table, the activation blocks and their scales all come from earlier kernels of this call.
-  pdl_wait();
   const int n_tiles = *P.tab.n_chunks * P.tiles_per_expert;
   const int tile_begin = static_cast<int>(static_cast<int64_t>(n_tiles) * blockIdx.x / gridDim.x);
   const int tile_end = static_cast<int>(static_cast<int64_t>(n_tiles) * (blockIdx.x + 1) / gridDim.x);
@@ -186,6 +189,7 @@ __global__ void __launch_bounds__(kExpertThreads, 1) tc_expert_kernel(const __gr
         }
       }
     } else if (lane == 1) {
+      pdl_wait();  // the blocks come from the kernel before this one
       Ring x;
       bool ok = true, wrapped = false;
       for (int tile = tile_begin; tile < tile_end && ok; ++tile) {
@@ -249,6 +253,7 @@ __global__ void __launch_bounds__(kExpertThreads, 1) tc_expert_kernel(const __gr
     // ================================ epilogue ================================
     const int r = tid;  // row of the tile = TMEM lane
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
+    pdl_wait();  // the rows' scales come from the kernel before this one, and what is written here may still be read by earlier ones
     for (int tile = tile_begin; tile < tile_end; ++tile) {
       const int t = tile - tile_begin, buf = t & 1;
       const int chunk = tile / P.tiles_per_expert, tt = tile - chunk * P.tiles_per_expert;
