@@ -39,7 +39,6 @@ namespace b200 {
 namespace {
 
 constexpr int kX16Threads = kGemvThreads + 64;
-constexpr int kX16Batch = 4;  // steps of 64 values a warp takes out of a slot at once: 12 registers each
 
 struct X16Ring {
   int cb;        // blocks of K per stage
@@ -376,52 +375,38 @@ __global__ void __launch_bounds__(kX16Threads, 1) gemv_x16_kernel(const GemvPara
       // release a slot's next lap before the others have released this one.
       x16_wait(full_bar(ring.slot), ring.lap, dead, R.status);
       if (R.whole) ca = cursor_at(hdr_a, ra), cb = cursor_at(hdr_b, rb);  // the headers came with the stage
-      // The slice's bytes go to registers kX16Batch steps at a time, and the slot is given back when the last are there, before they
-      // are decoded: the next copy then travels under this unit's decode instead of behind it.
-      const uint8_t* const slot = smem + R.ring_off + ring.slot * R.slot_bytes;
-      const uint8_t* const row_a = slot + blocks_a + 16u * t;
-      const uint8_t* const row_b = slot + blocks_b + 16u * t;
-      const uint8_t *const bases_a = hdr_a + 4 * slots, *const bases_b = hdr_b + 4 * slots;
-      int s = a;
-      do {
-        uint4 sm_a[kX16Batch], sm_b[kX16Batch];
-        uint2 cd_a[kX16Batch], cd_b[kX16Batch];
-        uint32_t base[kX16Batch];  // of the two rows' blocks, in bytes 0 and 1
-#pragma unroll
-        for (int i = 0; i < kX16Batch; ++i) {
-          if (s + i >= b) break;
-          const uint32_t half = static_cast<uint32_t>(s + i) & 1u, block = static_cast<uint32_t>(s + i) >> 1;
-          const uint32_t at = (block - static_cast<uint32_t>(blk_lo)) * 192u;
-          const uint8_t *const va = row_a + at + 64u * half, *const vb = row_b + at + 64u * half;
+      if (a < b) {
+        const uint8_t* slot = smem + R.ring_off + ring.slot * R.slot_bytes;
+        // The lane's place in the block step `a` lies in, and on from there block by block: nothing in the loop multiplies.
+        const uint32_t first = static_cast<uint32_t>(a >> 1) - static_cast<uint32_t>(blk_lo);
+        const uint8_t* row_a = slot + blocks_a + first * 192u + 16u * t;
+        const uint8_t* row_b = slot + blocks_b + first * 192u + 16u * t;
+        const uint8_t* base_at_a = hdr_a + 4 * slots + (a >> 1);
+        const uint8_t* base_at_b = hdr_b + 4 * slots + (a >> 1);
+        uint32_t xo = static_cast<uint32_t>(a) * kXStep;
+        uint32_t lim = (static_cast<uint32_t>(a) * 64u + 16u * t + 16u) << 8;  // the end of this lane's values of the step, as a patch word
+        uint32_t base_a = 0, base_b = 0;
+        // one step: half H of the block at row_a / row_b
+        auto step = [&](auto half_c) {
+          constexpr uint32_t H = decltype(half_c)::value;
+          uint4 sm_a, sm_b;
           if constexpr (A16) {
-            sm_a[i] = *reinterpret_cast<const uint4*>(va);
-            sm_b[i] = *reinterpret_cast<const uint4*>(vb);
+            sm_a = *reinterpret_cast<const uint4*>(row_a + 64u * H);
+            sm_b = *reinterpret_cast<const uint4*>(row_b + 64u * H);
           } else {
-            const uint2 a0 = *reinterpret_cast<const uint2*>(va), a1 = *reinterpret_cast<const uint2*>(va + 8);
-            const uint2 b0 = *reinterpret_cast<const uint2*>(vb), b1 = *reinterpret_cast<const uint2*>(vb + 8);
-            sm_a[i] = make_uint4(a0.x, a0.y, a1.x, a1.y);
-            sm_b[i] = make_uint4(b0.x, b0.y, b1.x, b1.y);
+            const uint2 a0 = *reinterpret_cast<const uint2*>(row_a + 64u * H), a1 = *reinterpret_cast<const uint2*>(row_a + 64u * H + 8);
+            const uint2 b0 = *reinterpret_cast<const uint2*>(row_b + 64u * H), b1 = *reinterpret_cast<const uint2*>(row_b + 64u * H + 8);
+            sm_a = make_uint4(a0.x, a0.y, a1.x, a1.y);
+            sm_b = make_uint4(b0.x, b0.y, b1.x, b1.y);
           }
-          // the codes of the lane's 16 values: 8 bytes at 128 + 32 half + 8 t of the block (va already stands 64 half + 16 t in)
-          cd_a[i] = *reinterpret_cast<const uint2*>(va + 128u - 32u * half - 8u * t);
-          cd_b[i] = *reinterpret_cast<const uint2*>(vb + 128u - 32u * half - 8u * t);
-          base[i] = bases_a[block] | static_cast<uint32_t>(bases_b[block]) << 8;
-        }
-        if (s + kX16Batch >= b) {
-          __syncwarp();
-          if (lane == 0) mbar_arrive(empty_bar(ring.slot));
-        }
-#pragma unroll
-        for (int i = 0; i < kX16Batch; ++i) {
-          if (s + i >= b) break;
-          const uint32_t xo = static_cast<uint32_t>(s + i) * kXStep;
-          const uint32_t lim = (static_cast<uint32_t>(s + i) * 64u + 16u * t + 16u) << 8;  // the end of this lane's values of the step, as a patch word
+          // the codes of the lane's 16 values: 8 bytes at 128 + 32 H + 8 t of the block (row_a already stands 16 t in)
+          const uint2 cd_a = *reinterpret_cast<const uint2*>(row_a + 128u + 32u * H - 8u * t);
+          const uint2 cd_b = *reinterpret_cast<const uint2*>(row_b + 128u + 32u * H - 8u * t);
           uint32_t wa[8], wb[8];
-          const uint32_t ba = __byte_perm(base[i], 0, 0x0000), bb = __byte_perm(base[i], 0, 0x1111);
-          x16_words8(sm_a[i].x, sm_a[i].y, cd_a[i].x, ba, wa);
-          x16_words8(sm_a[i].z, sm_a[i].w, cd_a[i].y, ba, wa + 4);
-          x16_words8(sm_b[i].x, sm_b[i].y, cd_b[i].x, bb, wb);
-          x16_words8(sm_b[i].z, sm_b[i].w, cd_b[i].y, bb, wb + 4);
+          x16_words8(sm_a.x, sm_a.y, cd_a.x, base_a, wa);
+          x16_words8(sm_a.z, sm_a.w, cd_a.y, base_a, wa + 4);
+          x16_words8(sm_b.x, sm_b.y, cd_b.x, base_b, wb);
+          x16_words8(sm_b.z, sm_b.w, cd_b.y, base_b, wb + 4);
           if (min(ca.next, cb.next) < lim) {  // rare: a patch of one of the two rows lies below the end of this lane's values
             const uint32_t k0 = (lim >> 8) - 16u;
             if (ca.next < lim) {
@@ -429,14 +414,14 @@ __global__ void __launch_bounds__(kX16Threads, 1) gemv_x16_kernel(const GemvPara
               f = x16_fix16(rec_of(ra), slots, k0, f);
               ca.next = f.next, ca.taken = f.taken;
 #pragma unroll
-              for (int q = 0; q < 8; ++q) wa[q] = f.w[q];
+              for (int i = 0; i < 8; ++i) wa[i] = f.w[i];
             }
             if (cb.next < lim) {
               X16Fix f{cb.next, cb.taken, {wb[0], wb[1], wb[2], wb[3], wb[4], wb[5], wb[6], wb[7]}};
               f = x16_fix16(rec_of(rb), slots, k0, f);
               cb.next = f.next, cb.taken = f.taken;
 #pragma unroll
-              for (int q = 0; q < 8; ++q) wb[q] = f.w[q];
+              for (int i = 0; i < 8; ++i) wb[i] = f.w[i];
             }
           }
 #pragma unroll
@@ -448,9 +433,35 @@ __global__ void __launch_bounds__(kX16Threads, 1) gemv_x16_kernel(const GemvPara
               mma_step<kMmaBf16>(acc[c], wa[4 * h + 2], wb[4 * h + 2], wa[4 * h + 3], wb[4 * h + 3], xv[c].z, xv[c].w);
             }
           }
+          xo += kXStep, lim += 64u << 8;
+        };
+        auto open_block = [&] {
+          base_a = *base_at_a * 0x01010101u, base_b = *base_at_b * 0x01010101u;
+        };
+        auto next_block = [&] {
+          row_a += 192, row_b += 192, ++base_at_a, ++base_at_b;
+        };
+        int s = a;
+        if (s & 1) {  // the slice begins in the second half of a block
+          open_block();
+          step(std::integral_constant<uint32_t, 1>{});
+          next_block();
+          ++s;
         }
-        s += kX16Batch;
-      } while (s < b);
+#pragma unroll 1
+        for (; s + 1 < b; s += 2) {
+          open_block();
+          step(std::integral_constant<uint32_t, 0>{});
+          step(std::integral_constant<uint32_t, 1>{});
+          next_block();
+        }
+        if (s < b) {  // and ends in the first half of one
+          open_block();
+          step(std::integral_constant<uint32_t, 0>{});
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(empty_bar(ring.slot));
       ring.advance(R.S);
     }
     if (!R.whole && lane == 0) mbar_arrive(hempty_bar(hs));  // after the __syncwarp of the last stage: every lane has read its bases
