@@ -14,7 +14,7 @@
 //      bf16(silu(gate) * up) to each member pair's row of the workspace.
 //   2. down: a block belongs to one (token, 16 or 8 output rows); a warp takes two or one and sums the token's top_k experts in k order in
 //      registers and writes out[t, l].
-// Each (pair, row) sum is two lane-ordered chains of fmaf over k (even and odd values) followed by a fixed shuffle tree, whatever else the
+// Each (pair, row) sum is one lane-ordered chain of fmaf over k followed by a fixed shuffle tree, whatever else the
 // block serves, which is what makes the rows batch-invariant and BF16X equal to bf16 bit for bit (both walk 8 values
 // per lane per step).
 #include <cuda_runtime.h>
@@ -95,19 +95,9 @@ __device__ __forceinline__ Raw load_raw(const Stack& S, const uint8_t* row, cons
   }
 }
 
-// Pairs of f32 values, multiplied and added by one instruction each (fma.rn.f32x2: two chains of fmaf side by side).
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("{ .reg .b64 x, y, z; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mov.b64 z, {%6, %7};\n"
-      "fma.rn.f32x2 z, x, y, z; mov.b64 {%0, %1}, z; }"
-      : "=f"(d.x), "=f"(d.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-  return d;
-}
-
-// V activations from value k0 of a bf16 row as pairs of f32, zero past K.
+// V activations from value k0 of a bf16 row as f32, zero past K.
 template <int V>
-__device__ __forceinline__ void load_x(const uint16_t* x, int k0, int K, bool vec, float2 (&xf)[V / 2]) {
+__device__ __forceinline__ void load_x(const uint16_t* x, int k0, int K, bool vec, float (&xf)[V]) {
   if (vec && k0 + V <= K) {
 #pragma unroll
     for (int q = 0; q < V / 8; ++q) {
@@ -115,15 +105,13 @@ __device__ __forceinline__ void load_x(const uint16_t* x, int k0, int K, bool ve
       const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        xf[4 * q + j] = make_float2(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xffff0000u));
+        xf[8 * q + 2 * j] = __uint_as_float(w[j] << 16);
+        xf[8 * q + 2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
       }
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < V / 2; ++j) {
-      xf[j].x = k0 + 2 * j < K ? bf16_bits_to_f32(x[k0 + 2 * j]) : 0.0f;
-      xf[j].y = k0 + 2 * j + 1 < K ? bf16_bits_to_f32(x[k0 + 2 * j + 1]) : 0.0f;
-    }
+    for (int j = 0; j < V; ++j) xf[j] = k0 + j < K ? bf16_bits_to_f32(x[k0 + j]) : 0.0f;
   }
 }
 
@@ -145,10 +133,10 @@ __device__ __noinline__ uint32_t patched_exponent(const uint8_t* row, int K, int
   return e;
 }
 
-// acc += sum_j x[j] * value_j of the word, j ascending, even j in acc.x and odd j in acc.y (NVFP4: the block's sums times its scale).
+// acc += sum_j x[j] * value_j of the word, j ascending (NVFP4: the block's sum times its scale).
 template <int F>
-__device__ __forceinline__ float2 dot_word(const Raw& r, const float2 (&xf)[kLaneValues<F> / 2], float2 acc, const uint8_t* row, int k0,
-                                           int K) {
+__device__ __forceinline__ float dot_word(const Raw& r, const float (&xf)[kLaneValues<F>], float acc, const uint8_t* row, int k0,
+                                          int K) {
   constexpr int V = kLaneValues<F>;
   const uint32_t w[4] = {r.w.x, r.w.y, r.w.z, r.w.w};
   if constexpr (F == LX_W_BF16 || F == LX_W_BF16X) {
@@ -173,16 +161,17 @@ __device__ __forceinline__ float2 dot_word(const Raw& r, const float2 (&xf)[kLan
       }
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc = fma2(xf[j], make_float2(__uint_as_float(v[j] << 16), __uint_as_float(v[j] & 0xffff0000u)), acc);
+    for (int j = 0; j < 4; ++j) {
+      acc = fmaf(xf[2 * j], __uint_as_float(v[j] << 16), acc);
+      acc = fmaf(xf[2 * j + 1], __uint_as_float(v[j] & 0xffff0000u), acc);
+    }
   } else if constexpr (F == LX_W_INT8) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const uint32_t b = w[j] ^ 0x80808080u;  // byte + 128 in the mantissa of 2^23, then minus (2^23 + 128): exact
-      float f[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) f[i] = __uint_as_float(__byte_perm(b, 0x4b000000u, 0x7540 + i)) - 8388736.0f;
-      acc = fma2(xf[2 * j], make_float2(f[0], f[1]), acc);
-      acc = fma2(xf[2 * j + 1], make_float2(f[2], f[3]), acc);
+      for (int i = 0; i < 4; ++i)
+        acc = fmaf(xf[4 * j + i], __uint_as_float(0x4b000000u | ((b >> (8 * i)) & 0xffu)) - 8388736.0f, acc);
     }
   } else if constexpr (F == LX_W_FP8) {
 #pragma unroll
@@ -190,11 +179,13 @@ __device__ __forceinline__ float2 dot_word(const Raw& r, const float2 (&xf)[kLan
       uint32_t lo, hi;
       asm("{ .reg .b16 a, b; mov.b32 {a, b}, %2; cvt.rn.f16x2.e4m3x2 %0, a; cvt.rn.f16x2.e4m3x2 %1, b; }" : "=r"(lo), "=r"(hi) : "r"(w[j]));
       const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&lo)), f1 = __half22float2(*reinterpret_cast<const __half2*>(&hi));
-      acc = fma2(xf[2 * j], f0, acc);
-      acc = fma2(xf[2 * j + 1], f1, acc);
+      acc = fmaf(xf[4 * j], f0.x, acc);
+      acc = fmaf(xf[4 * j + 1], f0.y, acc);
+      acc = fmaf(xf[4 * j + 2], f1.x, acc);
+      acc = fmaf(xf[4 * j + 3], f1.y, acc);
     }
   } else {
-    float2 part = make_float2(0.0f, 0.0f);
+    float part = 0.0f;
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       uint32_t v[4];
@@ -203,10 +194,13 @@ __device__ __forceinline__ float2 dot_word(const Raw& r, const float2 (&xf)[kLan
           : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
           : "r"(w[q]));
 #pragma unroll
-      for (int i = 0; i < 4; ++i) part = fma2(xf[4 * q + i], __half22float2(*reinterpret_cast<const __half2*>(&v[i])), part);
+      for (int i = 0; i < 4; ++i) {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&v[i]));
+        part = fmaf(xf[8 * q + 2 * i], f.x, part);
+        part = fmaf(xf[8 * q + 2 * i + 1], f.y, part);
+      }
     }
-    const float scale = e4m3_to_f32(r.s & 0xffu);
-    acc = fma2(make_float2(scale, scale), part, acc);
+    acc = fmaf(e4m3_to_f32(r.s & 0xffu), part, acc);
   }
   (void)V;
   return acc;
@@ -262,7 +256,7 @@ __device__ __forceinline__ Raw load_whole(const uint8_t* at, const uint8_t* scal
 template <int F, int NR, int NT, bool WHOLE, int STEPS = 4>
 __device__ __forceinline__ void dot_rows(const Stack& S, const uint8_t* const (&row)[NR], const uint8_t* const (&row_scale)[NR],
                                          const uint32_t (&flag)[NR], const uint16_t* const (&x)[NT], bool xvec, int lane,
-                                         float2 (&acc)[NR][NT]) {
+                                         float (&acc)[NR][NT]) {
   constexpr int V = kLaneValues<F>;
   constexpr int kSteps = NT == 1 ? STEPS : 2;
   constexpr int kStep = 32 * V;  // values of K a step covers
@@ -293,7 +287,7 @@ __device__ __forceinline__ void dot_rows(const Stack& S, const uint8_t* const (&
         if (j >= left) break;
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
-          float2 xf[V / 2];
+          float xf[V];
           load_x<V>(xp[t] + j * kStep, 0, V, true, xf);
 #pragma unroll
           for (int r = 0; r < NR; ++r) acc[r][t] = dot_word<F>(raw[j][r], xf, acc[r][t], row[r], k_done + j * kStep + lane * V, K);
@@ -319,7 +313,7 @@ __device__ __forceinline__ void dot_rows(const Stack& S, const uint8_t* const (&
     }
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
-      float2 xf[V / 2];
+      float xf[V];
       load_x<V>(x[t], k0, F == LX_W_BF16X ? K : k0 + V, true, xf);
 #pragma unroll
       for (int r = 0; r < NR; ++r) acc[r][t] = dot_word<F>(raw[r], xf, acc[r][t], row[r], k0, K);
@@ -340,7 +334,7 @@ __device__ __forceinline__ void dot_rows(const Stack& S, const uint8_t* const (&
         if (k0 >= K) continue;
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
-          float2 xf[V / 2];
+          float xf[V];
           load_x<V>(x[t], k0, K, xvec, xf);
 #pragma unroll
           for (int r = 0; r < NR; ++r) acc[r][t] = dot_word<F>(raw[j][r], xf, acc[r][t], row[r], k0, K);
@@ -370,14 +364,14 @@ __device__ __forceinline__ void gate_up_members(const Stack& S, int e, int i, in
   const uint16_t* x[NT];
 #pragma unroll
   for (int t = 0; t < NT; ++t) x[t] = latent + static_cast<int64_t>(member[t < count ? t : 0] / top_k) * ld;
-  float2 acc[2][NT];
+  float acc[2][NT];
 #pragma unroll
-  for (int t = 0; t < NT; ++t) acc[0][t] = acc[1][t] = make_float2(0.0f, 0.0f);
+  for (int t = 0; t < NT; ++t) acc[0][t] = acc[1][t] = 0.0f;
   dot_rows<F, 2, NT, WHOLE, LEAN ? 2 : 4>(S, row, row_scale, flag, x, xvec, lane, acc);
   const float fg = stack_row_factor<F>(S, ng, e), fu = stack_row_factor<F>(S, nu, e);
 #pragma unroll
   for (int t = 0; t < NT; ++t) {
-    const float g = fg * warp_sum(acc[0][t].x + acc[0][t].y), u = fu * warp_sum(acc[1][t].x + acc[1][t].y);
+    const float g = fg * warp_sum(acc[0][t]), u = fu * warp_sum(acc[1][t]);
     if (lane == 0 && t < count)
       mid[static_cast<int64_t>(member[t]) * I + i] = static_cast<uint16_t>(f32_to_bf16_bits(g / (1.0f + expf(-g)) * u));
   }
@@ -441,20 +435,20 @@ __global__ void __launch_bounds__(kDecodeThreads, WHOLE && F != LX_W_BF16X ? 4 :
     int64_t n[ROWS];
     const uint8_t *row[ROWS], *row_scale[ROWS];
     uint32_t flag[ROWS];
-    float2 acc[ROWS][1];
+    float acc[ROWS][1];
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) {
       n[r] = static_cast<int64_t>(e) * S.rows + min(l0 + r, L - 1);  // (past the last row: that row again, not written)
       row[r] = S.data + n[r] * S.row_bytes;
       row_scale[r] = scale_row<F>(S, n[r]);
       flag[r] = row_flag<F>(row[r]);
-      acc[r][0] = make_float2(0.0f, 0.0f);
+      acc[r][0] = 0.0f;
     }
     const uint16_t* const x[1] = {mid + static_cast<int64_t>(p) * S.K};
     dot_rows<F, ROWS, 1, WHOLE>(S, row, row_scale, flag, x, xvec != 0, lane, acc);
 #pragma unroll
     for (int r = 0; r < ROWS; ++r)
-      total[r] = __fadd_rn(total[r], __fmul_rn(weights[p], __fmul_rn(stack_row_factor<F>(S, n[r], e), warp_sum(acc[r][0].x + acc[r][0].y))));
+      total[r] = __fadd_rn(total[r], __fmul_rn(weights[p], __fmul_rn(stack_row_factor<F>(S, n[r], e), warp_sum(acc[r][0]))));
   }
 #pragma unroll
   for (int r = 0; r < ROWS; ++r)
