@@ -37,16 +37,8 @@ constexpr int kPairCols = 256;      // the most accumulator columns per tile
 constexpr int kPairStageK = 128;    // bytes of K per stage: one swizzled box
 constexpr int kPairEpilogueWarps = 8, kPairThreads = (kPairEpilogueWarps + 3) * 32;
 constexpr int kPairABytes = 128 * kPairStageK;
-constexpr int kPairMaxCuts = 80;                            // tiles cut between pairs of SMs: at most one per pair
-constexpr int kPairCutFlags = 2 * kPairEpilogueWarps;       // a flag per epilogue warp of the two CTAs
-constexpr int kPairCutBytes = kPairTile * kPairCols * 4;    // its sums
 
 struct PairParams {
-  // Tiles that are cut between two pairs (see Pieces): their sums so far, and a flag per epilogue warp of a cut.
-  uint4* partial;           // [cut][CTA][warp][columns of a warp / 16][4][32 lanes]
-  int* flags;               // [cut][CTA][warp], zero when the kernel starts
-  int rounds;               // whole tiles every pair takes in turn before its share of the others
-  int64_t cut_bytes;
   const float* row_scale;   // f32 [N] (INT8 / FP8), null for BF16
   const float* inv_scales;  // per activation row, null when all are 1
   int N, M, n_stages;
@@ -105,89 +97,18 @@ __device__ __forceinline__ void pair_umma(uint32_t d_tmem, uint32_t a_lo, uint32
 #undef B200_PAIR_UMMA
 }
 
-// ---- who multiplies what -----------------------------------------------------------------------------------------------------
-// P.rounds whole tiles are dealt in turn. What is left (the last pairs + 1 .. 2 pairs - 1 tiles where they do not come out even) lies
-// on one line of stages that is cut into equal shares, so that no pair waits for the last turn of others. A share is at least one
-// tile long: it begins with the end of a tile, of which it multiplies the FIRST stages of K, goes on with whole tiles and ends
-// with the beginning of one, of which it multiplies the last. The first stages are therefore done early by one pair and the last ones late
-// by the pair before it, which takes the sums over: the f32 accumulators travel through the workspace as they are, so that a row's
-// bits do not depend on where a tile is cut. The pair that waits is the one with the lower number, and pairs are numbered against
-// the order in which the grid starts: the pair waited for is running already, and what it leaves it leaves before it waits itself.
-struct Piece {
-  int tile, s0, s1;  // stages [s0, s1) of K
-  int in, out;       // the cut whose sums it goes on from, or leaves its own at; -1: none
-};
-constexpr int kPairMinPiece = 4;  // cuts nearer than this many stages to a tile's end move there
-struct Pieces {
-  int pair, pairs, left, n, rounds;
-  int at, end;  // this pair's share of the line, in stages from tile rounds * pairs on
-  int round = 0;
-  __device__ __forceinline__ int cut(int p) const {
-    if (left < pairs) return min(p, left) * n;  // fewer tiles than pairs: whole ones
-    const int u = static_cast<int>(static_cast<int64_t>(left) * n * p / pairs), r = u % n;
-    return r < kPairMinPiece ? u - r : n - r < kPairMinPiece ? u - r + n : u;
-  }
-  __device__ __forceinline__ Pieces(const PairParams& P, int pair, int pairs);
-  // The next piece; false when there is none.
-  __device__ __forceinline__ bool next(Piece& p) {
-    if (round < rounds) {
-      p = Piece{pair + round * pairs, 0, n, -1, -1};
-      ++round;
-      return true;
-    }
-    if (at >= end) return false;
-    const int k = at / n, first = k * n, last = min(first + n, end);
-    p.tile = rounds * pairs + k;
-    p.s0 = first + n - last;  // [at, last) of the line: the beginning of a tile that goes on in the next share is multiplied last
-    p.s1 = first + n - at;    // and the end of one first
-    p.in = last < first + n ? pair : -1;
-    p.out = at > first ? pair - 1 : -1;
-    at = last;
-    return true;
-  }
-};
-__device__ __forceinline__ Pieces::Pieces(const PairParams& P, int pair_, int pairs_)
-    : pair(pair_), pairs(pairs_), left(P.tiles - P.rounds * pairs_), n(P.n_stages), rounds(P.rounds) {
-  at = cut(pair), end = cut(pair + 1);
-}
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr), "r"(r[0]),
-               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]),
-               "r"(r[13]), "r"(r[14]), "r"(r[15])
-               : "memory");
-}
-// A wait for a flag that another pair's warp sets (at most 0.25 s, as tc_wait). All lanes of the warp call it and agree.
-__device__ __forceinline__ bool wait_flag(const int* flag, int lane, int* status) {
-  int v = 0;
-  if (lane == 0) {
-    const uint64_t t0 = global_timer_ns();
-    for (;;) {
-      asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
-      if (v) break;
-      if (global_timer_ns() - t0 > 250000000ull) {
-        if (status) atomicExch(status, kStatusTcWait);
-        break;
-      }
-    }
-  }
-  return __shfl_sync(0xffffffffu, v, 0) != 0;
-}
-
 // ---- activations, row-major by plane ------------------------------------------------------------------------------------
 // Block (chunk, u): 128 threads, each 16 bytes of K of every plane of activation row u (as tc_prep_kernel, which writes
 // core-matrix order); plane j of row u starts at out + (j * rows + u) * ld.
 template <int ACT, bool XBF, int MODE>
 __global__ void __launch_bounds__(128) pair_prep_kernel(const void* __restrict__ x, int ld_x, int rows, int K, int planes, int ld,
-                                                        uint8_t* __restrict__ out, float* __restrict__ inv_scales, int* __restrict__ flags,
-                                                        int n_flags) {
+                                                        uint8_t* __restrict__ out, float* __restrict__ inv_scales) {
   constexpr int kElem = act_elem(ACT), V = 16 / kElem;
   constexpr bool QUANT = MODE == kPrepQuant, AS_BF16 = XBF || MODE == kPrepRound;
   pdl_trigger();
   pdl_wait();  // the kernel before this one may still be reading the workspace
   __shared__ float part[4];
   const int u = blockIdx.y, tid = threadIdx.x;
-  if (u == 0 && blockIdx.x == 0)
-    for (int i = tid; i < n_flags; i += 128) flags[i] = 0;
   const int k0 = (blockIdx.x * 128 + tid) * V;
   const bool in_range = k0 < K;
   const int64_t row = static_cast<int64_t>(u) * ld_x;
@@ -221,13 +142,6 @@ __global__ void __launch_bounds__(128) pair_prep_kernel(const void* __restrict__
   else make_planes<ACT, AS_BF16, V>(v, sc, w);
   for (int j = 0; j < planes; ++j)
     *reinterpret_cast<uint4*>(out + static_cast<int64_t>(j * rows + u) * ld + static_cast<int64_t>(k0) * kElem) = make_uint4(w[j][0], w[j][1], w[j][2], w[j][3]);
-}
-
-// The flags of the cuts, where the activations need no preparation.
-__global__ void __launch_bounds__(256) pair_clear_kernel(int* __restrict__ flags, int n_flags) {
-  pdl_trigger();
-  pdl_wait();
-  for (int i = threadIdx.x; i < n_flags; i += 256) flags[i] = 0;
 }
 
 // ---- a tile's outputs ------------------------------------------------------------------------------------------------------
@@ -294,12 +208,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   auto empty_bar = [&](int s) { return bar0 + 8u * (S + s); };   // its products are done
   auto d_full = [&](int b) { return bar0 + 8u * (2 * S + b); };  // accumulator b is complete
   auto d_empty = [&](int b) { return bar0 + 8u * (2 * S + 2 + b); };  // (first CTA) read by the epilogue warps of both CTAs
-  const uint32_t d_filled = bar0 + 8u * (2 * S + 4);                  // (first CTA) the sums that a piece goes on from are in place
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S + 5);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S + 4);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_rank();
-  const int pairs = gridDim.x >> 1, pair = pairs - 1 - static_cast<int>(blockIdx.x >> 1);  // (Pieces: who waits for whom)
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int n_stages = P.n_stages;
 
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
@@ -310,7 +224,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       mbar_init(d_full(b), 1);
       mbar_init(d_empty(b), 2 * kPairEpilogueWarps);
     }
-    mbar_init(d_filled, 2 * kPairEpilogueWarps);
     mbar_init_fence();
   }
   if (warp == kPairEpilogueWarps + 1) {
@@ -334,10 +247,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       Ring r;
       bool ok = true, wrapped = false;
       int issued = 0;
-      Pieces pieces(P, pair, pairs);
-      for (Piece p; ok && pieces.next(p);) {
-        const int row = p.tile / P.col_tiles * kPairTile + static_cast<int>(rank) * 128;
-        for (int s = p.s0; s < p.s1; ++s) {
+      for (int tile = pair; tile < P.tiles && ok; tile += pairs) {
+        const int row = tile / P.col_tiles * kPairTile + static_cast<int>(rank) * 128;
+        for (int s = 0; s < n_stages; ++s) {
           if (wrapped && !tc_wait(empty_bar(r.slot), r.lap ^ 1u, P.status)) {
             ok = false;
             break;
@@ -361,10 +273,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       pdl_wait();  // they come from the kernel before this one
       Ring r;
       bool ok = true, wrapped = false;
-      Pieces pieces(P, pair, pairs);
-      for (Piece p; ok && pieces.next(p);) {
-        const int m0 = p.tile % P.col_tiles * 2 * P.half + static_cast<int>(rank) * P.half;
-        for (int s = p.s0; s < p.s1; ++s) {
+      for (int tile = pair; tile < P.tiles && ok; tile += pairs) {
+        const int m0 = tile % P.col_tiles * 2 * P.half + static_cast<int>(rank) * P.half;
+        for (int s = 0; s < n_stages; ++s) {
           if (wrapped && !tc_wait(empty_bar(r.slot), r.lap ^ 1u, P.status)) {
             ok = false;
             break;
@@ -387,20 +298,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       const uint32_t lo0 = ((ring0 & 0x3ffffu) >> 4) | (1u << 16);
       Ring r;
       bool ok = true;
-      Pieces pieces(P, pair, pairs);
-      int t = 0;
-      for (Piece p; ok && pieces.next(p); ++t) {
+      for (int tile = pair, t = 0; tile < P.tiles && ok; tile += pairs, ++t) {
         const int buf = t & 1;
         const uint32_t d_tmem = tmem_base + buf * kPairCols;
         if (t >= 2) {
           if (!tc_wait(d_empty(buf), ((t >> 1) - 1) & 1, P.status)) break;
           tc_fence_after();
         }
-        if (p.in >= 0) {  // (once: only a share's last piece goes on from sums)
-          if (!tc_wait(d_filled, 0, P.status)) break;
-          tc_fence_after();
-        }
-        for (int s = p.s0; s < p.s1; ++s) {
+        for (int s = 0; s < n_stages; ++s) {
           if (!tc_wait(full_bar(r.slot), r.lap, P.status)) {
             ok = false;
             break;
@@ -422,83 +327,29 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     const int row = quarter * 32 + lane;             // of this CTA's 128
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     pdl_wait();  // y and the activation scales come from earlier kernels
-    const int chunks = PLANES * P.half / 16, who = static_cast<int>(rank) * kPairEpilogueWarps + warp;  // this warp's columns, in 16s
-    auto sums_of = [&](int cut) { return P.partial + cut * (P.cut_bytes / 16) + static_cast<int64_t>(who * chunks) * 128 + lane; };
-    Pieces pieces(P, pair, pairs);
-    Piece p, ahead;
-    bool more = pieces.next(ahead);
-    // Where the next piece (the t-th) goes on from another pair's sums, they are put where it adds; that accumulator's last
-    // piece, the one before this, has been stored. False: given up.
-    auto take_over = [&](int t) {
-      if (!more || ahead.in < 0) return true;
-      if (!wait_flag(P.flags + ahead.in * kPairCutFlags + who, lane, P.status)) return false;
-      const uint4* from = sums_of(ahead.in);
-      const uint32_t to = lane_addr + (t & 1) * kPairCols + part * PLANES * P.half;
-      for (int c = 0; c < chunks; c += 2) {
-        uint32_t raw[2][16];
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          if (c + h < chunks) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const uint4 u = __ldcg(from + (c + h) * 128 + q * 32);
-              raw[h][4 * q] = u.x, raw[h][4 * q + 1] = u.y, raw[h][4 * q + 2] = u.z, raw[h][4 * q + 3] = u.w;
-            }
-          }
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          if (c + h < chunks) tmem_st16(to + 16 * (c + h), raw[h]);
-      }
-      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) pair_arrive_first(d_filled);
-      return true;
-    };
-    for (int t = 0; more; ++t) {
-      p = ahead;
-      more = pieces.next(ahead);
-      // under this piece's products; but sums that another pair waits for are left first
-      if (p.out < 0 && !take_over(t + 1)) break;
+    for (int tile = pair, t = 0; tile < P.tiles; tile += pairs, ++t) {
       const int buf = t & 1;
-      const uint32_t d_addr = lane_addr + buf * kPairCols + part * PLANES * P.half;
-      if (p.out >= 0) {  // the first stages of a tile that the pair before this one finishes
-        if (!tc_wait(d_full(buf), (t >> 1) & 1, P.status)) break;
-        tc_fence_after();
-        uint4* to = sums_of(p.out);
-        for (int c = 0; c < chunks; ++c) {
-          uint32_t raw[16];
-          tmem_ld16(d_addr + 16 * c, raw);
-          tmem_wait_ld();
-#pragma unroll
-          for (int q = 0; q < 4; ++q) __stcg(to + c * 128 + q * 32, make_uint4(raw[4 * q], raw[4 * q + 1], raw[4 * q + 2], raw[4 * q + 3]));
-        }
-        __threadfence();
-        __syncwarp();
-        if (lane == 0) asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(P.flags + p.out * kPairCutFlags + who), "r"(1) : "memory");
-        if (!take_over(t + 1)) break;
-      } else {
-        const int n = p.tile / P.col_tiles * kPairTile + static_cast<int>(rank) * 128 + row;
-        const int m0 = p.tile % P.col_tiles * 2 * P.half + part * P.half;
-        const int rows = min(P.half, P.M - m0);  // (none or fewer: the last tile of the columns is ragged)
-        const bool live = n < P.N;
-        float rf = 1.0f, bias = 0.0f;
-        if (live) {
-          if (P.row_scale) rf = P.row_scale[n];
-          if (P.bias) bias = load_f32(P.bias, P.bias_dtype, n);
-        }
-        float inv[4] = {1.0f, 1.0f, 1.0f, 1.0f};  // lane l: rows l, 32 + l, 64 + l, 96 + l of this half
-        if (P.inv_scales) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-            if (32 * q + lane < rows) inv[q] = P.inv_scales[m0 + 32 * q + lane];
-        }
-        if (!tc_wait(d_full(buf), (t >> 1) & 1, P.status)) break;
-        tc_fence_after();
-        const int64_t at = static_cast<int64_t>(m0) * P.ld_y + n;
-        if (P.y_dtype == LX_BF16) pair_store<kAct, PLANES, uint16_t>(P, static_cast<uint16_t*>(P.y) + at, d_addr, rows, live, rf, bias, inv);
-        else pair_store<kAct, PLANES, float>(P, static_cast<float*>(P.y) + at, d_addr, rows, live, rf, bias, inv);
+      const int n = tile / P.col_tiles * kPairTile + static_cast<int>(rank) * 128 + row;
+      const int m0 = tile % P.col_tiles * 2 * P.half + part * P.half;
+      const int rows = min(P.half, P.M - m0);  // (none or fewer: the last tile of the columns is ragged)
+      const bool live = n < P.N;
+      float rf = 1.0f, bias = 0.0f;
+      if (live) {
+        if (P.row_scale) rf = P.row_scale[n];
+        if (P.bias) bias = load_f32(P.bias, P.bias_dtype, n);
       }
+      float inv[4] = {1.0f, 1.0f, 1.0f, 1.0f};  // lane l: rows l, 32 + l, 64 + l, 96 + l of this half
+      if (P.inv_scales) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (32 * q + lane < rows) inv[q] = P.inv_scales[m0 + 32 * q + lane];
+      }
+      if (!tc_wait(d_full(buf), (t >> 1) & 1, P.status)) break;
+      tc_fence_after();
+      const uint32_t d_addr = lane_addr + buf * kPairCols + part * PLANES * P.half;
+      const int64_t at = static_cast<int64_t>(m0) * P.ld_y + n;
+      if (P.y_dtype == LX_BF16) pair_store<kAct, PLANES, uint16_t>(P, static_cast<uint16_t*>(P.y) + at, d_addr, rows, live, rf, bias, inv);
+      else pair_store<kAct, PLANES, float>(P, static_cast<float*>(P.y) + at, d_addr, rows, live, rf, bias, inv);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) pair_arrive_first(d_empty(buf));
@@ -511,19 +362,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 }
 
 // ---- host ------------------------------------------------------------------------------------------------------------------
-// What the busiest pair multiplies, in columns of products times stages, when `tiles` tiles of n stages and so many columns are
-// dealt out whole, or (cut) with the last ones cut between pairs. A product of fewer than ~160 columns is charged as that many:
-// its operands come in no faster (8 KB per SM at 256 columns, 6 KB at 128).
-constexpr int64_t kCutCost = 2000;  // leaving the sums and taking them over, ~2 us
-int64_t pair_cost(int64_t tiles, int n, int columns, int pairs, bool cut) {
-  const int64_t width = std::max(160, columns);
-  return cut ? (tiles * n + pairs - 1) / pairs * width + kCutCost : (tiles + pairs - 1) / pairs * n * width;
-}
-bool pair_cuts(int64_t tiles, int n, int columns, int pairs) {
-  return pairs <= kPairMaxCuts && tiles > pairs && tiles % pairs != 0 && pair_cost(tiles, n, columns, pairs, true) < pair_cost(tiles, n, columns, pairs, false);
-}
-// Activation rows per CTA and tile: the multiple of 8 or 16 with `planes` planes within 128 columns that costs least.
-int pair_half(int M, int N, int n, int planes, int pairs) {
+// Activation rows per CTA and tile: the multiple of 8 or 16 with `planes` planes within 128 columns for which the busiest pair
+// has the fewest columns of products. A product of fewer than ~160 columns is charged as that many: its operands come in
+// no faster (8 KB per SM at 256 columns, 6 KB at 128).
+int pair_half(int M, int N, int planes, int pairs) {
   const int step = planes == 2 ? 8 : 16;  // a product of a pair takes its columns in whole 32s
   const int most = 128 / planes / step * step;
   const int64_t row_tiles = (N + kPairTile - 1) / kPairTile;
@@ -531,7 +373,7 @@ int pair_half(int M, int N, int n, int planes, int pairs) {
   int64_t best_cost = -1;
   for (int h = most; h >= step; h -= step) {
     const int64_t tiles = row_tiles * ((M + 2 * h - 1) / (2 * h));
-    const int64_t cost = pair_cost(tiles, n, 2 * h * planes, pairs, pair_cuts(tiles, n, 2 * h * planes, pairs));
+    const int64_t cost = (tiles + pairs - 1) / pairs * std::max(160, 2 * h * planes);
     if (best_cost < 0 || cost < best_cost) best = h, best_cost = cost;
   }
   return best;
@@ -540,7 +382,7 @@ int pair_half(int M, int N, int n, int planes, int pairs) {
 template <int F, int PLANES>
 int launch_pair(const CUtensorMap& wmap, const CUtensorMap& xmap, const PairParams& P, int pairs, size_t smem, cudaStream_t stream) {
   if (int e = allow_big_smem<200 + F * 4 + PLANES>(tc_pair_kernel<F, PLANES>)) return e;
-  return launch_kernel(tc_pair_kernel<F, PLANES>, dim3(2 * static_cast<unsigned>(pairs)), dim3(kPairThreads), smem, stream, wmap, xmap, P);
+  return launch_kernel(tc_pair_kernel<F, PLANES>, dim3(2 * static_cast<unsigned>(std::min(P.tiles, pairs))), dim3(kPairThreads), smem, stream, wmap, xmap, P);
 }
 
 }  // namespace
@@ -548,10 +390,9 @@ int launch_pair(const CUtensorMap& wmap, const CUtensorMap& xmap, const PairPara
 // The most rows one call of the kernel takes (more come in passes of as many): bounds the workspace.
 constexpr int kPairMaxRows = 2048;
 
-// The activations with their scales, then the cuts: flags and sums.
-static int64_t pair_cuts_at(int64_t rows, int K) { return (rows * K * 3 + 15 + rows * 4 + 255) / 256 * 256; }  // int8: three planes of a byte
 int64_t pair_workspace_bytes(int M, int K) {
-  return pair_cuts_at(std::min(M, kPairMaxRows), K) + int64_t{kPairMaxCuts} * (kPairCutFlags * 4 + kPairCutBytes) + 256;
+  const int64_t rows = std::min(M, kPairMaxRows);
+  return rows * K * 3 + 15 + rows * 4 + 256;  // int8: three planes of a byte
 }
 
 // All of M, prepared activations and their scales in `workspace` (pair_workspace_bytes). kNotSupported: not a shape for this
@@ -575,7 +416,7 @@ int pair_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const
     P.n_stages = (K * elem + kPairStageK - 1) / kPairStageK;
     P.x_rows = rows;
     P.digit = act == kActS8 ? 0.0078125f : act == kActE4m3 ? 0.0625f : 1.0f;
-    P.half = pair_half(rows, N, P.n_stages, planes, pairs);
+    P.half = pair_half(rows, N, planes, pairs);
     P.b_bytes = planes * P.half * kPairStageK;
     P.col_tiles = (rows + 2 * P.half - 1) / (2 * P.half);
     P.tiles = (N + kPairTile - 1) / kPairTile * P.col_tiles;
@@ -585,19 +426,9 @@ int pair_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const
     P.alpha = alpha, P.beta = beta;
     P.status = status_word();
     if (w.type != LX_W_BF16) P.row_scale = static_cast<const float*>(w.scale);
-    const int grid_pairs = std::min(P.tiles, pairs);
-    const bool cuts = pair_cuts(P.tiles, P.n_stages, 2 * P.half * planes, pairs);
-    P.rounds = P.tiles / grid_pairs - (cuts ? 1 : 0);
-    const int n_flags = cuts ? grid_pairs * kPairCutFlags : 0;
-    uint8_t* const cuts_at = ws + pair_cuts_at(std::min(M, kPairMaxRows), K);
-    P.flags = reinterpret_cast<int*>(cuts_at);
-    P.partial = reinterpret_cast<uint4*>(cuts_at + kPairMaxCuts * kPairCutFlags * 4);
-    P.cut_bytes = kPairCutFlags * (planes * P.half / 16) * 2048;
     const bool in_place = w.type == LX_W_BF16 && x_bf16 && aligned(xrow, 16) && ld_x % 8 == 0;
     if (in_place) {
       if (int e = make_tile_map(&xmap, xrow, 2ll * K, rows, 128, P.half, 4, true, 2ll * ld_x)) return e;
-      if (cuts)
-        if (int e = launch_kernel(pair_clear_kernel, dim3(1), dim3(256), 0, stream, P.flags, n_flags)) return e;
     } else {
       const int64_t ld = static_cast<int64_t>(K) * elem;
       float* inv = reinterpret_cast<float*>(ws + (planes * rows * ld + 15) / 16 * 16);
@@ -605,8 +436,7 @@ int pair_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const
       const int per_block = 128 * 16 / elem;
       const dim3 grid((K + per_block - 1) / per_block, rows);
       auto prep = [&](auto kernel) {
-        return launch_kernel(kernel, grid, dim3(128), 0, stream, static_cast<const void*>(xrow), ld_x, rows, K, planes, static_cast<int>(ld), ws, inv,
-                             P.flags, n_flags);
+        return launch_kernel(kernel, grid, dim3(128), 0, stream, static_cast<const void*>(xrow), ld_x, rows, K, planes, static_cast<int>(ld), ws, inv);
       };
       int e;
       if (quantized) {
@@ -626,9 +456,9 @@ int pair_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const
     P.S = std::min(8, (200 * 1024) / stage);
     const size_t smem = std::max<size_t>(static_cast<size_t>(P.S) * stage + 1024, 120 * 1024);  // one CTA per SM: it takes all of tensor memory
     int e;
-    if (w.type == LX_W_BF16) e = launch_pair<LX_W_BF16, 1>(wmap, xmap, P, grid_pairs, smem, stream);
-    else if (w.type == LX_W_INT8) e = planes == 1 ? launch_pair<LX_W_INT8, 1>(wmap, xmap, P, grid_pairs, smem, stream) : launch_pair<LX_W_INT8, 3>(wmap, xmap, P, grid_pairs, smem, stream);
-    else e = planes == 1 ? launch_pair<LX_W_FP8, 1>(wmap, xmap, P, grid_pairs, smem, stream) : launch_pair<LX_W_FP8, 2>(wmap, xmap, P, grid_pairs, smem, stream);
+    if (w.type == LX_W_BF16) e = launch_pair<LX_W_BF16, 1>(wmap, xmap, P, pairs, smem, stream);
+    else if (w.type == LX_W_INT8) e = planes == 1 ? launch_pair<LX_W_INT8, 1>(wmap, xmap, P, pairs, smem, stream) : launch_pair<LX_W_INT8, 3>(wmap, xmap, P, pairs, smem, stream);
+    else e = planes == 1 ? launch_pair<LX_W_FP8, 1>(wmap, xmap, P, pairs, smem, stream) : launch_pair<LX_W_FP8, 2>(wmap, xmap, P, pairs, smem, stream);
     if (e) return e;
   }
   return kOk;
