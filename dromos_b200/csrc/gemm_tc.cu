@@ -182,14 +182,21 @@ __device__ __forceinline__ RowTerms row_terms(const TcParams& P, int tile, int r
   return t;
 }
 
-// The calling thread owns row r of the tile (accumulator lane r, its warp's lane quarter already in d_addr) and the
-// 8-row chunks of activations chunk0, chunk0 + chunk_step, ... inv_lo / inv_hi: lane l holds the inverse activation
+// The calling thread owns row r of the tile (accumulator lane r, its warp's lane quarter already in d_addr) and takes the
+// activations in chunks of 8 rows. inv_lo / inv_hi: lane l holds the inverse activation
 // scale of rows l and 32 + l. release_bar (0 = none) gets one arrival per warp as soon as the warp has read the
 // accumulator.
 // kPeers: the all-gather epilogue (stores into every rank's y) instead of the usual one (into P.y).
+// next: what y holds at the first chunk (first_old), asked for before the wait for the accumulator.
+template <bool kPeers>
+__device__ __forceinline__ void first_old(const TcParams& P, const RowTerms& T, float (&next)[8]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) next[j] = 0.0f;
+  if (!kPeers && P.beta != 0.0f && T.live) load_old(P, 0, T.n, next);
+}
 template <int F, bool kPeers>
-__device__ __forceinline__ void finish_tile(const TcParams& P, const RowTerms& T, uint32_t d_addr, int lane, int chunk0, int chunk_step,
-                                            float inv_lo, float inv_hi, uint32_t release_bar) {
+__device__ __forceinline__ void finish_tile(const TcParams& P, const RowTerms& T, uint32_t d_addr, int lane, float (&next)[8], float inv_lo,
+                                            float inv_hi, uint32_t release_bar) {
   constexpr int kAct = TcFmt<F>::kAct;
   const int Mp = P.Mp, chunks = Mp / 8;
   auto release = [&]() {
@@ -199,12 +206,11 @@ __device__ __forceinline__ void finish_tile(const TcParams& P, const RowTerms& T
   };
   uint32_t raw[3][8];
   const bool adds = !kPeers && P.beta != 0.0f && T.live;
-  float old[8] = {}, next[8] = {};  // y at this chunk and the next one
-  if (adds && chunk0 < chunks) load_old(P, chunk0 * 8, T.n, next);
-  for (int c = chunk0; c < chunks; c += chunk_step) {
+  float old[8];  // y at this chunk, next: at the one after
+  for (int c = 0; c < chunks; ++c) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) old[j] = next[j];
-    if (adds && c + chunk_step < chunks) load_old(P, (c + chunk_step) * 8, T.n, next);
+    if (adds && c + 1 < chunks) load_old(P, (c + 1) * 8, T.n, next);
 #pragma unroll
     for (int p = 0; p < 3; ++p)
       if (p < P.planes) tmem_ld8(d_addr + p * Mp + c * 8, raw[p]);
@@ -212,10 +218,9 @@ __device__ __forceinline__ void finish_tile(const TcParams& P, const RowTerms& T
 #pragma unroll
     for (int j = 0; j < 8; ++j) inv[j] = __shfl_sync(0xffffffffu, c < 4 ? inv_lo : inv_hi, (c * 8 + j) & 31);
     tmem_wait_ld();
-    if (c + chunk_step >= chunks) release();
+    if (c + 1 >= chunks) release();
     if (T.live) combine_and_store<kAct, kPeers>(P, raw, inv, c * 8, T.n, T.rf, T.bias, old);
   }
-  if (chunk0 >= chunks) release();
 }
 
 // The all-gather epilogue's hand-off. Every epilogue warp, once what it stored to the peers' buffers is visible
@@ -417,9 +422,11 @@ __global__ void __launch_bounds__(XMODE ? kOwnThreads : kDirectThreads, XMODE ? 
       for (int tile = tile_begin; tile < tile_end; ++tile) {
         const int t = tile - tile_begin, buf = t & 1;
         const RowTerms T = row_terms<F>(P, tile, r);
+        float old[8];
+        first_old<PEERS>(P, T, old);
         if (!tc_wait(d_full(buf), (t >> 1) & 1, P.status)) break;
         tc_fence_after();
-        finish_tile<F, PEERS>(P, T, lane_addr + buf * P.dstride, lane, 0, 1, inv_lo, inv_hi, d_empty(buf));
+        finish_tile<F, PEERS>(P, T, lane_addr + buf * P.dstride, lane, old, inv_lo, inv_hi, d_empty(buf));
       }
       if constexpr (PEERS) signal_peers(P, lane, cta_count);  // (a CTA whose wait gave up still counts itself: nobody hangs, the status word tells)
     } else {
@@ -565,9 +572,11 @@ __global__ void __launch_bounds__(XMODE ? kOwnThreads : kDirectThreads, XMODE ? 
       auto finish = [&](int tile) {
         const int t = tile - tile_begin, buf = t & 1;
         const RowTerms T = row_terms<F>(P, tile, r);
+        float old[8];
+        first_old<PEERS>(P, T, old);
         if (!tc_wait(d_full(buf), (t >> 1) & 1, P.status)) return false;
         tc_fence_after();
-        finish_tile<F, PEERS>(P, T, lane_addr + buf * P.dstride, lane, 0, 1, inv, 0.0f, d_empty(buf));
+        finish_tile<F, PEERS>(P, T, lane_addr + buf * P.dstride, lane, old, inv, 0.0f, d_empty(buf));
         return true;
       };
       Ring x[B];
