@@ -14,10 +14,12 @@
 //      bf16(silu(gate) * up) to each member pair's row of the workspace.
 //   2. down: a block belongs to one (token, 16 or 8 output rows); a warp takes two or one and sums the token's top_k experts in k order in
 //      registers and writes out[t, l].
-// Each (pair, row) sum is one lane-ordered chain of fmaf over k followed by a fixed shuffle tree, whatever else the
+// Each (pair, row) sum is one lane-ordered chain of fmaf over k (INT8: two, see Sum) followed by a fixed shuffle tree, whatever else the
 // block serves, which is what makes the rows batch-invariant and BF16X equal to bf16 bit for bit (both walk 8 values
 // per lane per step).
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 #include "launch.cuh"
 
@@ -133,10 +135,27 @@ __device__ __noinline__ uint32_t patched_exponent(const uint8_t* row, int K, int
   return e;
 }
 
+// What a lane adds up: one f32 sum; INT8 the sums of the even and of the odd values, two multiplications and additions per
+// instruction (fma.rn.f32x2). Whole calls, 64 experts, top 8, I = 1536, L = 4096: INT8, four / eight tokens 136 / 245 -> 117 / 203 us; 16 experts,
+// I = 768, L = 2048, two tokens 21.0 -> 16.0. The others lose by it: FP8, four tokens 102 -> 109 (its values come as pairs that have to be
+// copied into aligned registers), BF16 87 -> 92, NVFP4 and BF16X 123 and 533 either way.
+template <int F>
+using Sum = std::conditional_t<F == LX_W_INT8, float2, float>;
+__device__ __forceinline__ float whole(float s) { return s; }
+__device__ __forceinline__ float whole(float2 s) { return s.x + s.y; }
+__device__ __forceinline__ float2 fma2(float a0, float a1, float b0, float b1, float2 c) {
+  float2 d;
+  asm("{ .reg .b64 x, y, z; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mov.b64 z, {%6, %7};\n"
+      "fma.rn.f32x2 z, x, y, z; mov.b64 {%0, %1}, z; }"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a0), "f"(a1), "f"(b0), "f"(b1), "f"(c.x), "f"(c.y));
+  return d;
+}
+
 // acc += sum_j x[j] * value_j of the word, j ascending (NVFP4: the block's sum times its scale).
 template <int F>
-__device__ __forceinline__ float dot_word(const Raw& r, const float (&xf)[kLaneValues<F>], float acc, const uint8_t* row, int k0,
-                                          int K) {
+__device__ __forceinline__ Sum<F> dot_word(const Raw& r, const float (&xf)[kLaneValues<F>], Sum<F> acc, const uint8_t* row, int k0,
+                                           int K) {
   constexpr int V = kLaneValues<F>;
   const uint32_t w[4] = {r.w.x, r.w.y, r.w.z, r.w.w};
   if constexpr (F == LX_W_BF16 || F == LX_W_BF16X) {
@@ -169,9 +188,11 @@ __device__ __forceinline__ float dot_word(const Raw& r, const float (&xf)[kLaneV
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const uint32_t b = w[j] ^ 0x80808080u;  // byte + 128 in the mantissa of 2^23, then minus (2^23 + 128): exact
+      float f[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        acc = fmaf(xf[4 * j + i], __uint_as_float(0x4b000000u | ((b >> (8 * i)) & 0xffu)) - 8388736.0f, acc);
+      for (int i = 0; i < 4; ++i) f[i] = __uint_as_float(__byte_perm(b, 0x4b000000u, 0x7540 + i)) - 8388736.0f;
+      acc = fma2(xf[4 * j], xf[4 * j + 1], f[0], f[1], acc);
+      acc = fma2(xf[4 * j + 2], xf[4 * j + 3], f[2], f[3], acc);
     }
   } else if constexpr (F == LX_W_FP8) {
 #pragma unroll
@@ -256,7 +277,7 @@ __device__ __forceinline__ Raw load_whole(const uint8_t* at, const uint8_t* scal
 template <int F, int NR, int NT, bool WHOLE, int STEPS = 4>
 __device__ __forceinline__ void dot_rows(const Stack& S, const uint8_t* const (&row)[NR], const uint8_t* const (&row_scale)[NR],
                                          const uint32_t (&flag)[NR], const uint16_t* const (&x)[NT], bool xvec, int lane,
-                                         float (&acc)[NR][NT]) {
+                                         Sum<F> (&acc)[NR][NT]) {
   constexpr int V = kLaneValues<F>;
   constexpr int kSteps = NT == 1 ? STEPS : 2;
   constexpr int kStep = 32 * V;  // values of K a step covers
@@ -364,14 +385,14 @@ __device__ __forceinline__ void gate_up_members(const Stack& S, int e, int i, in
   const uint16_t* x[NT];
 #pragma unroll
   for (int t = 0; t < NT; ++t) x[t] = latent + static_cast<int64_t>(member[t < count ? t : 0] / top_k) * ld;
-  float acc[2][NT];
+  Sum<F> acc[2][NT];
 #pragma unroll
-  for (int t = 0; t < NT; ++t) acc[0][t] = acc[1][t] = 0.0f;
+  for (int t = 0; t < NT; ++t) acc[0][t] = acc[1][t] = Sum<F>{};
   dot_rows<F, 2, NT, WHOLE, LEAN ? 2 : 4>(S, row, row_scale, flag, x, xvec, lane, acc);
   const float fg = stack_row_factor<F>(S, ng, e), fu = stack_row_factor<F>(S, nu, e);
 #pragma unroll
   for (int t = 0; t < NT; ++t) {
-    const float g = fg * warp_sum(acc[0][t]), u = fu * warp_sum(acc[1][t]);
+    const float g = fg * warp_sum(whole(acc[0][t])), u = fu * warp_sum(whole(acc[1][t]));
     if (lane == 0 && t < count)
       mid[static_cast<int64_t>(member[t]) * I + i] = static_cast<uint16_t>(f32_to_bf16_bits(g / (1.0f + expf(-g)) * u));
   }
@@ -381,7 +402,7 @@ __device__ __forceinline__ void gate_up_members(const Stack& S, int e, int i, in
 // time (more members than two read the rows again, from L1 / L2: the registers of wider passes would halve the warps
 // an SM holds for the common case of one or two).
 template <int F, bool WHOLE, bool LEAN>
-__global__ void __launch_bounds__(kDecodeThreads, LEAN ? 4 : WHOLE && F == LX_W_BF16 ? 3 : 2) decode_gate_up_kernel(const Stack S, const uint16_t* __restrict__ latent, int ld,
+__global__ void __launch_bounds__(kDecodeThreads, LEAN ? (F == LX_W_INT8 ? 3 : 4) : WHOLE && F == LX_W_BF16 ? 3 : 2) decode_gate_up_kernel(const Stack S, const uint16_t* __restrict__ latent, int ld,
                                                                         int xvec, const int32_t* __restrict__ ids,
                                                                         uint16_t* __restrict__ mid, int P, int top_k, int I,
                                                                         int dedupe) {
@@ -435,20 +456,20 @@ __global__ void __launch_bounds__(kDecodeThreads, WHOLE && F != LX_W_BF16X ? 4 :
     int64_t n[ROWS];
     const uint8_t *row[ROWS], *row_scale[ROWS];
     uint32_t flag[ROWS];
-    float acc[ROWS][1];
+    Sum<F> acc[ROWS][1];
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) {
       n[r] = static_cast<int64_t>(e) * S.rows + min(l0 + r, L - 1);  // (past the last row: that row again, not written)
       row[r] = S.data + n[r] * S.row_bytes;
       row_scale[r] = scale_row<F>(S, n[r]);
       flag[r] = row_flag<F>(row[r]);
-      acc[r][0] = 0.0f;
+      acc[r][0] = Sum<F>{};
     }
     const uint16_t* const x[1] = {mid + static_cast<int64_t>(p) * S.K};
     dot_rows<F, ROWS, 1, WHOLE>(S, row, row_scale, flag, x, xvec != 0, lane, acc);
 #pragma unroll
     for (int r = 0; r < ROWS; ++r)
-      total[r] = __fadd_rn(total[r], __fmul_rn(weights[p], __fmul_rn(stack_row_factor<F>(S, n[r], e), warp_sum(acc[r][0]))));
+      total[r] = __fadd_rn(total[r], __fmul_rn(weights[p], __fmul_rn(stack_row_factor<F>(S, n[r], e), warp_sum(whole(acc[r][0])))));
   }
 #pragma unroll
   for (int r = 0; r < ROWS; ++r)
