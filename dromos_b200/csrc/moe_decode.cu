@@ -53,7 +53,7 @@ constexpr int kLaneValues = F == LX_W_BF16 || F == LX_W_BF16X ? 8 : 16;
 // A lane's bytes of one row and step, as loaded.
 struct Raw {
   uint4 w;     // BF16X: x, y = sign|mantissa bytes, z = 4-bit codes, w = the block's base exponent
-  uint32_t s;  // NVFP4: the block's scale byte; BF16X: 1 when the row has patches
+  uint32_t s;  // NVFP4: the block's scale byte; BF16X: 1 when a value of the word may be patched
 };
 
 __device__ __forceinline__ uint4 ldg16(const void* p) { return __ldg(static_cast<const uint4*>(p)); }
@@ -117,20 +117,41 @@ __device__ __forceinline__ void load_x(const uint16_t* x, int k0, int K, bool ve
   }
 }
 
-// The exponent a patch list gives value k of a BF16X row, or `e` when the list does not name it.
-__device__ __noinline__ uint32_t patched_exponent(const uint8_t* row, int K, int k, uint32_t e) {
+// The patch list of a BF16X row: in its header's slots (ascending, unused ones behind hold kNoPatch), or, for a row with more
+// patches than slots, in an overflow record behind the rows.
+struct PatchList {
+  const uint32_t* list;
+  int n;
+};
+__device__ __forceinline__ PatchList patch_list(const uint8_t* row, int K) {
   const uint32_t* list = reinterpret_cast<const uint32_t*>(row);
-  int n_list = x16::patch_slots(K);
-  const uint32_t s0 = list[0];
-  if (s0 & 0x80000000u) {  // the row's patches live in an overflow record behind the rows
-    const uint32_t* rec = reinterpret_cast<const uint32_t*>(row + static_cast<int64_t>(s0 & 0x7fffffffu) * 8);
-    n_list = static_cast<int>(rec[0]);
-    list = rec + 1;
+  const uint32_t s0 = __ldg(list);
+  if (s0 == x16::kNoPatch || !(s0 & 0x80000000u)) return PatchList{list, x16::patch_slots(K)};
+  const uint32_t* rec = reinterpret_cast<const uint32_t*>(row + static_cast<int64_t>(s0 & 0x7fffffffu) * 8);
+  return PatchList{rec + 1, static_cast<int>(__ldg(rec))};
+}
+// The positions of a row's first and last patch; (~0, 0) when it has none.
+__device__ __noinline__ uint2 patched_range(const uint8_t* row, int K) {
+  const PatchList p = patch_list(row, K);
+  uint2 range = make_uint2(~0u, 0u);
+  for (int i = p.n - 1; i >= 0; --i) {
+    const uint32_t last = __ldg(p.list + i);
+    if (last == x16::kNoPatch) continue;
+    range = make_uint2(__ldg(p.list) >> 8, last >> 8);
+    break;
   }
-  for (int i = 0; i < n_list; ++i) {
-    const uint32_t p = list[i];
-    if (p == x16::kNoPatch || (p >> 8) > static_cast<uint32_t>(k)) break;
-    if ((p >> 8) == static_cast<uint32_t>(k)) e = p & 0xffu;
+  return range;
+}
+// The exponents of the eight values from k0 on (a byte each) with the row's patches in place of theirs.
+__device__ __noinline__ uint2 patched_exponents(const uint8_t* row, int K, int k0, uint2 e) {
+  const PatchList p = patch_list(row, K);
+  for (int i = 0; i < p.n; ++i) {
+    const uint32_t patch = __ldg(p.list + i), at = (patch >> 8) - static_cast<uint32_t>(k0);
+    if (patch == x16::kNoPatch || (patch >> 8) >= static_cast<uint32_t>(k0) + 8u) break;
+    if (at >= 8u) continue;
+    const uint32_t sh = 8 * (at & 3), clear = ~(0xffu << sh), set = (patch & 0xffu) << sh;
+    if (at < 4) e.x = (e.x & clear) | set;
+    else e.y = (e.y & clear) | set;
   }
   return e;
 }
@@ -138,7 +159,7 @@ __device__ __noinline__ uint32_t patched_exponent(const uint8_t* row, int K, int
 // What a lane adds up: one f32 sum; INT8 the sums of the even and of the odd values, two multiplications and additions per
 // instruction (fma.rn.f32x2). Whole calls, 64 experts, top 8, I = 1536, L = 4096: INT8, four / eight tokens 136 / 245 -> 117 / 203 us; 16 experts,
 // I = 768, L = 2048, two tokens 21.0 -> 16.0. The others lose by it: FP8, four tokens 102 -> 109 (its values come as pairs that have to be
-// copied into aligned registers), BF16 87 -> 92, NVFP4 and BF16X 123 and 533 either way.
+// copied into aligned registers), BF16 87 -> 92, NVFP4 and BF16X as long either way.
 template <int F>
 using Sum = std::conditional_t<F == LX_W_INT8, float2, float>;
 __device__ __forceinline__ float whole(float s) { return s; }
@@ -162,16 +183,9 @@ __device__ __forceinline__ Sum<F> dot_word(const Raw& r, const float (&xf)[kLane
     uint32_t v[4] = {w[0], w[1], w[2], w[3]};
     if constexpr (F == LX_W_BF16X) {  // four values at a time to the bf16 words they encode, then like those
       const uint32_t base4 = w[3] * 0x01010101u;
-      uint32_t e[2] = {base4 - (w[2] & 0x0f0f0f0fu), base4 - ((w[2] >> 4) & 0x0f0f0f0fu)};
-      if (r.s) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int sh = 8 * (j & 3);
-          const uint32_t p = patched_exponent(row, K, k0 + j, (e[j >> 2] >> sh) & 0xffu);
-          e[j >> 2] = (e[j >> 2] & ~(0xffu << sh)) | (p << sh);
-        }
-      }
-      const uint2 lo = x16_assemble(w[0], e[0]), hi = x16_assemble(w[1], e[1]);
+      uint2 e = make_uint2(base4 - (w[2] & 0x0f0f0f0fu), base4 - ((w[2] >> 4) & 0x0f0f0f0fu));
+      if (r.s) e = patched_exponents(row, K, k0, e);
+      const uint2 lo = x16_assemble(w[0], e.x), hi = x16_assemble(w[1], e.y);
       v[0] = lo.x, v[1] = lo.y, v[2] = hi.x, v[3] = hi.y;
       if (k0 + 8 > K) {  // padding of the last block decodes to 2^(base - 127), not to zero
 #pragma unroll
@@ -239,12 +253,16 @@ template <int F>
 __device__ __forceinline__ const uint8_t* scale_row(const Stack& S, int64_t n) {
   return F == LX_W_NVFP4 ? S.scale + n * (S.K / 16) : nullptr;
 }
-// BF16X: whether the row has patches (Raw::s of its words)
+// BF16X: the values of a row from its first to its last patch; a word outside needs no look at the list. (One row in six of 4096 N(0, 0.02)
+// values has a patch, seldom two. While such a row's every value was looked up, four tokens of 64 experts, I = 768, took 534 us; 198 now.)
 template <int F>
-__device__ __forceinline__ uint32_t row_flag(const uint8_t* row) {
-  if constexpr (F == LX_W_BF16X) return __ldg(reinterpret_cast<const uint32_t*>(row)) != x16::kNoPatch;
-  else return 0;
+__device__ __forceinline__ uint2 patches_of(const uint8_t* row, int K) {
+  if constexpr (F == LX_W_BF16X) {
+    if (__ldg(reinterpret_cast<const uint32_t*>(row)) != x16::kNoPatch) return patched_range(row, K);
+  }
+  return make_uint2(~0u, 0u);
 }
+__device__ __forceinline__ uint32_t may_have_patches(uint2 range, int k0) { return static_cast<uint32_t>(k0) + 8u > range.x && static_cast<uint32_t>(k0) <= range.y; }
 
 // A lane's word of a step that lies whole within the row, its address a running pointer: no bounds, no test of the alignment.
 // (`row` and k0 are for BF16X, whose three pieces of a word are found from the value's place in its record.)
@@ -276,7 +294,7 @@ __device__ __forceinline__ Raw load_whole(const uint8_t* at, const uint8_t* scal
 // fma.rn.f32.f16 (128, but one token 61 where this took 53: the part has no such instruction and converts both operands).
 template <int F, int NR, int NT, bool WHOLE, int STEPS = 4>
 __device__ __forceinline__ void dot_rows(const Stack& S, const uint8_t* const (&row)[NR], const uint8_t* const (&row_scale)[NR],
-                                         const uint32_t (&flag)[NR], const uint16_t* const (&x)[NT], bool xvec, int lane,
+                                         const uint2 (&patches)[NR], const uint16_t* const (&x)[NT], bool xvec, int lane,
                                          Sum<F> (&acc)[NR][NT]) {
   constexpr int V = kLaneValues<F>;
   constexpr int kSteps = NT == 1 ? STEPS : 2;
@@ -300,7 +318,7 @@ __device__ __forceinline__ void dot_rows(const Stack& S, const uint8_t* const (&
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
           raw[j][r] = load_whole<F>(at[r] + j * kStepBytes, scale_at[r] + j * 32, row[r], k_done + j * kStep + lane * V, hdr, slots);
-          if constexpr (F == LX_W_BF16X) raw[j][r].s = flag[r];
+          if constexpr (F == LX_W_BF16X) raw[j][r].s = may_have_patches(patches[r], k_done + j * kStep + lane * V);
         }
       }
 #pragma unroll
@@ -330,7 +348,7 @@ __device__ __forceinline__ void dot_rows(const Stack& S, const uint8_t* const (&
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
       raw[r] = load_whole<F>(at[r] + back / V * kWord, scale_at[r] + back / 16, row[r], k0, hdr, slots);
-      if constexpr (F == LX_W_BF16X) raw[r].s = flag[r];
+      if constexpr (F == LX_W_BF16X) raw[r].s = may_have_patches(patches[r], k0);
     }
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
@@ -347,7 +365,7 @@ __device__ __forceinline__ void dot_rows(const Stack& S, const uint8_t* const (&
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
           raw[j][r] = load_raw<F>(S, row[r], row_scale[r], k_base + (32 * j + lane) * V);
-          if constexpr (F == LX_W_BF16X) raw[j][r].s = flag[r];
+          if constexpr (F == LX_W_BF16X) raw[j][r].s = may_have_patches(patches[r], k_base + (32 * j + lane) * V);
         }
 #pragma unroll
       for (int j = 0; j < kSteps; ++j) {
@@ -381,14 +399,14 @@ __device__ __forceinline__ void gate_up_members(const Stack& S, int e, int i, in
   const int64_t ng = static_cast<int64_t>(e) * S.rows + i, nu = ng + I;
   const uint8_t* const row[2] = {S.data + ng * S.row_bytes, S.data + nu * S.row_bytes};
   const uint8_t* const row_scale[2] = {scale_row<F>(S, ng), scale_row<F>(S, nu)};
-  const uint32_t flag[2] = {row_flag<F>(row[0]), row_flag<F>(row[1])};
+  const uint2 patches[2] = {patches_of<F>(row[0], S.K), patches_of<F>(row[1], S.K)};
   const uint16_t* x[NT];
 #pragma unroll
   for (int t = 0; t < NT; ++t) x[t] = latent + static_cast<int64_t>(member[t < count ? t : 0] / top_k) * ld;
   Sum<F> acc[2][NT];
 #pragma unroll
   for (int t = 0; t < NT; ++t) acc[0][t] = acc[1][t] = Sum<F>{};
-  dot_rows<F, 2, NT, WHOLE, LEAN ? 2 : 4>(S, row, row_scale, flag, x, xvec, lane, acc);
+  dot_rows<F, 2, NT, WHOLE, LEAN ? 2 : 4>(S, row, row_scale, patches, x, xvec, lane, acc);
   const float fg = stack_row_factor<F>(S, ng, e), fu = stack_row_factor<F>(S, nu, e);
 #pragma unroll
   for (int t = 0; t < NT; ++t) {
@@ -455,18 +473,18 @@ __global__ void __launch_bounds__(kDecodeThreads, WHOLE && F != LX_W_BF16X ? 4 :
     const int p = t * top_k + k, e = ids[p];
     int64_t n[ROWS];
     const uint8_t *row[ROWS], *row_scale[ROWS];
-    uint32_t flag[ROWS];
+    uint2 patches[ROWS];
     Sum<F> acc[ROWS][1];
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) {
       n[r] = static_cast<int64_t>(e) * S.rows + min(l0 + r, L - 1);  // (past the last row: that row again, not written)
       row[r] = S.data + n[r] * S.row_bytes;
       row_scale[r] = scale_row<F>(S, n[r]);
-      flag[r] = row_flag<F>(row[r]);
+      patches[r] = patches_of<F>(row[r], S.K);
       acc[r][0] = Sum<F>{};
     }
     const uint16_t* const x[1] = {mid + static_cast<int64_t>(p) * S.K};
-    dot_rows<F, ROWS, 1, WHOLE>(S, row, row_scale, flag, x, xvec != 0, lane, acc);
+    dot_rows<F, ROWS, 1, WHOLE>(S, row, row_scale, patches, x, xvec != 0, lane, acc);
 #pragma unroll
     for (int r = 0; r < ROWS; ++r)
       total[r] = __fadd_rn(total[r], __fmul_rn(weights[p], __fmul_rn(stack_row_factor<F>(S, n[r], e), warp_sum(whole(acc[r][0])))));
