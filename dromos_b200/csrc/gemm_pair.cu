@@ -148,9 +148,21 @@ __global__ void __launch_bounds__(128) pair_prep_kernel(const void* __restrict__
 // The calling thread owns one weight row (accumulator lane) and `rows` activation rows from y on, P.ld_y apart; inv: lane l
 // holds the inverse scales of rows l, 32 + l, ... Sixteen rows at a time, the addresses in one running pointer: with an
 // index multiplied out per output the epilogue of a 128 x 256 tile took 10 us, longer than an FP8 tile's products.
-template <int kAct, int PLANES, typename Y>
-__device__ __forceinline__ void pair_store(const PairParams& P, Y* __restrict__ y, uint32_t d_addr, int rows, bool live, float rf, float bias,
-                                           const float (&inv)[4]) {
+// BETA: what y holds at up to sixteen of them. Those of the next sixteen are asked for before these are stored, the first before the
+// wait for the accumulator: asked for in turn, each sixteen cost a round trip to memory. (Kernels of their own: the 32 registers that
+// are in flight leave the next kernel in the stream no room beside this one's CTAs.)
+template <typename Y>
+__device__ __forceinline__ void pair_old(const PairParams& P, const Y* y, int rows, bool live, float (&old)[16]) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) old[j] = 0.0f;
+  if (!live) return;
+#pragma unroll
+  for (int j = 0; j < 16; ++j, y += P.ld_y)
+    if (j < rows) old[j] = sizeof(Y) == 4 ? static_cast<float>(*y) : bf16_bits_to_f32(static_cast<uint32_t>(*y));
+}
+template <int kAct, int PLANES, bool BETA, typename Y>
+__device__ __forceinline__ void pair_store(const PairParams& P, Y* y, uint32_t d_addr, int rows, bool live, float rf, float bias,
+                                           const float (&inv)[4], float (&next)[16]) {
   const int64_t ld = P.ld_y;
   auto value = [&](const uint32_t (&raw)[PLANES][16], int j, float scale) {
     float sum = 0.0f, digit = 1.0f;
@@ -163,7 +175,7 @@ __device__ __forceinline__ void pair_store(const PairParams& P, Y* __restrict__ 
     return P.alpha * (rf * (sum * scale) + bias);
   };
   auto put = [&](Y* at, float v, float old) {
-    if (P.beta != 0.0f) v = fmaf(P.beta, old, v);
+    if constexpr (BETA) v = fmaf(P.beta, old, v);
     if constexpr (sizeof(Y) == 4) *at = v;
     else *at = static_cast<uint16_t>(f32_to_bf16_bits(v));
   };
@@ -174,28 +186,25 @@ __device__ __forceinline__ void pair_store(const PairParams& P, Y* __restrict__ 
 #pragma unroll
     for (int p = 0; p < PLANES; ++p) tmem_ld16(d_addr + p * P.half + 16 * q, raw[p]);
     const int left = rows - 16 * q;
-    float old[16];  // with beta: all sixteen asked for before the first is stored (see gemm_tc.cu)
+    float old[16];
+    if constexpr (BETA) {
 #pragma unroll
-    for (int j = 0; j < 16; ++j) old[j] = 0.0f;
-    if (P.beta != 0.0f && live) {
-      const Y* from = y;
-#pragma unroll
-      for (int j = 0; j < 16; ++j, from += ld)
-        if (j < left) old[j] = sizeof(Y) == 4 ? static_cast<float>(*from) : bf16_bits_to_f32(static_cast<uint32_t>(*from));
+      for (int j = 0; j < 16; ++j) old[j] = next[j];
+      if (left > 16) pair_old(P, y + 16 * ld, left - 16, live, next);
     }
     tmem_wait_ld();
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       const float scale = PLANES == 1 && kAct == kActBf16 ? 1.0f : __shfl_sync(0xffffffffu, inv[q / 2], 16 * (q & 1) + j);
       const float v = value(raw, j, scale);
-      if (live && j < left) put(y, v, old[j]);
+      if (live && j < left) put(y, v, BETA ? old[j] : 0.0f);
       y += ld;
     }
   }
 }
 
 // ---- the product ----------------------------------------------------------------------------------------------------------
-template <int F, int PLANES>
+template <int F, int PLANES, bool BETA>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     tc_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const PairParams P) {
   constexpr int kAct = TcFmt<F>::kAct;
@@ -344,12 +353,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
         for (int q = 0; q < 4; ++q)
           if (32 * q + lane < rows) inv[q] = P.inv_scales[m0 + 32 * q + lane];
       }
-      if (!tc_wait(d_full(buf), (t >> 1) & 1, P.status)) break;
-      tc_fence_after();
       const uint32_t d_addr = lane_addr + buf * kPairCols + part * PLANES * P.half;
       const int64_t at = static_cast<int64_t>(m0) * P.ld_y + n;
-      if (P.y_dtype == LX_BF16) pair_store<kAct, PLANES, uint16_t>(P, static_cast<uint16_t*>(P.y) + at, d_addr, rows, live, rf, bias, inv);
-      else pair_store<kAct, PLANES, float>(P, static_cast<float*>(P.y) + at, d_addr, rows, live, rf, bias, inv);
+      float next[16];
+      if constexpr (BETA) {
+        if (P.y_dtype == LX_BF16) pair_old(P, static_cast<const uint16_t*>(P.y) + at, rows, live, next);
+        else pair_old(P, static_cast<const float*>(P.y) + at, rows, live, next);
+      }
+      if (!tc_wait(d_full(buf), (t >> 1) & 1, P.status)) break;
+      tc_fence_after();
+      if (P.y_dtype == LX_BF16) pair_store<kAct, PLANES, BETA, uint16_t>(P, static_cast<uint16_t*>(P.y) + at, d_addr, rows, live, rf, bias, inv, next);
+      else pair_store<kAct, PLANES, BETA, float>(P, static_cast<float*>(P.y) + at, d_addr, rows, live, rf, bias, inv, next);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) pair_arrive_first(d_empty(buf));
@@ -379,10 +393,14 @@ int pair_half(int M, int N, int planes, int pairs) {
   return best;
 }
 
+template <int F, int PLANES, bool BETA>
+int launch_pair(const CUtensorMap& wmap, const CUtensorMap& xmap, const PairParams& P, int pairs, size_t smem, cudaStream_t stream) {
+  if (int e = allow_big_smem<200 + F * 8 + PLANES * 2 + BETA>(tc_pair_kernel<F, PLANES, BETA>)) return e;
+  return launch_kernel(tc_pair_kernel<F, PLANES, BETA>, dim3(2 * static_cast<unsigned>(std::min(P.tiles, pairs))), dim3(kPairThreads), smem, stream, wmap, xmap, P);
+}
 template <int F, int PLANES>
 int launch_pair(const CUtensorMap& wmap, const CUtensorMap& xmap, const PairParams& P, int pairs, size_t smem, cudaStream_t stream) {
-  if (int e = allow_big_smem<200 + F * 4 + PLANES>(tc_pair_kernel<F, PLANES>)) return e;
-  return launch_kernel(tc_pair_kernel<F, PLANES>, dim3(2 * static_cast<unsigned>(std::min(P.tiles, pairs))), dim3(kPairThreads), smem, stream, wmap, xmap, P);
+  return P.beta != 0.0f ? launch_pair<F, PLANES, true>(wmap, xmap, P, pairs, smem, stream) : launch_pair<F, PLANES, false>(wmap, xmap, P, pairs, smem, stream);
 }
 
 }  // namespace
