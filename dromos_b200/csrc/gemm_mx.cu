@@ -27,10 +27,9 @@
 // column; up to 64 rows are 448 columns in two instructions of four and three digits. A launch takes up to 1024 rows in
 // chunks of at most 64, the chunks of a weight panel next to each other so that its later readers find it in L2.
 //
-// Measured (replayed graphs; before: the f16 expansion): 28672 x 8192, 16 / 32 / 48 / 64 rows 70.7 / 72.1 / 74.2 / 80.3 -> 43.2 / 48.1
-// / 62.7 / 77.5 us; 14336 x 4096, 64 / 100 / 500 / 1000 rows 26.8 / 49.5 / 205 / 406 -> 25.4 / 43.6 / 136 / 248; with an outlier in every
-// block, 28672 x 8192, 16 / 64 rows 81 / 139. What a stage takes at 16 rows is its copies (39 us with products and scales left out); at
-// 64 rows the 60 KB of digits that every SM fetches from L2 per 12 KB of weights. Error against 64 bits, N(0, 1) rows: 4e-8 at
+// Measured (replayed graphs; before: the f16 expansion): 28672 x 8192, 16 / 32 / 48 / 64 rows 70.7 / 72.1 / 74.2 / 80.3 -> 36.1 / 47.4
+// / 64.7 / 78.5 us; 14336 x 4096, 64 / 100 / 500 / 1000 rows 26.8 / 49.5 / 205 / 406 -> 25.4 / 43.6 / 136 / 248. At
+// 64 rows it is the 60 KB of digits that every SM fetches from L2 per 12 KB of weights. Error against 64 bits, N(0, 1) rows: 4e-8 at
 // every K (f16: 9e-8 at K = 512, 2.3e-6 at 8192); with an outlier of 2^6 .. 2^20 in every block, outputs whose weights are zero there:
 // 5e-8 .. 7.5e-7 at K = 8192 (f16: 2.3e-6; seven base-8 digits alone, as this kernel began: 4e-6 .. 0.4).
 //   * The block scales go to tensor memory with tcgen05.st. Written to shared memory for tcgen05.cp they needed the proxy fence,
@@ -56,7 +55,7 @@ constexpr int kMxDigits = 7;
 constexpr int kMxBase = 13;
 constexpr int kMxUnit = 23;                     // a block's values are whole numbers of 2^(e - kMxUnit), e the exponent of its largest
 constexpr int kMxThreads = 11 * 32;
-constexpr int kMxScaleBytes = 2 * 128 * 16;     // shared memory in which the scale warps exchange rows: two stages of 128 rows x 16 bytes
+constexpr int kMxScaleBytes = 2 * 128 * 16;     // shared memory in which the scale warps exchange rows, for each stage of a slot: two of 128 rows x 16 bytes
 constexpr int kAhead = 8;                       // stages whose weight scales a thread has in flight
 
 struct MxParams {
@@ -71,7 +70,7 @@ struct MxParams {
   int R, box_bytes;         // weight rows per tile; shared memory of a stage's box (1024-aligned)
   int Mp;                   // accumulator columns per digit
   int cols0, cols1;         // columns of a step's first instruction and of its second (0: one takes all digits)
-  int sf0, sf_stages;       // where in tensor memory the scales begin, and for how many stages in turn (4, 2 or 1)
+  int sf0, sf_turns;        // where in tensor memory the scales begin, and for how many slots in turn (4, 2 or 1)
   int x_bytes, sf_off;      // a stage's activations: digits, and from sf_off on the block scales
   const uint8_t* xprep;
   int64_t remainders;       // from a stage's digits to those of its remainders
@@ -321,16 +320,21 @@ __device__ __noinline__ float infinite_sum(const void* x, int x_bf16, const uint
 
 // ---- the product -------------------------------------------------------------------------------------------------------------
 // ATOMS: 128-column pieces of a step's activation scales; TWO: two instructions per step.
+// SUB: stages per slot of the rings. What bounds a product of few rows is neither copies nor products but what every role does once per
+// slot (waits, commits, the meeting of the scale warps and their store to tensor memory: ~650 ns, where the copies of a stage take 370
+// and its products 200), so up to 32 rows, where two or more slots of twice the size fit, a slot holds two stages: 28672 x 8192, 1 / 8 / 16 /
+// 24 / 32 rows 42.4 / 43.4 / 44.7 / 48.0 / 50.3 -> 34.0 / 34.9 / 36.1 / 44.3 / 47.4 us; 14336 x 4096 and 4096 x 4096, 16 rows 17.7 / 16.5 ->
+// 15.6 / 14.3. (Beyond, where a step is two instructions, a slot of two stages would take more than half of the shared memory.)
 // Tensor memory columns of a stage's scales: 4 products x 4 columns of the weights', then 4 x 4 per piece of the activations'.
-template <int ATOMS, bool TWO>
+template <int ATOMS, bool TWO, int SUB>
 __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_constant__ CUtensorMap wmap, const MxParams P) {
   extern __shared__ __align__(1024) uint8_t smem[];
   constexpr int kSfCols = 16 + 16 * ATOMS;
   const int SW = P.SW, SX = P.SX, x_bytes = P.x_bytes, box_bytes = P.box_bytes;
   // The tensor core reads 128 rows from every box, whatever R is: behind the boxes come the scales and the activations.
-  uint8_t* const sring = smem + static_cast<size_t>(SW) * box_bytes;
-  uint8_t* const xring = sring + kMxScaleBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(xring + static_cast<size_t>(SX) * x_bytes);
+  uint8_t* const sring = smem + static_cast<size_t>(SW) * SUB * box_bytes;
+  uint8_t* const xring = sring + SUB * kMxScaleBytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(xring + static_cast<size_t>(SX) * SUB * x_bytes);
   const uint32_t bar0 = smem_u32(bars);
   auto w_full = [&](int s) { return bar0 + 8u * s; };                       // weights landed
   auto w_empty = [&](int s) { return bar0 + 8u * (SW + s); };               // products done
@@ -353,14 +357,18 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
   const int tile_begin = static_cast<int>(static_cast<int64_t>(n_tiles) * blockIdx.x / gridDim.x);
   const int tile_end = static_cast<int>(static_cast<int64_t>(n_tiles) * (blockIdx.x + 1) / gridDim.x);
   const int groups = P.groups;
-  // stage(s, rest) for each of a chunk's stages in turn, then for those that go again; false as soon as one gives up
-  auto all_stages = [&](int chunk, auto&& stage) __attribute__((always_inline)) {
-    for (int s = 0; s < n_stages; ++s)
-      if (!stage(s, false)) return false;
+  // slot(s, second, rest) for each of a chunk's stages in turn (second: the other stage of a slot, n_stages if there is none), then for
+  // those that go again; false as soon as one gives up
+  auto all_slots = [&](int chunk, auto&& slot) __attribute__((always_inline)) {
+    for (int s = 0; s < n_stages; s += SUB)
+      if (!slot(s, SUB == 2 ? s + 1 : n_stages, false)) return false;
     if (!tc_wait(a_full, 0, P.status)) return false;
     const uint8_t* bits = again + chunk * groups;
-    for (int s = again_after(bits, n_stages, -1); s < n_stages; s = again_after(bits, n_stages, s))
-      if (!stage(s, true)) return false;
+    for (int s = again_after(bits, n_stages, -1); s < n_stages;) {
+      const int second = SUB == 2 ? again_after(bits, n_stages, s) : n_stages;
+      if (!slot(s, second, true)) return false;
+      s = again_after(bits, n_stages, SUB == 2 ? second : s);
+    }
     return true;
   };
 
@@ -403,16 +411,19 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
       int issued = 0;
       for (int tile = tile_begin; tile < tile_end && ok; ++tile) {
         const int row = tile / chunks * P.R, chunk = tile % chunks;
-        auto stage = [&](int s, bool) __attribute__((always_inline)) {
+        auto slot = [&](int s, int second, bool) __attribute__((always_inline)) {
           if (wrapped && !tc_wait(w_empty(w.slot), w.lap ^ 1u, P.status)) return false;
-          mbar_arrive_expect_tx(w_full(w.slot), P.R * 128);
-          tile_g2s(smem_u32(smem) + static_cast<uint32_t>(w.slot) * box_bytes, &wmap, s * 32, row, w_full(w.slot));
+          const bool both = SUB == 2 && second < n_stages;
+          const uint32_t dst = smem_u32(smem) + static_cast<uint32_t>(w.slot) * SUB * box_bytes;
+          mbar_arrive_expect_tx(w_full(w.slot), (both ? 2 : 1) * P.R * 128);
+          tile_g2s(dst, &wmap, s * 32, row, w_full(w.slot));
+          if (both) tile_g2s(dst + box_bytes, &wmap, second * 32, row, w_full(w.slot));
           ++issued;
           w.advance(SW);
           wrapped |= w.slot == 0;
           return true;
         };
-        ok = all_stages(chunk, stage);
+        ok = all_slots(chunk, slot);
       }
       if (!ok)  // the copies in flight land before the CTA leaves
         for (int i = max(0, issued - SW); i < issued; ++i) tc_wait(w_full(i % SW), (i / SW) & 1, P.status);
@@ -426,16 +437,20 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
       int i = 0, chunk = tile_begin % chunks;
       for (int tile = tile_begin; tile < tile_end && ok; ++tile) {
         const uint8_t* src = P.xprep + chunk * P.chunk_bytes;
-        auto stage = [&](int s, bool rest) __attribute__((always_inline)) {
+        auto slot = [&](int s, int second, bool rest) __attribute__((always_inline)) {
           if (wrapped && !tc_wait(x_empty(x.slot), x.lap ^ 1u, P.status)) return false;
-          mbar_arrive_expect_tx(x_full(x.slot), x_bytes);
-          bulk_g2s(smem_u32(xring) + static_cast<uint32_t>(x.slot) * x_bytes, src + (rest ? P.remainders : 0) + static_cast<size_t>(s) * x_bytes, x_bytes, x_full(x.slot));
+          const bool both = SUB == 2 && second < n_stages;
+          const uint32_t dst = smem_u32(xring) + static_cast<uint32_t>(x.slot) * SUB * x_bytes;
+          const uint8_t* from = src + (rest ? P.remainders : 0);
+          mbar_arrive_expect_tx(x_full(x.slot), (both ? 2 : 1) * x_bytes);
+          bulk_g2s(dst, from + static_cast<size_t>(s) * x_bytes, x_bytes, x_full(x.slot));
+          if (both) bulk_g2s(dst + x_bytes, from + static_cast<size_t>(second) * x_bytes, x_bytes, x_full(x.slot));
           ++i;
           x.advance(SX);
           wrapped |= x.slot == 0;
           return true;
         };
-        ok = all_stages(chunk, stage);
+        ok = all_slots(chunk, slot);
         if (++chunk == chunks) chunk = 0;
       }
       if (!ok)
@@ -455,7 +470,7 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
       const uint32_t b_step = (2u * lbo) >> 4, b_second = static_cast<uint32_t>(P.cols0 / 8) * 128 >> 4;
       Ring w, x;
       bool ok = true;
-      const uint32_t sf_mask = P.sf_stages - 1, sf_shift = P.sf_stages == 4 ? 2 : P.sf_stages == 2 ? 1 : 0;
+      const uint32_t sf_mask = P.sf_turns - 1, sf_shift = P.sf_turns == 4 ? 2 : P.sf_turns == 2 ? 1 : 0;
       uint32_t i = 0;
       int chunk = tile_begin % chunks;
       for (int tile = tile_begin, t = 0; tile < tile_end && ok; ++tile, ++t) {
@@ -463,18 +478,24 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
         const uint32_t d_tmem = tmem_base + buf * NC;
         if (use > 0 && !tc_wait(d_empty(buf), (use - 1) & 1, P.status)) break;
         tc_fence_after();
-        auto stage = [&](int s, bool rest) __attribute__((always_inline)) {
-          const uint32_t turn = i & sf_mask, sfa = tmem_base + P.sf0 + turn * kSfCols, sfb = sfa + 16;
+        auto slot = [&](int s, int second, bool rest) __attribute__((always_inline)) {
+          const uint32_t turn = i & sf_mask;
           if (!tc_wait(x_full(x.slot), x.lap, P.status) || !tc_wait(w_full(w.slot), w.lap, P.status) || !tc_wait(s_full(turn), (i >> sf_shift) & 1, P.status)) {
             return false;
           }
           tc_fence_after();
-          const uint32_t x_at = (static_cast<uint32_t>(x.slot) * x_bytes) >> 4;
-          const uint32_t a_lo = a_lo0 + ((static_cast<uint32_t>(w.slot) * box_bytes) >> 4), b_lo = b_lo0 + x_at;
 #pragma unroll
-          for (int ks = 0; ks < 4; ++ks) {
-            mx_umma(d_tmem, a_lo + 2 * ks, a_hi, b_lo + ks * b_step, b_hi, idesc0, sfa + 4 * ks, sfb + 4 * ATOMS * ks, (rest || (s | ks)) ? 1u : 0u);
-            if constexpr (TWO) mx_umma(d_tmem + P.cols0, a_lo + 2 * ks, a_hi, b_lo + ks * b_step + b_second, b_hi, idesc1, sfa + 4 * ks, sfb + 4 * ATOMS * ks, (rest || (s | ks)) ? 1u : 0u);
+          for (int h = 0; h < SUB; ++h) {
+            if (h > 0 && second >= n_stages) break;
+            const uint32_t sfa = tmem_base + P.sf0 + (turn * SUB + h) * kSfCols, sfb = sfa + 16;
+            const uint32_t x_at = ((static_cast<uint32_t>(x.slot) * SUB + h) * x_bytes) >> 4;
+            const uint32_t a_lo = a_lo0 + (((static_cast<uint32_t>(w.slot) * SUB + h) * box_bytes) >> 4), b_lo = b_lo0 + x_at;
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) {
+              const uint32_t adds = rest || (s | h | ks) ? 1u : 0u;
+              mx_umma(d_tmem, a_lo + 2 * ks, a_hi, b_lo + ks * b_step, b_hi, idesc0, sfa + 4 * ks, sfb + 4 * ATOMS * ks, adds);
+              if constexpr (TWO) mx_umma(d_tmem + P.cols0, a_lo + 2 * ks, a_hi, b_lo + ks * b_step + b_second, b_hi, idesc1, sfa + 4 * ks, sfb + 4 * ATOMS * ks, adds);
+            }
           }
           umma_commit(w_empty(w.slot));
           umma_commit(x_empty(x.slot));
@@ -484,7 +505,7 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
           ++i;
           return true;
         };
-        ok = all_stages(chunk, stage);
+        ok = all_slots(chunk, slot);
         if (ok) umma_commit(d_full(buf));
         if (++chunk == chunks) chunk = 0;
       }
@@ -507,51 +528,65 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
     Ring w, x;
     bool ok = true;
     uint32_t count = 0;  // stages so far
-    const uint32_t sf_mask = P.sf_stages - 1, sf_shift = P.sf_stages == 4 ? 2 : P.sf_stages == 2 ? 1 : 0;
-    // One stage: this thread's scales s to the tensor core; `fetch` asks for the ones that come later. (A warp whose wait gave up still
-    // comes to the meetings.)
-    auto stage = [&](uint4& s, auto&& fetch) __attribute__((always_inline)) {
+    const uint32_t sf_mask = P.sf_turns - 1, sf_shift = P.sf_turns == 4 ? 2 : P.sf_turns == 2 ? 1 : 0;
+    // One slot: this thread's scales of its stages to the tensor core (both: there is a second stage); `fetch` asks for the ones that
+    // come later. (A warp whose wait gave up still comes to the meetings.)
+    auto slot = [&](uint4 (&s)[SUB], bool both, auto&& fetch) __attribute__((always_inline)) {
       const uint32_t turn = count & sf_mask, use = count >> sf_shift;
-      if ((s.x | s.y | s.z | s.w) & 0x80808080u) {  // scales have no sign here: it goes to the block's values
-        ok = ok && tc_wait(w_full(w.slot), w.lap, P.status);
-        const uint32_t sc[4] = {s.x, s.y, s.z, s.w};
-        uint8_t* box = smem + static_cast<size_t>(w.slot) * box_bytes + r * 128;
-        for (int b = 0; b < 16 && ok && r < P.R; ++b)
-          if (sc[b >> 2] >> (8 * (b & 3)) & 0x80u) {
-            uint2* at = reinterpret_cast<uint2*>(box + (((b >> 1) ^ (r & 7)) << 4) + 8 * (b & 1));
-            *at = make_uint2(at->x ^ 0x88888888u, at->y ^ 0x88888888u);
-          }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor core reads what this thread wrote
+      uint4* rows = reinterpret_cast<uint4*>(sring) + (count & 1) * SUB * 128;  // (two slots in turn: one meeting per slot is enough)
+#pragma unroll
+      for (int h = 0; h < SUB; ++h) {
+        if (h > 0 && !both) break;
+        if ((s[h].x | s[h].y | s[h].z | s[h].w) & 0x80808080u) {  // scales have no sign here: it goes to the block's values
+          ok = ok && tc_wait(w_full(w.slot), w.lap, P.status);
+          const uint32_t sc[4] = {s[h].x, s[h].y, s[h].z, s[h].w};
+          uint8_t* box = smem + (static_cast<size_t>(w.slot) * SUB + h) * box_bytes + r * 128;
+          for (int b = 0; b < 16 && ok && r < P.R; ++b)
+            if (sc[b >> 2] >> (8 * (b & 3)) & 0x80u) {
+              uint2* at = reinterpret_cast<uint2*>(box + (((b >> 1) ^ (r & 7)) << 4) + 8 * (b & 1));
+              *at = make_uint2(at->x ^ 0x88888888u, at->y ^ 0x88888888u);
+            }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor core reads what this thread wrote
+        }
+        rows[h * 128 + r] = make_uint4(s[h].x & 0x7f7f7f7fu, s[h].y & 0x7f7f7f7fu, s[h].z & 0x7f7f7f7fu, s[h].w & 0x7f7f7f7fu);
       }
-      uint4* rows = reinterpret_cast<uint4*>(sring) + (count & 1) * 128;  // (two stages in turn: one meeting per stage is enough)
-      rows[r] = make_uint4(s.x & 0x7f7f7f7fu, s.y & 0x7f7f7f7fu, s.z & 0x7f7f7f7fu, s.w & 0x7f7f7f7fu);
       fetch(s);
       __syncwarp();
       named_bar_sync(1, 128);
-      uint32_t v[16];
+      uint32_t v[16], xv[ATOMS][16];
+      auto read_rows = [&](int h) __attribute__((always_inline)) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const uint4 u = rows[32 * c + lane];
-        v[c] = u.x, v[4 + c] = u.y, v[8 + c] = u.z, v[12 + c] = u.w;
-      }
-      // the activations' scales lie behind their digits as the four words of each lane and product
+        for (int c = 0; c < 4; ++c) {
+          const uint4 u = rows[h * 128 + 32 * c + lane];
+          v[c] = u.x, v[4 + c] = u.y, v[8 + c] = u.z, v[12 + c] = u.w;
+        }
+      };
+      auto read_x = [&](int h) __attribute__((always_inline)) {
+        // the activations' scales lie behind their digits as the four words of each lane and product
+        const uint4* xsf = reinterpret_cast<const uint4*>(xring + (static_cast<size_t>(x.slot) * SUB + h) * x_bytes + P.sf_off) + lane;
+#pragma unroll
+        for (int j = 0; j < 4 * ATOMS; ++j) {
+          const uint4 u = xsf[32 * j];
+          uint32_t* to = xv[j / 4] + 4 * (j % 4);
+          to[0] = u.x, to[1] = u.y, to[2] = u.z, to[3] = u.w;
+        }
+      };
+      read_rows(0);
       ok = ok && tc_wait(x_full(x.slot), x.lap, P.status);
-      const uint4* xsf = reinterpret_cast<const uint4*>(xring + static_cast<size_t>(x.slot) * x_bytes + P.sf_off) + lane;
-      uint32_t xv[ATOMS][16];
-#pragma unroll
-      for (int j = 0; j < 4 * ATOMS; ++j) {
-        const uint4 u = xsf[32 * j];
-        uint32_t* to = xv[j / 4] + 4 * (j % 4);
-        to[0] = u.x, to[1] = u.y, to[2] = u.z, to[3] = u.w;
-      }
+      read_x(0);  // before the wait for their place (the second stage's after: 154 registers leave the next preparation no room)
       if (use > 0 && ok) ok = tc_wait(s_empty(turn), (use - 1) & 1, P.status);
       ok = __all_sync(0xffffffffu, ok);
       if (ok) {
-        const uint32_t at = lane_addr + turn * kSfCols;
         tc_fence_after();
-        tmem_st16(at, v);
 #pragma unroll
-        for (int a = 0; a < ATOMS; ++a) tmem_st16(at + 16 + 16 * a, xv[a]);
+        for (int h = 0; h < SUB; ++h) {
+          if (h > 0 && !both) break;
+          if (h > 0) read_rows(h), read_x(h);
+          const uint32_t at = lane_addr + (turn * SUB + h) * kSfCols;
+          tmem_st16(at, v);
+#pragma unroll
+          for (int a = 0; a < ATOMS; ++a) tmem_st16(at + 16 + 16 * a, xv[a]);
+        }
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
@@ -567,23 +602,38 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
       const uint8_t* const bits = again + chunk * groups;
       for (int s0 = 0; s0 < n_stages; s0 += kAhead) {
 #pragma unroll
-        for (int i = 0; i < kAhead; ++i) {
+        for (int i = 0; i < kAhead; i += SUB) {
           if (s0 + i >= n_stages) break;
-          stage(q[i], [&](uint4& s) {  // stage s0 + i + kAhead, or stage i of the next tile
-            const bool here = s0 + i + kAhead < n_stages;
-            const uint4* from = here ? scales : scales_next;
-            if (from) s = __ldg(from + (here ? s0 + i + kAhead : i));
+          uint4 now[SUB];
+#pragma unroll
+          for (int h = 0; h < SUB; ++h) now[h] = q[i + h];
+          slot(now, SUB == 2 && s0 + i + 1 < n_stages, [&](uint4 (&)[SUB]) {  // stage s0 + i + kAhead, or stage i of the next tile
+#pragma unroll
+            for (int h = 0; h < SUB; ++h) {
+              const bool here = s0 + i + h + kAhead < n_stages;
+              const uint4* from = here ? scales : scales_next;
+              if (from && (here || i + h < n_stages)) q[i + h] = __ldg(from + (here ? s0 + i + h + kAhead : i + h));
+            }
           });
         }
       }
       if (!named_bar_and(1, 128, tc_wait(a_full, 0, P.status))) break;  // all four warps leave together
-      int a = again_after(bits, n_stages, -1);  // the stage that goes again next: its scales are asked for a stage ahead
-      uint4 ahead = a < n_stages && scales ? __ldg(scales + a) : make_uint4(0, 0, 0, 0);
+      // the stages that go again next: their scales are asked for a slot ahead
+      auto scales_at = [&](int a) { return a < n_stages && scales ? __ldg(scales + a) : make_uint4(0, 0, 0, 0); };
+      int a = again_after(bits, n_stages, -1), second = SUB == 2 ? again_after(bits, n_stages, a) : n_stages;
+      uint4 ahead[SUB];
+      ahead[0] = scales_at(a);
+      if constexpr (SUB == 2) ahead[1] = scales_at(second);
       while (a < n_stages) {
-        uint4 now = ahead;
-        a = again_after(bits, n_stages, a);
-        stage(now, [&](uint4&) {
-          if (a < n_stages && scales) ahead = __ldg(scales + a);
+        uint4 now[SUB];
+#pragma unroll
+        for (int h = 0; h < SUB; ++h) now[h] = ahead[h];
+        const bool both = SUB == 2 && second < n_stages;
+        a = again_after(bits, n_stages, SUB == 2 ? second : a);
+        second = SUB == 2 ? again_after(bits, n_stages, a) : n_stages;
+        slot(now, both, [&](uint4 (&)[SUB]) {
+          ahead[0] = scales_at(a);
+          if constexpr (SUB == 2) ahead[1] = scales_at(second);
         });
       }
       scales = scales_next;
@@ -739,8 +789,10 @@ int mx_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const v
     // tensor memory from its end: the scales, then the accumulators, more than one of each where they fit
     const int cols = L.cols0 + L.cols1;
     const int sf_cols = 16 + 16 * ((L.cols0 + 127) / 128);
-    P.sf_stages = cols + 4 * sf_cols <= kTmemColumns ? 4 : cols + 2 * sf_cols <= kTmemColumns ? 2 : 1;
-    P.sf0 = kTmemColumns - P.sf_stages * sf_cols;
+    const bool two_atoms = L.cols0 > 128;
+    const int sub = L.cols1 ? 1 : 2;  // stages per slot: see the kernel
+    P.sf_turns = cols + 4 * sub * sf_cols <= kTmemColumns ? 4 : cols + 2 * sub * sf_cols <= kTmemColumns ? 2 : 1;
+    P.sf0 = kTmemColumns - P.sf_turns * sub * sf_cols;
     P.buffers = 2 * cols <= P.sf0 ? 2 : 1;
     P.remainders = P.chunks * P.chunk_bytes;
     P.groups = (K / kMxStageK + 7) / 8;
@@ -759,14 +811,13 @@ int mx_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const v
     // A ring of as many stages of activations as of weights: a block of them, the same for every SM, travels as long as the weights
     // do. Where that is fewer than four, the weights keep six.
     const int tail = std::max(1024, 448 + P.chunks * P.groups);  // barriers, and the stages that go again
-    const int room = 224 * 1024 - kMxScaleBytes - tail;
-    const int even = room / (P.box_bytes + L.x_bytes);
-    P.SX = even >= 4 ? std::min(8, even) : std::max(2, std::min(4, (room - 6 * P.box_bytes) / L.x_bytes));
-    P.SW = std::min(12, (room - P.SX * L.x_bytes) / P.box_bytes);
+    const int room = 224 * 1024 - sub * kMxScaleBytes - tail, box = sub * P.box_bytes, block = sub * L.x_bytes;
+    const int even = room / (box + block);
+    P.SX = sub == 2 ? std::max(2, std::min(6, even)) : even >= 4 ? std::min(8, even) : std::max(2, std::min(4, (room - 6 * P.box_bytes) / L.x_bytes));
+    P.SW = std::min(12, (room - P.SX * block) / box);
     if (P.SW < 2) return kNotSupported;
-    const size_t smem = std::max<size_t>(static_cast<size_t>(P.SW) * P.box_bytes + kMxScaleBytes + static_cast<size_t>(P.SX) * L.x_bytes + tail, 120 * 1024);
-    const bool two_atoms = L.cols0 > 128;
-    auto kernel = !two_atoms ? tc_mx_kernel<1, false> : L.cols1 ? tc_mx_kernel<2, true> : tc_mx_kernel<2, false>;
+    const size_t smem = std::max<size_t>(static_cast<size_t>(P.SW) * box + sub * kMxScaleBytes + static_cast<size_t>(P.SX) * block + tail, 120 * 1024);
+    auto kernel = !two_atoms ? tc_mx_kernel<1, false, 2> : L.cols1 ? tc_mx_kernel<2, true, 1> : tc_mx_kernel<2, false, 2>;
     if (int e = !two_atoms ? allow_big_smem<300>(kernel) : L.cols1 ? allow_big_smem<301>(kernel) : allow_big_smem<302>(kernel)) return e;
     const int tiles = (N + P.R - 1) / P.R * P.chunks;
     if (int e = launch_kernel(kernel, dim3(std::min(tiles, sms)), dim3(kMxThreads), smem, stream, wmap, P)) return e;
