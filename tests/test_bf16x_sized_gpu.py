@@ -14,7 +14,7 @@ from tests import util
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("rows,K,every", [(1, 128, 0), (9, 1000, 0), (5, 1024, 2), (300, 1000, 7), (3000, 512, 1), (2, 8192, 1)])
+@pytest.mark.parametrize("rows,K,every", [(1, 128, 0), (9, 1000, 0), (5, 1024, 2), (300, 1000, 7), (3000, 512, 1), (2, 8192, 1), (6000, 256, 1)])
 def test_size_and_bytes(lx, rows, K, every):
     w = util.bf16_normal((rows, K), 0.02, rows)
     if every:
