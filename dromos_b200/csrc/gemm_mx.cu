@@ -736,20 +736,25 @@ struct MxLayout {
 // The most rows one launch takes (more come in launches of as many): bounds the workspace.
 constexpr int kMxMaxRows = 1024;
 
-// Chunks of the fewest that hold M rows, all of the same size (a multiple of 8).
-static int mx_chunk_rows(int M) {
-  const int chunks = (M + kMaxRows - 1) / kMaxRows;
+// The fewest chunks of at most `most` rows that hold M, all of the same size (a multiple of 8).
+constexpr int kMxChunkMost[] = {kMaxRows, 32, 16};
+static int mx_chunk_rows(int M, int most) {
+  const int chunks = (M + most - 1) / most;
   return ((M + chunks - 1) / chunks + 7) / 8 * 8;
 }
+// What a stage of a tile takes with so many activation rows, in tens of ns (28672 x 8192, two tiles per SM).
+static int mx_stage_cost(int rows) { return rows <= 16 ? 49 : rows <= 24 ? 61 : rows <= 32 ? 66 : 88 + (rows - 40) * 11 / 10; }
 
 int64_t mx_workspace_bytes(int M, int K) {
   int64_t need = 0;
   for (int rows : {std::min(M, kMxMaxRows), M % kMxMaxRows}) {  // a launch of the most rows, and the last one
     if (rows == 0) continue;
-    const int chunk = mx_chunk_rows(rows);
-    const MxLayout L(chunk);
-    const int stages = (K + kMxStageK - 1) / kMxStageK;
-    need = std::max(need, static_cast<int64_t>((rows + chunk - 1) / chunk) * (int64_t{2} * stages * L.x_bytes + (stages + 7) / 8 * kMaxRows) + 4 * rows + 256);
+    for (int most : kMxChunkMost) {  // (which of them N decides)
+      const int chunk = mx_chunk_rows(rows, most);
+      const MxLayout L(chunk);
+      const int stages = (K + kMxStageK - 1) / kMxStageK;
+      need = std::max(need, static_cast<int64_t>((rows + chunk - 1) / chunk) * (int64_t{2} * stages * L.x_bytes + (stages + 7) / 8 * kMaxRows) + 4 * rows + 256);
+    }
   }
   return need;
 }
@@ -776,15 +781,22 @@ int mx_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const v
   P.xprep = ws;
   for (int first = 0; first < M; first += kMxMaxRows) {
     P.M = std::min(kMxMaxRows, M - first);
-    P.chunk_rows = mx_chunk_rows(P.M);
+    // Chunks of up to 64 rows, or of 32 or 16 where the busiest SM is done sooner with more, shorter tiles: a weight of few rows
+    // leaves most SMs without a tile otherwise. (A row's bits do not depend on its chunk.)
+    auto turns_of = [&](int R, int chunk) { return (static_cast<int64_t>((N + R - 1) / R) * ((P.M + chunk - 1) / chunk) + sms - 1) / sms; };
+    int64_t least = -1;
+    for (int most : kMxChunkMost) {
+      const int chunk = mx_chunk_rows(P.M, most);
+      const int64_t cost = std::min(turns_of(kBM, chunk), turns_of(even_rows, chunk)) * mx_stage_cost(chunk);
+      if (least < 0 || cost < least) least = cost, P.chunk_rows = chunk;
+    }
     P.chunks = (P.M + P.chunk_rows - 1) / P.chunk_rows;
     const MxLayout L(P.chunk_rows);
     P.Mp = L.Mp, P.cols0 = L.cols0, P.cols1 = L.cols1, P.sf_off = L.sf_off, P.x_bytes = L.x_bytes;
     P.chunk_bytes = static_cast<int64_t>(K / kMxStageK) * L.x_bytes;
     // A tile takes as long with 128 weight rows as with fewer (its steps do), so what counts is the busiest SM's tiles; rows dealt
     // evenly where that is the same.
-    auto turns = [&](int R) { return (static_cast<int64_t>((N + R - 1) / R) * P.chunks + sms - 1) / sms; };
-    P.R = turns(kBM) < turns(even_rows) ? kBM : even_rows;
+    P.R = turns_of(kBM, P.chunk_rows) < turns_of(even_rows, P.chunk_rows) ? kBM : even_rows;
     P.box_bytes = (P.R + 7) / 8 * 1024;
     // tensor memory from its end: the scales, then the accumulators, more than one of each where they fit
     const int cols = L.cols0 + L.cols1;
