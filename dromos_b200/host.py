@@ -74,13 +74,14 @@ def store_weight(lib: abi.Library, w_bf16: torch.Tensor, wtype: int) -> StoredWe
         return StoredWeight(wtype, w_bf16, rows=rows, cols=cols)
     if wtype == abi.W_BF16X:
         if lib.has("lx_b200_bf16x_encode_sized"):
-            # one pass over the matrix: few have overflow records, so the buffer is first one without (sizing 14336 x 4096
-            # before encoding it cost 40 of 150 us)
-            n = max(rows * lib.lx_bf16x_row_bytes(cols), 8)
+            # one pass over the matrix (sizing 14336 x 4096 before encoding it cost 40 of 150 us), into a buffer with room for the
+            # overflow records of some rows (one matrix in 20 of that size has a row with more patches than slots)
+            n = rows * lib.lx_bf16x_row_bytes(cols)
+            n = max(n + min(1 << 18, n >> 6), 8)
             data, need = torch.empty(n, dtype=torch.uint8, device=w_bf16.device), ctypes.c_int64(0)
             st = lib.lx_b200_bf16x_encode_sized(abi.ptr(w_bf16), rows, cols, abi.ptr(data), n, ctypes.byref(need), _stream())
             if st == 0:
-                return StoredWeight(wtype, data, rows=rows, cols=cols)
+                return StoredWeight(wtype, data[: need.value], rows=rows, cols=cols)
             if st != abi.ERR_SCRATCH:
                 raise RuntimeError(f"lx_b200_bf16x_encode_sized failed: {st}")
             n, data = need.value, None
