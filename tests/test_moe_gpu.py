@@ -151,6 +151,45 @@ def test_token_bits_do_not_depend_on_batch(lx):
     assert np.array_equal(outs[1], outs[8][:1]) and np.array_equal(outs[3], outs[8][:3])
 
 
+@pytest.mark.parametrize("wtype", [O.W_BF16, O.W_INT8, O.W_FP8], ids=lambda w: NAMES[w])
+@pytest.mark.parametrize("T", [32, 160])  # 160: more than 1024 pairs, grouped by the other kernel
+def test_calls_with_other_routings_on_one_workspace(lx, wtype, T):
+    """Calls one behind the other, nothing between them, whose routings differ in everything: how many chunks there are, which experts
+    they belong to. The tables lie at the same addresses in each, and the weights are asked for before the activations are ready: each
+    call has to stream the experts of its own routing."""
+    L, I, E, top_k = 512, 256, 64, 8
+    gu, dn = (util.DeviceWeight(O.quantize_weight(util.bf16_normal(s, 0.02, 1), wtype)) for s in ((E, 2 * I, L), (E, L, I)))
+    latent = util.dev(util.bf16_normal((T, L), 1.0, 3))
+    weights = util.dev(np.abs(util.f32_normal((T, top_k), 1.0, 4)))
+    rng = np.random.default_rng(5)
+    routings = [np.stack([rng.permutation(E)[:top_k] for _ in range(T)]) for _ in range(4)]          # spread over all experts
+    routings += [np.tile(rng.permutation(E)[:top_k], (T, 1)) for _ in range(4)]                      # the same eight for every token
+    routings += [np.stack([first + rng.permutation(top_k) for _ in range(T)]) for first in (0, 56)]  # the first eight, the last eight
+    ids = [util.dev(np.ascontiguousarray(r, dtype=np.int32)) for r in routings]
+    nbytes = lx.lx_moe_grouped_workspace_bytes(T, L, I, E, top_k, 0)
+
+    def call(i, ws, out):
+        assert lx.lx_moe_experts_grouped(abi.ptr(latent), abi.ptr(ids[i]), abi.ptr(weights), gu.ref(), dn.ref(), 0, abi.ptr(out), abi.ptr(ws), T, L, I,
+                                         E, top_k, util.stream_ptr()) == 0
+
+    def workspace():
+        return torch.full((nbytes,), 0xFF, dtype=torch.uint8, device="cuda")
+
+    order = [int(i) for i in rng.integers(0, len(ids), 40)]
+    alone, together = (torch.full((n, T, L), float("nan"), device="cuda") for n in (len(ids), len(order)))
+    for i in range(len(ids)):
+        call(i, workspace(), alone[i])
+        torch.cuda.synchronize()
+    shared = workspace()
+    torch.cuda.synchronize()
+    for n, i in enumerate(order):
+        call(i, shared, together[n])
+    util.check_status(lx)
+    assert not bool(torch.isnan(alone).any())
+    for n, (i, y) in enumerate(zip(order, together)):
+        assert torch.equal(y, alone[i]), f"call {n}, routing {i}"
+
+
 def router_case(lx, M, E, K, top_k, with_bias, seed, tie=False):
     rng = np.random.default_rng(seed)
     ld_x = K + 3
