@@ -490,6 +490,12 @@ extern "C" int lx_b200_gemv_ring_plan(int wtype, int K, int M, int x_is_bf16, in
   return kOk;
 }
 
+// How lx_gemm_w cuts a product on NVFP4 weights up (gemm_mx.cu), without launching anything: the function the launches use.
+extern "C" int lx_b200_gemm_mx_plan(int M, int N, int K, int sms, int32_t* out) {
+  if (!out || M < 1 || M > 1024 || N < 1 || K <= 0 || K % 256 != 0 || sms < 1) return kInvalid;
+  return mx_plan_numbers(M, N, K, sms, tile_rows(N, sms), out);
+}
+
 extern "C" int lx_b200_wait_arrivals(int* counter, int total, void* stream) {
   if (!counter || total <= 0) return kInvalid;
   return tc_wait_arrivals(counter, total, static_cast<cudaStream_t>(stream));

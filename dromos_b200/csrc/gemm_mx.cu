@@ -58,6 +58,26 @@ constexpr int kMxThreads = 11 * 32;
 constexpr int kMxScaleBytes = 2 * 128 * 16;     // shared memory in which the scale warps exchange rows, for each stage of a slot: two of 128 rows x 16 bytes
 constexpr int kAhead = 8;                       // stages whose weight scales a thread has in flight
 
+// How a chunk's rows lie in accumulator columns and in the workspace. An instruction has at most 256 columns, in whole 16s. A stage's
+// activations are its digits and, from sf_off on, its block scales: as they go to tensor memory, those of whole 128 columns per product (64
+// values of K), or (compact, what small chunks take) those of sf_rows rows, a word each.
+struct MxLayout {
+  int Mp = 0;                // accumulator columns per digit
+  int cols0 = 0, cols1 = 0;  // columns of a step's first instruction and of its second (0: one takes all digits)
+  int sf_off = 0, sf_rows = 0, x_bytes = 0;
+  static constexpr __host__ __device__ int compact_rows(bool two_atoms) { return two_atoms ? 32 : 16; }  // as many as chunks of the same kernel can have
+  MxLayout() = default;
+  explicit MxLayout(int rows, int compact_as = 0) {
+    auto whole = [](int c) { return (c + 15) / 16 * 16; };
+    Mp = (rows + 7) / 8 * 8;
+    cols0 = whole(kMxDigits * Mp);
+    if (cols0 > 256) cols0 = 4 * Mp, cols1 = whole((kMxDigits - 4) * Mp);  // four digits, then the rest
+    sf_off = (cols0 + cols1) * (kMxStageK / 2);
+    sf_rows = compact_as;
+    x_bytes = sf_off + (compact_as ? 16 * compact_as : 4 * ((cols0 + 127) / 128) * 512);
+  }
+};
+
 struct MxParams {
   const void* x;            // the activations themselves, for rows with infinities
   int x_bf16, ld_x;
@@ -68,10 +88,8 @@ struct MxParams {
   int chunks, chunk_rows;   // the activation rows are multiplied in chunks of at most 64
   int64_t chunk_bytes;      // a chunk's prepared activations
   int R, box_bytes;         // weight rows per tile; shared memory of a stage's box (1024-aligned)
-  int Mp;                   // accumulator columns per digit
-  int cols0, cols1;         // columns of a step's first instruction and of its second (0: one takes all digits)
+  MxLayout lay[2];          // the chunks' and the last one's, which may have fewer rows
   int sf0, sf_turns;        // where in tensor memory the scales begin, and for how many slots in turn (4, 2 or 1)
-  int x_bytes, sf_off;      // a stage's activations: digits, and from sf_off on the block scales
   const uint8_t* xprep;
   int64_t remainders;       // from a stage's digits to those of its remainders
   const uint8_t* again;     // [chunks][groups][64]: bit b of byte (c, g, m): row m of chunk c has remainders in stage 8 g + b
@@ -148,8 +166,8 @@ __device__ __forceinline__ float exp2_of(int e) { return __uint_as_float(e >= -1
 constexpr int kPrepThreads = 256;  // (at most 40 registers each: a block fits beside the product's CTA and starts under its end. With 48,
                                    // and 140 in the product, it did not: 14336 x 4096 at 32 rows 23 us instead of 19)
 template <bool XBF>
-__global__ void __launch_bounds__(kPrepThreads, 6) mx_prep_kernel(const void* __restrict__ x, int ld_x, int K, int chunk_rows, int64_t chunk_bytes, int Mp, int cols0,
-                                                               int cols1, int x_bytes, int sf_off, uint8_t* __restrict__ out, int64_t remainders,
+__global__ void __launch_bounds__(kPrepThreads, 6) mx_prep_kernel(const void* __restrict__ x, int ld_x, int K, int chunks, int chunk_rows, int64_t chunk_bytes,
+                                                               const MxLayout lay, const MxLayout lay_last, uint8_t* __restrict__ out, int64_t remainders,
                                                                uint8_t* __restrict__ again, float* __restrict__ row_scale) {
   pdl_trigger();
   __shared__ uint32_t part[kPrepThreads / 32], stages_again;
@@ -235,8 +253,10 @@ __global__ void __launch_bounds__(kPrepThreads, 6) mx_prep_kernel(const void* __
   }
   if (tid == 0) again[(static_cast<int64_t>(chunk) * gridDim.x + blockIdx.x) * kMaxRows + m] = static_cast<uint8_t>(stages);
   if (k0 >= K) return;
-  uint8_t* stage = out + chunk * chunk_bytes + static_cast<size_t>(k0 / kMxStageK) * x_bytes;
-  const int kb = (k0 % kMxStageK) / 2, NC = cols0 + cols1, atoms = (cols0 + 127) / 128;
+  const bool last = chunk + 1 == chunks;
+  const int Mp = last ? lay_last.Mp : lay.Mp, NC = last ? lay_last.cols0 + lay_last.cols1 : lay.cols0 + lay.cols1;
+  uint8_t* stage = out + chunk * chunk_bytes + static_cast<size_t>(k0 / kMxStageK) * (last ? lay_last.x_bytes : lay.x_bytes);
+  const int kb = (k0 % kMxStageK) / 2;
 #pragma unroll
   for (int j = 0; j < kMxDigits; ++j) *reinterpret_cast<uint32_t*>(stage + block_offset(NC, kb & ~15, j * Mp + m) + (kb & 15)) = w[j];
   const bool block_rest = (with_rest >> (tid & 30) & 3u) != 0;  // this thread's eight values' or its neighbour's
@@ -258,9 +278,18 @@ __global__ void __launch_bounds__(kPrepThreads, 6) mx_prep_kernel(const void* __
     }
   }
   if (k0 % 16 != 0) return;
-  // scales: product k0 / 64 of the stage; 128 columns are 32 lanes of 16 bytes, a column's 4 bytes at word column / 32
   const uint8_t sf = static_cast<uint8_t>(finite ? ue4m3_pow2(e - e_row + 8) : 0x38u), sf_rest = static_cast<uint8_t>(block_rest ? ue4m3_pow2(zeros - 9) : 0u);
-  uint8_t* sfs = stage + sf_off + (k0 % kMxStageK) / 64 * (atoms * 512) + (k0 % 64) / 16;
+  uint8_t* sfs = stage + (last ? lay_last.sf_off : lay.sf_off) + (k0 % 64) / 16;
+  const int product = (k0 % kMxStageK) / 64;
+  if (lay.sf_rows) {  // once for all digits of the row
+    const int at = product * (4 * lay.sf_rows) + 4 * m;
+    sfs[at] = sf;
+    sfs[remainders + at] = sf_rest;
+    return;
+  }
+  // 128 columns are 32 lanes of 16 bytes, a column's 4 bytes at word column / 32
+  const int cols0 = lay.cols0, atoms = (cols0 + 127) / 128;
+  sfs += product * (atoms * 512);
 #pragma unroll
   for (int j = 0; j < kMxDigits; ++j) {
     const int c = j * Mp + m;
@@ -325,16 +354,17 @@ __device__ __noinline__ float infinite_sum(const void* x, int x_bf16, const uint
 // and its products 200), so up to 32 rows, where two or more slots of twice the size fit, a slot holds two stages: 28672 x 8192, 1 / 8 / 16 /
 // 24 / 32 rows 42.4 / 43.4 / 44.7 / 48.0 / 50.3 -> 34.0 / 34.9 / 36.1 / 44.3 / 47.4 us; 14336 x 4096 and 4096 x 4096, 16 rows 17.7 / 16.5 ->
 // 15.6 / 14.3. (Beyond, where a step is two instructions, a slot of two stages would take more than half of the shared memory.)
+// COMPACT: the activations' scales come once per row, and the last chunk may have fewer rows (see mx_cut).
 // Tensor memory columns of a stage's scales: 4 products x 4 columns of the weights', then 4 x 4 per piece of the activations'.
-template <int ATOMS, bool TWO, int SUB>
+template <int ATOMS, bool TWO, int SUB, bool COMPACT>
 __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_constant__ CUtensorMap wmap, const MxParams P) {
   extern __shared__ __align__(1024) uint8_t smem[];
   constexpr int kSfCols = 16 + 16 * ATOMS;
-  const int SW = P.SW, SX = P.SX, x_bytes = P.x_bytes, box_bytes = P.box_bytes;
+  const int SW = P.SW, SX = P.SX, x_slot = P.lay[0].x_bytes, box_bytes = P.box_bytes;
   // The tensor core reads 128 rows from every box, whatever R is: behind the boxes come the scales and the activations.
   uint8_t* const sring = smem + static_cast<size_t>(SW) * SUB * box_bytes;
   uint8_t* const xring = sring + SUB * kMxScaleBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(xring + static_cast<size_t>(SX) * SUB * x_bytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(xring + static_cast<size_t>(SX) * SUB * x_slot);
   const uint32_t bar0 = smem_u32(bars);
   auto w_full = [&](int s) { return bar0 + 8u * s; };                       // weights landed
   auto w_empty = [&](int s) { return bar0 + 8u * (SW + s); };               // products done
@@ -437,14 +467,15 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
       int i = 0, chunk = tile_begin % chunks;
       for (int tile = tile_begin; tile < tile_end && ok; ++tile) {
         const uint8_t* src = P.xprep + chunk * P.chunk_bytes;
+        const int x_bytes = P.lay[COMPACT && chunk + 1 == chunks].x_bytes;
         auto slot = [&](int s, int second, bool rest) __attribute__((always_inline)) {
           if (wrapped && !tc_wait(x_empty(x.slot), x.lap ^ 1u, P.status)) return false;
           const bool both = SUB == 2 && second < n_stages;
-          const uint32_t dst = smem_u32(xring) + static_cast<uint32_t>(x.slot) * SUB * x_bytes;
+          const uint32_t dst = smem_u32(xring) + static_cast<uint32_t>(x.slot) * SUB * x_slot;
           const uint8_t* from = src + (rest ? P.remainders : 0);
           mbar_arrive_expect_tx(x_full(x.slot), (both ? 2 : 1) * x_bytes);
           bulk_g2s(dst, from + static_cast<size_t>(s) * x_bytes, x_bytes, x_full(x.slot));
-          if (both) bulk_g2s(dst + x_bytes, from + static_cast<size_t>(second) * x_bytes, x_bytes, x_full(x.slot));
+          if (both) bulk_g2s(dst + x_slot, from + static_cast<size_t>(second) * x_bytes, x_bytes, x_full(x.slot));
           ++i;
           x.advance(SX);
           wrapped |= x.slot == 0;
@@ -459,15 +490,11 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
   } else if (warp == 9) {
     // ================================ issuer ================================
     if (lane == 0) {
-      const int NC = P.cols0 + P.cols1;
       // e2m1 x e2m1, ue4m3 scales, 128 rows
       const uint32_t idesc = (1u << 7) | (1u << 10) | (1u << 27);
-      const uint32_t idesc0 = idesc | (static_cast<uint32_t>(P.cols0 >> 3) << 17), idesc1 = idesc | (static_cast<uint32_t>(P.cols1 >> 3) << 17);
-      const uint32_t lbo = static_cast<uint32_t>(NC / 8) * 128, sbo = 128;
+      const uint32_t sbo = 128;
       const uint32_t a_hi = (1024u >> 4) | (1u << 14) | (2u << 29), b_hi = (sbo >> 4) | (1u << 14);
       const uint32_t a_lo0 = ((smem_u32(smem) & 0x3ffffu) >> 4) | (1u << 16);
-      const uint32_t b_lo0 = ((smem_u32(xring) & 0x3ffffu) >> 4) | ((lbo >> 4) << 16);
-      const uint32_t b_step = (2u * lbo) >> 4, b_second = static_cast<uint32_t>(P.cols0 / 8) * 128 >> 4;
       Ring w, x;
       bool ok = true;
       const uint32_t sf_mask = P.sf_turns - 1, sf_shift = P.sf_turns == 4 ? 2 : P.sf_turns == 2 ? 1 : 0;
@@ -475,7 +502,12 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
       int chunk = tile_begin % chunks;
       for (int tile = tile_begin, t = 0; tile < tile_end && ok; ++tile, ++t) {
         const int buf = P.buffers == 2 ? t & 1 : 0, use = P.buffers == 2 ? t >> 1 : t;  // this accumulator's use-th use
-        const uint32_t d_tmem = tmem_base + buf * NC;
+        const MxLayout& L = P.lay[COMPACT && chunk + 1 == chunks];
+        const uint32_t cols0 = L.cols0, cols1 = L.cols1, lbo = (cols0 + cols1) / 8 * 128;
+        const uint32_t idesc0 = idesc | (cols0 >> 3 << 17), idesc1 = idesc | (cols1 >> 3 << 17);
+        const uint32_t b_lo0 = ((smem_u32(xring) & 0x3ffffu) >> 4) | ((lbo >> 4) << 16);
+        const uint32_t b_step = (2u * lbo) >> 4, b_second = cols0 / 8 * 128 >> 4;
+        const uint32_t d_tmem = tmem_base + buf * (P.lay[0].cols0 + P.lay[0].cols1);
         if (use > 0 && !tc_wait(d_empty(buf), (use - 1) & 1, P.status)) break;
         tc_fence_after();
         auto slot = [&](int s, int second, bool rest) __attribute__((always_inline)) {
@@ -488,13 +520,13 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
           for (int h = 0; h < SUB; ++h) {
             if (h > 0 && second >= n_stages) break;
             const uint32_t sfa = tmem_base + P.sf0 + (turn * SUB + h) * kSfCols, sfb = sfa + 16;
-            const uint32_t x_at = ((static_cast<uint32_t>(x.slot) * SUB + h) * x_bytes) >> 4;
+            const uint32_t x_at = ((static_cast<uint32_t>(x.slot) * SUB + h) * x_slot) >> 4;
             const uint32_t a_lo = a_lo0 + (((static_cast<uint32_t>(w.slot) * SUB + h) * box_bytes) >> 4), b_lo = b_lo0 + x_at;
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks) {
               const uint32_t adds = rest || (s | h | ks) ? 1u : 0u;
               mx_umma(d_tmem, a_lo + 2 * ks, a_hi, b_lo + ks * b_step, b_hi, idesc0, sfa + 4 * ks, sfb + 4 * ATOMS * ks, adds);
-              if constexpr (TWO) mx_umma(d_tmem + P.cols0, a_lo + 2 * ks, a_hi, b_lo + ks * b_step + b_second, b_hi, idesc1, sfa + 4 * ks, sfb + 4 * ATOMS * ks, adds);
+              if constexpr (TWO) mx_umma(d_tmem + cols0, a_lo + 2 * ks, a_hi, b_lo + ks * b_step + b_second, b_hi, idesc1, sfa + 4 * ks, sfb + 4 * ATOMS * ks, adds);
             }
           }
           umma_commit(w_empty(w.slot));
@@ -527,7 +559,8 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + P.sf0;
     Ring w, x;
     bool ok = true;
-    uint32_t count = 0;  // stages so far
+    uint32_t count = 0;  // slots so far
+    uint32_t x_rows[ATOMS] = {}, sf_off = 0;  // compact, the chunk's: the rows of columns lane, 32 + lane, ..., a byte each, and where their scales begin
     const uint32_t sf_mask = P.sf_turns - 1, sf_shift = P.sf_turns == 4 ? 2 : P.sf_turns == 2 ? 1 : 0;
     // One slot: this thread's scales of its stages to the tensor core (both: there is a second stage); `fetch` asks for the ones that
     // come later. (A warp whose wait gave up still comes to the meetings.)
@@ -562,18 +595,28 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
         }
       };
       auto read_x = [&](int h) __attribute__((always_inline)) {
-        // the activations' scales lie behind their digits as the four words of each lane and product
-        const uint4* xsf = reinterpret_cast<const uint4*>(xring + (static_cast<size_t>(x.slot) * SUB + h) * x_bytes + P.sf_off) + lane;
+        // The activations' scales lie behind their digits, as the four words of each lane and product or, compact, a word per product and row:
+        // column c is a digit of row c % Mp, word q of a product is that of column 32 q + lane. (Words: the four products' of a row at once
+        // would have to change places before they are stored.)
+        const uint8_t* const xsf = xring + static_cast<size_t>(x.slot * SUB + h) * x_slot + (COMPACT ? sf_off : P.lay[0].sf_off);
 #pragma unroll
-        for (int j = 0; j < 4 * ATOMS; ++j) {
-          const uint4 u = xsf[32 * j];
-          uint32_t* to = xv[j / 4] + 4 * (j % 4);
-          to[0] = u.x, to[1] = u.y, to[2] = u.z, to[3] = u.w;
+        for (int q = 0; q < 4 * ATOMS; ++q) {
+          if constexpr (COMPACT) {
+            uint32_t row = x_rows[q / 4];
+            asm volatile("" : "+r"(row));  // (taken out for each slot: the addresses of all words, kept, would take the next preparation's registers)
+            const uint32_t* from = reinterpret_cast<const uint32_t*>(xsf + 4 * (row >> 8 * (q % 4) & 255u));
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) xv[(4 * ATOMS * ks + q) / 16][(4 * ATOMS * ks + q) % 16] = from[ks * MxLayout::compact_rows(ATOMS == 2)];
+          } else {
+            const uint4 u = *reinterpret_cast<const uint4*>(xsf + 512 * q + 16 * lane);
+            uint32_t* to = xv[q / 4] + 4 * (q % 4);
+            to[0] = u.x, to[1] = u.y, to[2] = u.z, to[3] = u.w;
+          }
         }
       };
       read_rows(0);
       ok = ok && tc_wait(x_full(x.slot), x.lap, P.status);
-      read_x(0);  // before the wait for their place (the second stage's after: 154 registers leave the next preparation no room)
+      read_x(0);  // before the wait for their place (the second stage's after: they would take more registers than there are)
       if (use > 0 && ok) ok = tc_wait(s_empty(turn), (use - 1) & 1, P.status);
       ok = __all_sync(0xffffffffu, ok);
       if (ok) {
@@ -600,6 +643,15 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
       const bool turns = chunk + 1 == chunks;
       const uint4* const scales_next = tile + 1 >= tile_end ? nullptr : turns ? scales_of(panel + 1) : scales;
       const uint8_t* const bits = again + chunk * groups;
+      if constexpr (COMPACT) {
+        const MxLayout& L = P.lay[chunk + 1 == chunks];
+        sf_off = L.sf_off;
+#pragma unroll
+        for (int q = 0, m = lane; q < 4 * ATOMS; ++q, m += 32) {
+          while (m >= L.Mp) m -= L.Mp;
+          x_rows[q / 4] = q % 4 ? x_rows[q / 4] | static_cast<uint32_t>(m) << 8 * (q % 4) : static_cast<uint32_t>(m);
+        }
+      }
       for (int s0 = 0; s0 < n_stages; s0 += kAhead) {
 #pragma unroll
         for (int i = 0; i < kAhead; i += SUB) {
@@ -664,18 +716,19 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
     mbar_arrive(a_full);
     for (int tile = tile_begin, t = 0; tile < tile_end; ++tile, ++t) {
       const int buf = P.buffers == 2 ? t & 1 : 0, use = P.buffers == 2 ? t >> 1 : t;
-      const int panel = tile / chunks, m0 = (tile - panel * chunks) * P.chunk_rows, rows = min(P.chunk_rows, P.M - m0);
+      const int panel = tile / chunks, chunk = tile - panel * chunks, m0 = chunk * P.chunk_rows, rows = min(P.chunk_rows, P.M - m0);
+      const int Mp = P.lay[COMPACT && chunk + 1 == chunks].Mp;
       const int n = panel * P.R + r;
       const bool live = r < P.R && n < P.N;
       const float inv_lo = lane < rows ? P.row_scale[m0 + lane] : 0.0f, inv_hi = 32 + lane < rows ? P.row_scale[m0 + 32 + lane] : 0.0f;
       const float bias = live && P.bias ? load_f32(P.bias, P.bias_dtype, n) : 0.0f;
       if (!tc_wait(d_full(buf), use & 1, P.status)) break;
       tc_fence_after();
-      const uint32_t d_addr = lane_addr + buf * (P.cols0 + P.cols1);
+      const uint32_t d_addr = lane_addr + buf * (P.lay[0].cols0 + P.lay[0].cols1);
       for (int c = 0; c < rows; c += 8) {
         uint32_t raw[kMxDigits][8];
 #pragma unroll
-        for (int j = 0; j < kMxDigits; ++j) tmem_ld8(d_addr + j * P.Mp + c, raw[j]);
+        for (int j = 0; j < kMxDigits; ++j) tmem_ld8(d_addr + j * Mp + c, raw[j]);
         float old[8] = {};  // with beta: all eight asked for before the first is stored (see gemm_tc.cu)
         if (P.beta != 0.0f && live) {
 #pragma unroll
@@ -718,25 +771,12 @@ __global__ void __launch_bounds__(kMxThreads, 1) tc_mx_kernel(const __grid_const
   if (warp == 9) tmem_dealloc(tmem_base, kTmemColumns);
 }
 
-// How a pass of M rows lies in accumulator columns and in the workspace. An instruction has at most 256 columns, in whole 16s.
-struct MxLayout {
-  int Mp, cols0, cols1, sf_off, x_bytes;
-  explicit MxLayout(int M) {
-    auto whole = [](int c) { return (c + 15) / 16 * 16; };
-    Mp = (M + 7) / 8 * 8;
-    cols0 = whole(kMxDigits * Mp), cols1 = 0;
-    if (cols0 > 256) cols0 = 4 * Mp, cols1 = whole((kMxDigits - 4) * Mp);  // four digits, then the rest
-    sf_off = (cols0 + cols1) * (kMxStageK / 2);
-    x_bytes = sf_off + 4 * ((cols0 + 127) / 128) * 512;
-  }
-};
-
 }  // namespace
 
 // The most rows one launch takes (more come in launches of as many): bounds the workspace.
 constexpr int kMxMaxRows = 1024;
 
-// The fewest chunks of at most `most` rows that hold M, all of the same size (a multiple of 8).
+// The fewest chunks of at most `most` rows that hold M, all of the same size (a multiple of 8) but the last.
 constexpr int kMxChunkMost[] = {kMaxRows, 32, 16};
 static int mx_chunk_rows(int M, int most) {
   const int chunks = (M + most - 1) / most;
@@ -745,22 +785,100 @@ static int mx_chunk_rows(int M, int most) {
 // What a stage of a tile takes with so many activation rows, in tens of ns (28672 x 8192, two tiles per SM).
 static int mx_stage_cost(int rows) { return rows <= 16 ? 49 : rows <= 24 ? 61 : rows <= 32 ? 66 : 88 + (rows - 40) * 11 / 10; }
 
+// How P.M <= kMxMaxRows rows lie in the workspace when they go in chunks of at most `most`; returns the bytes. Rows that are split further
+// than into chunks of 64 have their block scales there once, not for each of their digits, and a last chunk of fewer rows takes the room of
+// those only: so no split takes more than the chunks of 64 do (which split, N decides, and who asks for the size has no N to give).
+// Whole chunks keep the scales as they go to tensor memory: 28672 x 8192, 16 / 64 rows 36.0 / 78.0 us, compact 37.1 / 80.0.
+static int64_t mx_cut(MxParams& P, int most) {
+  const int stages = (P.K + kMxStageK - 1) / kMxStageK, whole = mx_chunk_rows(P.M, kMaxRows);
+  P.chunk_rows = mx_chunk_rows(P.M, most);
+  P.chunks = (P.M + P.chunk_rows - 1) / P.chunk_rows;
+  P.lay[0] = P.lay[1] = MxLayout(P.chunk_rows);
+  if (P.chunk_rows < whole) {
+    const int as = MxLayout::compact_rows(P.lay[0].cols0 > 128);
+    P.lay[0] = MxLayout(P.chunk_rows, as), P.lay[1] = MxLayout(P.M - (P.chunks - 1) * P.chunk_rows, as);
+  }
+  P.chunk_bytes = static_cast<int64_t>(stages) * P.lay[0].x_bytes;
+  P.remainders = (P.chunks - 1) * P.chunk_bytes + static_cast<int64_t>(stages) * P.lay[1].x_bytes;
+  P.groups = (stages + 7) / 8;
+  return 2 * P.remainders + static_cast<int64_t>(P.chunks) * P.groups * kMaxRows + 4 * P.M + 256;
+}
+
 int64_t mx_workspace_bytes(int M, int K) {
   int64_t need = 0;
-  for (int rows : {std::min(M, kMxMaxRows), M % kMxMaxRows}) {  // a launch of the most rows, and the last one
-    if (rows == 0) continue;
-    for (int most : kMxChunkMost) {  // (which of them N decides)
-      const int chunk = mx_chunk_rows(rows, most);
-      const MxLayout L(chunk);
-      const int stages = (K + kMxStageK - 1) / kMxStageK;
-      need = std::max(need, static_cast<int64_t>((rows + chunk - 1) / chunk) * (int64_t{2} * stages * L.x_bytes + (stages + 7) / 8 * kMaxRows) + 4 * rows + 256);
+  MxParams P{};
+  P.K = K;
+  for (int rows : {std::min(M, kMxMaxRows), M % kMxMaxRows})  // a launch of the most rows, and the last one
+    for (int most : kMxChunkMost) {                           // (which of them N decides)
+      if (rows == 0) continue;
+      P.M = rows;
+      need = std::max(need, mx_cut(P, most));
     }
-  }
   return need;
 }
 
-// K % 256 == 0; weights, scales and workspace (mx_workspace_bytes) on 16 bytes. even_rows: the weight rows per tile that deal N
-// out evenly over the SMs.
+// Everything about a launch that follows from the sizes (P.M, P.N, P.K) and the number of SMs. *sub: stages per slot, *smem: dynamic
+// shared memory. even_rows: the weight rows per tile that deal N out evenly over the SMs.
+static int mx_plan(MxParams& P, int sms, int even_rows, int* sub, size_t* smem) {
+  constexpr int kMostFlags = 8192;  // of a chunk's groups, in shared memory: a split does not take room from the rings for more
+  // Chunks of up to 64 rows, or of 32 or 16 where the busiest SM is done sooner with more, shorter tiles: a weight of few rows
+  // leaves most SMs without a tile otherwise. (A row's bits do not depend on its chunk.)
+  auto turns_of = [&](int R, int chunk) { return (static_cast<int64_t>((P.N + R - 1) / R) * ((P.M + chunk - 1) / chunk) + sms - 1) / sms; };
+  int64_t least = -1;
+  int best = kMaxRows;
+  for (int most : kMxChunkMost) {
+    mx_cut(P, most);
+    const int64_t cost = std::min(turns_of(kBM, P.chunk_rows), turns_of(even_rows, P.chunk_rows)) * mx_stage_cost(P.chunk_rows);
+    if (least >= 0 && (cost >= least || P.chunks * P.groups > kMostFlags)) continue;
+    least = cost, best = most;
+  }
+  mx_cut(P, best);
+  const MxLayout& L = P.lay[0];
+  // A tile takes as long with 128 weight rows as with fewer (its steps do), so what counts is the busiest SM's tiles; rows dealt
+  // evenly where that is the same.
+  P.R = turns_of(kBM, P.chunk_rows) < turns_of(even_rows, P.chunk_rows) ? kBM : even_rows;
+  P.box_bytes = (P.R + 7) / 8 * 1024;
+  // tensor memory from its end: the scales, then the accumulators, more than one of each where they fit
+  const int cols = L.cols0 + L.cols1;
+  const int sf_cols = 16 + 16 * ((L.cols0 + 127) / 128);
+  *sub = L.cols1 ? 1 : 2;  // see the kernel
+  P.sf_turns = cols + 4 * *sub * sf_cols <= kTmemColumns ? 4 : cols + 2 * *sub * sf_cols <= kTmemColumns ? 2 : 1;
+  P.sf0 = kTmemColumns - P.sf_turns * *sub * sf_cols;
+  P.buffers = 2 * cols <= P.sf0 ? 2 : 1;
+  // A ring of as many stages of activations as of weights: a block of them, the same for every SM, travels as long as the weights
+  // do. Where that is fewer than four, the weights keep six.
+  const int tail = std::max(1024, 448 + P.chunks * P.groups);  // barriers, and the stages that go again
+  const int room = 224 * 1024 - *sub * kMxScaleBytes - tail, box = *sub * P.box_bytes, block = *sub * L.x_bytes;
+  const int even = room / (box + block);
+  P.SX = *sub == 2 ? std::max(2, std::min(6, even)) : even >= 4 ? std::min(8, even) : std::max(2, std::min(4, (room - 6 * P.box_bytes) / L.x_bytes));
+  P.SW = std::min(12, (room - P.SX * block) / box);
+  if (P.SW < 2) return kNotSupported;
+  *smem = std::max<size_t>(static_cast<size_t>(P.SW) * box + *sub * kMxScaleBytes + static_cast<size_t>(P.SX) * block + tail, 120 * 1024);
+  return kOk;
+}
+
+int mx_plan_numbers(int M, int N, int K, int sms, int even_rows, int32_t* out) {
+  MxParams P{};
+  P.M = M, P.N = N, P.K = K;
+  int sub = 0;
+  size_t smem = 0;
+  if (int e = mx_plan(P, sms, even_rows, &sub, &smem)) return e;
+  const int64_t bytes = 2 * P.remainders + static_cast<int64_t>(P.chunks) * P.groups * kMaxRows + 4 * P.M;
+  const int32_t v[] = {P.chunk_rows, P.chunks,  P.lay[0].cols0, P.lay[0].cols1, P.lay[0].x_bytes, P.lay[1].cols0, P.lay[1].x_bytes, sub, P.R,
+                       P.SW,         P.SX,      P.sf_turns,     P.sf0,          P.buffers,        static_cast<int32_t>(smem), static_cast<int32_t>(bytes)};
+  std::copy(v, v + 16, out);
+  return kOk;
+}
+
+template <int ATOMS, bool TWO, bool COMPACT>
+static int launch_mx(const MxParams& P, const CUtensorMap& wmap, size_t smem, int sms, cudaStream_t stream) {
+  constexpr auto kernel = tc_mx_kernel<ATOMS, TWO, TWO ? 1 : 2, COMPACT>;
+  if (int e = allow_big_smem<300 + ATOMS * 4 + TWO * 2 + COMPACT>(kernel)) return e;
+  const int tiles = (P.N + P.R - 1) / P.R * P.chunks;
+  return launch_kernel(kernel, dim3(std::min(tiles, sms)), dim3(kMxThreads), smem, stream, wmap, P);
+}
+
+// K % 256 == 0; weights, scales and workspace (mx_workspace_bytes) on 16 bytes.
 int mx_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const void* bias, int bias_dtype, void* y, int y_dtype, int ld_y,
                int M, int N, int K, float alpha, float beta, void* workspace, int even_rows, cudaStream_t stream) {
   if (K % kMxStageK != 0) return kNotSupported;
@@ -781,33 +899,9 @@ int mx_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const v
   P.xprep = ws;
   for (int first = 0; first < M; first += kMxMaxRows) {
     P.M = std::min(kMxMaxRows, M - first);
-    // Chunks of up to 64 rows, or of 32 or 16 where the busiest SM is done sooner with more, shorter tiles: a weight of few rows
-    // leaves most SMs without a tile otherwise. (A row's bits do not depend on its chunk.)
-    auto turns_of = [&](int R, int chunk) { return (static_cast<int64_t>((N + R - 1) / R) * ((P.M + chunk - 1) / chunk) + sms - 1) / sms; };
-    int64_t least = -1;
-    for (int most : kMxChunkMost) {
-      const int chunk = mx_chunk_rows(P.M, most);
-      const int64_t cost = std::min(turns_of(kBM, chunk), turns_of(even_rows, chunk)) * mx_stage_cost(chunk);
-      if (least < 0 || cost < least) least = cost, P.chunk_rows = chunk;
-    }
-    P.chunks = (P.M + P.chunk_rows - 1) / P.chunk_rows;
-    const MxLayout L(P.chunk_rows);
-    P.Mp = L.Mp, P.cols0 = L.cols0, P.cols1 = L.cols1, P.sf_off = L.sf_off, P.x_bytes = L.x_bytes;
-    P.chunk_bytes = static_cast<int64_t>(K / kMxStageK) * L.x_bytes;
-    // A tile takes as long with 128 weight rows as with fewer (its steps do), so what counts is the busiest SM's tiles; rows dealt
-    // evenly where that is the same.
-    P.R = turns_of(kBM, P.chunk_rows) < turns_of(even_rows, P.chunk_rows) ? kBM : even_rows;
-    P.box_bytes = (P.R + 7) / 8 * 1024;
-    // tensor memory from its end: the scales, then the accumulators, more than one of each where they fit
-    const int cols = L.cols0 + L.cols1;
-    const int sf_cols = 16 + 16 * ((L.cols0 + 127) / 128);
-    const bool two_atoms = L.cols0 > 128;
-    const int sub = L.cols1 ? 1 : 2;  // stages per slot: see the kernel
-    P.sf_turns = cols + 4 * sub * sf_cols <= kTmemColumns ? 4 : cols + 2 * sub * sf_cols <= kTmemColumns ? 2 : 1;
-    P.sf0 = kTmemColumns - P.sf_turns * sub * sf_cols;
-    P.buffers = 2 * cols <= P.sf0 ? 2 : 1;
-    P.remainders = P.chunks * P.chunk_bytes;
-    P.groups = (K / kMxStageK + 7) / 8;
+    int sub = 0;
+    size_t smem = 0;
+    if (int e = mx_plan(P, sms, even_rows, &sub, &smem)) return e;
     uint8_t* again = ws + 2 * P.remainders;
     P.again = again;
     float* row_scale = reinterpret_cast<float*>(again + static_cast<int64_t>(P.chunks) * P.groups * kMaxRows);
@@ -818,21 +912,13 @@ int mx_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const v
     alignas(64) CUtensorMap wmap;
     if (int e = make_tile_map(&wmap, w.data, K / 2, N, 128, P.R, 4, true)) return e;
     if (int e = launch_kernel(x_bf16 ? mx_prep_kernel<true> : mx_prep_kernel<false>, dim3(P.groups, P.M), dim3(kPrepThreads), 0, stream, xrow, ld_x, K,
-                              P.chunk_rows, P.chunk_bytes, L.Mp, L.cols0, L.cols1, L.x_bytes, L.sf_off, ws, P.remainders, again, row_scale))
+                              P.chunks, P.chunk_rows, P.chunk_bytes, P.lay[0], P.lay[1], ws, P.remainders, again, row_scale))
       return e;
-    // A ring of as many stages of activations as of weights: a block of them, the same for every SM, travels as long as the weights
-    // do. Where that is fewer than four, the weights keep six.
-    const int tail = std::max(1024, 448 + P.chunks * P.groups);  // barriers, and the stages that go again
-    const int room = 224 * 1024 - sub * kMxScaleBytes - tail, box = sub * P.box_bytes, block = sub * L.x_bytes;
-    const int even = room / (box + block);
-    P.SX = sub == 2 ? std::max(2, std::min(6, even)) : even >= 4 ? std::min(8, even) : std::max(2, std::min(4, (room - 6 * P.box_bytes) / L.x_bytes));
-    P.SW = std::min(12, (room - P.SX * block) / box);
-    if (P.SW < 2) return kNotSupported;
-    const size_t smem = std::max<size_t>(static_cast<size_t>(P.SW) * box + sub * kMxScaleBytes + static_cast<size_t>(P.SX) * block + tail, 120 * 1024);
-    auto kernel = !two_atoms ? tc_mx_kernel<1, false, 2> : L.cols1 ? tc_mx_kernel<2, true, 1> : tc_mx_kernel<2, false, 2>;
-    if (int e = !two_atoms ? allow_big_smem<300>(kernel) : L.cols1 ? allow_big_smem<301>(kernel) : allow_big_smem<302>(kernel)) return e;
-    const int tiles = (N + P.R - 1) / P.R * P.chunks;
-    if (int e = launch_kernel(kernel, dim3(std::min(tiles, sms)), dim3(kMxThreads), smem, stream, wmap, P)) return e;
+    const int e = P.lay[0].cols0 <= 128 ? (P.lay[0].sf_rows ? launch_mx<1, false, true>(P, wmap, smem, sms, stream) : launch_mx<1, false, false>(P, wmap, smem, sms, stream))
+                  : P.lay[0].cols1      ? launch_mx<2, true, false>(P, wmap, smem, sms, stream)
+                  : P.lay[0].sf_rows    ? launch_mx<2, false, true>(P, wmap, smem, sms, stream)
+                                        : launch_mx<2, false, false>(P, wmap, smem, sms, stream);
+    if (e) return e;
   }
   return kOk;
 }

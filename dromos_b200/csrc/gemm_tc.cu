@@ -673,6 +673,8 @@ int small_min_stages() {
   return n;
 }
 
+}  // namespace
+
 // Rows per tile: the fewest whole tiles per SM that keep a tile within 128 rows, then the rows that spread N evenly
 // over that many tiles.
 int tile_rows(int N, int sms) {
@@ -680,6 +682,8 @@ int tile_rows(int N, int sms) {
   const int rows = (N + per_sm * sms - 1) / (per_sm * sms);
   return std::min(kBM, std::max(kMinTileRows, rows));
 }
+
+namespace {
 
 template <int F, int XMODE>
 int tc_launch(const lx_weight& w, TcParams P, cudaStream_t stream, int* grid_out = nullptr) {

@@ -202,6 +202,8 @@ int64_t pair_workspace_bytes(int M, int K);
 int mx_product(const void* x, int x_dtype, int ld_x, const lx_weight& w, const void* bias, int bias_dtype, void* y, int y_dtype, int ld_y,
                int M, int N, int K, float alpha, float beta, void* workspace, int even_rows, cudaStream_t stream);
 int64_t mx_workspace_bytes(int M, int K);
+int mx_plan_numbers(int M, int N, int K, int sms, int even_rows, int32_t* out);  // lx_b200_gemm_mx_plan
+int tile_rows(int N, int sms);  // gemm_tc.cu
 bool tc_enabled();
 // Where the all-gather epilogue of a sharded product stores: every rank's copy of the whole y and arrival counter.
 struct PeerTargets {

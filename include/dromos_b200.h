@@ -191,6 +191,13 @@ LX_API int lx_b200_last_error(void);
  * of a header slot, and the offsets of the header ring, the ring and the barriers in dynamic shared memory, and its total.
  * Returns 0, or 1 for a null pointer, K <= 0 or M outside 1..8. For tests of the layout on machines without a GPU. */
 LX_API int lx_b200_gemv_ring_plan(int wtype, int K, int M, int x_is_bf16, int32_t* out);
+/* How lx_gemm_w cuts up a product of M <= 1024 activation rows on NVFP4 weights on a GPU of `sms` SMs (larger ones are launches of
+ * 1024 rows and one of the rest); nothing is launched. out[0..15] = activation rows per chunk, chunks, accumulator columns of a chunk's
+ * first and of its second instruction (0: there is one), bytes of a stage of its activations, columns and bytes of the last chunk's,
+ * stages of K per ring slot, weight rows per tile, slots of the weights' and of the activations' ring, slots whose scales tensor
+ * memory holds in turn and the column they begin at, accumulators, dynamic shared memory, bytes of workspace used. Returns 0,
+ * LX_ERR_NOT_SUPPORTED where no ring fits, 1 for a null pointer or sizes outside (K % 256 == 0). For tests without a GPU. */
+LX_API int lx_b200_gemm_mx_plan(int M, int N, int K, int sms, int32_t* out);
 
 /* A row-sharded product whose epilogue is the all-gather (no counterpart in the reference, which is single-GPU). Every
  * rank calls it with its rows of W (N rows, the columns col0 .. col0 + N - 1 of the whole y): the outputs are stored
