@@ -1,6 +1,7 @@
 """lx_gemm_w on NVFP4 weights (weights multiplied as stored, activations as base-13 digits): against 64-bit sums at the edges of its
-layouts (digit columns in one instruction or two, chunks of 64 rows, launches of 1024, weight panels, 256 values of K), rows that
-do not depend on the call they come in, small values beside large ones, and the values that have no digits.
+layouts (chunks of 8 to 64 rows, launches of 1024, weight panels, 256 values of K; weights of so few rows go in chunks of 16 or 32, and
+the kernel of two instructions per step is in test_gemm_mx_kernels_gpu.py), rows that do not depend on the call they come in,
+small values beside large ones, and the values that have no digits.
 
 Bound: digits and remainders hold a value exactly, or within 2^-41 of its row's largest, or leave out what is below 2^-24 * K / 512 of the
 row's typical values; products of digits are exact, their sums f32, and seven sums are put together with one f32 rounding each (the
