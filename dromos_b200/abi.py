@@ -100,6 +100,7 @@ EXTENSIONS = {
     "lx_b200_kernel_launches": (c_i64, []),
     "lx_b200_last_error": (c_int, []),
     "lx_b200_bf16x_encode_sized": (c_int, [c_ptr, c_i64, c_int, c_ptr, c_i64, ctypes.POINTER(c_i64), c_ptr]),
+    "lx_b200_bf16x_encode_rest": (c_int, [c_ptr, c_i64, c_int, c_ptr, c_ptr, c_i64, c_ptr]),
     "lx_b200_gemv_ring_plan": (c_int, [c_int, c_int, c_int, c_int, c_ptr]),
     "lx_b200_gemm_mx_plan": (c_int, [c_int, c_int, c_int, c_int, c_ptr]),
     "lx_b200_moe_experts_grouped_static": (c_int, [c_ptr, c_ptr, c_ptr, _W, _W, c_int, c_ptr, c_int, c_int, c_int, c_int, c_int, c_ptr]),

@@ -17,10 +17,10 @@ constexpr int kBlock = 256;
 constexpr int kWarpsPerBlock = kBlock / 32;
 // Iterations of 256 values a warp keeps in flight. What bounds these kernels is HBM once a lane's loads are 16 bytes and
 // several are in flight: with 2-byte loads, one 128-value block at a time, sizing, encoding and decoding 14336 x 4096 took
-// 390 us in all, 6.3 x the time its bytes take; now 153, of which ~90 are the matrix read three times and the records once
-// each way, the rest two round trips to the host (the size is a host number) and launches.
+// 390 us in all, 6.3 x the time its bytes take; with both 153; with sizing and encoding in one pass (lx_b200_bf16x_encode_sized) 107, of which
+// ~76 are the matrix read once and written once and the records once each way, the rest a round trip to the host (the size is a
+// host number) and launches.
 constexpr int kInFlight = 4;
-constexpr int64_t kAlwaysEncoded = 4736;  // 148 SMs x 4 blocks x 8 rows
 
 __host__ __device__ inline int64_t record_bytes(int64_t patches) { return (4 * (patches + 2) + 7) / 8 * 8; }
 
@@ -58,10 +58,17 @@ __device__ __forceinline__ uint32_t patch_mask(const uint4& v, uint32_t base, in
   return mask;
 }
 
-// A warp: *area += bytes of a row's overflow record if it has more patches than slots. (A sum of whole numbers: the order in
-// which rows add does not matter.)
+// One warp per row: *area += bytes of the row's overflow record, for rows with more patches than slots. (A sum of whole
+// numbers: the order in which rows add does not matter.)
 template <bool VEC>
-__device__ __forceinline__ void count_row(const uint16_t* __restrict__ src, int K, int lane, unsigned long long* __restrict__ area) {
+__global__ void __launch_bounds__(kBlock) count_kernel(const uint16_t* __restrict__ w, int64_t rows, int K, unsigned long long* __restrict__ area) {
+  // no early trigger: what this kernel writes may be the weight of the next product, whose kernels read weights
+  // before their own wait
+  pdl_wait();
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const int lane = threadIdx.x & 31;
+  const uint16_t* src = w + row * K;
   int n = 0;
   for (int k_base = 0; k_base < K; k_base += 256 * kInFlight) {
     uint4 v[kInFlight];
@@ -73,15 +80,6 @@ __device__ __forceinline__ void count_row(const uint16_t* __restrict__ src, int 
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
   if (lane == 0 && n > x16::patch_slots(K)) atomicAdd(area, static_cast<unsigned long long>(record_bytes(n)));
-}
-template <bool VEC>
-__global__ void __launch_bounds__(kBlock) count_kernel(const uint16_t* __restrict__ w, int64_t rows, int K, unsigned long long* __restrict__ area) {
-  // no early trigger: what this kernel writes may be the weight of the next product, whose kernels read weights
-  // before their own wait
-  pdl_wait();
-  const int64_t row = static_cast<int64_t>(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
-  if (row >= rows) return;
-  count_row<VEC>(w + row * K, K, threadIdx.x & 31, area);
 }
 
 // Where a lane's patches go in its row's list: after those of the lanes below it. Returns the warp's count.
@@ -102,26 +100,15 @@ __device__ __forceinline__ int place_patches(uint32_t mask, int lane, int& befor
 // common matrix is read once, and nothing but *area has to be known before.
 // A lane holds eight consecutive values: eight sign|mantissa bytes, and one word of codes (byte j holds value j low and
 // value 4 + j high), so a block's 192 bytes leave in 16 stores of 8 and 16 of 4 bytes.
-// room: the bytes there are for overflow records. Once the rows so far have more, what is written is of no use any more, and the
-// rest are only counted (a matrix whose every row overflows then costs what counting it costs). The first kAlwaysEncoded rows, which run
-// together and would find nothing counted yet, do not look: the look comes before a warp's first loads (1253 x 1280: 4.7 us without, 6.1 with).
 template <bool VEC>
 __global__ void __launch_bounds__(kBlock) encode_kernel(const uint16_t* __restrict__ w, int64_t rows, int K, uint8_t* __restrict__ out,
-                                                        unsigned long long* __restrict__ area, unsigned long long room) {
+                                                        unsigned long long* __restrict__ area) {
   // no early trigger: what this kernel writes may be the weight of the next product, whose kernels read weights
   // before their own wait
   pdl_wait();
   const int64_t row = static_cast<int64_t>(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int lane = threadIdx.x & 31;
-  if (room != ~0ull && row >= kAlwaysEncoded) {
-    unsigned long long so_far = 0;
-    if (lane == 0) asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(so_far) : "l"(area) : "memory");
-    if (__shfl_sync(0xffffffffu, so_far, 0) > room) {
-      count_row<VEC>(w + row * K, K, lane, area);
-      return;
-    }
-  }
   const int H = x16::header_bytes(K), P = x16::patch_slots(K), B = x16::blocks(K);
   const uint16_t* src = w + row * K;
   uint8_t* rec = out + row * x16::row_bytes(K);
@@ -185,8 +172,9 @@ __global__ void __launch_bounds__(kBlock) encode_kernel(const uint16_t* __restri
 __device__ __forceinline__ bool overflowed(uint32_t slot0) { return slot0 != x16::kNoPatch && (slot0 & 0x80000000u); }
 
 // One CTA, after encode_kernel: the places of the overflow records, in row order (an exclusive prefix sum over the counts
-// that encode_kernel left), take the place of the counts in slot 0.
-__global__ void __launch_bounds__(1024) place_records_kernel(uint8_t* __restrict__ out, int64_t rows, int64_t rb) {
+// that encode_kernel left), take the place of the counts in slot 0. room: the bytes there are for records; a row whose record would end
+// past them is left without its patches.
+__global__ void __launch_bounds__(1024) place_records_kernel(uint8_t* __restrict__ out, int64_t rows, int64_t rb, int64_t room) {
   // no early trigger: what this kernel writes may be the weight of the next product, whose kernels read weights
   // before their own wait
   pdl_wait();
@@ -213,8 +201,9 @@ __global__ void __launch_bounds__(1024) place_records_kernel(uint8_t* __restrict
   for (int64_t r = r0; r < r1; ++r) {
     const uint32_t s = *slot0(r);
     if (!overflowed(s)) continue;
-    *slot0(r) = 0x80000000u | static_cast<uint32_t>((rows * rb + run - r * rb) / 8);  // from the row's own start, in 8 bytes
+    const int64_t at = run;
     run += record_bytes(s & 0x7fffffffu);
+    *slot0(r) = run <= room ? 0x80000000u | static_cast<uint32_t>((rows * rb + at - r * rb) / 8) : x16::kNoPatch;  // from the row's own start, in 8 bytes
   }
 }
 
@@ -354,30 +343,25 @@ extern "C" int64_t lx_bf16x_bytes(const void* w, int64_t rows, int K, void* stre
   return rows * x16::row_bytes(K) + static_cast<int64_t>(bytes);
 }
 
-// What the two encoders share. *total: the bytes the encoding takes, as lx_bf16x_bytes answers. count_on: a buffer that turns out
-// too small is not filled any further, and what it holds is undefined; else it is left as lx_bf16x_encode leaves it.
-static int encode_matrix(const void* w, int64_t rows, int K, void* out, int64_t out_bytes, int64_t* total, bool count_on, cudaStream_t stream) {
-  const int64_t rb = x16::row_bytes(K);
-  const bool vec = whole_rows(w, K);
+// The rows, and what the whole encoding takes (*total, as lx_bf16x_bytes answers): rows with more patches than slots are left with their counts.
+static int encode_rows(const void* w, int64_t rows, int K, void* out, int64_t* total, cudaStream_t stream) {
   ResultWord area(stream);
   if (area.status) return area.status;
-  const auto* src = static_cast<const uint16_t*>(w);
-  auto* dst = static_cast<uint8_t*>(out);
-  const unsigned long long room = static_cast<unsigned long long>(out_bytes - rows * rb);
-  if (int e = launch_kernel(vec ? encode_kernel<true> : encode_kernel<false>, row_grid(rows), dim3(kBlock), 0, area.stream, src, rows, K, dst, area.dev,
-                            count_on ? room : ~0ull))
+  if (int e = launch_kernel(whole_rows(w, K) ? encode_kernel<true> : encode_kernel<false>, row_grid(rows), dim3(kBlock), 0, area.stream,
+                            static_cast<const uint16_t*>(w), rows, K, static_cast<uint8_t*>(out), area.dev))
     return e;
   unsigned long long bytes = 0;
   if (int e = area.read(&bytes)) return e;
-  *total = rows * rb + static_cast<int64_t>(bytes);
-  if (!bytes) return kOk;
-  if (bytes > room) {
-    if (count_on) return LX_B200_ERR_SCRATCH;
-    const int e = launch_kernel(drop_counts_kernel, dim3(static_cast<unsigned>((rows + kBlock - 1) / kBlock)), dim3(kBlock), 0, area.stream, dst, rows, rb);
-    return e ? e : kInvalid;
-  }
-  if (int e = launch_kernel(place_records_kernel, dim3(1), dim3(1024), 0, area.stream, dst, rows, rb)) return e;
-  return launch_kernel(vec ? overflow_kernel<true> : overflow_kernel<false>, row_grid(rows), dim3(kBlock), 0, area.stream, src, rows, K, dst);
+  *total = rows * x16::row_bytes(K) + static_cast<int64_t>(bytes);
+  return kOk;
+}
+// The overflow records of encoded rows, which take the place of their counts.
+static int encode_records(const void* w, int64_t rows, int K, void* out, int64_t out_bytes, cudaStream_t stream) {
+  const int64_t rb = x16::row_bytes(K);
+  auto* dst = static_cast<uint8_t*>(out);
+  if (int e = launch_kernel(place_records_kernel, dim3(1), dim3(1024), 0, stream, dst, rows, rb, out_bytes - rows * rb)) return e;
+  return launch_kernel(whole_rows(w, K) ? overflow_kernel<true> : overflow_kernel<false>, row_grid(rows), dim3(kBlock), 0, stream, static_cast<const uint16_t*>(w), rows,
+                       K, dst);
 }
 
 // A buffer too small for the overflow records is refused after the rows themselves (which fit) have been written: whether it is, only the
@@ -386,17 +370,36 @@ extern "C" int lx_bf16x_encode(const void* w, int64_t rows, int K, void* out, in
   if (rows <= 0) return kOk;
   const int64_t rb = K > 0 && K < (1 << 23) ? x16::row_bytes(K) : 0;
   if (!rb || !w || !out || !aligned(out, 8) || out_bytes < rows * rb) return kInvalid;
+  auto s = static_cast<cudaStream_t>(stream);
   int64_t total = 0;
-  return encode_matrix(w, rows, K, out, out_bytes, &total, false, static_cast<cudaStream_t>(stream));
+  if (int e = encode_rows(w, rows, K, out, &total, s)) return e;
+  if (total == rows * rb) return kOk;
+  if (total <= out_bytes) return encode_records(w, rows, K, out, out_bytes, s);
+  const int e = launch_kernel(drop_counts_kernel, dim3(static_cast<unsigned>((rows + kBlock - 1) / kBlock)), dim3(kBlock), 0, s, static_cast<uint8_t*>(out), rows, rb);
+  return e ? e : kInvalid;
 }
 
-// Sizing and encoding in one call, the matrix read once: few matrices have overflow records at all, so a caller begins with
-// a buffer of rows * lx_bf16x_row_bytes(K) and comes back with a larger one only when the answer is LX_B200_ERR_SCRATCH. *bytes: what the
-// encoding takes (lx_bf16x_bytes), filled in with either answer.
+// Sizing and encoding in one call, the matrix read once: few matrices have overflow records at all, so a caller begins with a buffer of
+// rows * lx_bf16x_row_bytes(K). One that turns out too small keeps the encoded rows, and lx_b200_bf16x_encode_rest takes them from there
+// (copied, 3 bytes per value; encoded again, 3.5 and the host waits once more).
 extern "C" int lx_b200_bf16x_encode_sized(const void* w, int64_t rows, int K, void* out, int64_t out_bytes, int64_t* bytes, void* stream) {
   const int64_t rb = K > 0 && K < (1 << 23) ? x16::row_bytes(K) : 0;
   if (rows <= 0 || !rb || !w || !out || !bytes || !aligned(out, 8) || out_bytes < rows * rb) return kInvalid;
-  return encode_matrix(w, rows, K, out, out_bytes, bytes, true, static_cast<cudaStream_t>(stream));
+  auto s = static_cast<cudaStream_t>(stream);
+  if (int e = encode_rows(w, rows, K, out, bytes, s)) return e;
+  if (*bytes == rows * rb) return kOk;
+  return *bytes <= out_bytes ? encode_records(w, rows, K, out, out_bytes, s) : LX_B200_ERR_SCRATCH;
+}
+extern "C" int lx_b200_bf16x_encode_rest(const void* w, int64_t rows, int K, const void* encoded, void* out, int64_t out_bytes, void* stream) {
+  const int64_t rb = K > 0 && K < (1 << 23) ? x16::row_bytes(K) : 0;
+  if (rows <= 0 || !rb || !w || !encoded || !out || !aligned(out, 8) || out_bytes < rows * rb) return kInvalid;
+  auto s = static_cast<cudaStream_t>(stream);
+  const cudaError_t e = out == encoded ? cudaSuccess : cudaMemcpyAsync(out, encoded, static_cast<size_t>(rows * rb), cudaMemcpyDeviceToDevice, s);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return static_cast<int>(e);
+  }
+  return encode_records(w, rows, K, out, out_bytes, s);
 }
 
 extern "C" int lx_bf16x_decode(const void* data, int64_t rows, int K, void* w, void* stream) {

@@ -73,18 +73,24 @@ def store_weight(lib: abi.Library, w_bf16: torch.Tensor, wtype: int) -> StoredWe
     if wtype == abi.W_BF16:
         return StoredWeight(wtype, w_bf16, rows=rows, cols=cols)
     if wtype == abi.W_BF16X:
-        if lib.has("lx_b200_bf16x_encode_sized"):
-            # one pass over the matrix (sizing 14336 x 4096 before encoding it cost 40 of 150 us), into a buffer with room for the
-            # overflow records of some rows (one matrix in 20 of that size has a row with more patches than slots)
+        if lib.has("lx_b200_bf16x_encode_rest"):
+            # one pass over the matrix (sizing 14336 x 4096 before encoding it cost 40 of 150 us); the rows of a matrix with overflow records
+            # (one in 20 of that size) move to a buffer with room for these, so that a weight's buffer is its encoding and no more
             n = rows * lib.lx_bf16x_row_bytes(cols)
-            n = max(n + min(1 << 18, n >> 6), 8)
-            data, need = torch.empty(n, dtype=torch.uint8, device=w_bf16.device), ctypes.c_int64(0)
+            data, need = torch.empty(max(n, 8), dtype=torch.uint8, device=w_bf16.device), ctypes.c_int64(0)
             st = lib.lx_b200_bf16x_encode_sized(abi.ptr(w_bf16), rows, cols, abi.ptr(data), n, ctypes.byref(need), _stream())
-            if st == 0:
-                return StoredWeight(wtype, data[: need.value], rows=rows, cols=cols)
-            if st != abi.ERR_SCRATCH:
+            encoded, n = data, need.value
+            if st == abi.ERR_SCRATCH:
+                try:
+                    data = torch.empty(n, dtype=torch.uint8, device=w_bf16.device)
+                    st = lib.lx_b200_bf16x_encode_rest(abi.ptr(w_bf16), rows, cols, abi.ptr(encoded), abi.ptr(data), n, _stream())
+                except torch.OutOfMemoryError:  # no room for both: the rows go, and are encoded again
+                    data = None
+            if st not in (0, abi.ERR_SCRATCH):
                 raise RuntimeError(f"lx_b200_bf16x_encode_sized failed: {st}")
-            n, data = need.value, None
+            if data is not None:
+                return StoredWeight(wtype, data, rows=rows, cols=cols)
+            del encoded
         else:
             n = lib.lx_bf16x_bytes(abi.ptr(w_bf16), rows, cols, _stream())
             if n <= 0:

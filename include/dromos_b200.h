@@ -279,8 +279,11 @@ LX_API int lx_b200_moe_sum_rows(const float* rows, float* out, int T, int L, int
 #define LX_B200_ERR_SCRATCH 804
 /* lx_bf16x_bytes and lx_bf16x_encode in one call that reads the matrix once. out_bytes >= rows * lx_bf16x_row_bytes(K), out on 8
  * bytes. Returns 0 with the bytes of the encoding in *bytes (which lx_bf16x_bytes would answer), or LX_B200_ERR_SCRATCH when they are
- * more than out_bytes: *bytes says how many, what out holds is undefined. Synchronizes the stream, as both do. */
+ * more than out_bytes: *bytes says how many, and out holds rows that are no encoding yet. lx_b200_bf16x_encode_rest, with the same w and
+ * these rows as `encoded` (which may be `out`), writes the encoding to a buffer `out` of that many bytes (nothing is written past
+ * out_bytes, and what a smaller one holds is no encoding of w). The first synchronizes the stream, the second does not. */
 LX_API int lx_b200_bf16x_encode_sized(const void* w, int64_t rows, int K, void* out, int64_t out_bytes, int64_t* bytes, void* stream);
+LX_API int lx_b200_bf16x_encode_rest(const void* w, int64_t rows, int K, const void* encoded, void* out, int64_t out_bytes, void* stream);
 LX_API int lx_b200_moe_experts_grouped_static(const void* latent, const int32_t* ids, const float* weights,
                                               const lx_weight* gate_up, const lx_weight* down, lx_math math, float* out,
                                               int T, int L, int I, int E, int top_k, void* stream);
