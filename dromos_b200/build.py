@@ -44,6 +44,24 @@ def compile_one(src, verbose):
     return src, r.returncode, r.stdout + r.stderr
 
 
+def build_calls(stale):
+    """The module of csrc/calls.cpp. Without it abi.Library calls through ctypes, slower and otherwise the same, so a machine without a C++
+    compiler or Python's headers gets a warning and the library all the same."""
+    if not stale:
+        return
+    if os.path.exists(CALLS):
+        os.remove(CALLS)  # of other sources
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-I", INCLUDE, "-I", sysconfig.get_paths()["include"],
+           CALLS_SRC, "-o", CALLS]
+    try:
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        why = r.stdout + r.stderr if r.returncode else None
+    except OSError as e:
+        why = str(e)
+    if why is not None:
+        print(f"{why}\nwarning: {os.path.basename(CALLS)} not built (it needs a C++ compiler and Python's headers): calls go through ctypes", file=sys.stderr)
+
+
 def build(force=False, verbose=False):
     os.makedirs(OBJ, exist_ok=True)
     hdr = headers_mtime()
@@ -67,13 +85,7 @@ def build(force=False, verbose=False):
         if r.returncode != 0:
             print(r.stdout + r.stderr, file=sys.stderr)
             raise RuntimeError("link failed")
-    if force or not os.path.exists(CALLS) or os.path.getmtime(CALLS) < max(hdr, os.path.getmtime(CALLS_SRC)):
-        cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-I", INCLUDE, "-I", sysconfig.get_paths()["include"],
-               CALLS_SRC, "-o", CALLS]
-        r = subprocess.run(cmd, capture_output=True, text=True)
-        if r.returncode != 0:
-            print(r.stdout + r.stderr, file=sys.stderr)
-            raise RuntimeError("g++ failed on calls.cpp")
+    build_calls(force or not os.path.exists(CALLS) or os.path.getmtime(CALLS) < max(hdr, os.path.getmtime(CALLS_SRC)))
     return LIB
 
 

@@ -2,13 +2,20 @@
 results, the same refusals of arguments. Calls of no rows, and sizes, need no GPU."""
 
 import ctypes
+import os
+import sysconfig
 
 import pytest
 import torch
 
-from dromos_b200 import abi, host
+from dromos_b200 import abi, build, host
 
-calls = pytest.importorskip("dromos_b200._calls", reason="built by python -m dromos_b200.build")
+if abi._calls is None and not os.path.exists(os.path.join(sysconfig.get_paths()["include"], "Python.h")):
+    pytest.skip("no Python headers: the module cannot be built here", allow_module_level=True)
+
+
+def test_the_module_is_there():
+    assert abi._calls is not None, "not built (python -m dromos_b200.build)"
 
 
 @pytest.fixture()
@@ -69,3 +76,13 @@ def test_without_the_module_ctypes_converts(monkeypatch):
     monkeypatch.setattr(abi, "_calls", None)
     lib = abi.Library(abi.default_library_path())
     assert lib.lx_gemv_w is lib.fn("lx_gemv_w") and lib.lx_gemv_w(*gemv_args()) == 0
+
+
+@pytest.mark.parametrize("compiler", ["false", "/no/such/compiler"])
+def test_a_build_without_the_module_is_no_error(monkeypatch, tmp_path, capsys, compiler):
+    module = tmp_path / os.path.basename(build.CALLS)
+    module.write_bytes(b"of other sources")
+    monkeypatch.setattr(build, "CALLS", str(module))
+    monkeypatch.setenv("CXX", compiler)
+    build.build_calls(stale=True)
+    assert not module.exists() and "not built" in capsys.readouterr().err
