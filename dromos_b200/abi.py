@@ -38,6 +38,10 @@ class WeightRef:
     def __init__(self, struct: LxWeight):
         self.struct, self.address, self._as_parameter_ = struct, ctypes.addressof(struct), ctypes.byref(struct)
 
+    @property
+    def _obj(self):  # as ctypes.byref(struct) has it
+        return self.struct
+
 
 if _calls is not None:
     _calls.setup(c_ptr, WeightRef)

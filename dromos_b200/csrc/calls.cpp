@@ -1,10 +1,11 @@
 // The entry points of the C ABI as Python callables that convert their arguments in C++ (module dromos_b200._calls).
 //
-// A decode step is hundreds of calls of 10 to 17 arguments whose kernels take a few microseconds each; ctypes takes 3 to 6 us
-// to convert one call's arguments, here it is 0.5. What is converted: ints, floats, None, c_void_p objects and
+// A decode step is hundreds of calls of 10 to 17 arguments whose kernels take a few microseconds each; a GEMV's 15 arguments took ctypes
+// 5.1 us, here it is 0.9. What is converted: ints, floats, None, c_void_p objects and
 // abi.WeightRef, which is what this package passes. A call with anything else goes, as it is, to the ctypes function that is kept
-// behind the callable, so it is accepted, refused or converted as it always was. The interpreter lock is released during a call, as
-// ctypes does.
+// behind the callable, so it is accepted, refused or converted as it always was. That function also stands in for the callable as an
+// argument of ctypes (cast), and once one of its attributes is set (errcheck, restype) it takes all calls. The interpreter lock is
+// released during a call, as ctypes does.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -28,6 +29,7 @@ struct Function {
   vectorcallfunc vectorcall;
   void* fn;
   PyObject* slow;
+  bool plain;  // an attribute of `slow` has been set: what it does to calls is for ctypes to do
 };
 
 // An address from an int; false for anything else (no Python error is left set).
@@ -92,7 +94,7 @@ struct Call<R(A...)> {
   static PyObject* run(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* names) {
     auto* f = reinterpret_cast<Function*>(self);
     std::tuple<A...> to;
-    if (names || PyVectorcall_NARGS(nargsf) != static_cast<Py_ssize_t>(sizeof...(A)) || !convert(args, to, std::index_sequence_for<A...>{}))
+    if (f->plain || names || PyVectorcall_NARGS(nargsf) != static_cast<Py_ssize_t>(sizeof...(A)) || !convert(args, to, std::index_sequence_for<A...>{}))
       return PyObject_Vectorcall(f->slow, args, nargsf, names);
     R r;
     Py_BEGIN_ALLOW_THREADS
@@ -130,7 +132,15 @@ void function_dealloc(PyObject* self) {
   Py_TYPE(self)->tp_free(self);
 }
 PyObject* function_getattro(PyObject* self, PyObject* name) {  // restype, argtypes and the like: the ctypes function's
-  return PyObject_GetAttr(reinterpret_cast<Function*>(self)->slow, name);
+  PyObject* slow = reinterpret_cast<Function*>(self)->slow;
+  if (PyUnicode_Check(name) && PyUnicode_CompareWithASCIIString(name, "_as_parameter_") == 0) return Py_NewRef(slow);
+  return PyObject_GetAttr(slow, name);
+}
+int function_setattro(PyObject* self, PyObject* name, PyObject* value) {
+  auto* f = reinterpret_cast<Function*>(self);
+  if (PyObject_SetAttr(f->slow, name, value) != 0) return -1;
+  f->plain = true;
+  return 0;
 }
 
 PyTypeObject g_function_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
@@ -143,6 +153,7 @@ bool ready_function_type() {
   t.tp_vectorcall_offset = offsetof(Function, vectorcall);
   t.tp_call = PyVectorcall_Call;
   t.tp_getattro = function_getattro;
+  t.tp_setattro = function_setattro;
   t.tp_flags = Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_VECTORCALL;
   t.tp_doc = "An entry point; calls with unusual arguments go to the ctypes function it was made from.";
   return PyType_Ready(&t) == 0;
@@ -161,6 +172,7 @@ PyObject* bind(PyObject*, PyObject* args) {
     f->vectorcall = e.call;
     f->fn = reinterpret_cast<void*>(static_cast<uintptr_t>(address));
     f->slow = Py_NewRef(slow);
+    f->plain = false;
     return reinterpret_cast<PyObject*>(f);
   }
   return Py_NewRef(slow);

@@ -63,6 +63,34 @@ def test_counts_of_arguments_and_names(lib):
     assert lib.lx_bf16x_row_bytes(4096) == 6192 and lib.lx_bf16x_row_bytes(0) == -1  # a 64-bit result with its sign
 
 
+def test_the_callables_pass_for_ctypes_functions(lib):
+    fast, slow = lib.lx_gemm_workspace_bytes, lib.fn("lx_gemm_workspace_bytes")
+    assert ctypes.cast(fast, ctypes.c_void_p).value == ctypes.cast(slow, ctypes.c_void_p).value
+    assert ctypes.CFUNCTYPE(ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.c_int)(ctypes.cast(fast, ctypes.c_void_p).value)(9, 4096, 0) == slow(9, 4096, 0)
+    with pytest.raises(AttributeError):
+        fast.no_such_attribute
+
+
+def test_attributes_that_are_set_count(lib):
+    seen = []
+    want = lib.lx_gemm_workspace_bytes(9, 4096, 0)
+    lib.lx_gemm_workspace_bytes.errcheck = lambda result, f, args: seen.append((result, args)) or -result
+    assert lib.lx_gemm_workspace_bytes(9, 4096, 0) == -want and seen == [(want, (9, 4096, 0))]
+    lib.lx_bf16x_row_bytes.restype = ctypes.c_int8
+    assert lib.lx_bf16x_row_bytes(4096) == ctypes.c_int8(6192).value
+    lib.lx_gemv_w.argtypes = None
+    assert lib.lx_gemv_w.argtypes is None
+    with pytest.raises(TypeError):
+        lib.lx_gemv_w.argtypes = 5
+
+
+def test_a_weight_reference_is_as_byref_has_it():
+    ref = host.StoredWeight(abi.W_BF16, torch.zeros(64, dtype=torch.uint8)).ref()
+    assert ref._obj is ref.struct
+    assert ctypes.cast(ref, ctypes.POINTER(abi.LxWeight)).contents.data == ref.struct.data
+    assert ctypes.cast(ref, ctypes.c_void_p).value == ctypes.cast(ctypes.byref(ref.struct), ctypes.c_void_p).value == ref.address
+
+
 def test_a_weight_follows_its_struct():
     a, b = torch.zeros(64, dtype=torch.uint8), torch.zeros(64, dtype=torch.uint8)
     w = host.StoredWeight(abi.W_BF16, a)
