@@ -17,7 +17,7 @@ constexpr int kBlock = 256;
 constexpr int kWarpsPerBlock = kBlock / 32;
 // Iterations of 256 values a warp keeps in flight. What bounds these kernels is HBM once a lane's loads are 16 bytes and
 // several are in flight: with 2-byte loads, one 128-value block at a time, sizing, encoding and decoding 14336 x 4096 took
-// 390 us in all, 6.3 x the time its bytes take; with both 153; with sizing and encoding in one pass (lx_b200_bf16x_encode_sized) 107, of which
+// 390 us in all, 6.3 x the time its bytes take; with both 153; with sizing and encoding in one pass (lx_b200_bf16x_encode_sized) 102, of which
 // ~76 are the matrix read once and written once and the records once each way, the rest a round trip to the host (the size is a
 // host number) and launches.
 constexpr int kInFlight = 4;

@@ -822,7 +822,8 @@ int64_t mx_workspace_bytes(int M, int K) {
 static int mx_plan(MxParams& P, int sms, int even_rows, int* sub, size_t* smem) {
   constexpr int kMostFlags = 8192;  // of a chunk's groups, in shared memory: a split does not take room from the rings for more
   // Chunks of up to 64 rows, or of 32 or 16 where the busiest SM is done sooner with more, shorter tiles: a weight of few rows
-  // leaves most SMs without a tile otherwise. (A row's bits do not depend on its chunk.)
+  // leaves most SMs without a tile otherwise. (A row's bits do not depend on its chunk.) Replayed graphs, chunks of 64 and as the rule has it:
+  // 4096 x 4096 at 64 rows 25.3 and 17.3 us, 1000 x 2048 at 64 rows 16.3 and 12.2, 293 x 2048 at 525 rows 21.6 and 15.1.
   auto turns_of = [&](int R, int chunk) { return (static_cast<int64_t>((P.N + R - 1) / R) * ((P.M + chunk - 1) / chunk) + sms - 1) / sms; };
   int64_t least = -1;
   int best = kMaxRows;

@@ -287,8 +287,8 @@ __device__ __forceinline__ Raw load_whole(const uint8_t* at, const uint8_t* scal
 // acc[r][t] += rows[r] . x[t] over all of K: the warp's lanes take consecutive words, kSteps words of each row in
 // flight per lane. A token's sum is the same chain of operations whatever NT is.
 // WHOLE (rows, scales and activations on their word's boundary): the steps all of whose 32 words lie within the row go
-// without bounds, by running pointers. The same words in the same order either way. These kernels are bound by instruction
-// issue: at 5.4-6.4 instructions per FP8 value (where converting and adding take 3) four tokens of the 64-expert case (FP8,
+// without bounds, by running pointers. The same words in the same order either way. What bounds these kernels is instruction issue
+// and what 24 to 32 warps per SM have in flight, each at two thirds of its limit: at 5.4-6.4 instructions per FP8 value (where converting and adding take 3) four tokens of the 64-expert case (FP8,
 // 4096 x 1536, top 8) took 152 us, at half the copy bandwidth; 137 this way, 115 with the blocks per SM of the two kernels. Measured and dropped: a word asked for as soon as one
 // is used, across rows and experts (161 against 137: more registers, fewer warps); f16 activations staged in shared memory for
 // fma.rn.f32.f16 (128, but one token 61 where this took 53: the part has no such instruction and converts both operands).
@@ -383,11 +383,12 @@ __device__ __forceinline__ void dot_rows(const Stack& S, const uint8_t* const (&
   }
 }
 
-// Gate/up rows of the 8-bit formats (LEAN): two steps in flight per warp and four blocks per SM (64 registers) instead of four steps and
-// two (96 to 99). Measured with the rest of the call, weights of a few experts in L2: I = 1536, L = 4096, two / four / eight FP8 tokens of 16
-// experts 43 / 65 / 105 -> 37 / 54 / 91 us. A grid of fewer than two blocks per SM has no use for the third, and more to wait for with two
-// steps: I = 768, L = 2048, one INT8 / FP8 token (192 blocks) 20.6 / 15.2 with LEAN, 14.0 / 10.9 without. BF16, whose words need no
-// conversion, is faster with more in flight (98 against 105), NVFP4 and BF16X do not fit 64 registers.
+// Gate/up rows of the 8-bit formats (LEAN): two steps in flight per warp and four blocks per SM (FP8: 64 registers) or three (INT8, whose sums
+// are pairs: 77) instead of four steps and two blocks (111, 115). Measured with the rest of the call (replayed graphs), 16 experts, top 8:
+// I = 1536, L = 4096, two / four / eight tokens FP8 62 / 108 / 180 -> 54 / 93 / 164 us, INT8 65 / 114 / 194 -> 59 / 103 / 185. A grid of fewer than two
+// blocks per SM has no use for the third, and more to wait for with two steps: one INT8 token, L = 2048, I = 512 (256 blocks) 15.1 with LEAN,
+// 13.5 without; I = 768 (384 blocks) 19.0 and 19.8. BF16, whose words need no conversion, is faster with more in flight (98 against 105),
+// NVFP4 and BF16X do not fit 64 registers.
 template <int F>
 constexpr bool kLeanFormat = F == LX_W_FP8 || F == LX_W_INT8;
 constexpr unsigned kLeanBlocks = 2 * 148;
